@@ -65,6 +65,83 @@ static __device__ __forceinline__ int dv_itmax(double a, double b) {
 #define MR3_U 4     // rows per chunk of the software-pipelined sweeps
 #endif
 
+// ------------------------------------------------------------------------
+// Correctly rounded quotients with a deferred check.
+//
+// The sweeps below are chains of one division per row, and a lane that runs
+// one alone waits for the division's latency: 112 cycles for a / b here.
+// dv_qdiv gives the same quotient in four dependent operations after the
+// residual e = 1 - b y0 of a reciprocal seed y0: with a y0 = qh + ql exactly
+// (error-free product by FMA), a / b = a y0 / (1 - e) is the sum
+// qh + [ql + qh e + e^2 (qh + qh e)] up to e^4, rounded once.  That the
+// result q is the correctly rounded one is then checked, not assumed
+// (Markstein's residual test): r = a - b q is exact, t = RN(q + r y0 (1 +
+// 2^-16)) overshoots a / b on r's side because y0 = (1 - e) / b with
+// |e| < 2^-17, so t == q means RN(a/b) == q by the monotonicity of rounding.
+// The conditions (t == q; |e| < 2^-17, which also rules out zero, infinite
+// and NaN divisors; |a| and |q| >= 2^-960, so that r does not underflow)
+// are only recorded (qdiv_chk); a sweep tests them once per chunk of rows
+// and repeats a chunk that fails, 1.5e-5 per division, with plain
+// divisions.  So every result is that of a / b, whatever the seed.
+//
+// The seed of the next row may come from a divisor predicted with *qt =
+// qh (1 + e), 40 bits of the quotient two operations earlier, which takes
+// the seed's latency out of the chain.
+//
+// One warp, Sturm count on T: 193 cycles a row with a / b, 90 so (99
+// without the prediction).  With the SM full of warps both are bound by the
+// FP64 pipe and take the same time (0.74 against 0.70 T rows/s), so the
+// kernels that run a thread per eigenvalue of a large batch keep a / b.
+// ------------------------------------------------------------------------
+#define QDIV_KK   1.0000152587890625      // 1 + 2^-16
+#define QDIV_EMAX (0x3ee00000u << 1)      // high word of 2^-17, sign shifted out
+#define QDIV_AMIN (0x03f00000u << 1)      // high word of 2^-960
+#define QDIV_U    8                       // rows per checked chunk
+
+struct qdiv_chk {
+  unsigned acc, emax, amin;
+};
+
+static __device__ __forceinline__ double dv_rcp_seed(double b) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+  return y;
+}
+
+// The high word of |x| shifted left by one: ordered as |x| is.
+static __device__ __forceinline__ unsigned dv_habs(double x) {
+  return (unsigned)__double2hiint(x) << 1;
+}
+
+static __device__ __forceinline__ int dv_signbit(double x) {
+  return (int)((unsigned)__double2hiint(x) >> 31);
+}
+
+static __device__ __forceinline__ void qdiv_begin(qdiv_chk *k) {
+  k->acc = 0u;
+  k->emax = 0u;
+  k->amin = 0xffffffffu;
+}
+
+static __device__ __forceinline__ bool qdiv_failed(const qdiv_chk &k) {
+  return k.acc != 0u || k.emax >= QDIV_EMAX || k.amin < QDIV_AMIN;
+}
+
+static __device__ __forceinline__ double dv_qdiv(double a, double b, double y0, qdiv_chk *k,
+                                                 double *qt) {
+  const double e = __fma_rn(-b, y0, 1.0);
+  const double qh = __dmul_rn(a, y0), ql = __fma_rn(a, y0, -qh);
+  *qt = __fma_rn(qh, e, qh);
+  const double s = __fma_rn(qh, e, ql), f = __dmul_rn(e, e);
+  const double q = __dadd_rn(qh, __fma_rn(f, *qt, s));
+  const double r = __fma_rn(-b, q, a), t = __fma_rn(r, __dmul_rn(y0, QDIV_KK), q);
+  k->acc |= (unsigned)(__double2loint(t) ^ __double2loint(q));
+  k->acc |= (unsigned)(__double2hiint(t) ^ __double2hiint(q));
+  k->emax = max(k->emax, dv_habs(e));
+  k->amin = min(k->amin, min(dv_habs(a), dv_habs(q)));
+  return q;
+}
+
 // Sturm count of T - x, IJOB=1 rule of dlaebz (SRC/LAPACK/odebz.f:255-270).
 // tp[j] = (d[j], e2[j-1]); tp[0].y unused.  The threads of a warp count the
 // same matrix, so every load is a broadcast that L1 serves; the plain loop
@@ -99,31 +176,74 @@ static __device__ __forceinline__ int dv_count_bisect(int n, const double2 *__re
   return cnt;
 }
 
-// One interval of dlaebz IJOB=3 from the user-supplied point c.
-static __device__ __noinline__ void dv_ijob3(int n, const double2 *__restrict__ tp, double pivmin,
-                                      double abstol, double reltol, int nitmax, int nval,
-                                      double c, double *a, double *b, int *na, int *nb) {
-  for (int it = 1; it <= nitmax; it++) {
-    int cnt = dv_count_bisect(n, tp, pivmin, c);
-    if (cnt <= nval) { *a = c; *na = cnt; }
-    if (cnt >= nval) { *b = c; *nb = cnt; }
-    double w = fabs(*b - *a);
-    double t = fmax(fabs(*b), fabs(*a));
-    if (w < fmax(fmax(abstol, pivmin), reltol * t) || *na >= *nb) break;
-    c = 0.5 * (*a + *b);
+// dv_count_bisect for the launches that wait for the chain (a lane group
+// per interval): quotients by dv_qdiv, rows in checked chunks loaded one
+// chunk ahead.  The clamp at pivmin, 34 cycles of compare and select in the
+// chain, becomes part of the chunk's check: a pivot above pivmin in
+// magnitude is not changed by it, and its sign bit is its count.
+static __device__ __noinline__ int dv_count_bisect_lat(int n, const double2 *__restrict__ tp,
+                                                double pivmin, double c) {
+  constexpr int U = QDIV_U;
+  double t = tp[0].x - c;
+  int cnt = 0;
+  if (t <= pivmin) { cnt = 1; t = fmin(t, -pivmin); }
+  int j = 1;
+  if (n > U) {
+    const unsigned hp = dv_habs(pivmin);
+    double y0 = dv_rcp_seed(t);
+    double2 v[U], nx[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) v[u] = tp[1 + u];
+    for (; j + U <= n; j += U) {
+#pragma unroll
+      for (int u = 0; u < U; u++) nx[u] = tp[d_imin(j + U + u, n - 1)];
+      const double t0 = t;
+      const int cnt0 = cnt;
+      unsigned tmin = 0xffffffffu;
+      qdiv_chk k;
+      qdiv_begin(&k);
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        double qt;
+        const double q = dv_qdiv(v[u].y, t, y0, &k, &qt);
+        y0 = dv_rcp_seed(v[u].x - qt - c);
+        t = v[u].x - q - c;
+        cnt += dv_signbit(t);
+        tmin = min(tmin, dv_habs(t));
+      }
+      if (qdiv_failed(k) || tmin <= hp) {
+        t = t0;
+        cnt = cnt0;
+#pragma unroll 1
+        for (int u = 0; u < U; u++) {
+          const double2 w = tp[j + u];
+          t = w.x - w.y / t - c;
+          if (t <= pivmin) { cnt++; t = fmin(t, -pivmin); }
+        }
+        y0 = dv_rcp_seed(t);
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++) v[u] = nx[u];
+    }
   }
+  for (; j < n; j++) {
+    const double2 w = tp[j];
+    t = w.x - w.y / t - c;
+    if (t <= pivmin) { cnt++; t = fmin(t, -pivmin); }
+  }
+  return cnt;
 }
 
-// dv_ijob3 by a group of L lanes (L = 2..32, a power of two; every lane of
-// the group passes the same arguments and gets the same results).  The
-// first count is at the given point c, as in the loop; after it the points
-// are midpoints, and the midpoints of the next log2(L) steps form a binary
+// One interval of dlaebz IJOB=3 from the user-supplied point c, by a group of
+// L lanes (L = 2..32, a power of two; every lane of the group passes the same
+// arguments and gets the same results).  The first count is at the given
+// point c, as in the sequential loop; after it the points are midpoints, and the midpoints of the next log2(L) steps form a binary
 // tree that follows from the current interval: lane t of the group counts
 // at node max(t,1) (heap numbering; its interval computed along the node's
 // path with the loop's operations), then the group walks the tree applying
 // the loop's updates and tests after each step.  A count equal to nval
 // closes the interval (a = b = c), which the width test then stops.  The
-// same points, counts and results as dv_ijob3; log2(L) steps per count.
+// same points, counts and results as the loop; log2(L) steps per count.
 static __device__ __noinline__ void dv_ijob3_tree(int L, int n, const double2 *__restrict__ tp,
                                            double pivmin, double abstol, double reltol,
                                            int nitmax, int nval, double c, double *a_,
@@ -137,7 +257,7 @@ static __device__ __noinline__ void dv_ijob3_tree(int L, int n, const double2 *_
   int na = *na_, nb = *nb_, it = 0;
   bool done = nitmax < 1;
   if (!done) {   // the first step, at the given point
-    const int cnt = dv_count_bisect(n, tp, pivmin, c);
+    const int cnt = dv_count_bisect_lat(n, tp, pivmin, c);
     if (cnt <= nval) { a = c; na = cnt; }
     if (cnt >= nval) { b = c; nb = cnt; }
     it = 1;
@@ -150,7 +270,7 @@ static __device__ __noinline__ void dv_ijob3_tree(int L, int n, const double2 *_
       const double m = 0.5 * (l + r);
       if ((node_t >> k) & 1) l = m; else r = m;
     }
-    const int raw = dv_count_bisect(n, tp, pivmin, 0.5 * (l + r));
+    const int raw = dv_count_bisect_lat(n, tp, pivmin, 0.5 * (l + r));
     int node = 1;
     for (int d = 0; d < depth; d++) {
       const int cv = __shfl_sync(gm, raw, g0 + node);
@@ -215,7 +335,7 @@ static __device__ __noinline__ int dv_bisect_tree(int L, int n, const double2 *_
       const double m = 0.5 * (l + r);
       if ((node_t >> k) & 1) l = m; else r = m;
     }
-    const int raw = dv_count_bisect(n, tp, pivmin, 0.5 * (l + r));
+    const int raw = dv_count_bisect_lat(n, tp, pivmin, 0.5 * (l + r));
     int node = 1;
     for (int d = 0; d < depth; d++) {
       const int cv = __shfl_sync(gm, raw, g0 + node);
@@ -237,12 +357,14 @@ static __device__ __noinline__ int dv_bisect_tree(int L, int n, const double2 *_
 }
 
 // dlaneg (SRC/LAPACK/odneg.f:98-163) on packed rows P[(i)*ps]; r is 1-based.
-// U > 1: rows are read in chunks of U with the next chunk's loads issued
-// ahead of the current chunk's arithmetic (see the dlar1v sweeps below),
-// for representations that the threads of a warp do not share (cluster
-// groups in the level arenas); the NaN re-run of a 128-row block reads its
-// rows again.  U == 1: the plain row loop, best when a warp's threads all
-// read the same rows (a block's root representation), which L1 serves.
+// U > 1: quotients by dv_qdiv in checked chunks of U rows, the next chunk's
+// rows loaded ahead of the current chunk's arithmetic: for launches that
+// wait for the chain, and for representations that the threads of a warp do
+// not share (cluster groups in the level arenas).  A NaN makes its chunk's
+// check fail, so it comes out of the plain divisions as in the row loop; the
+// NaN re-run of a 128-row block reads its rows again.  U == 1: the plain
+// row loop, best when a warp's threads all read the same rows (a block's
+// root representation) and fill the SM.
 template <int U>
 static __device__ __noinline__ int dv_dlaneg(int n, const double2 *__restrict__ P, int ps, double sigma,
                                       int r) {
@@ -311,36 +433,62 @@ static __device__ __noinline__ int dv_dlaneg(int n, const double2 *__restrict__ 
     double2 c[U], nx[U];
 #pragma unroll
     for (int u = 0; u < U; u++) c[u] = P[(size_t)(d_imin(1 + u, last) - 1) * ps];
+    double y0 = dv_rcp_seed(c[0].x + t);
     for (int bj = 1; bj <= last; bj += blklen) {
       const int jend = d_imin(bj + blklen - 1, last);
-      int neg1 = 0;
+      int neg1 = 0, j = bj;
       const double bsav = t;
-      for (int j0 = bj; j0 <= jend; j0 += U) {
+      for (; j + U - 1 <= jend; j += U) {
 #pragma unroll
-        for (int u = 0; u < U; u++) nx[u] = P[(size_t)(d_imin(j0 + U + u, last) - 1) * ps];
+        for (int u = 0; u < U; u++) nx[u] = P[(size_t)(d_imin(j + U + u, last) - 1) * ps];
+        const double t0 = t;
+        const int n0 = neg1;
+        qdiv_chk k;
+        qdiv_begin(&k);
 #pragma unroll
         for (int u = 0; u < U; u++) {
-          if (j0 + u <= jend) {
-            double dplus = c[u].x + t;
+          const double dplus = c[u].x + t;
+          double qt;
+          const double tmp = dv_qdiv(t, dplus, y0, &k, &qt);
+          y0 = dv_rcp_seed((u + 1 < U ? c[u + 1].x : nx[0].x) + (qt * c[u].y - sigma));
+          neg1 += dv_signbit(dplus);
+          t = tmp * c[u].y - sigma;
+        }
+        if (qdiv_failed(k)) {
+          t = t0;
+          neg1 = n0;
+#pragma unroll 1
+          for (int u = 0; u < U; u++) {
+            const double2 v = P[(size_t)(j + u - 1) * ps];
+            const double dplus = v.x + t;
             neg1 += (dplus < 0.0);
-            double tmp = t / dplus;
-            t = tmp * c[u].y - sigma;
+            const double tmp = t / dplus;
+            t = tmp * v.y - sigma;
           }
+          y0 = dv_rcp_seed(nx[0].x + t);
         }
 #pragma unroll
         for (int u = 0; u < U; u++) c[u] = nx[u];
       }
+      for (; j <= jend; j++) {   // the last rows, fewer than a chunk
+        const double2 v = P[(size_t)(j - 1) * ps];
+        const double dplus = v.x + t;
+        neg1 += (dplus < 0.0);
+        const double tmp = t / dplus;
+        t = tmp * v.y - sigma;
+      }
       if (isnan(t)) {
         neg1 = 0;
         t = bsav;
-        for (int j = bj; j <= jend; j++) {
-          const double2 v = P[(size_t)(j - 1) * ps];
+        for (int i = bj; i <= jend; i++) {
+          const double2 v = P[(size_t)(i - 1) * ps];
           double dplus = v.x + t;
           neg1 += (dplus < 0.0);
           double tmp = t / dplus;
           if (isnan(tmp)) tmp = 1.0;
           t = tmp * v.y - sigma;
         }
+        y0 = dv_rcp_seed(c[0].x + t);
       }
       negcnt += neg1;
     }
@@ -350,36 +498,62 @@ static __device__ __noinline__ int dv_dlaneg(int n, const double2 *__restrict__ 
     double2 c[U], nx[U];
 #pragma unroll
     for (int u = 0; u < U; u++) c[u] = P[(size_t)(d_imax(n - 1 - u, r) - 1) * ps];
+    double y0 = dv_rcp_seed(c[0].y + p);
     for (int bj = n - 1; bj >= r; bj -= blklen) {
       const int jend = d_imax(bj - blklen + 1, r);
-      int neg2 = 0;
+      int neg2 = 0, j = bj;
       const double bsav = p;
-      for (int j0 = bj; j0 >= jend; j0 -= U) {
+      for (; j - U + 1 >= jend; j -= U) {
 #pragma unroll
-        for (int u = 0; u < U; u++) nx[u] = P[(size_t)(d_imax(j0 - U - u, r) - 1) * ps];
+        for (int u = 0; u < U; u++) nx[u] = P[(size_t)(d_imax(j - U - u, r) - 1) * ps];
+        const double p0 = p;
+        const int n0 = neg2;
+        qdiv_chk k;
+        qdiv_begin(&k);
 #pragma unroll
         for (int u = 0; u < U; u++) {
-          if (j0 - u >= jend) {
-            double dminus = c[u].y + p;
+          const double dminus = c[u].y + p;
+          double qt;
+          const double tmp = dv_qdiv(p, dminus, y0, &k, &qt);
+          y0 = dv_rcp_seed((u + 1 < U ? c[u + 1].y : nx[0].y) + (qt * c[u].x - sigma));
+          neg2 += dv_signbit(dminus);
+          p = tmp * c[u].x - sigma;
+        }
+        if (qdiv_failed(k)) {
+          p = p0;
+          neg2 = n0;
+#pragma unroll 1
+          for (int u = 0; u < U; u++) {
+            const double2 v = P[(size_t)(j - u - 1) * ps];
+            const double dminus = v.y + p;
             neg2 += (dminus < 0.0);
-            double tmp = p / dminus;
-            p = tmp * c[u].x - sigma;
+            const double tmp = p / dminus;
+            p = tmp * v.x - sigma;
           }
+          y0 = dv_rcp_seed(nx[0].y + p);
         }
 #pragma unroll
         for (int u = 0; u < U; u++) c[u] = nx[u];
       }
+      for (; j >= jend; j--) {
+        const double2 v = P[(size_t)(j - 1) * ps];
+        const double dminus = v.y + p;
+        neg2 += (dminus < 0.0);
+        const double tmp = p / dminus;
+        p = tmp * v.x - sigma;
+      }
       if (isnan(p)) {
         neg2 = 0;
         p = bsav;
-        for (int j = bj; j >= jend; j--) {
-          const double2 v = P[(size_t)(j - 1) * ps];
+        for (int i = bj; i >= jend; i--) {
+          const double2 v = P[(size_t)(i - 1) * ps];
           double dminus = v.y + p;
           neg2 += (dminus < 0.0);
           double tmp = p / dminus;
           if (isnan(tmp)) tmp = 1.0;
           p = tmp * v.x - sigma;
         }
+        y0 = dv_rcp_seed(c[0].y + p);
       }
       negcnt += neg2;
     }
@@ -484,7 +658,7 @@ static __device__ __noinline__ int dv_dlarrb_tree(int L, int n, const double2 *_
       for (int j = 0; j < k; j++) { x = side ? x + back : x - back; back = 2.0 * back; }
       const bool mine = side ? need1 : need0;
       int cnt = 0;
-      if (mine) cnt = dv_dlaneg<MR3_U>(n, R, ps, x, r);
+      if (mine) cnt = dv_dlaneg<QDIV_U>(n, R, ps, x, r);
       const bool ok = mine && (side ? (cnt >= i) : (cnt <= i - 1));
       const unsigned gb = (__ballot_sync(full, ok) >> g0) & gbits;
       for (int sd = 0; sd < 2; sd++) {
@@ -527,7 +701,7 @@ static __device__ __noinline__ int dv_dlarrb_tree(int L, int n, const double2 *_
       if ((node_t >> b) & 1) l = m; else rr = m;
     }
     int cnt = 0;
-    if (!done) cnt = dv_dlaneg<MR3_U>(n, R, ps, 0.5 * (l + rr), r);
+    if (!done) cnt = dv_dlaneg<QDIV_U>(n, R, ps, 0.5 * (l + rr), r);
     int node = 1;
     for (int d = 0; d < depth; d++) {
       const int c = __shfl_sync(full, cnt, g0 + node);

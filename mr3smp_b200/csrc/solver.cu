@@ -1562,7 +1562,7 @@ k_cl_ext(int ncl, int L, const ClusterDev *cl, const ProbDev *probs, const Block
     int nc = 0;
     if (!TREE) {
       if (valid)
-        dv_dlarrb_one<MR3_U>(nb, Pp, ps, i, 1, II > 1, 0.0, 0.0, tol.rqtol, tol.rqtol, p->pivmin,
+        dv_dlarrb_one<QDIV_U>(nb, Pp, ps, i, 1, II > 1, 0.0, 0.0, tol.rqtol, tol.rqtol, p->pivmin,
                              maxitr, nb, &wv, &ev, &nc);
     } else {
       dv_dlarrb_tree(L, nb, Pp, ps, i, 1, II > 1, 0.0, 0.0, tol.rqtol, tol.rqtol, p->pivmin, maxitr,
@@ -1691,29 +1691,35 @@ __device__ __forceinline__ unsigned long long refine_cl_body(
   const int maxitr = dv_itmax(C.bl_spdiam + p->pivmin, p->pivmin);
   double w = Wsh[s], e = Werr[s];
   int nc = 0;
-  dv_dlarrb_one<MR3_U>(B.nbl, P, ps, i, i == pidx, II > 1, rgap, lgap, tol.rtol1, tol.rtol2, p->pivmin,
+  dv_dlarrb_one<QDIV_U>(B.nbl, P, ps, i, i == pidx, II > 1, rgap, lgap, tol.rtol1, tol.rtol2, p->pivmin,
                 maxitr, B.nbl, &w, &e, &nc);
   Wsh[s] = w;
   Werr[s] = e;
   return (unsigned long long)nc * (unsigned long long)B.nbl;
 }
 
-// Threads per SM that the tree forms may fill (a launch of few intervals
-// gets as many lanes per interval as fit; more than the resident threads
-// run in waves, which the tree's steps per count outweigh)
-#ifndef MR3_TREE_BUDGET
-#define MR3_TREE_BUDGET 2048
-#endif
-
-// Lanes per interval for a launch of `items` independent dlarrb intervals:
-// a thread each when they fill the GPU, else groups of 4..32 lanes running
-// the tree bisection (the same intervals, fewer sequential sweeps).
-__host__ __device__ __forceinline__ int tree_lanes(long long items, long long lanes,
-                                                   int maxL = 32) {
-  if (maxL < 4) return 1;
-  int L = maxL > 32 ? 32 : maxL;
-  while (L > 4 && items * L > lanes) L >>= 1;
-  return items * L > lanes ? 1 : L;
+// Lanes per interval for a launch of `items` independent intervals: the
+// form with the shortest time per bisection step.  A group of L lanes takes
+// log2(L) steps per count, a thread (L = 1) one.  A count's row costs the
+// larger of the chain's latency (90 cycles with dv_qdiv, 193 with plain
+// divisions) and the FP64 pipe's time for the warps of a quarter SM (50
+// cycles a warp for either form, measured with the SM full).  So lanes are
+// added while the chain's latency hides them and not beyond: 9000 intervals
+// take 4 lanes each (47 cycles a step; 32 lanes, which fill the SM with 15
+// warps a quarter, 103), 1000 take 32.
+#define MR3_ROW_LAT 90
+#define MR3_ROW_LAT1 193
+#define MR3_ROW_PIPE 50
+__host__ __device__ __forceinline__ int tree_lanes(long long items, int nsm, int maxL = 32) {
+  int best = 1;
+  double best_cost = 0.0;
+  for (int L = 1; L <= 32 && L <= maxL; L = L == 1 ? 4 : 2 * L) {
+    const double pipe = MR3_ROW_PIPE * (double)(items * L) / (32.0 * 4.0 * nsm);
+    const double lat = L == 1 ? MR3_ROW_LAT1 : MR3_ROW_LAT, row = lat > pipe ? lat : pipe;
+    const int steps = L == 32 ? 5 : L == 16 ? 4 : L == 8 ? 3 : L == 4 ? 2 : 1;
+    if (L == 1 || row / steps < best_cost) { best = L; best_cost = row / steps; }
+  }
+  return best;
 }
 
 template <bool TREE>
@@ -1721,10 +1727,10 @@ __global__ void LB_REF
 k_refine_cl(const int *rl, const int *rl_n, const ClusterDev *cl, const ProbDev *probs,
             const BlockDev *blocks, const double *arena_cur, double *Wsh, double *Werr,
             const double *Wgap, const int *Windex, const int *cl_of_slot, const int *lvl_of_slot,
-            int level, Tol tol, long long lanes, int tree_max, unsigned long long *stats) {
+            int level, Tol tol, int nsm, int tree_max, unsigned long long *stats) {
   const int cnt = *rl_n;
   unsigned long long work = 0;
-  const int L0 = cnt > 0 ? tree_lanes(cnt, lanes, tree_max) : 1;
+  const int L0 = cnt > 0 ? tree_lanes(cnt, nsm, tree_max) : 1;
   if (cnt > 0 && (L0 > 1) == TREE) {   // the other instantiation has the other form
     const int L = L0;
     const long long gt = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -3450,8 +3456,10 @@ extern "C" int mr3_cuda_solve_cb(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void
   // host's syncs (the kernels that wrote them have finished)
   std::vector<int> mest(L, 0);
   size_t ntiles = 0;
+  long long nwant = 0;   // eigenvalues wanted (range V: at most)
   for (int k = 0; k < L; k++) {
     const mr3_cuda_prob &q = pr[idx[k]];
+    nwant += q.range == MR3_RANGE_I ? q.iu - q.il + 1 : q.n;
     if (q.jobz == MR3_JOB_V && q.range != MR3_RANGE_V)
       mest[k] = q.range == MR3_RANGE_I ? q.iu - q.il + 1 : q.n;
     ntiles += (mest[k] + ZT_COLS - 1) / ZT_COLS;
@@ -3559,7 +3567,7 @@ extern "C" int mr3_cuda_solve_cb(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void
   LAUNCH(k_blocks, L, MR3_THREADS, c->probs, c->blocks, c->D, c->E, c->gers, c->TP, tol);
   unsigned long long *stats = c->prof ? c->stats : nullptr;
   {
-    const int Lb = tree_lanes(NN, (long long)c->nsm * MR3_TREE_BUDGET, tree_max);
+    const int Lb = tree_lanes(nwant, c->nsm, tree_max);
     if (Lb == 1) {
       // shared intervals breadth-first, then a thread per eigenvalue
       CK(cudaMemsetAsync(c->bis_st, 0xff, N * sizeof(BisState), st), "bis st");
@@ -3593,7 +3601,7 @@ extern "C" int mr3_cuda_solve_cb(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void
   LAUNCH(k_root, L, MR3_THREADS, c->probs, c->blocks, c->D, c->E, c->TP, c->Dt, c->Lt, c->W,
          c->Werr, c->Wgap, c->RP, c->RQ);
   {
-    const int Lr = tree_lanes(NN, (long long)c->nsm * MR3_TREE_BUDGET, tree_max);
+    const int Lr = tree_lanes(nwant, c->nsm, tree_max);
     if (Lr == 1)
       LAUNCH(k_refine_root<false>, gN128, 128, NN, 1, c->probs, c->blocks, c->iblk, c->RP, c->W,
              c->Werr, c->Wgap, tol, stats);
@@ -3638,14 +3646,14 @@ extern "C" int mr3_cuda_solve_cb(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void
     const int DEPTH_CAP = 512;
     ClsScratch xs;
     xs.ns = c->cls_ns; xs.soff = c->cls_soff; xs.cbase = c->cls_cbase; xs.abase = c->cls_abase;
-    const long long lanes = (long long)c->nsm * MR3_TREE_BUDGET;   // lanes a launch can keep busy
+    const long long lanes = (long long)c->nsm * 2048;   // lanes a launch can keep resident
     bool rounds_pending = false;
     for (int level = 0; ncl > 0; level++) {
       if (level >= DEPTH_CAP) { snprintf(c->err, sizeof(c->err), "representation tree too deep"); return MR3_EMISC; }
       const int cur = level & 1, nxt = cur ^ 1;
       const int gW = (ncl * 32 + MR3_THREADS - 1) / MR3_THREADS;
       if (level > 0) {
-        const int Lx = tree_lanes(2LL * ncl, lanes, tree_max);
+        const int Lx = tree_lanes(2LL * ncl, c->nsm, tree_max);
         if (Lx == 1)
           LAUNCH(k_cl_ext<false>, (int)((2LL * ncl + 127) / 128), 128, ncl, 1, c->cl[cur], c->probs,
                  c->blocks, c->RP, c->RQ, c->arena[nxt], c->Wsh, c->Werr, c->Windex, c->Wt, c->Et,
@@ -3676,10 +3684,10 @@ extern "C" int mr3_cuda_solve_cb(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void
         // length returns at once (the length is known on the device only)
         LAUNCH(k_refine_cl<false>, gN128, 128, c->rl, c->rl_n, c->cl[cur], c->probs, c->blocks,
                c->arena[cur], c->Wsh, c->Werr, c->Wgap, c->Windex, c->cl_of_slot, c->lvl_of_slot,
-               level, tol, lanes, tree_max, stats);
+               level, tol, c->nsm, tree_max, stats);
         LAUNCH(k_refine_cl<true>, (int)(lanes / 128), 128, c->rl, c->rl_n, c->cl[cur], c->probs,
                c->blocks, c->arena[cur], c->Wsh, c->Werr, c->Wgap, c->Windex, c->cl_of_slot,
-               c->lvl_of_slot, level, tol, lanes, tree_max, stats);
+               c->lvl_of_slot, level, tol, c->nsm, tree_max, stats);
         LAUNCH(k_gaps_cl, gN, 256, NN, c->cl[cur], c->Wsh, c->Werr, c->Wgap, c->W, c->cl_of_slot,
                c->lvl_of_slot, level);
       }
