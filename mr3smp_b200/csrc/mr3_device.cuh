@@ -2713,63 +2713,143 @@ static __device__ __noinline__ void dv_r1s_call(int n, double lambda, const doub
 // (SRC/LAPACK/odrrf.f:226-252) for one shift: DPLUS into dp[i*os], LPLUS
 // into lp[i*os]; returns max |DPLUS|, sawnan when a pivot was replaced by
 // -pivmin.  The running pivot stays in a register (it is written out, never
-// read back) and the rows are read in chunks of MR3_U issued one chunk
-// ahead of the arithmetic.
+// read back); quotients by dv_qdiv in checked chunks, rows loaded one chunk
+// ahead of the arithmetic.  A pivot that may be below pivmin in magnitude
+// fails its chunk's check, so the replacement is left to the plain rows.
 static __device__ __forceinline__ double rrf_sweep(int n, const double2 *__restrict__ P,
                                                    const double2 *__restrict__ Q, int ps,
-                                                   double sig, double pivmin, double *dp,
-                                                   double *lp, int os, bool *sawnan) {
-  constexpr int U = MR3_U;
+                                                   double sig, double pivmin,
+                                                   double *__restrict__ dp,
+                                                   double *__restrict__ lp, int os, bool *sawnan) {
+  constexpr int U = QDIV_U;
   double s = -sig;
   double d = P[0].x + s;
   if (fabs(d) < pivmin) { d = -pivmin; *sawnan = true; }
   dp[0] = d;
   double mx = fabs(d);
   const int last = n - 2;   // rows i = 0..n-2 produce LPLUS(i), DPLUS(i+1)
-  if (last >= 0) {
+  int i0 = 0;
+  if (last + 1 >= U) {
+    const unsigned hp = dv_habs(pivmin);
+    double y0 = dv_rcp_seed(d);
     double2 cq[U], nq[U];
     double cp[U], np_[U];
 #pragma unroll
     for (int u = 0; u < U; u++) {
-      const int i = d_imin(u, last);
-      cq[u] = Q[(size_t)i * ps];
-      cp[u] = P[(size_t)(i + 1) * ps].x;
+      cq[u] = Q[(size_t)u * ps];
+      cp[u] = P[(size_t)(u + 1) * ps].x;
     }
-    for (int i0 = 0; i0 <= last; i0 += U) {
+    for (; i0 + U - 1 <= last; i0 += U) {
 #pragma unroll
       for (int u = 0; u < U; u++) {
         const int i = d_imin(i0 + U + u, last);
         nq[u] = Q[(size_t)i * ps];
         np_[u] = P[(size_t)(i + 1) * ps].x;
       }
+      const double s0 = s, d0 = d, mx0 = mx;
+      unsigned dmin = 0xffffffffu;
+      qdiv_chk k;
+      qdiv_begin(&k);
 #pragma unroll
       for (int u = 0; u < U; u++) {
-        const int i = i0 + u;
-        if (i <= last) {
-          const double l = cq[u].y / d;
+        double qt;
+        const double l = dv_qdiv(cq[u].y, d, y0, &k, &qt);
+        y0 = dv_rcp_seed(cp[u] + (s * qt * cq[u].x - sig));
+        lp[(size_t)(i0 + u) * os] = l;
+        s = s * l * cq[u].x - sig;
+        d = cp[u] + s;
+        dmin = min(dmin, dv_habs(d));
+        dp[(size_t)(i0 + u + 1) * os] = d;
+        mx = fmax(mx, fabs(d));
+      }
+      if (qdiv_failed(k) || dmin <= hp) {
+        s = s0;
+        d = d0;
+        mx = mx0;
+#pragma unroll 1
+        for (int u = 0; u < U; u++) {
+          const int i = i0 + u;
+          const double2 q = Q[(size_t)i * ps];
+          const double l = q.y / d;
           lp[(size_t)i * os] = l;
-          s = s * l * cq[u].x - sig;
-          d = cp[u] + s;
+          s = s * l * q.x - sig;
+          d = P[(size_t)(i + 1) * ps].x + s;
           if (fabs(d) < pivmin) { d = -pivmin; *sawnan = true; }
           dp[(size_t)(i + 1) * os] = d;
           mx = fmax(mx, fabs(d));
         }
+        y0 = dv_rcp_seed(d);
       }
 #pragma unroll
       for (int u = 0; u < U; u++) { cq[u] = nq[u]; cp[u] = np_[u]; }
     }
   }
+  for (; i0 <= last; i0++) {
+    const double2 q = Q[(size_t)i0 * ps];
+    const double l = q.y / d;
+    lp[(size_t)i0 * os] = l;
+    s = s * l * q.x - sig;
+    d = P[(size_t)(i0 + 1) * ps].x + s;
+    if (fabs(d) < pivmin) { d = -pivmin; *sawnan = true; }
+    dp[(size_t)(i0 + 1) * os] = d;
+    mx = fmax(mx, fabs(d));
+  }
   return mx;
+}
+
+// The growth quantity RRR1 (RRR2) of dlarrf (odrrf.f:268-303): a = DPLUS and
+// b = LPLUS of the accepted side's mate as its loops pair them; rows are read
+// in chunks one chunk ahead (each row of one shift is os doubles apart).
+static __device__ __noinline__ double rrf_rrr(int n, const double *a, const double *b, int os,
+                                              double spdiam) {
+  constexpr int U = 8;
+  const double eps = MR3_EPS;
+  double ai = a[(size_t)(n - 1) * os], bi = 0.0;   // a(i), b(i); b(n-1) is not used (prod = 1)
+  double tmp = fabs(ai), znm2 = 1.0, prod = 1.0, oldp = 1.0;
+  double ca[U], cb[U], na[U], nb[U];
+#pragma unroll
+  for (int u = 0; u < U; u++) {
+    const int i = d_imax(n - 2 - u, 0);
+    ca[u] = a[(size_t)i * os];
+    cb[u] = b[(size_t)i * os];
+  }
+  for (int i0 = n - 1; i0 >= 1; i0 -= U) {
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int i = d_imax(i0 - U - u - 1, 0);
+      na[u] = a[(size_t)i * os];
+      nb[u] = b[(size_t)i * os];
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (i0 - u >= 1) {
+        if (prod <= eps)
+          prod = ((ai * bi) / (ca[u] * cb[u])) * oldp;
+        else
+          prod = prod * fabs(cb[u]);
+        oldp = prod;
+        znm2 = znm2 + prod * prod;
+        tmp = fmax(tmp, fabs(ca[u] * prod));
+        ai = ca[u];
+        bi = cb[u];
+      }
+#pragma unroll
+    for (int u = 0; u < U; u++) { ca[u] = na[u]; cb[u] = nb[u]; }
+  }
+  return tmp / (spdiam * sqrt(znm2));
 }
 
 // dlarrf, LAPACK 3.2.2 with NOFAIL (SRC/LAPACK/odrrf.f:140-378), one thread.
 // Parent rows: d = P[i].x, l = Q[i].x, ld = Q[i].y.  w/wgap/werr point at the
-// cluster's first eigenvalue (CLSTRT = 1, CLEND = clend).  dplus, lplus: out;
-// work: 2n scratch.  Returns the shift sigma.
+// cluster's first eigenvalue (CLSTRT = 1, CLEND = clend).  dplus, lplus: the
+// left shift's factors; work: the right shift's (2n).  Returns the shift
+// sigma; *alt tells that the accepted factors are the right shift's, left in
+// work (one lane's copy of 2n strided rows took longer than their sweep).
 // PAIR: two lanes (an even lane and the next odd one) per cluster, with the
 // same arguments; the even lane sweeps the left shift while the odd one
-// sweeps the right shift, so that a try costs one sweep's time instead of
-// two when the left shift fails.  The right sweep is run even when the left
+// sweeps the right shift, in lock-step (one call on the lane's own shift and
+// arrays), so that a try costs one sweep's time instead of two when the left
+// shift fails.  The right sweep is run even when the left
 // one is accepted; its output (the work array) is then not used, so the
 // result -- the shift and the representation in dplus/lplus -- is the
 // sequential one bit for bit.  Both lanes return the shift.
@@ -2779,10 +2859,7 @@ static __device__ __noinline__ double dv_dlarrf(int n, const double2 *__restrict
                                          const double *w, const double *wgap, const double *werr,
                                          double spdiam, double clgapl, double clgapr,
                                          double pivmin, double *dp_, double *lp_, double *wk_,
-                                         int os) {
-#define dplus(i) dp_[(size_t)(i) * os]
-#define lplus(i) lp_[(size_t)(i) * os]
-#define work(i) wk_[(size_t)(i) * os]
+                                         int os, int *alt) {
   const double maxgrowth1 = 8.0, maxgrowth2 = 8.0, eps = MR3_EPS, fact = 2.0;
   const int ktrymax = 1;
   int shift = 0, indx = 0, ktry = 0;
@@ -2813,9 +2890,8 @@ static __device__ __noinline__ double dv_dlarrf(int n, const double2 *__restrict
       const unsigned pm = 3u << ((threadIdx.x & 31) & ~1);   // this lane pair
       const bool right = (threadIdx.x & 1) != 0;
       bool sn = false;
-      const double mx = right ? rrf_sweep(n, P, Q, ps, rsigma, pivmin, wk_, wk_ + (size_t)n * os,
-                                          os, &sn)
-                              : rrf_sweep(n, P, Q, ps, lsigma, pivmin, dp_, lp_, os, &sn);
+      const double mx = rrf_sweep(n, P, Q, ps, right ? rsigma : lsigma, pivmin, right ? wk_ : dp_,
+                                  right ? wk_ + (size_t)n * os : lp_, os, &sn);
       const int src = (threadIdx.x & 31) & ~1;
       max1 = __shfl_sync(pm, mx, src);
       sawnan1 = __shfl_sync(pm, (int)sn, src) != 0;
@@ -2848,31 +2924,12 @@ static __device__ __noinline__ double dv_dlarrf(int n, const double2 *__restrict
       bool dorrr1 = (clwdth < mingap / 128.0) && (fmin(max1, max2) < fail2) && !sawnan1 &&
                     !sawnan2;
       if (dorrr1) {
+        // the two loops pair the arrays crosswise, as in odrrf.f
         if (indx == 1) {
-          double tmp = fabs(dplus(n - 1)), znm2 = 1.0, prod = 1.0, oldp = 1.0;
-          for (int i = n - 1; i >= 1; i--) {
-            if (prod <= eps)
-              prod = ((dplus(i) * work(n + i)) / (dplus(i - 1) * work(n + i - 1))) * oldp;
-            else
-              prod = prod * fabs(work(n + i - 1));
-            oldp = prod;
-            znm2 = znm2 + prod * prod;
-            tmp = fmax(tmp, fabs(dplus(i - 1) * prod));
-          }
-          double rrr1 = tmp / (spdiam * sqrt(znm2));
+          const double rrr1 = rrf_rrr(n, dp_, wk_ + (size_t)n * os, os, spdiam);
           if (rrr1 <= maxgrowth2) { sigma = lsigma; shift = 1; break; }
         } else if (indx == 2) {
-          double tmp = fabs(work(n - 1)), znm2 = 1.0, prod = 1.0, oldp = 1.0;
-          for (int i = n - 1; i >= 1; i--) {
-            if (prod <= eps)
-              prod = ((work(i) * lplus(i)) / (work(i - 1) * lplus(i - 1))) * oldp;
-            else
-              prod = prod * fabs(lplus(i - 1));
-            oldp = prod;
-            znm2 = znm2 + prod * prod;
-            tmp = fmax(tmp, fabs(work(i - 1) * prod));
-          }
-          double rrr2 = tmp / (spdiam * sqrt(znm2));
+          const double rrr2 = rrf_rrr(n, wk_, lp_, os, spdiam);
           if (rrr2 <= maxgrowth2) { sigma = rsigma; shift = 2; break; }
         }
       }
@@ -2890,17 +2947,8 @@ static __device__ __noinline__ double dv_dlarrf(int n, const double2 *__restrict
     rsigma = bestshift;
     forcer = true;
   }
-  if (shift == 2) {
-    // PAIR: the even lane copies DPLUS, the odd one LPLUS
-    if (!PAIR || (threadIdx.x & 1) == 0)
-      for (int i = 0; i < n; i++) dplus(i) = work(i);
-    if (!PAIR || (threadIdx.x & 1) != 0)
-      for (int i = 0; i < n - 1; i++) lplus(i) = work(n + i);
-  }
+  *alt = shift == 2;
   return sigma;
-#undef dplus
-#undef lplus
-#undef work
 }
 
 // One interval of dlarrj (SRC/LAPACK/odrrj.f:100-281): bisection on T to

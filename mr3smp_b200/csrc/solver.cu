@@ -98,6 +98,7 @@ struct ClusterDev {
   int pG, pg;                   // parent's group size and position
   long long grp_off;            // this cluster's group base in the current arena (depth >= 1)
   int G, g;                     // group size and position
+  int alt;                      // the accepted factors are in the dlarrf work array
   double par_sigma, sigma, tau;
 };
 
@@ -1496,7 +1497,7 @@ __global__ void k_level0(ProbDev *probs, BlockDev *blocks, const double *E, cons
       C.begin = wb; C.end = we; C.depth = 0; C.blk = p->off + b;
       C.bl_spdiam = gu - gl; C.lgap = lgap; C.par_off = -1; C.pG = 1; C.pg = 0;
       C.grp_off = -1; C.G = 1; C.g = 0;
-      C.par_sigma = sigma; C.sigma = sigma; C.tau = 0.0;
+      C.par_sigma = sigma; C.sigma = sigma; C.tau = 0.0; C.alt = 0;
       cl[c] = C;
     }
   }
@@ -1613,11 +1614,13 @@ k_cl_rrf(int ncl, ClusterDev *cl, const ProbDev *probs, const BlockDev *blocks, 
       Wsh[ce] = w1; Werr[ce] = e1;
     }
     if (PAIR) __syncwarp(3u << ((threadIdx.x & 31) & ~1));
+    int alt = 0;
     const double tau = dv_dlarrf<PAIR>(nb, Pp, Qp, ps, ce - cb + 1, Wsh + cb, Wgap + cb,
                                        Werr + cb, C.bl_spdiam, C.lgap, Wgap[ce], p->pivmin, dplus,
-                                       lplus, wk, C.G);
+                                       lplus, wk, C.G, &alt);
     if (lead) {
       cl[w].tau = tau;
+      cl[w].alt = alt;
       cl[w].sigma = C.par_sigma + tau;
       work = 2ull * nb;
     }
@@ -1639,7 +1642,6 @@ __global__ void k_cl_pack(int ncl, const ClusterDev *cl, const BlockDev *blocks,
     double *grp = arena_cur + L0.grp_off;
     double2 *Pn = reinterpret_cast<double2 *>(grp);
     double2 *Qn = reinterpret_cast<double2 *>(grp + 2 * nG);
-    const double *dplus = grp + 4 * nG, *lplus = grp + 5 * nG;
     for (int m = 0; m < G; m++) {
       const ClusterDev C = cl[w + m];
       const double tau = C.tau;
@@ -1657,16 +1659,18 @@ __global__ void k_cl_pack(int ncl, const ClusterDev *cl, const BlockDev *blocks,
       if (threadIdx.x == 0) atomicAdd(rl_n, C.end - C.begin + 1);
     }
     for (long long idx = threadIdx.x; idx < nG; idx += blockDim.x) {
-      const int i = (int)(idx / G);
+      const int i = (int)(idx / G), m = (int)(idx - (long long)i * G);
+      // DPLUS and LPLUS of the accepted shift (dlarrf's outputs or its work array)
+      const double *dplus = grp + (cl[w + m].alt ? 6 : 4) * nG;
       double dv = dplus[idx];
       if (i < nb - 1) {
-        double lv = lplus[idx];
+        double lv = dplus[nG + idx];
         double ld = dv * lv;
         Pn[idx] = make_double2(dv, ld * lv);
         Qn[idx] = make_double2(lv, ld);
       } else {
         Pn[idx] = make_double2(dv, 0.0);
-        Qn[idx] = make_double2(cl[w + (int)(idx % G)].sigma, 0.0);
+        Qn[idx] = make_double2(cl[w + m].sigma, 0.0);
       }
     }
   }
@@ -1926,7 +1930,7 @@ k_classify(int ncl, const ClusterDev *cl, const BlockDev *blocks, const double *
   proto.depth = depth + 1; proto.blk = C.blk; proto.bl_spdiam = C.bl_spdiam;
   proto.par_off = (depth == 0) ? -1 : C.grp_off;
   proto.pG = C.G; proto.pg = C.g;
-  proto.par_sigma = C.sigma; proto.sigma = 0.0; proto.tau = 0.0;
+  proto.par_sigma = C.sigma; proto.sigma = 0.0; proto.tau = 0.0; proto.alt = 0;
   proto.grp_off = 0; proto.G = 1; proto.g = 0;
   int s_base = 0, c_base = 0, nc_tot = 0;
   long long a_base = 0;
