@@ -2516,187 +2516,280 @@ static __device__ __noinline__ void dv_r1w_solve(bool active, int n, double lamb
 }
 
 // ------------------------------------------------------------------------
-// dlar1v for one eigenvector on a whole warp (the short lists at the end of
-// a level, where latency rather than throughput counts).  The stationary
-// sweep (lane 0) and the progressive sweep (lane 1) are independent chains
-// and run at the same time, each keeping every row's values in the warp's
-// scratch (SI and LPLUS of the stationary rows, P and UMINUS of the
-// progressive ones); the twist index is then chosen by all 32 lanes (the
-// smallest |gamma(i)|, the largest i among equal ones: what odr1v.f's upward
-// scan with .LE. selects); the back-substitution runs upward on lane 0 and
-// downward on lane 1, and lane 0 adds the downward squares to ztz after its
-// own, in odr1v.f's order.  Every value is computed by the operations of
-// odr1v.f:158-362 in their order, so the results are those of
+// dlar1v for one eigenvector on a group of L lanes (lists short enough that
+// latency counts).  The stationary sweep (lane 0 of the group) and the
+// progressive sweep (lane 1) are independent chains and run at the same
+// time, each keeping every row's values in the group's scratch (SI and LPLUS
+// of the stationary rows, P and UMINUS of the progressive ones); the twist
+// index is then chosen by all L lanes (the smallest |gamma(i)|, the largest
+// i among equal ones: what odr1v.f's upward scan with .LE. selects); the
+// back-substitution runs upward on lane 0 and downward on lane 1, and lane 0
+// adds the downward squares to ztz after its own, in odr1v.f's order.  Every
+// value is the one of odr1v.f:158-362, so the results are those of
 // dv_r1c_factor + dv_r1c_solve bit for bit.
-// Scratch per warp (nmax doubles each): SI, LP, PA, UM, ZV, rows 1-based at
-// [row]: SI[i], LP[i] of stationary row i; PA[i] the progressive value after
-// row i (PA[n] = D(n) - lambda); UM[i] of row i; ZV[i] the vector.
+//
+// A sweep is a chain of n rows, and a warp's two branches of an if would run
+// one after the other, so both lanes run one instruction stream: row by row
+//   t = a / (d + x);  v = (x t) f;  x = v - lambda
+// with d, a, f = D, L D, L (stationary) and D L^2, D, 1 (progressive; the
+// product with 1 is exact), quotients by dv_qdiv in checked chunks.  The
+// back-substitution forms a chunk of z and tests its rows for truncation
+// afterwards, instead of one dependent branch a row.  One group a warp:
+// 270 cycles a row and call with two branches, 150 so (n = 4096).
+//
+// Scratch per group: SI, LP, PA, UM, ZV, row i (1-based) at [i * st]; groups
+// of a warp are interleaved (st = groups per warp), so that their sweeps,
+// which mostly stand at the same row, write whole sectors.  PA[i] is the
+// progressive value after row i (PA[n] = D(n) - lambda); ZV is the vector.
 // ------------------------------------------------------------------------
 struct r1s_buf {
   double *SI, *LP, *PA, *UM, *ZV;
+  int st;
 };
 
-// Rows the split form's sweeping lanes prefetch ahead of their arithmetic
-// (0: none).  A lane sweeps alone, so nothing else hides the latency of its
-// loads; the child representations live in DRAM.
-#ifndef MR3_R1S_PF
-#define MR3_R1S_PF 32
-#endif
-static __device__ __forceinline__ void pf_l2(const void *p) {
-  asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
-}
-
-static __device__ __noinline__ void dv_r1s_call(int n, double lambda, const double2 *__restrict__ P,
+static __device__ __noinline__ void dv_r1s_call(bool active, int L, int n, double lambda,
+                                         const double2 *__restrict__ P,
                                          const double2 *__restrict__ Q, int ps, double pivmin,
-                                         bool wantnc, int r_in, double gaptol, r1s_buf b,
+                                         bool wantnc, int r_in, double gaptol, const r1s_buf &b,
                                          int *negcnt_o, dlar1v_out *o) {
-  const unsigned full = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
+  constexpr int U = QDIV_U;
+  const int lane = threadIdx.x & 31, t = lane & (L - 1), g0 = lane - t;
+  const unsigned gm = ((L == 32) ? 0xffffffffu : ((1u << L) - 1u)) << g0;
   const double eps = MR3_EPS;
+  const long long st = b.st;
+  if (!active) return;   // a whole group
   int r1 = 1, r2 = n;
   if (r_in != 0) { r1 = r_in; r2 = r_in; }
+  const bool up = t == 0;
   // ---- the two sweeps, rerun with the NaN-safe formulas where needed
-  int neg1 = 0, neg2 = 0;
-  bool slowA = false, slowB = false;
-  double sr1 = 0.0;   // SI of row r1-1 (0 for r1 = 1)
-  if (lane == 0) {
-    for (int pass = 0; pass < 2; pass++) {
-      const bool SLOW = pass == 1;
-      double s = 0.0 - lambda;
-      bool sawnan = false;
-      neg1 = 0;
-      sr1 = 0.0;
-#pragma unroll 4
-      for (int i = 1; i <= r2 - 1; i++) {
-        if (MR3_R1S_PF && i + MR3_R1S_PF <= r2 - 1) {
-          pf_l2(&P[(size_t)(i + MR3_R1S_PF - 1) * ps]);
-          pf_l2(&Q[(size_t)(i + MR3_R1S_PF - 1) * ps]);
-        }
-        const double2 pp = P[(size_t)(i - 1) * ps], q = Q[(size_t)(i - 1) * ps];
-        double dplus = pp.x + s;
-        if (SLOW && fabs(dplus) < pivmin) dplus = -pivmin;
-        const double lp = q.y / dplus;
-        if (i <= r1 - 1) neg1 += (dplus < 0.0);
-        double si = s * lp * q.x;
-        if (SLOW && lp == 0.0) si = pp.y;
-        s = si - lambda;
-        b.LP[i] = lp;
-        b.SI[i] = si;
-        if (i == r1 - 1) {
-          sr1 = si;
-          if (!SLOW && isnan(s)) sawnan = true;
-        }
-        if (sawnan) break;
+  int neg = 0;
+  bool slow1 = false;   // this lane's sweep needed the NaN-safe formulas
+  double sr1 = 0.0;     // SI of row r1-1 (0 for r1 = 1)
+  if (t < 2) {
+    const int m = up ? r2 - 1 : n - r1;   // rows of this lane's sweep
+    const long long first = up ? 0 : 2LL * (n - 2) * ps, step = up ? 2LL * ps : -2LL * ps;
+    const double *Pd = reinterpret_cast<const double *>(P), *Qd = reinterpret_cast<const double *>(Q);
+    const double *pd = Pd + first + (up ? 0 : 1);
+    const double *pa = up ? Qd + 1 : Pd + first;
+    const double *pc = Qd + first;
+    const long long ostep = up ? st : -st;
+    double *__restrict__ o1 = up ? b.LP + st : b.UM + (n - 1) * st;
+    double *__restrict__ o2 = up ? b.SI + st : b.PA + (n - 1) * st;
+    const double x_in = up ? 0.0 - lambda : Pd[2LL * (n - 1) * ps] - lambda;
+    if (!up) b.PA[n * st] = x_in;
+    double x = x_in, v = 0.0;
+    int k = 0;
+    // full: rows k .. m-1 by plain divisions; up to `upto` rows
+    auto plain = [&](int upto) {
+#pragma unroll 1
+      for (; k < upto; k++) {
+        const double c = pc[k * step];
+        const double den = pd[k * step] + x;
+        const double q = pa[k * step] / den;
+        neg += (den < 0.0);
+        v = x * q * (up ? c : 1.0);
+        x = v - lambda;
+        o1[k * ostep] = q * (up ? 1.0 : c);
+        o2[k * ostep] = up ? v : x;
       }
-      if (!SLOW && !sawnan) sawnan = isnan(s);
-      if (SLOW || !sawnan) break;
-      slowA = true;
+    };
+    if (m >= U) {
+      double cd[U], ca[U], cc[U], nd[U], na[U], nc[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) { cd[u] = pd[u * step]; ca[u] = pa[u * step]; cc[u] = pc[u * step]; }
+      double y0 = dv_rcp_seed(cd[0] + x);
+#pragma unroll 1
+      while (k + U <= m) {
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+          const long long e = d_imin(k + U + u, m - 1) * step;
+          nd[u] = pd[e]; na[u] = pa[e]; nc[u] = pc[e];
+        }
+        const double x0 = x, v0 = v;
+        const int neg0 = neg;
+        qdiv_chk ck;
+        qdiv_begin(&ck);
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+          const double den = cd[u] + x, f = up ? cc[u] : 1.0;
+          double qt;
+          const double q = dv_qdiv(ca[u], den, y0, &ck, &qt);
+          y0 = dv_rcp_seed((u + 1 < U ? cd[u + 1] : nd[0]) + (x * qt * f - lambda));
+          neg += dv_signbit(den);
+          v = x * q * f;
+          x = v - lambda;
+          o1[(k + u) * ostep] = q * (up ? 1.0 : cc[u]);
+          o2[(k + u) * ostep] = up ? v : x;
+        }
+        if (qdiv_failed(ck)) {
+          x = x0;
+          v = v0;
+          neg = neg0;
+          plain(k + U);
+          y0 = dv_rcp_seed(nd[0] + x);
+        } else {
+          k += U;
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) { cd[u] = nd[u]; ca[u] = na[u]; cc[u] = nc[u]; }
+      }
     }
-  } else if (lane == 1) {
-    for (int pass = 0; pass < 2; pass++) {
-      const bool SLOW = pass == 1;
-      double p = P[(size_t)(n - 1) * ps].x - lambda;
-      b.PA[n] = p;
-      neg2 = 0;
-#pragma unroll 4
-      for (int i = n - 1; i >= r1; i--) {
-        if (MR3_R1S_PF && i - MR3_R1S_PF >= r1) {
-          pf_l2(&P[(size_t)(i - MR3_R1S_PF - 1) * ps]);
-          pf_l2(&Q[(size_t)(i - MR3_R1S_PF - 1) * ps]);
+    plain(m);
+    if (isnan(x)) {   // odr1v.f:199-205, 234-250
+      slow1 = true;
+      neg = 0;
+      x = x_in;
+      v = 0.0;
+      for (k = 0; k < m; k++) {
+        const double c = pc[k * step], a = pa[k * step];
+        double den = pd[k * step] + x;
+        if (fabs(den) < pivmin) den = -pivmin;
+        const double q = a / den;
+        neg += (den < 0.0);
+        if (up) {
+          v = x * q * c;
+          if (q == 0.0) v = Pd[2LL * k * ps + 1];
+          x = v - lambda;
+          o1[k * ostep] = q;
+          o2[k * ostep] = v;
+        } else {
+          o1[k * ostep] = c * q;
+          x = q == 0.0 ? a - lambda : x * q - lambda;
+          o2[k * ostep] = x;
         }
-        const double2 pp = P[(size_t)(i - 1) * ps];
-        double dminus = pp.y + p;
-        if (SLOW && fabs(dminus) < pivmin) dminus = -pivmin;
-        const double tmp = pp.x / dminus;
-        neg2 += (dminus < 0.0);
-        b.UM[i] = Q[(size_t)(i - 1) * ps].x * tmp;
-        double pn = p * tmp - lambda;
-        if (SLOW && tmp == 0.0) pn = pp.x - lambda;
-        p = pn;
-        b.PA[i] = p;
       }
-      if (SLOW || !isnan(p)) break;
-      slowB = true;
+    }
+    if (up) {
+      sr1 = r_in != 0 && m > 0 ? v : 0.0;
+      if (r_in == 0) neg = 0;   // only rows 1..r1-1 are counted
     }
   }
-  neg1 = __shfl_sync(full, neg1, 0);
-  sr1 = __shfl_sync(full, sr1, 0);
-  slowA = __shfl_sync(full, slowA, 0);
-  neg2 = __shfl_sync(full, neg2, 1);
-  slowB = __shfl_sync(full, slowB, 1);
-  __syncwarp();
+  sr1 = __shfl_sync(gm, sr1, g0);
+  int negt = __shfl_sync(gm, neg, g0) + __shfl_sync(gm, neg, g0 + 1);
+  const bool slow = __any_sync(gm, slow1);
+  __syncwarp(gm);
   // ---- the twist index: gamma(i) = SI(i-1) + P(i-1) for i in (r1, r2]
   double best = 0.0;
   int rbest = 0;
-  for (int i = r1 + 1 + lane; i <= r2; i += 32) {
-    const double sprev = b.SI[i - 1];
-    double c = sprev + b.PA[i];
+#pragma unroll 4
+  for (int i = r1 + 1 + t; i <= r2; i += L) {
+    const double sprev = b.SI[(i - 1) * st];
+    double c = sprev + b.PA[i * st];
     if (c == 0.0) c = eps * sprev;
-    if (isnan(c)) continue;
-    if (rbest == 0 || fabs(c) <= fabs(best)) { best = c; rbest = i; }   // i increases
+    if (!isnan(c) && (rbest == 0 || fabs(c) <= fabs(best))) { best = c; rbest = i; }   // i increases
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    const double ob = __shfl_xor_sync(full, best, o);
-    const int orb = __shfl_xor_sync(full, rbest, o);
+  for (int s = L >> 1; s > 0; s >>= 1) {
+    const double ob = __shfl_xor_sync(gm, best, s);
+    const int orb = __shfl_xor_sync(gm, rbest, s);
     if (orb != 0 && (rbest == 0 || fabs(ob) < fabs(best) || (fabs(ob) == fabs(best) && orb > rbest))) {
       best = ob;
       rbest = orb;
     }
   }
-  const double pr1 = b.PA[r1];
+  const double pr1 = b.PA[r1 * st];
   double mg = sr1 + pr1;
-  if (mg < 0.0) neg1++;
-  *negcnt_o = wantnc ? neg1 + neg2 : -1;
+  if (mg < 0.0) negt++;
+  *negcnt_o = wantnc ? negt : -1;
   if (fabs(mg) == 0.0) mg = eps * sr1;
   int r = r1;
   if (rbest != 0 && fabs(best) <= fabs(mg)) { mg = best; r = rbest; }
-  const bool slow = slowA || slowB;
   // ---- back-substitution: upward on lane 0, downward on lane 1
-  int is1 = 1, is2 = n;
+  int stop = up ? 1 : n;   // first (last) row of the support
   double ztz = 1.0;
-  if (lane == 0) {
-    b.ZV[r] = 1.0;
-    double zp = 1.0, zpp = 0.0;
-    for (int i = r - 1; i >= 1; i--) {
-      if (MR3_R1S_PF && i - 16 >= 1) {   // the rows ahead into L1
-        pf_l1(&Q[(size_t)(i - 17) * ps]);
-        pf_l1(&b.LP[i - 16]);
+  if (t < 2) {
+    const int m = up ? r - 1 : n - r;
+    const double *Qd = reinterpret_cast<const double *>(Q);
+    const long long zs = up ? -st : st, qs = up ? -2LL * ps : 2LL * ps;
+    // step k: row i = r-1-k (upward, z(i) from z(i+1)), r+k (downward, z(i+1) from z(i))
+    const double *pm = up ? b.LP + (r - 1) * st : b.UM + r * st;
+    const double *pq = Qd + 2LL * ((up ? r - 2 : r - 1)) * ps + 1;
+    double *pz = b.ZV + (up ? r - 1 : r + 1) * st;
+    if (up) b.ZV[r * st] = 1.0;
+    double z = 1.0;
+    int k = 0;
+    if (slow) {
+      double zp = 0.0;   // the value before z
+      for (; k < m; k++) {
+        const double ldi = pq[k * qs];
+        double zn;
+        // a zero z: the quotient of the off-diagonals beside it
+        if (z == 0.0) zn = -(pq[(k - 1) * qs] / ldi) * zp;
+        else zn = -(pm[k * zs] * z);
+        if ((fabs(zn) + fabs(z)) * fabs(ldi) < gaptol) { stop = up ? r - k : r + k; break; }
+        ztz = ztz + zn * zn;
+        pz[k * zs] = zn;
+        zp = z;
+        z = zn;
       }
-      const double ldi = Q[(size_t)(i - 1) * ps].y;
-      double zi;
-      if (!slow) zi = -(b.LP[i] * zp);
-      else if (zp == 0.0) zi = -(Q[(size_t)i * ps].y / ldi) * zpp;
-      else zi = -(b.LP[i] * zp);
-      if ((fabs(zi) + fabs(zp)) * fabs(ldi) < gaptol) { is1 = i + 1; break; }
-      ztz = ztz + zi * zi;
-      b.ZV[i] = zi;
-      zpp = zp;
-      zp = zi;
-    }
-  } else if (lane == 1) {
-    double zc = 1.0, zcp = 0.0;
-    for (int i = r; i <= n - 1; i++) {
-      if (MR3_R1S_PF && i + 16 <= n - 1) {
-        pf_l1(&Q[(size_t)(i + 15) * ps]);
-        pf_l1(&b.UM[i + 16]);
+    } else {
+      double cm[U], cq[U], nm[U], nq[U];
+      if (m >= U) {
+#pragma unroll
+        for (int u = 0; u < U; u++) { cm[u] = pm[u * zs]; cq[u] = pq[u * qs]; }
       }
-      const double ldi = Q[(size_t)(i - 1) * ps].y;
-      double zn;
-      if (!slow) zn = -(b.UM[i] * zc);
-      else if (zc == 0.0) zn = -(Q[(size_t)(i - 2) * ps].y / ldi) * zcp;
-      else zn = -(b.UM[i] * zc);
-      if ((fabs(zc) + fabs(zn)) * fabs(ldi) < gaptol) { is2 = i; break; }
-      b.ZV[i + 1] = zn;
-      zcp = zc;
-      zc = zn;
+      bool go = true;
+#pragma unroll 1
+      for (; go && k + U <= m; k += U) {
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+          const long long e = d_imin(k + U + u, m - 1);
+          nm[u] = pm[e * zs];
+          nq[u] = pq[e * qs];
+        }
+        double zz[U], zl = z;
+        unsigned cut = 0u;
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+          zz[u] = -(cm[u] * zl);
+          if ((fabs(zz[u]) + fabs(zl)) * fabs(cq[u]) < gaptol) cut |= 1u << u;
+          zl = zz[u];
+        }
+        if (cut == 0u) {
+#pragma unroll
+          for (int u = 0; u < U; u++) {
+            ztz = ztz + zz[u] * zz[u];
+            pz[(k + u) * zs] = zz[u];
+          }
+          z = zl;
+        } else {
+          const int w = __ffs(cut) - 1;
+#pragma unroll
+          for (int u = 0; u < U; u++)
+            if (u < w) {
+              ztz = ztz + zz[u] * zz[u];
+              pz[(k + u) * zs] = zz[u];
+            }
+          stop = up ? r - (k + w) : r + (k + w);
+          go = false;
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) { cm[u] = nm[u]; cq[u] = nq[u]; }
+      }
+      for (; go && k < m; k++) {
+        const double zn = -(pm[k * zs] * z), ldi = pq[k * qs];
+        if ((fabs(zn) + fabs(z)) * fabs(ldi) < gaptol) { stop = up ? r - k : r + k; break; }
+        ztz = ztz + zn * zn;
+        pz[k * zs] = zn;
+        z = zn;
+      }
     }
   }
-  is2 = __shfl_sync(full, is2, 1);
-  __syncwarp();
-  if (lane == 0)
-    for (int i = r + 1; i <= is2; i++) ztz = ztz + b.ZV[i] * b.ZV[i];
-  ztz = __shfl_sync(full, ztz, 0);
-  is1 = __shfl_sync(full, is1, 0);
+  const int is1 = __shfl_sync(gm, stop, g0), is2 = __shfl_sync(gm, stop, g0 + 1);
+  __syncwarp(gm);
+  if (up) {
+    const double *pz = b.ZV + (r + 1) * st;
+    const int m = is2 - r;
+    int k = 0;
+    double c[U];
+    for (; k + U <= m; k += U) {
+#pragma unroll
+      for (int u = 0; u < U; u++) c[u] = pz[(k + u) * st];
+#pragma unroll
+      for (int u = 0; u < U; u++) ztz = ztz + c[u] * c[u];
+    }
+    for (; k < m; k++) ztz = ztz + pz[k * st] * pz[k * st];
+  }
+  ztz = __shfl_sync(gm, ztz, g0);
   o->r = r;
   o->mingma = mg;
   o->isupp1 = is1;

@@ -120,10 +120,10 @@ struct SngCounters {
   int act_n[2], act_next[2];   // round lists: entries, next entry to take
   int bs_n, bs_next, err, nin; // bisection list; err: a list outlived the
                                // rounds; nin: entries of this round's list
+  int fb_n, fb_next;           // k_sng_finish's bisection list
   int done_n, done_exp;        // finished column tiles: listed, exported to the host
   int mode, fin_ctas;          // 0 rounds; 1 the next list is finished by k_sng_finish;
-                               // 3 by k_sng_round<SNG_ITER>; 2 finished (later
-                               // rounds are empty)
+                               // 2 finished (later rounds are empty)
 };
 
 // Output column zind of a problem is written.  Columns are counted in tiles
@@ -2112,6 +2112,8 @@ __global__ void k_round_reset(SngCounters *sc, int in, int first) {
   sc->nin = first ? sc->n_sng : sc->act_n[in];
   sc->act_next[in] = 0;
   sc->bs_next = 0;
+  sc->fb_n = 0;
+  sc->fb_next = 0;
   if (first) { sc->mode = 0; sc->fin_ctas = 0; }
 }
 
@@ -2187,7 +2189,7 @@ __global__ void __launch_bounds__(256) k_list_count(const SngCounters *sc,
 // Exclusive scan of the block counts (one block of 1024 threads); the totals
 // become the next list's length and the bisection list's length.
 __global__ void __launch_bounds__(1024) k_list_scan(int nblk, SngCounters *sc, int *bcnt, int out,
-                                                    int last_round, int finish_max, int iter_max) {
+                                                    int last_round, int finish_max) {
   __shared__ int wa[32], wb[32];
   __shared__ int carry[2];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -2223,13 +2225,9 @@ __global__ void __launch_bounds__(1024) k_list_scan(int nblk, SngCounters *sc, i
     sc->act_n[out] = carry[0];
     sc->bs_n = carry[1];
     if (last_round && (carry[0] | carry[1])) sc->err = 1;
-    // a short list is finished in one launch, a warp per singleton (mode 1)
-    // or a lane per singleton (mode 3: no more than a chunk per warp)
+    // a short list is finished in one launch (k_sng_finish)
     const int left = carry[0] + carry[1];
-    if (!last_round && sc->mode == 0 && left > 0) {
-      if (left <= finish_max) sc->mode = 1;
-      else if (left <= iter_max) sc->mode = 3;
-    }
+    if (!last_round && sc->mode == 0 && left > 0 && left <= finish_max) sc->mode = 1;
   }
 }
 
@@ -2267,18 +2265,28 @@ __global__ void __launch_bounds__(256) k_list_scatter(int first, const SngCounte
   }
 }
 
-// ITER (SngCounters.mode 3, a level's tail): every lane runs its singleton's
-// remaining Rayleigh-quotient loop to the end in this launch -- one dlar1v
-// call per pass of the warp, a bisection (SRC/process_singleton.c:178-192)
-// by the whole warp with the tree bisection when a lane's step left its
-// interval -- instead of one call per round.  A tail round lasts as long as
-// the largest block's dlar1v whatever the list's length; here the tail's
-// calls follow one another without the rounds' launches between them.
-// Every call and state update is the one the rounds make (the same bits).
-// The last block to finish empties the list (mode 2).
 // KIND: SNG_LATER (rounds after the first), SNG_FIRST (the first round of a
-// level: the state starts from the eigenvalue's refinement), SNG_ITER.
-enum { SNG_LATER = 0, SNG_FIRST = 1, SNG_ITER = 2 };
+// level: the state starts from the eigenvalue's refinement).
+enum { SNG_LATER = 0, SNG_FIRST = 1 };
+// A singleton's loop variables before its first dlar1v.
+__device__ __forceinline__ SngState sng_start(int s, const SngDev &S, const BlockDev &B,
+                                              const double *Wsh, const double *Werr,
+                                              const double *Wgap) {
+  SngState st;
+  st.lambda = Wsh[s]; st.wsh = st.lambda; st.werr = Werr[s];
+  st.left = st.lambda - st.werr; st.right = st.lambda + st.werr;
+  // the reference compares the eigenvalue index with the block's first
+  // and last row (SRC/process_singleton.c:142-157); W slots and rows of
+  // a problem start at the same offset, so the same comparison is s == row
+  const double lgap = (s == B.ibgn) ? MR3_EPS * fmax(fabs(st.left), fabs(st.right)) : S.lgap;
+  const double rgap = (s == B.iend) ? MR3_EPS * fmax(fabs(st.left), fabs(st.right)) : Wgap[s];
+  st.gap = fmin(lgap, rgap);
+  st.gaptol = (s == B.ibgn || s == B.iend) ? 0.0 : st.gap * MR3_EPS;
+  st.bstres = 0.0; st.bstw = 0.0; st.resid = 0.0;
+  st.r = 0; st.k = 1; st.flags = 0; st.pad = 0;
+  return st;
+}
+
 template <int KIND>
 __global__ void __launch_bounds__(SNG_WARPS * 32, SNG_MINB)
 k_sng_round(int in, const SngDev *sng, const ClusterDev *cl, ProbDev *probs,
@@ -2287,8 +2295,7 @@ k_sng_round(int in, const SngDev *sng, const ClusterDev *cl, ProbDev *probs,
             const int *Zindex, SngState *sst, const int *act0, const int *act1,
             unsigned char *flag, SngCounters *sc, double *scratch, long long nmax,
             int2 *done_list, int *tile_left, unsigned long long *stats) {
-  constexpr bool FIRST = KIND == SNG_FIRST, ITER = KIND == SNG_ITER;
-  if (ITER && sc->mode != 3) return;
+  constexpr bool FIRST = KIND == SNG_FIRST;
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const long long gw = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
@@ -2304,7 +2311,7 @@ k_sng_round(int in, const SngDev *sng, const ClusterDev *cl, ProbDev *probs,
 #if MR3_SNG_LOCKSTEP
   extern __shared__ double ztile[];   // SNG_WARPS tiles of 32 x 33 doubles
 #endif
-  unsigned long long w_r1v = 0, w_sweep = 0, w_chunks = 0, w_neg = 0;
+  unsigned long long w_r1v = 0, w_sweep = 0, w_chunks = 0;
   for (;;) {
     int base = 0;
     if (lane == 0) base = atomicAdd(&sc->act_next[in], 32);
@@ -2316,10 +2323,8 @@ k_sng_round(int in, const SngDev *sng, const ClusterDev *cl, ProbDev *probs,
     const int j = active ? base + lane : base;
     const int idx = FIRST ? j : Ain[j];
     const int s = sng[idx].slot;
-    bool live = active;   // ITER: this lane's singleton is not finished yet
-    do {
     int nb;
-    double pivmin, lam_call, gaptol, bspd;
+    double pivmin, lam_call, gaptol;
     const double2 *P, *Q;
     double *zcol;   // the eigenvector's column of Z at the block's first row
     int ps, r_in;
@@ -2333,25 +2338,9 @@ k_sng_round(int in, const SngDev *sng, const ClusterDev *cl, ProbDev *probs,
       nb = B.nbl;
       const ProbDev *pd = &probs[B.prob];
       pivmin = pd->pivmin;
-      bspd = C.bl_spdiam;
       zcol = pd->Z + (size_t)Zindex[s] * pd->ldz + (B.ibgn - pd->off);
       own_rrr(C, B, RP, RQ, arena, &P, &Q, &ps);
-      SngState st;
-      if (FIRST) {
-        st.lambda = Wsh[s]; st.wsh = st.lambda; st.werr = Werr[s];
-        st.left = st.lambda - st.werr; st.right = st.lambda + st.werr;
-        // the reference compares the eigenvalue index with the block's first
-        // and last row (SRC/process_singleton.c:142-157); W slots and rows of
-        // a problem start at the same offset, so the same comparison is s == row
-        const double lgap = (s == B.ibgn) ? MR3_EPS * fmax(fabs(st.left), fabs(st.right)) : S.lgap;
-        const double rgap = (s == B.iend) ? MR3_EPS * fmax(fabs(st.left), fabs(st.right)) : Wgap[s];
-        st.gap = fmin(lgap, rgap);
-        st.gaptol = (s == B.ibgn || s == B.iend) ? 0.0 : st.gap * MR3_EPS;
-        st.bstres = 0.0; st.bstw = 0.0; st.resid = 0.0;
-        st.r = 0; st.k = 1; st.flags = 0; st.pad = 0;
-      } else {
-        st = sst[idx];
-      }
+      const SngState st = FIRST ? sng_start(s, S, B, Wsh, Werr, Wgap) : sst[idx];
       sm_st[threadIdx.x] = st;
       usedBS = (st.flags & SF_USEDBS) != 0;
       lam_call = (st.flags & SF_STEP2) ? st.bstw : st.lambda;
@@ -2368,27 +2357,27 @@ k_sng_round(int in, const SngDev *sng, const ClusterDev *cl, ProbDev *probs,
     r1c_state rs;
     rs.r = 0; rs.mingma = 0.0; rs.sawnan = false; rs.slowA = false; rs.slowB = false;
     int negc = 0;
-    dv_r1c_factor(live, nb, lam_call, P, Q, ps, pivmin, !usedBS, r_in, ck, &negc, &rs);
+    dv_r1c_factor(active, nb, lam_call, P, Q, ps, pivmin, !usedBS, r_in, ck, &negc, &rs);
     dlar1v_out o;
     o.isupp1 = 1; o.isupp2 = nb; o.nrminv = 0.0; o.r = 0; o.resid = 0.0; o.rqcorr = 0.0;
     // z of the support goes to the column unscaled; an accepted vector is
     // scaled below (z * nrminv, the reference's dscal after dlar1v)
 #if MR3_SNG_LOCKSTEP
-    dv_r1w_solve(live, nb, lam_call, P, Q, ps, pivmin, gaptol, rs.r, rs.sawnan, rs.slowA,
+    dv_r1w_solve(active, nb, lam_call, P, Q, ps, pivmin, gaptol, rs.r, rs.sawnan, rs.slowA,
                  rs.slowB, ck.S, ck.P, rs.mingma, zcol, write, ztile + (threadIdx.x >> 5) * 32 * 33,
                  &o);
 #else
-    if (live)
+    if (active)
       dv_r1c_solve(nb, lam_call, P, Q, ps, pivmin, gaptol, rs.r, rs.sawnan, rs.slowA, rs.slowB,
                    ck.S, ck.P, rs.mingma, write ? zcol : nullptr, 1.0, &o);
 #endif
     SngState st = sm_st[threadIdx.x];
     const bool step2 = (st.flags & SF_STEP2) != 0;
     const bool rewrite = (st.flags & SF_REWRITE) != 0;
-    const int nb_sweep = __reduce_max_sync(full, live ? nb : 0);
+    const int nb_sweep = __reduce_max_sync(full, active ? nb : 0);
     if (lane == 0) { w_chunks++; w_sweep += nb_sweep; }
     bool done = false, tobs = false;
-    if (live) {
+    if (active) {
       w_r1v += nb;
       st.r = o.r;
       if (rewrite) {
@@ -2429,43 +2418,12 @@ k_sng_round(int in, const SngDev *sng, const ClusterDev *cl, ProbDev *probs,
         }
       }
     }
-    if (!ITER) {
-      // unfinished singletons: state saved, flagged for the next round's
-      // list (or the bisection list); the compaction keeps the list order
-      if (live && !done) sst[idx] = st;
-      if (live) flag[base + lane] = done ? 0 : (tobs ? 2 : 1);
-    } else {
-      // the bisections the rounds would send to k_sng_bisect, one lane's
-      // singleton at a time by the whole warp (same bits as k_sng_bisect)
-      for (unsigned bm = __ballot_sync(full, tobs); bm; bm &= bm - 1) {
-        const int v = __ffs(bm) - 1;
-        const int nbv = __shfl_sync(full, nb, v), psv = __shfl_sync(full, ps, v);
-        const int wiv = __shfl_sync(full, Windex[s], v);
-        const double pvm = __shfl_sync(full, pivmin, v), spd = __shfl_sync(full, bspd, v);
-        const double2 *Pv = (const double2 *)__shfl_sync(full, (unsigned long long)P, v);
-        const int rv = __shfl_sync(full, st.r, v);
-        double wsh = __shfl_sync(full, st.wsh, v), werr = __shfl_sync(full, st.werr, v);
-        const int maxitr = dv_itmax(spd + pvm, pvm);
-        const int tw = (rv < 1 || rv > nbv) ? nbv : rv;
-        int nc = 0;
-        dv_dlarrb_tree(32, nbv, Pv, psv, wiv, 1, 0, 0.0, 0.0, 0.0, 2.0 * MR3_EPS, pvm, maxitr, tw,
-                       &wsh, &werr, &nc);
-        wsh = __shfl_sync(full, wsh, 0);
-        werr = __shfl_sync(full, werr, 0);
-        if (lane == 0) w_neg += (unsigned long long)nc * nbv;
-        if (lane == v) {
-          st.wsh = wsh;
-          st.werr = werr;
-          st.flags = (st.flags | SF_USEDBS) & ~SF_NEEDBS;
-          st.lambda = st.wsh;
-          st.r = 0;
-        }
-      }
-      if (live && !done) sst[idx] = st;
-    }
+    // unfinished singletons: state saved, flagged for the next round's
+    // list (or the bisection list); the compaction keeps the list order
+    if (active && !done) sst[idx] = st;
+    if (active) flag[base + lane] = done ? 0 : (tobs ? 2 : 1);
     // finished eigenvectors out
     const unsigned fin = __ballot_sync(full, done);
-    live = live && !done;
     if (fin) {
       const ClusterDev &Cf = cl[sng[idx].cl];
       const BlockDev &B = blocks[Cf.blk];
@@ -2504,23 +2462,11 @@ k_sng_round(int in, const SngDev *sng, const ClusterDev *cl, ProbDev *probs,
         column_done(p, B.prob, zind, sc, done_list, tile_left);
       }
     }
-    } while (ITER && __any_sync(full, live));
   }
   stat_add(stats, KID_SNG * 4 + 2, w_r1v);
-  if (ITER) stat_add(stats, KID_SNG * 4 + 1, w_neg);
   // diagnostics: warp-level row sweeps and warp chunks
   stat_add(stats, KID_OTHER * 4 + 0, w_sweep);
   stat_add(stats, KID_OTHER * 4 + 1, w_chunks);
-  if (ITER) {
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      __threadfence();
-      if (atomicAdd(&sc->fin_ctas, 1) == (int)gridDim.x - 1) {
-        sc->nin = 0;
-        sc->mode = 2;
-      }
-    }
-  }
 }
 
 // The bisection of a singleton whose Rayleigh-quotient step left its
@@ -2580,114 +2526,162 @@ k_sng_bisect(int out, const SngDev *sng, const ClusterDev *cl, const ProbDev *pr
   stat_add(stats, KID_SNG * 4 + 1, w_neg);
 }
 
-// The rest of a level's singletons when few are left (SngCounters.mode 1):
-// a warp per singleton (the warps take them in turn) runs its remaining
-// Rayleigh-quotient loop (SRC/process_singleton.c:159-292) to the end in one
-// launch -- each dlar1v on lanes 0 and 1 (SPLIT, the default) or on lane 0
-// with its checkpoints, a bisection by all 32 lanes with the tree
-// bisection -- instead of one call per round with a launch
-// sequence (round, compaction, bisection, sort) between calls.  Every call
-// and every state update is the one the rounds make, so the results are the
-// same bits.  The last block to finish empties the list (mode 2).
-// SPLIT: each dlar1v is dv_r1s_call (the two sweeps on two lanes at once,
-// the twist chosen by the warp, the vector in the warp's row scratch
-// fscratch, 5 (nmax + 2) doubles per warp) instead of lane 0's checkpointed
-// dlar1v; the results are the same bits.
-template <bool SPLIT>
-__global__ void __launch_bounds__(SNG_WARPS * 32, 2)
+// A level's singletons when its list is short (FIN_FIRST: from their first
+// call on), or the rest of them when few are left after some rounds
+// (FIN_LATER, SngCounters.mode 1): a group of L lanes per singleton runs its
+// Rayleigh-quotient loop (SRC/process_singleton.c:159-292) to the end --
+// each dlar1v on the group's lanes 0 and 1 (dv_r1s_call), a bisection by all
+// L lanes with the tree bisection -- instead of one call per round with a
+// launch sequence (round, compaction, bisection, sort) between calls.  Every
+// call and every state update is the one the rounds make, so the results are
+// the same bits; the vector stays in the group's scratch until it is
+// accepted, so the first call needs no rewrite.  The last block to finish
+// empties the list (mode 2).
+//
+// A warp holds G = 32 / L groups in lock-step; a group that finishes its
+// singleton takes the next one of the list.  A sweep's row takes one warp
+// about 110 cycles of latency and 45 of issue, whatever its number of groups,
+// so two warps a quarter SM fill it (one CTA of 8 warps per SM: 8 against 16
+// warps, 4.5 and 5.7 ms for the n = 1000 problem, 343 and 378 for the glued
+// n = 20010 one) and a longer list gets more groups per warp, not more warps.
+//
+// A bisection takes as long as about ten calls.  With several groups a warp
+// the others would wait for each group's, so singletons that need one leave
+// their group for a second list (bsl) and FIN_BISECT serves that: all groups
+// of a warp bisect at the same time, then make the one or two calls left.
+#ifndef FIN_CTAS
+#define FIN_CTAS 1
+#endif
+#ifndef FIN_MAXG
+#define FIN_MAXG 8
+#endif
+#ifndef FIN_LIST
+#define FIN_LIST 16      // singletons per warp up to which a list is taken
+#endif
+enum { FIN_LATER = 0, FIN_FIRST = 1, FIN_BISECT = 2 };
+
+// Groups per warp for a list of n: the fewest that hold it at once; for the
+// bisections those with the fewest turns times steps, the steps growing as
+// 1 / log2(L).
+__device__ __forceinline__ int fin_groups(int n, int nwarps, int maxG, bool bisect) {
+  int G = 1;
+  if (!bisect) {
+    while (G < maxG && (long long)G * nwarps < n) G <<= 1;
+    return G;
+  }
+  float best = 0.f;
+  for (int g = 1, depth = 5; g <= maxG; g <<= 1, depth--) {
+    const int turns = (n + nwarps * g - 1) / (nwarps * g);
+    const float cost = turns / (float)depth;
+    if (g == 1 || cost < best) { best = cost; G = g; }
+  }
+  return G;
+}
+
+template <int KIND>
+__global__ void __launch_bounds__(SNG_WARPS * 32, FIN_CTAS)
 k_sng_finish(int in, const SngDev *sng, const ClusterDev *cl, ProbDev *probs,
              const BlockDev *blocks, const double2 *RP, const double2 *RQ, const double *arena,
              double *W, double *Wsh, double *Werr, double *Wgap, const int *Windex,
-             const int *Zindex, SngState *sst, const int *act0, const int *act1, SngCounters *sc,
-             double *scratch, double *fscratch, long long nmax, int2 *done_list, int *tile_left,
-             unsigned long long *stats) {
-  if (sc->mode != 1) return;
+             const int *Zindex, SngState *sst, const int *act0, const int *act1, int *bsl,
+             SngCounters *sc, double *fscratch, long long nmax, int maxG, int2 *done_list,
+             int *tile_left, unsigned long long *stats) {
+  constexpr bool FIRST = KIND == FIN_FIRST, BISECT = KIND == FIN_BISECT;
+  if (BISECT ? sc->fb_n == 0 : !FIRST && sc->mode != 1) return;
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const long long gw = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-  const long long nck = nmax / CK_K + 1;
-  r1c_ck ck;
-  ck.S = scratch + gw * 3 * nck * 32 + lane;
-  ck.I = ck.S + nck * 32;
-  ck.P = ck.I + nck * 32;
+  const int nwarps = (gridDim.x * blockDim.x) >> 5;
+  const int *Ain = BISECT ? bsl : in ? act1 : act0;
+  const int nin = BISECT ? sc->fb_n : sc->nin;
+  int *next = BISECT ? &sc->fb_next : &sc->act_next[in];
+  const int G = fin_groups(nin, nwarps, maxG, BISECT);
+  const int L = 32 / G, gi = lane / L, t = lane & (L - 1), g0 = lane - t;
+  const unsigned gm = ((L == 32) ? 0xffffffffu : ((1u << L) - 1u)) << g0;
   r1s_buf rb;
   {
-    const long long len = nmax + 2;
-    rb.SI = (SPLIT ? fscratch : scratch) + gw * 5 * len;
+    const long long len = (nmax + 2) * G;
+    rb.SI = fscratch + gw * 5 * (nmax + 2) * maxG + gi;
     rb.LP = rb.SI + len;
     rb.PA = rb.LP + len;
     rb.UM = rb.PA + len;
     rb.ZV = rb.UM + len;
+    rb.st = G;
   }
-  const int *Ain = in ? act1 : act0;
-  const int nin = sc->nin;
   const double rqtol = 2.0 * MR3_EPS;
   unsigned long long w_r1v = 0, w_neg = 0;
+  bool have = false;      // this group holds a singleton
+  int idx = 0, s = 0, nb = 0, ps = 1, wi = 0;
+  double pivmin = 0.0, spd = 0.0;
+  const double2 *P = nullptr, *Q = nullptr;
+  SngState st = {};       // identical in the group's lanes
   for (;;) {
-    int j = 0;
-    if (lane == 0) j = atomicAdd(&sc->act_next[in], 1);
-    j = __shfl_sync(full, j, 0);
-    if (j >= nin) break;
-    const int idx = Ain[j];
-    const SngDev S = sng[idx];
-    const int s = S.slot;
-    const ClusterDev C = cl[S.cl];
-    const BlockDev &B = blocks[C.blk];
-    ProbDev *p = &probs[B.prob];
-    const int nb = B.nbl;
-    const double pivmin = p->pivmin;
-    const double2 *P, *Q;
-    int ps;
-    own_rrr(C, B, RP, RQ, arena, &P, &Q, &ps);
-    double *zcol = p->Z + (size_t)Zindex[s] * p->ldz + (B.ibgn - p->off);
-    const int wi = Windex[s];
-    SngState st = sst[idx];   // identical in every lane
+    // groups without a singleton take the next ones of the list (the
+    // bisecting ones together, when the whole warp is free)
+    const unsigned want = __ballot_sync(full, !have && t == 0);
+    if (want && (!BISECT || __popc(want) == G)) {
+      int base = 0;
+      if (lane == 0) base = atomicAdd(next, __popc(want));
+      base = __shfl_sync(full, base, 0);
+      if (!have) {
+        const int j = base + __popc(want & ((1u << g0) - 1u));
+        if (j < nin) {
+          have = true;
+          idx = FIRST ? j : Ain[j];
+          const SngDev S = sng[idx];
+          s = S.slot;
+          const ClusterDev C = cl[S.cl];
+          const BlockDev &B = blocks[C.blk];
+          nb = B.nbl;
+          pivmin = probs[B.prob].pivmin;
+          spd = C.bl_spdiam;
+          own_rrr(C, B, RP, RQ, arena, &P, &Q, &ps);
+          wi = Windex[s];
+          st = FIRST ? sng_start(s, S, B, Wsh, Werr, Wgap) : sst[idx];
+        }
+      }
+    }
+    if (!__any_sync(full, have)) break;
+    // the bisection a round would have sent this singleton to (a second
+    // step or a rewrite follows the loop's end: no bisection then)
+    const bool needbs = have && (st.flags & SF_NEEDBS) && !(st.flags & (SF_STEP2 | SF_REWRITE));
+    if (!BISECT && G > 1) {
+      if (needbs) {
+        if (t == 0) {
+          sst[idx] = st;
+          bsl[atomicAdd(&sc->fb_n, 1)] = idx;
+        }
+        have = false;
+      }
+    } else if (needbs) {
+      const int maxitr = dv_itmax(spd + pivmin, pivmin);
+      const int tw = (st.r < 1 || st.r > nb) ? nb : st.r;
+      int nc = 0;
+      dv_dlarrb_tree(L, nb, P, ps, wi, 1, 0, 0.0, 0.0, 0.0, 2.0 * MR3_EPS, pivmin, maxitr, tw,
+                     &st.wsh, &st.werr, &nc);
+      st.flags = (st.flags | SF_USEDBS) & ~SF_NEEDBS;
+      st.lambda = st.wsh;
+      st.r = 0;
+      if (t == 0) w_neg += (unsigned long long)nc * nb;
+    }
+    __syncwarp();
+    if (!BISECT && !__any_sync(full, have)) continue;   // all sent to the second list
+    const bool usedBS = (st.flags & SF_USEDBS) != 0;
+    int negc = 0;
     dlar1v_out o;
-    for (;;) {
-      // the bisection a round would have sent this singleton to (a second
-      // step or a rewrite follows the loop's end: no bisection then)
-      if ((st.flags & SF_NEEDBS) && !(st.flags & (SF_STEP2 | SF_REWRITE))) {
-        const int maxitr = dv_itmax(C.bl_spdiam + pivmin, pivmin);
-        const int tw = (st.r < 1 || st.r > nb) ? nb : st.r;
-        int nc = 0;
-        dv_dlarrb_tree(32, nb, P, ps, wi, 1, 0, 0.0, 0.0, 0.0, 2.0 * MR3_EPS, pivmin, maxitr, tw,
-                       &st.wsh, &st.werr, &nc);
-        st.flags = (st.flags | SF_USEDBS) & ~SF_NEEDBS;
-        st.lambda = st.wsh;
-        st.r = 0;
-        if (lane == 0) w_neg += (unsigned long long)nc * nb;
-      }
-      const bool usedBS = (st.flags & SF_USEDBS) != 0;
-      const double lam_call = (st.flags & SF_STEP2) ? st.bstw : st.lambda;
-      const int r_in = (st.flags & SF_REWRITE) ? 0 : st.r;
-      const bool write = (st.flags & (SF_REWRITE | SF_STEP2 | SF_USEDBS)) || st.k > 1;
-      int negc = 0;
-      o.isupp1 = 1; o.isupp2 = nb; o.nrminv = 0.0; o.r = 0; o.resid = 0.0; o.rqcorr = 0.0;
-      if (SPLIT) {
-        dv_r1s_call(nb, lam_call, P, Q, ps, pivmin, !usedBS, r_in, st.gaptol, rb, &negc, &o);
-      } else {
-        r1c_state rs;
-        rs.r = 0; rs.mingma = 0.0; rs.sawnan = false; rs.slowA = false; rs.slowB = false;
-        dv_r1c_factor(lane == 0, nb, lam_call, P, Q, ps, pivmin, !usedBS, r_in, ck, &negc, &rs);
-        if (lane == 0)
-          dv_r1c_solve(nb, lam_call, P, Q, ps, pivmin, st.gaptol, rs.r, rs.sawnan, rs.slowA,
-                       rs.slowB, ck.S, ck.P, rs.mingma, write ? zcol : nullptr, 1.0, &o);
-      }
-      o.r = __shfl_sync(full, o.r, 0);
-      o.isupp1 = __shfl_sync(full, o.isupp1, 0);
-      o.isupp2 = __shfl_sync(full, o.isupp2, 0);
-      o.nrminv = __shfl_sync(full, o.nrminv, 0);
-      o.resid = __shfl_sync(full, o.resid, 0);
-      o.rqcorr = __shfl_sync(full, o.rqcorr, 0);
-      negc = __shfl_sync(full, negc, 0);
-      if (lane == 0) w_r1v += nb;
-      // the state update of k_sng_round, in every lane
-      bool done = false;
-      const bool step2 = (st.flags & SF_STEP2) != 0;
+    o.isupp1 = 1; o.isupp2 = nb; o.nrminv = 0.0; o.r = 0; o.resid = 0.0; o.rqcorr = 0.0;
+    // a rewrite repeats the accepted first call (twist searched, r = 0)
+    dv_r1s_call(have, L, nb, (st.flags & SF_STEP2) ? st.bstw : st.lambda, P, Q, ps, pivmin, !usedBS,
+                (st.flags & SF_REWRITE) ? 0 : st.r, st.gaptol, rb, &negc, &o);
+    __syncwarp();
+    // the state update of k_sng_round, in every lane
+    bool done = false;
+    if (have) {
+      if (t == 0) w_r1v += nb;
       st.r = o.r;
       if (st.flags & SF_REWRITE) {
         done = true;
-      } else if (step2) {
+      } else if (st.flags & SF_STEP2) {
         st.lambda = st.bstw;
         done = true;
       } else {
@@ -2714,42 +2708,45 @@ k_sng_finish(int in, const SngDev *sng, const ClusterDev *cl, ProbDev *probs,
         if (!more) {
           if ((st.flags & SF_USEDRQ) && (st.flags & SF_USEDBS) && st.bstres <= st.resid)
             st.flags |= SF_STEP2;
-          else if (write)
-            done = true;
           else
-            st.flags |= SF_REWRITE;
+            done = true;
         }
       }
-      if (done) break;
     }
-    // outputs and the finished column (support scaled, the rest zero)
-    const int bl0 = B.ibgn - p->off;
-    const int zind = Zindex[s];
-    if (lane == 0) {
-      Wsh[s] = st.lambda;
-      Werr[s] = st.werr;
-      Wgap[s] = st.gap;
-      W[s] = st.lambda + C.sigma;
-      p->Zsupp[2 * (size_t)zind] = o.isupp1 + bl0;
-      p->Zsupp[2 * (size_t)zind + 1] = o.isupp2 + bl0;
+    if (done) {
+      // outputs and the finished column (support scaled, the rest zero)
+      const ClusterDev &C = cl[sng[idx].cl];
+      const BlockDev &B = blocks[C.blk];
+      ProbDev *p = &probs[B.prob];
+      const int bl0 = B.ibgn - p->off;
+      const int zind = Zindex[s];
+      if (t == 0) {
+        Wsh[s] = st.lambda;
+        Werr[s] = st.werr;
+        Wgap[s] = st.gap;
+        W[s] = st.lambda + C.sigma;
+        p->Zsupp[2 * (size_t)zind] = o.isupp1 + bl0;
+        p->Zsupp[2 * (size_t)zind + 1] = o.isupp2 + bl0;
+      }
+      const int a = bl0 + o.isupp1 - 1, b = bl0 + o.isupp2;
+      double *Zc = p->Z + (size_t)zind * p->ldz;
+      for (int row = t; row < a; row += L) Zc[row] = 0.0;
+#pragma unroll 4
+      for (int row = a + t; row < b; row += L)
+        Zc[row] = rb.ZV[(row - bl0 + 1) * (long long)G] * o.nrminv;
+      for (int row = b + t; row < p->n; row += L) Zc[row] = 0.0;
+      __syncwarp(gm);
+      if (t == 0) {
+        __threadfence();
+        column_done(p, B.prob, zind, sc, done_list, tile_left);
+      }
+      have = false;
     }
-    const int a = bl0 + o.isupp1 - 1, b = bl0 + o.isupp2;
-    double *Zc = p->Z + (size_t)zind * p->ldz;
     __syncwarp();
-    for (int row = lane; row < a; row += 32) Zc[row] = 0.0;
-    if (SPLIT)   // the vector is in the warp's scratch (rows of the block, 1-based)
-      for (int row = a + lane; row < b; row += 32) Zc[row] = rb.ZV[row - bl0 + 1] * o.nrminv;
-    else
-      for (int row = a + lane; row < b; row += 32) Zc[row] = Zc[row] * o.nrminv;
-    for (int row = b + lane; row < p->n; row += 32) Zc[row] = 0.0;
-    __syncwarp();
-    if (lane == 0) {
-      __threadfence();
-      column_done(p, B.prob, zind, sc, done_list, tile_left);
-    }
   }
   stat_add(stats, KID_SNG * 4 + 2, w_r1v);
   stat_add(stats, KID_SNG * 4 + 1, w_neg);
+  if (BISECT) return;
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
@@ -3111,8 +3108,6 @@ extern "C" int mr3_cuda_ctx_create_prio(int device, int high, mr3_cuda_ctx **out
   }
   int nb = 0;
   if (cudaFuncSetAttribute(k_sng_round<SNG_LATER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           SNG_TILE_BYTES) != cudaSuccess ||
-      cudaFuncSetAttribute(k_sng_round<SNG_ITER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            SNG_TILE_BYTES) != cudaSuccess ||
       cudaFuncSetAttribute(k_sng_round<SNG_FIRST>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            SNG_TILE_BYTES) != cudaSuccess) {
@@ -3642,10 +3637,6 @@ extern "C" int mr3_cuda_solve_cb(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void
     const size_t resident = (size_t)c->nsm * (size_t)c->sng_ctas_per_sm * SNG_WARPS;
     size_t nwarps = std::min<size_t>(resident, std::max<size_t>(c->nsm, budget / (per_warp * 8)));
     nwarps = (nwarps + SNG_WARPS - 1) / SNG_WARPS * SNG_WARPS;
-    if (nwarps * per_warp > c->capScratch) {
-      CK(regrow(&c->scratch, nwarps * per_warp), "scratch");
-      c->capScratch = nwarps * per_warp;
-    }
     int ncl = c->h_lc[0].n_cl;
     const int DEPTH_CAP = 512;
     ClsScratch xs;
@@ -3733,43 +3724,30 @@ extern "C" int mr3_cuda_solve_cb(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void
         const size_t smem = SNG_TILE_BYTES;
         const int bis_ctas = c->nsm * 4;
         const int nblk = (nsng + LIST_T - 1) / LIST_T;
-        // a list of at most this many singletons (four per persistent warp)
-        // is finished in one launch (k_sng_finish), a warp each in turn;
-        // MR3_FINISH_MAX overrides it (0: never).  A level's last few
-        // thousand singletons are mostly ones that run all MAXITER calls and
-        // the bisection; one round per call for them cost more than their
-        // warps running the calls back to back (4096-problem batch: 44 ms
-        // less per step with four per warp than with one)
-        int finish_max = (int)std::min<size_t>(4 * nwarps, 1u << 30);
+        // k_sng_finish: fw warps of up to maxG groups each, their row scratch
+        // (5 (nmax + 2) doubles a group) within 2 GB (one group a warp at least)
+        const size_t per = 5ull * ((size_t)nmaxV + 2) * sizeof(double);
+        const size_t fw = (size_t)c->nsm * FIN_CTAS * SNG_WARPS;
+        int maxG = FIN_MAXG;
+        while (maxG > 1 && (fw * maxG * per > ((size_t)2 << 30) || fw * (maxG / 2) >= (size_t)nsng))
+          maxG >>= 1;
+        const int fin_ctas = (int)(fw / SNG_WARPS);
+        if (fw * maxG * per > c->capFscratch) {
+          CK(cudaStreamSynchronize(c->own), "fscratch sync");
+          CK(cudaStreamSynchronize(c->rnd), "fscratch sync");
+          CK(regrow(&c->fscratch, fw * maxG * per / sizeof(double)), "fscratch");
+          c->capFscratch = fw * maxG * per;
+        }
+        // a list of at most this many singletons is finished in one launch
+        // (k_sng_finish), from the level's start or after some rounds;
+        // MR3_FINISH_MAX overrides it (0: never)
+        int finish_max = (int)std::min<size_t>(FIN_LIST * fw, 1u << 30);
         if (const char *ev = getenv("MR3_FINISH_MAX")) finish_max = atoi(ev);
-        // MR3_ITER_MAX: a list of at most this many is finished in one launch,
-        // a lane each (k_sng_round<SNG_ITER>).  Off by default: a warp then
-        // waits for its slowest lane and runs its lanes' bisections one after
-        // another, and the step took longer than with the rounds (1049 ms
-        // against 1009 ms on the 4096-problem batch, 279 ms against 178 ms on
-        // a 256-problem one).
-        int iter_max = 0;
-        if (const char *ev = getenv("MR3_ITER_MAX")) iter_max = atoi(ev);
-        // the split form of the finish (two sweeps at once, about half the
-        // latency of a call); MR3_FINISH_SPLIT=0 gives lane 0's checkpointed
-        // form
-        bool split = true;
-        if (const char *ev = getenv("MR3_FINISH_SPLIT")) split = atoi(ev) != 0;
-        int fin_ctas = ctas_all;
-        if (split) {
-          // warps of the split finish: their row scratch (5 (nmax + 2) doubles
-          // each) kept within 2 GB, at least one CTA per SM
-          const size_t per = 5ull * ((size_t)nmaxV + 2) * sizeof(double);
-          size_t fw = std::min<size_t>(nwarps, std::max<size_t>((size_t)c->nsm * SNG_WARPS,
-                                                                ((size_t)2 << 30) / per));
-          fw = fw / SNG_WARPS * SNG_WARPS;
-          fin_ctas = (int)(fw / SNG_WARPS);
-          if (fw * per > c->capFscratch) {
-            CK(cudaStreamSynchronize(c->own), "fscratch sync");
-            CK(cudaStreamSynchronize(c->rnd), "fscratch sync");
-            CK(regrow(&c->fscratch, fw * per / sizeof(double)), "fscratch");
-            c->capFscratch = fw * per;
-          }
+        const bool direct = nsng <= finish_max;
+        if (!direct && nwarps * per_warp > c->capScratch) {
+          CK(cudaStreamSynchronize(st), "scratch sync");
+          CK(regrow(&c->scratch, nwarps * per_warp), "scratch");
+          c->capScratch = nwarps * per_warp;
         }
         const bool trace_rounds = getenv("MR3_TRACE_ROUNDS") != nullptr;
         auto trace_t0 = std::chrono::steady_clock::now();
@@ -3778,29 +3756,28 @@ extern "C" int mr3_cuda_solve_cb(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void
         for (int rd = 0; rd < SNG_ROUNDS; rd++) {
           const int in = rd & 1, last = rd == SNG_ROUNDS - 1;
           LAUNCH(k_round_reset, 1, 1, c->sc, in, rd == 0);
-          if (rd > 0 && split)
-            LAUNCH(k_sng_finish<true>, fin_ctas, SNG_WARPS * 32, in, c->sng, c->cl[cur],
-                   c->probs, c->blocks, c->RP, c->RQ, c->arena[cur], c->W, c->Wsh, c->Werr,
-                   c->Wgap, c->Windex, c->Zindex, c->sst, c->act[0], c->act[1], c->sc,
-                   c->scratch, c->fscratch, (long long)nmaxV, c->done_list, c->tile_left, stats);
+          if (direct)
+            LAUNCH(k_sng_finish<FIN_FIRST>, fin_ctas, SNG_WARPS * 32, in, c->sng, c->cl[cur], c->probs,
+                   c->blocks, c->RP, c->RQ, c->arena[cur], c->W, c->Wsh, c->Werr, c->Wgap,
+                   c->Windex, c->Zindex, c->sst, c->act[0], c->act[1], c->bsl, c->sc, c->fscratch,
+                   (long long)nmaxV, maxG, c->done_list, c->tile_left, stats);
           else if (rd > 0)
-            LAUNCH(k_sng_finish<false>, ctas_all, SNG_WARPS * 32, in, c->sng, c->cl[cur],
-                   c->probs, c->blocks, c->RP, c->RQ, c->arena[cur], c->W, c->Wsh, c->Werr,
-                   c->Wgap, c->Windex, c->Zindex, c->sst, c->act[0], c->act[1], c->sc,
-                   c->scratch, nullptr, (long long)nmaxV, c->done_list, c->tile_left, stats);
-          if (rd > 0)
-            LAUNCH_SMEM(k_sng_round<SNG_ITER>, ctas_all, SNG_WARPS * 32, smem, in, c->sng,
-                        c->cl[cur], c->probs, c->blocks, c->RP, c->RQ, c->arena[cur], c->W, c->Wsh,
-                        c->Werr, c->Wgap, c->Windex, c->Zindex, c->sst, c->act[0], c->act[1],
-                        c->sflag, c->sc, c->scratch, (long long)nmaxV, c->done_list, c->tile_left,
-                        stats);
-          if (rd == 0)
+            LAUNCH(k_sng_finish<FIN_LATER>, fin_ctas, SNG_WARPS * 32, in, c->sng, c->cl[cur], c->probs,
+                   c->blocks, c->RP, c->RQ, c->arena[cur], c->W, c->Wsh, c->Werr, c->Wgap,
+                   c->Windex, c->Zindex, c->sst, c->act[0], c->act[1], c->bsl, c->sc, c->fscratch,
+                   (long long)nmaxV, maxG, c->done_list, c->tile_left, stats);
+          if (maxG > 1 && (direct || rd > 0))
+            LAUNCH(k_sng_finish<FIN_BISECT>, fin_ctas, SNG_WARPS * 32, in, c->sng, c->cl[cur], c->probs,
+                   c->blocks, c->RP, c->RQ, c->arena[cur], c->W, c->Wsh, c->Werr, c->Wgap,
+                   c->Windex, c->Zindex, c->sst, c->act[0], c->act[1], c->bsl, c->sc, c->fscratch,
+                   (long long)nmaxV, maxG, c->done_list, c->tile_left, stats);
+          if (!direct && rd == 0)
             LAUNCH_SMEM(k_sng_round<SNG_FIRST>, ctas_first, SNG_WARPS * 32, smem, in, c->sng,
                         c->cl[cur], c->probs, c->blocks, c->RP, c->RQ, c->arena[cur], c->W, c->Wsh,
                         c->Werr, c->Wgap, c->Windex, c->Zindex, c->sst, c->act[0], c->act[1],
                         c->sflag, c->sc, c->scratch, (long long)nmaxV, c->done_list, c->tile_left,
                         stats);
-          else
+          else if (!direct)
             LAUNCH_SMEM(k_sng_round<SNG_LATER>, ctas_all, SNG_WARPS * 32, smem, in, c->sng,
                         c->cl[cur], c->probs, c->blocks, c->RP, c->RQ, c->arena[cur], c->W, c->Wsh,
                         c->Werr, c->Wgap, c->Windex, c->Zindex, c->sst, c->act[0], c->act[1],
@@ -3812,8 +3789,9 @@ extern "C" int mr3_cuda_solve_cb(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void
             CK(cudaEventRecord(c->rev[npend], st), "round record");
             npend++;
           }
+          if (direct) break;
           LAUNCH(k_list_count, nblk, 256, c->sc, c->sflag, c->sbcnt);
-          LAUNCH(k_list_scan, 1, 1024, nblk, c->sc, c->sbcnt, in ^ 1, last, finish_max, iter_max);
+          LAUNCH(k_list_scan, 1, 1024, nblk, c->sc, c->sbcnt, in ^ 1, last, finish_max);
           if (trace_rounds) {
             // MR3_TRACE_ROUNDS=1: each round's list lengths and wall time on
             // stderr (synchronises after every round; diagnostics only)

@@ -38,3 +38,19 @@ def test_sizes_around_the_chunks(kind, lanes, monkeypatch):
             assert_same(g, o, f"{kind} n={n} {rng} lanes={lanes}")
         g, o = M.mrrr("N", "A", D, E), oracle.mrrr("N", "A", D, E)
         assert_same(g, o, f"{kind} n={n} N lanes={lanes}")
+
+
+@pytest.mark.parametrize("finish_max", [None, "0", "700"])
+def test_several_singletons_per_warp(finish_max, monkeypatch):
+    """A list longer than the finish's warps (several groups of lanes per warp,
+    bisections on the second list), finished from the level's start, in rounds
+    only, and after some rounds."""
+    if finish_max is not None:
+        monkeypatch.setenv("MR3_FINISH_MAX", finish_max)
+    probs = [dict(jobz="V", range="A", D=D, E=E)
+             for D, E, _ in wl.mixed_batch(24, seed=77, nmin=5, nmax=500)]
+    for n in (201, 335):
+        D, E = wl.glued_wilkinson(5, n // 5 | 1, 1e-9)
+        probs.append(dict(jobz="V", range="A", D=D, E=E))
+    for k, (p, r) in enumerate(zip(probs, M.mrrr_batched(probs))):
+        assert_same(r, oracle.mrrr("V", "A", p["D"], p["E"]), f"batch[{k}] {finish_max}")
