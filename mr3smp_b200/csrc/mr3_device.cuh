@@ -234,6 +234,75 @@ static __device__ __noinline__ int dv_count_bisect_lat(int n, const double2 *__r
   return cnt;
 }
 
+// ------------------------------------------------------------------------
+// Guessed bisections.  The bisection of eigenvalue j follows the counts
+// N(c) at its midpoints only through N(c) >= j, and N, the count of
+// dv_count_bisect with its rounding errors, does not decrease with c: by
+// induction over the rows the pair (count so far, pivot) of a larger c is
+// never behind that of a smaller one in the order "count, then negative
+// before positive pivots, then decreasing pivot", since subtraction, the
+// quotient of a nonnegative e^2, rounding and the clamp at pivmin are all
+// monotone (Kahan; Demmel, Dhillon, Ren 1995).  So if the bisection is run
+// with any other counts and ends in [a, b], two counts at its ends,
+// N(a) < j <= N(b), show that N would have taken every turn the same way:
+// all midpoints on the way are <= a or >= b.  The interval, and with it the
+// result, is then the sequential one bit for bit; otherwise the bisection is
+// run again with N itself.
+//
+// dv_count_guess is that other count: quotients from the reciprocal seed and
+// a cubic step, e^2 y0 (1 + e + e^2), in 6 FP64 operations and 48 cycles a
+// row instead of 13 and 193 (plain) or 90 (checked).  Their error, some units
+// in the last place, moves an eigenvalue by about 2^-51 ||T||, and the final
+// interval is 2^-27 |lambda| or wider, so only eigenvalues below 1e-6 ||T|| are
+// ever repeated.  (A Newton step alone, 4 operations and 2^-40, had one
+// eigenvalue in most warps repeated: host_batch's k_bisect_cont took 12.3 ms,
+// with exact counts alone 6.8.)  A chunk that meets a zero, subnormal or
+// overflowing pivot is repeated with plain divisions.
+// ------------------------------------------------------------------------
+static __device__ __noinline__ int dv_count_guess(int n, const double2 *__restrict__ tp,
+                                                  double pivmin, double c) {
+  constexpr int U = QDIV_U;
+  double t = tp[0].x - c;
+  int cnt = 0;
+  if (t <= pivmin) { cnt = 1; t = fmin(t, -pivmin); }
+  int j = 1;
+  if (n > U) {
+    double2 v[U], nx[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) v[u] = tp[1 + u];
+    for (; j + U <= n; j += U) {
+#pragma unroll
+      for (int u = 0; u < U; u++) nx[u] = tp[d_imin(j + U + u, n - 1)];
+      const double t0 = t;
+      const int cnt0 = cnt;
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const double y0 = dv_rcp_seed(t), e = __fma_rn(-t, y0, 1.0), qh = v[u].y * y0;
+        t = __fma_rn(-qh, __fma_rn(e, e, e), (v[u].x - c) - qh);
+        cnt += dv_signbit(t);
+      }
+      if (dv_habs(t) >= (0x7fe00000u << 1)) {   // infinite, NaN or about to be
+        t = t0;
+        cnt = cnt0;
+#pragma unroll 1
+        for (int u = 0; u < U; u++) {
+          const double2 w = tp[j + u];
+          t = w.x - w.y / t - c;
+          if (t <= pivmin) { cnt++; t = fmin(t, -pivmin); }
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++) v[u] = nx[u];
+    }
+  }
+  for (; j < n; j++) {
+    const double2 w = tp[j];
+    t = w.x - w.y / t - c;
+    if (t <= pivmin) { cnt++; t = fmin(t, -pivmin); }
+  }
+  return cnt;
+}
+
 // One interval of dlaebz IJOB=3 from the user-supplied point c, by a group of
 // L lanes (L = 2..32, a power of two; every lane of the group passes the same
 // arguments and gets the same results).  The first count is at the given
@@ -293,14 +362,16 @@ static __device__ __noinline__ void dv_ijob3_tree(int L, int n, const double2 *_
 
 // The interval of eigenvalue j under dlaebz IJOB=2 started from [a,b] with
 // counts (na,nb): midpoint bisection of that one interval (odebz.f 90-120).
-// it0 > 0 continues a bisection whose first it0 steps ended in [a,b].
+// it0 > 0 continues a bisection whose first it0 steps ended in [a,b].  GUESS:
+// with dv_count_guess, to be confirmed by the counts at the ends.
+template <bool GUESS>
 static __device__ __noinline__ int dv_bisect_one(int n, const double2 *__restrict__ tp, double pivmin,
                                           double abstol, double reltol, int itmax, int j,
                                           double *a, double *b, int na, int nb, int *iters,
                                           int it0 = 0) {
   double c = 0.5 * (*a + *b);
   for (int it = it0 + 1; it <= itmax; it++) {
-    int cnt = dv_count_bisect(n, tp, pivmin, c);
+    int cnt = GUESS ? dv_count_guess(n, tp, pivmin, c) : dv_count_bisect(n, tp, pivmin, c);
     cnt = d_imin(nb, d_imax(na, cnt));
     if (j <= cnt) { *b = c; nb = cnt; } else { *a = c; na = cnt; }
     double w = fabs(*b - *a);
@@ -318,42 +389,58 @@ static __device__ __noinline__ int dv_bisect_one(int n, const double2 *__restric
 // interval computed along the node's path with the loop's operations), then
 // the group walks the tree, clamping each count to the walk's (na, nb) and
 // applying the loop's convergence test after each step, as the sequential
-// loop does.  The same sequence of intervals; log2(L) steps per count.
-static __device__ __noinline__ int dv_bisect_tree(int L, int n, const double2 *__restrict__ tp,
-                                           double pivmin, double abstol, double reltol, int itmax,
-                                           int j, double *a_, double *b_, int na, int nb,
-                                           int *iters) {
+// loop does.  The same sequence of intervals; log2(L) steps per count.  The
+// counts are guessed; lanes 0 and 1 then confirm the two ends, and the walk
+// is repeated with exact counts if one fails.
+static __device__ __noinline__ void dv_bisect_tree(int L, int n, const double2 *__restrict__ tp,
+                                            double pivmin, double abstol, double reltol, int itmax,
+                                            int j, double *a_, double *b_, const int na0,
+                                            const int nb0, int *iters) {
   const int lane = threadIdx.x & 31;
   const int t = lane & (L - 1), g0 = lane - t, depth = 31 - __clz(L);
   const unsigned gm = ((L == 32) ? 0xffffffffu : ((1u << L) - 1u)) << g0;
   const int node_t = t == 0 ? 1 : t;
-  double a = *a_, b = *b_;
-  int it = 0, done = itmax < 1, conv = 0;
-  while (!done) {
-    double l = a, r = b;
-    for (int k = 30 - __clz(node_t); k >= 0; k--) {
-      const double m = 0.5 * (l + r);
-      if ((node_t >> k) & 1) l = m; else r = m;
-    }
-    const int raw = dv_count_bisect_lat(n, tp, pivmin, 0.5 * (l + r));
-    int node = 1;
-    for (int d = 0; d < depth; d++) {
-      const int cv = __shfl_sync(gm, raw, g0 + node);
-      if (!done) {
-        const double c = 0.5 * (a + b);
-        const int cnt = d_imin(nb, d_imax(na, cv));
-        if (j <= cnt) { b = c; nb = cnt; node = 2 * node; } else { a = c; na = cnt; node = 2 * node + 1; }
-        it++;
-        const double w = fabs(b - a), tt = fmax(fabs(b), fabs(a));
-        if (w < fmax(fmax(abstol, pivmin), reltol * tt) || na >= nb) { done = 1; conv = 1; }
-        else if (it >= itmax) done = 1;
+  const double a0 = *a_, b0 = *b_;
+  double a = a0, b = b0;
+  int it = 0;
+#pragma unroll 1
+  for (int pass = 0; pass < 2; pass++) {
+    int na = na0, nb = nb0;
+    bool done = itmax < 1;
+    a = a0;
+    b = b0;
+    it = 0;
+    while (!done) {
+      double l = a, r = b;
+      for (int k = 30 - __clz(node_t); k >= 0; k--) {
+        const double m = 0.5 * (l + r);
+        if ((node_t >> k) & 1) l = m; else r = m;
+      }
+      const double x = 0.5 * (l + r);
+      const int raw = pass == 0 ? dv_count_guess(n, tp, pivmin, x)
+                                : dv_count_bisect_lat(n, tp, pivmin, x);
+      int node = 1;
+      for (int d = 0; d < depth; d++) {
+        const int cv = __shfl_sync(gm, raw, g0 + node);
+        if (!done) {
+          const double c = 0.5 * (a + b);
+          const int cnt = d_imin(nb, d_imax(na, cv));
+          if (j <= cnt) { b = c; nb = cnt; node = 2 * node; } else { a = c; na = cnt; node = 2 * node + 1; }
+          it++;
+          const double w = fabs(b - a), tt = fmax(fabs(b), fabs(a));
+          if (w < fmax(fmax(abstol, pivmin), reltol * tt) || na >= nb || it >= itmax) done = true;
+        }
       }
     }
+    if (pass == 1) { it += 2; break; }
+    const int cv = t < 2 ? dv_count_bisect_lat(n, tp, pivmin, t == 0 ? a : b) : 0;
+    const int ca = __shfl_sync(gm, cv, g0), cb = __shfl_sync(gm, cv, g0 + 1);
+    it = 2;
+    if (ca < j && cb >= j) break;
   }
   *a_ = a;
   *b_ = b;
-  *iters = it;
-  return conv;
+  *iters = it;   // exact counts
 }
 
 // dlaneg (SRC/LAPACK/odneg.f:98-163) on packed rows P[(i)*ps]; r is 1-based.

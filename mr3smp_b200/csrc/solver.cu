@@ -204,7 +204,7 @@ __device__ int cta_exscan(int v, int *sh, int *total) {
 __device__ __forceinline__ void set_status(ProbDev *p, int s) { atomicMax(&p->status, s); }
 
 // Device work counters for the roofline: stats[kernel * 4 + kind], kinds
-// 0 = Sturm-count steps on T, 1 = Sturm-count steps on L D L^T (dlaneg),
+// 0 = Sturm-count steps on T (the exact ones), 1 = Sturm-count steps on L D L^T (dlaneg),
 // 2 = twisted-factorisation rows (dlar1v), 3 = dlarrf rows.  Every lane of a
 // warp must call stat_add (it reduces over the full warp).
 enum { KID_BISECT = 0, KID_REFROOT, KID_NEWRRR, KID_REFCL, KID_SNG, KID_OTHER, KID_COUNT };
@@ -574,41 +574,18 @@ k_blocks(ProbDev *probs, BlockDev *blocks, const double *D, double *E, const dou
 
 // ------------------------------------------------------------------------
 // Stage A2: initial approximations by bisection, one thread per eigenvalue
-// (dlarrd/dlaebz IJOB=2, SRC/LAPACK/odrrd.f:450-520).  Thread k of a block
-// bisects eigenvalue nab1+1+k; a block never has more than nbl of them.
+// (dlarrd/dlaebz IJOB=2, SRC/LAPACK/odrrd.f:450-520).  Slot k of a block
+// bisects eigenvalue nab1+1+k; a block never has more than nbl of them.  The
+// counts on the way are guessed and the final interval is confirmed by exact
+// counts at its ends (see dv_count_guess).
 // ------------------------------------------------------------------------
-__device__ __forceinline__ unsigned long long bisect_body(int g, const ProbDev *probs,
-                                                          const BlockDev *blocks,
-                                                          const int *blk_of_row, const double2 *TP,
-                                                          double *Wt, double *Et, int *It, Tol tol) {
-  const BlockDev *B = &blocks[blk_of_row[g]];
-  const ProbDev *p = &probs[B->prob];
-  if (p->trivial || p->jobz == MR3_JOB_C || p->status) return 0;
-  int k = g - B->ibgn;
-  if (B->nbl < 2 || B->mbl <= 0 || B->none || k >= B->nab2 - B->nab1) return 0;
-  int j = B->nab1 + 1 + k;
-  double a = B->gl3, b = B->gu3;
-  int it = 0;
-  dv_bisect_one(B->nbl, TP + B->ibgn, p->pivmin, B->atoli, tol.bsrtol, B->itmax2, j, &a, &b,
-                B->nab1, B->nab2, &it);
-  Wt[g] = 0.5 * (a + b);
-  Et[g] = 0.5 * fabs(a - b);
-  It[g] = j;
-  return (unsigned long long)it * (unsigned long long)B->nbl;
-}
-
-// TREE = false: a thread per eigenvalue (L = 1).  The two forms are separate
-// instantiations so that the thread form keeps its own register budget.
-template <bool TREE>
+// L lanes per eigenvalue (few eigenvalues: single large problems).
 __global__ void __launch_bounds__(128)
 k_bisect(int N, int L, const ProbDev *probs, const BlockDev *blocks, const int *blk_of_row,
          const double2 *TP, double *Wt, double *Et, int *It, Tol tol, unsigned long long *stats) {
   const long long gt = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   unsigned long long work = 0;
-  if (!TREE) {
-    if (gt < N) work = bisect_body((int)gt, probs, blocks, blk_of_row, TP, Wt, Et, It, tol);
-  } else if (gt / L < N) {
-    // L lanes per eigenvalue (few eigenvalues: single large problems)
+  if (gt / L < N) {
     const int g = (int)(gt / L);
     const BlockDev *B = &blocks[blk_of_row[g]];
     const ProbDev *p = &probs[B->prob];
@@ -641,17 +618,20 @@ k_bisect(int N, int L, const ProbDev *probs, const BlockDev *blocks, const int *
 // node's eigenvalues continue in its children.  A child holding one
 // eigenvalue leaves the tree with its state (k_bisect_cont continues it, a
 // thread per eigenvalue); a converged child, or one at the iteration
-// limit, writes its eigenvalues' results.  Every eigenvalue sees the
-// operations of dv_bisect_one in the same order, so the results are those
-// of the thread form bit for bit, and the first levels, which all of a
-// block's eigenvalues share, are counted once per node.
+// limit, leaves it with its eigenvalues' final interval.  Every eigenvalue
+// sees the operations of dv_bisect_one in the same order, and the first
+// levels, which all of a block's eigenvalues share, are counted once per
+// node.  All these counts are guessed (dv_count_guess); k_bisect_cont
+// confirms each eigenvalue's final interval by exact counts at its two ends
+// and repeats the bisection with exact counts where they disagree, so the
+// results are those of the exact sequential bisection bit for bit.
 // ------------------------------------------------------------------------
 struct BisNode {
   double a, b;
   int na, nb, it, blk;   // counts at a and b, steps done, block
 };
 struct BisState {
-  int na, nb, it, pad;   // a single eigenvalue's state (a, b in Wt, Et); it < 0: none
+  int na, nb, it, done;  // a single eigenvalue's state (a, b in Wt, Et); it < 0: none
 };
 #define BIS_DEPTH 16     // tree levels before the remaining nodes are split up
 
@@ -660,23 +640,17 @@ __device__ __forceinline__ bool bis_block_ok(const BlockDev *B, const ProbDev *p
          !(B->nbl < 2 || B->mbl <= 0 || B->none) && B->nab2 > B->nab1;
 }
 
-// Eigenvalues na+1..nb of an interval: results (done) or single states.
+// Eigenvalues na+1..nb of an interval as single states (done: final).
 __device__ __forceinline__ void bis_finish(const BlockDev *B, double a, double b, int na, int nb,
-                                           int it, bool done, double *Wt, double *Et, int *It,
+                                           int it, bool done, double *Wt, double *Et,
                                            BisState *st) {
   for (int j = na + 1; j <= nb; j++) {
     const int g = B->ibgn + (j - B->nab1 - 1);
-    if (done) {
-      Wt[g] = 0.5 * (a + b);
-      Et[g] = 0.5 * fabs(a - b);
-      It[g] = j;
-    } else {
-      Wt[g] = a;
-      Et[g] = b;
-      BisState q;
-      q.na = na; q.nb = nb; q.it = it; q.pad = 0;
-      st[g] = q;
-    }
+    Wt[g] = a;
+    Et[g] = b;
+    BisState q;
+    q.na = na; q.nb = nb; q.it = it; q.done = done;
+    st[g] = q;
   }
 }
 
@@ -699,7 +673,7 @@ __device__ __forceinline__ int bis_child(const BisNode &nd, int cnt, int side, d
 
 __global__ void __launch_bounds__(256)
 k_bis_roots(int N, const ProbDev *probs, const BlockDev *blocks, const int *blk_of_row,
-            BisNode *out, int *n_out, double *Wt, double *Et, int *It, BisState *st) {
+            BisNode *out, int *n_out, double *Wt, double *Et, BisState *st) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= N) return;
   const int bk = blk_of_row[g];
@@ -708,9 +682,9 @@ k_bis_roots(int N, const ProbDev *probs, const BlockDev *blocks, const int *blk_
   const ProbDev *p = &probs[B->prob];
   if (!bis_block_ok(B, p)) return;
   if (B->itmax2 <= 0) {
-    bis_finish(B, B->gl3, B->gu3, B->nab1, B->nab2, 0, true, Wt, Et, It, st);
+    bis_finish(B, B->gl3, B->gu3, B->nab1, B->nab2, 0, true, Wt, Et, st);
   } else if (B->nab2 - B->nab1 == 1) {
-    bis_finish(B, B->gl3, B->gu3, B->nab1, B->nab2, 0, false, Wt, Et, It, st);
+    bis_finish(B, B->gl3, B->gu3, B->nab1, B->nab2, 0, false, Wt, Et, st);
   } else {
     BisNode nd;
     nd.a = B->gl3; nd.b = B->gu3; nd.na = B->nab1; nd.nb = B->nab2; nd.it = 0; nd.blk = bk;
@@ -722,8 +696,8 @@ k_bis_roots(int N, const ProbDev *probs, const BlockDev *blocks, const int *blk_
 // the number of next-level children per CTA in bcnt.
 __global__ void __launch_bounds__(256)
 k_bis_count(const BisNode *in, const int *n_in_dev, const ProbDev *probs, const BlockDev *blocks,
-            const double2 *TP, Tol tol, int *ccnt, int *bcnt, double *Wt, double *Et, int *It,
-            BisState *st, unsigned long long *stats) {
+            const double2 *TP, Tol tol, int *ccnt, int *bcnt, double *Wt, double *Et,
+            BisState *st) {
   __shared__ int sint[32];
   // the level's length is on the device (the grid covers its bound, N/2)
   const int n_in = *n_in_dev;
@@ -733,20 +707,18 @@ k_bis_count(const BisNode *in, const int *n_in_dev, const ProbDev *probs, const 
   }
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   int nnext = 0;
-  unsigned long long work = 0;
   if (i < n_in) {
     const BisNode nd = in[i];
     const BlockDev *B = &blocks[nd.blk];
     const double pivmin = probs[B->prob].pivmin;
-    int cnt = dv_count_bisect(B->nbl, TP + B->ibgn, pivmin, 0.5 * (nd.a + nd.b));
+    int cnt = dv_count_guess(B->nbl, TP + B->ibgn, pivmin, 0.5 * (nd.a + nd.b));
     cnt = d_imin(nd.nb, d_imax(nd.na, cnt));
     ccnt[i] = cnt;
-    work = (unsigned long long)B->nbl;
     for (int side = 0; side < 2; side++) {
       BisNode ch;
       const int kind = bis_child(nd, cnt, side, pivmin, B->atoli, tol.bsrtol, B->itmax2, &ch);
       if (kind == 1 || kind == 2)
-        bis_finish(B, ch.a, ch.b, ch.na, ch.nb, ch.it, kind == 1, Wt, Et, It, st);
+        bis_finish(B, ch.a, ch.b, ch.na, ch.nb, ch.it, kind == 1, Wt, Et, st);
       else if (kind == 3)
         nnext++;
     }
@@ -754,7 +726,6 @@ k_bis_count(const BisNode *in, const int *n_in_dev, const ProbDev *probs, const 
   int total;
   cta_exscan(nnext, sint, &total);
   if (threadIdx.x == 0) bcnt[blockIdx.x] = total;
-  stat_add(stats, KID_BISECT * 4 + 0, work);
 }
 
 // Exclusive scan of the per-CTA counts (one CTA of 1024 threads); the total
@@ -783,7 +754,7 @@ __global__ void __launch_bounds__(1024) k_bis_scan(int nblk, int *bcnt, int *n_o
 __global__ void __launch_bounds__(256)
 k_bis_scatter(const BisNode *in, const int *n_in_dev, const ProbDev *probs, const BlockDev *blocks,
               Tol tol, const int *ccnt, const int *bcnt, BisNode *out, int split, double *Wt,
-              double *Et, int *It, BisState *st) {
+              double *Et, BisState *st) {
   __shared__ int sint[32];
   const int n_in = *n_in_dev;
   if (blockIdx.x * blockDim.x >= n_in) return;
@@ -805,13 +776,13 @@ k_bis_scatter(const BisNode *in, const int *n_in_dev, const ProbDev *probs, cons
   for (int side = 0; side < 2; side++)
     if (kind[side] == 3) {
       if (split) bis_finish(B, ch[side].a, ch[side].b, ch[side].na, ch[side].nb, ch[side].it, false,
-                            Wt, Et, It, st);
+                            Wt, Et, st);
       else out[pos++] = ch[side];
     }
 }
 
-// The single eigenvalues that left the tree, a thread each, continued with
-// dv_bisect_one from their state.
+// The single eigenvalues that left the tree, a thread each: continued with
+// dv_bisect_one from their state, then confirmed.
 __global__ void LB_BIS
 k_bisect_cont(int N, const ProbDev *probs, const BlockDev *blocks, const int *blk_of_row,
               const double2 *TP, double *Wt, double *Et, int *It, const BisState *st, Tol tol,
@@ -823,15 +794,25 @@ k_bisect_cont(int N, const ProbDev *probs, const BlockDev *blocks, const int *bl
     if (q.it >= 0) {
       const BlockDev *B = &blocks[blk_of_row[g]];
       const ProbDev *p = &probs[B->prob];
-      const int j = B->nab1 + 1 + (g - B->ibgn);
+      const double2 *tp = TP + B->ibgn;
+      const double pivmin = p->pivmin;
+      const int j = B->nab1 + 1 + (g - B->ibgn), n = B->nbl;
       double a = Wt[g], b = Et[g];
       int it = q.it;
-      dv_bisect_one(B->nbl, TP + B->ibgn, p->pivmin, B->atoli, tol.bsrtol, B->itmax2, j, &a, &b,
-                    q.na, q.nb, &it, q.it);
+      if (!q.done)
+        dv_bisect_one<true>(n, tp, pivmin, B->atoli, tol.bsrtol, B->itmax2, j, &a, &b, q.na, q.nb,
+                            &it, q.it);
+      it = 2;   // exact counts
+      if (dv_count_bisect(n, tp, pivmin, a) >= j || dv_count_bisect(n, tp, pivmin, b) < j) {
+        a = B->gl3;
+        b = B->gu3;
+        dv_bisect_one<false>(n, tp, pivmin, B->atoli, tol.bsrtol, B->itmax2, j, &a, &b, B->nab1,
+                             B->nab2, &it);
+      }
+      work = (unsigned long long)it * (unsigned long long)n;
       Wt[g] = 0.5 * (a + b);
       Et[g] = 0.5 * fabs(a - b);
       It[g] = j;
-      work = (unsigned long long)(it - q.it) * (unsigned long long)B->nbl;
     }
   }
   stat_add(stats, KID_BISECT * 4 + 0, work);
@@ -1711,15 +1692,15 @@ __device__ __forceinline__ unsigned long long refine_cl_body(
 // added while the chain's latency hides them and not beyond: 9000 intervals
 // take 4 lanes each (47 cycles a step; 32 lanes, which fill the SM with 15
 // warps a quarter, 103), 1000 take 32.
-#define MR3_ROW_LAT 90
-#define MR3_ROW_LAT1 193
-#define MR3_ROW_PIPE 50
-__host__ __device__ __forceinline__ int tree_lanes(long long items, int nsm, int maxL = 32) {
+// The guessed counts of stage A: 48 cycles, 18 a warp, for both forms.
+struct RowCost { int lat1, lat, pipe; };   // thread form, group form, per warp
+__host__ __device__ __forceinline__ int tree_lanes(long long items, int nsm, int maxL = 32,
+                                                   RowCost rc = {193, 90, 50}) {
   int best = 1;
   double best_cost = 0.0;
   for (int L = 1; L <= 32 && L <= maxL; L = L == 1 ? 4 : 2 * L) {
-    const double pipe = MR3_ROW_PIPE * (double)(items * L) / (32.0 * 4.0 * nsm);
-    const double lat = L == 1 ? MR3_ROW_LAT1 : MR3_ROW_LAT, row = lat > pipe ? lat : pipe;
+    const double pipe = rc.pipe * (double)(items * L) / (32.0 * 4.0 * nsm);
+    const double lat = L == 1 ? rc.lat1 : rc.lat, row = lat > pipe ? lat : pipe;
     const int steps = L == 32 ? 5 : L == 16 ? 4 : L == 8 ? 3 : L == 4 ? 2 : 1;
     if (L == 1 || row / steps < best_cost) { best = L; best_cost = row / steps; }
   }
@@ -3566,13 +3547,13 @@ extern "C" int mr3_cuda_solve_cb(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void
   LAUNCH(k_blocks, L, MR3_THREADS, c->probs, c->blocks, c->D, c->E, c->gers, c->TP, tol);
   unsigned long long *stats = c->prof ? c->stats : nullptr;
   {
-    const int Lb = tree_lanes(nwant, c->nsm, tree_max);
+    const int Lb = tree_lanes(nwant, c->nsm, tree_max, RowCost{48, 48, 18});
     if (Lb == 1) {
       // shared intervals breadth-first, then a thread per eigenvalue
       CK(cudaMemsetAsync(c->bis_st, 0xff, N * sizeof(BisState), st), "bis st");
       CK(cudaMemsetAsync(c->bis_n, 0, 2 * sizeof(int), st), "bis n");
       LAUNCH(k_bis_roots, gN, 256, NN, c->probs, c->blocks, c->blk_of_row, c->bis_nodes[0],
-             c->bis_n, c->Wt, c->Et, c->It, c->bis_st);
+             c->bis_n, c->Wt, c->Et, c->bis_st);
       // BIS_DEPTH levels without a host synchronisation: each level's length
       // stays on the device (bis_n[level parity]); a node holds at least two
       // eigenvalues, so no level exceeds N/2 nodes, the grid's bound
@@ -3581,17 +3562,17 @@ extern "C" int mr3_cuda_solve_cb(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void
       for (int depth = 0; depth < BIS_DEPTH; depth++) {
         const int split = depth + 1 >= BIS_DEPTH;
         LAUNCH(k_bis_count, nbmax, 256, c->bis_nodes[cur], c->bis_n + cur, c->probs, c->blocks,
-               c->TP, tol, c->bis_cnt, c->bis_bcnt, c->Wt, c->Et, c->It, c->bis_st, stats);
+               c->TP, tol, c->bis_cnt, c->bis_bcnt, c->Wt, c->Et, c->bis_st);
         if (!split) LAUNCH(k_bis_scan, 1, 1024, nbmax, c->bis_bcnt, c->bis_n + (cur ^ 1));
         LAUNCH(k_bis_scatter, nbmax, 256, c->bis_nodes[cur], c->bis_n + cur, c->probs, c->blocks,
-               tol, c->bis_cnt, c->bis_bcnt, c->bis_nodes[cur ^ 1], split, c->Wt, c->Et, c->It,
+               tol, c->bis_cnt, c->bis_bcnt, c->bis_nodes[cur ^ 1], split, c->Wt, c->Et,
                c->bis_st);
         cur ^= 1;
       }
       LAUNCH(k_bisect_cont, gN128, 128, NN, c->probs, c->blocks, c->blk_of_row, c->TP, c->Wt,
              c->Et, c->It, c->bis_st, tol, stats);
     } else
-      LAUNCH(k_bisect<true>, (int)(((long long)NN * Lb + 127) / 128), 128, NN, Lb, c->probs,
+      LAUNCH(k_bisect, (int)(((long long)NN * Lb + 127) / 128), 128, NN, Lb, c->probs,
              c->blocks, c->blk_of_row, c->TP, c->Wt, c->Et, c->It, tol, stats);
   }
   LAUNCH(k_compact, L, MR3_THREADS, c->probs, c->blocks, c->D, c->Wt, c->Et, c->It, c->W, c->Werr,
