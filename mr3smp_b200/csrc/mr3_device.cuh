@@ -715,9 +715,11 @@ static __device__ __noinline__ int dv_dlarrb_one(int n, const double2 *__restric
 // at node max(t,1) (heap numbering, computed along the node's path with the
 // same operations the sequential loop uses), then the group walks the tree
 // with the counts, applying the sequential loop's convergence test before
-// each step.  The widening loops are evaluated the same way, L/2 candidate
-// ends per side in one sweep.  The sequence of intervals is exactly the
-// sequential one.
+// each step (and before the next pass, which it may spare).  The first pass
+// counts at the two ends (lanes 0 and 1) and, for the usual case that
+// neither has to be widened, at nodes 1..L-2 of the tree between them.  The
+// widening loops are evaluated the same way, L/2 candidate ends per side in
+// one sweep.  The sequence of intervals is exactly the sequential one.
 static __device__ __noinline__ int dv_dlarrb_tree(int L, int n, const double2 *__restrict__ R, int ps,
                                            int i, int first, int has_left, double rgap_own,
                                            double lgap_in, double rtol1, double rtol2,
@@ -725,28 +727,40 @@ static __device__ __noinline__ int dv_dlarrb_tree(int L, int n, const double2 *_
                                            double *werr, int *ncount) {
   const int lane = threadIdx.x & 31;
   const int t = lane & (L - 1), g0 = lane - t, half = L >> 1;
-  const int depth = 31 - __clz(L);
   const unsigned gbits = (L == 32) ? 0xffffffffu : ((1u << L) - 1u);
   const unsigned full = gbits << g0;   // the group's lanes: groups run independently
   const double mnwdth = 2.0 * pivmin;
   double left = *w - *werr, right = *w + *werr;
-  double gap = fmin(first ? rgap_own : lgap_in, rgap_own);
   int status = 0;
-  // widening: the first L/2 lanes hold the left end after 0..L/2-1 widening
-  // steps, the others the right end; the first candidate that passes is the
-  // end the sequential loop stops at
-  {
+  // the count at this lane's point: an end, a candidate end or a tree node
+  auto node_mid = [&](int node) {
+    double l = left, rr = right;
+    for (int b = 30 - __clz(node); b >= 0; b--) {
+      const double m = 0.5 * (l + rr);
+      if ((node >> b) & 1) l = m; else rr = m;
+    }
+    return 0.5 * (l + rr);
+  };
+  int cnt = dv_dlaneg<QDIV_U>(n, R, ps, t == 0 ? left : t == 1 ? right : node_mid(t - 1), r);
+  bool need0 = __shfl_sync(full, cnt, g0) > i - 1, need1 = __shfl_sync(full, cnt, g0 + 1) < i;
+  *ncount += 2;
+  int shift = 1, known = L - 2;   // lane of node v: v + shift; nodes counted
+  if (need0 || need1) {
+    // widening: the first L/2 lanes hold the left end after the next 0..L/2-1
+    // widening steps, the others the right end; the first candidate that
+    // passes is the end the sequential loop stops at
+    known = 0;
     const int side = t >= half, k = t & (half - 1);
-    double xs0 = left, xs1 = right, bs0 = *werr, bs1 = *werr;
-    bool need0 = true, need1 = true;
-    int steps0 = 0, steps1 = 0;
-    while (__any_sync(full, need0 || need1)) {
+    double xs0 = need0 ? left - *werr : left, xs1 = need1 ? right + *werr : right;
+    double bs0 = 2.0 * *werr, bs1 = 2.0 * *werr;
+    int steps0 = 1, steps1 = 1;
+    while (need0 || need1) {
       double x = side ? xs1 : xs0, back = side ? bs1 : bs0;
       for (int j = 0; j < k; j++) { x = side ? x + back : x - back; back = 2.0 * back; }
       const bool mine = side ? need1 : need0;
-      int cnt = 0;
-      if (mine) cnt = dv_dlaneg<QDIV_U>(n, R, ps, x, r);
-      const bool ok = mine && (side ? (cnt >= i) : (cnt <= i - 1));
+      int c = 0;
+      if (mine) c = dv_dlaneg<QDIV_U>(n, R, ps, x, r);
+      const bool ok = mine && (side ? (c >= i) : (c <= i - 1));
       const unsigned gb = (__ballot_sync(full, ok) >> g0) & gbits;
       for (int sd = 0; sd < 2; sd++) {
         const unsigned pass = (gb >> (half * sd)) & ((1u << half) - 1u);
@@ -775,42 +789,34 @@ static __device__ __noinline__ int dv_dlarrb_tree(int L, int n, const double2 *_
   }
   double width = 0.5 * fabs(left - right);
   double tmp = fmax(fabs(left), fabs(right));
+  double gap = fmin(first ? rgap_own : lgap_in, rgap_own);
   double cvrgd = fmax(rtol1 * gap, rtol2 * tmp);
-  const bool early = (width <= cvrgd || width <= mnwdth);   // W, WERR kept
-  bool done = early;
+  if (width <= cvrgd || width <= mnwdth) return status;   // W, WERR kept
   gap = fmin(has_left ? lgap_in : rgap_own, rgap_own);
-  int iter = 0;
-  const int node_t = t == 0 ? 1 : t;
-  while (__any_sync(full, !done)) {
-    double l = left, rr = right;
-    for (int b = 30 - __clz(node_t); b >= 0; b--) {
-      const double m = 0.5 * (l + rr);
-      if ((node_t >> b) & 1) l = m; else rr = m;
-    }
-    int cnt = 0;
-    if (!done) cnt = dv_dlaneg<QDIV_U>(n, R, ps, 0.5 * (l + rr), r);
+  for (int iter = 0;;) {
+    // walk the counted nodes
     int node = 1;
-    for (int d = 0; d < depth; d++) {
-      const int c = __shfl_sync(full, cnt, g0 + node);
-      if (!done) {
-        const double mid = 0.5 * (left + right);
-        width = right - mid;
-        tmp = fmax(fabs(left), fabs(right));
-        cvrgd = fmax(rtol1 * gap, rtol2 * tmp);
-        if (width <= cvrgd || width <= mnwdth || iter == maxitr) {
-          done = true;
-        } else {
-          *ncount += 1;
-          if (c <= i - 1) { left = mid; node = 2 * node + 1; } else { right = mid; node = 2 * node; }
-          iter++;
-        }
-      }
+    bool done = false;
+    double mid;
+    for (;;) {
+      mid = 0.5 * (left + right);
+      width = right - mid;
+      tmp = fmax(fabs(left), fabs(right));
+      cvrgd = fmax(rtol1 * gap, rtol2 * tmp);
+      done = width <= cvrgd || width <= mnwdth || iter == maxitr;
+      if (done || node > known) break;
+      const int c = __shfl_sync(full, cnt, g0 + node + shift);
+      *ncount += 1;
+      if (c <= i - 1) { left = mid; node = 2 * node + 1; } else { right = mid; node = 2 * node; }
+      iter++;
     }
+    if (done) break;
+    cnt = dv_dlaneg<QDIV_U>(n, R, ps, node_mid(t == 0 ? 1 : t), r);
+    shift = 0;
+    known = L - 1;
   }
-  if (!early) {
-    *w = 0.5 * (left + right);
-    *werr = right - *w;
-  }
+  *w = 0.5 * (left + right);
+  *werr = right - *w;
   return status;
 }
 

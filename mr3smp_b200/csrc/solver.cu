@@ -1686,16 +1686,16 @@ __device__ __forceinline__ unsigned long long refine_cl_body(
 // Lanes per interval for a launch of `items` independent intervals: the
 // form with the shortest time per bisection step.  A group of L lanes takes
 // log2(L) steps per count, a thread (L = 1) one.  A count's row costs the
-// larger of the chain's latency (90 cycles with dv_qdiv, 193 with plain
-// divisions) and the FP64 pipe's time for the warps of a quarter SM (50
-// cycles a warp for either form, measured with the SM full).  So lanes are
-// added while the chain's latency hides them and not beyond: 9000 intervals
-// take 4 lanes each (47 cycles a step; 32 lanes, which fill the SM with 15
-// warps a quarter, 103), 1000 take 32.
-// The guessed counts of stage A: 48 cycles, 18 a warp, for both forms.
+// larger of the chain's latency and the FP64 pipe's time for the warps of a
+// quarter SM.  So lanes are added while the chain's latency hides them and
+// not beyond: 9000 intervals take 4 lanes each (65 cycles a step; 32 lanes,
+// which fill the SM with 15 warps a quarter, 152), 1000 take 32.  Measured in
+// cycles a row: dlaneg 250 (thread, plain divisions) and 115-135 (checked;
+// more when the rows are strided), 50 a warp with the SM full for either;
+// the guessed counts of stage A 48 and 18.
 struct RowCost { int lat1, lat, pipe; };   // thread form, group form, per warp
 __host__ __device__ __forceinline__ int tree_lanes(long long items, int nsm, int maxL = 32,
-                                                   RowCost rc = {193, 90, 50}) {
+                                                   RowCost rc = {130, 130, 50}) {
   int best = 1;
   double best_cost = 0.0;
   for (int L = 1; L <= 32 && L <= maxL; L = L == 1 ? 4 : 2 * L) {
@@ -1723,6 +1723,9 @@ k_refine_cl(const int *rl, const int *rl_n, const ClusterDev *cl, const ProbDev 
     for (long long b0 = 0; b0 < cnt; b0 += per) {
       const long long it = b0 + gt / L;
       const bool valid = it < cnt;
+      // a warp past the list's end has nothing to do (the spare groups of
+      // the last warp mirror its last interval)
+      if (b0 + (gt & ~31LL) / L >= cnt) break;
       const int s = rl[valid ? it : cnt - 1];
       if (!TREE) {
         if (valid)
@@ -3581,7 +3584,7 @@ extern "C" int mr3_cuda_solve_cb(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void
   LAUNCH(k_root, L, MR3_THREADS, c->probs, c->blocks, c->D, c->E, c->TP, c->Dt, c->Lt, c->W,
          c->Werr, c->Wgap, c->RP, c->RQ);
   {
-    const int Lr = tree_lanes(nwant, c->nsm, tree_max);
+    const int Lr = tree_lanes(nwant, c->nsm, tree_max, RowCost{250, 115, 50});
     if (Lr == 1)
       LAUNCH(k_refine_root<false>, gN128, 128, NN, 1, c->probs, c->blocks, c->iblk, c->RP, c->W,
              c->Werr, c->Wgap, tol, stats);
