@@ -23,6 +23,16 @@
 //   P[i] = (D(i), D(i)L(i)^2)   read by every Sturm count (dlaneg)
 //   Q[i] = (L(i), D(i)L(i))     read in addition by the twisted factorization
 
+// The item (interval, eigenvalue) of this lane's group when 32 / L groups of
+// L lanes share a warp (L = 1: a lane each); -1 for the lanes left over.
+// *base: the warp's first item.
+static __device__ __forceinline__ long long group_item(int L, long long *base) {
+  const long long warp = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
+  const int G = 32 / L, g = (threadIdx.x & 31) / L;
+  *base = warp * G;
+  return g < G ? *base + g : -1;
+}
+
 static __device__ __forceinline__ int d_imin(int a, int b) { return a < b ? a : b; }
 static __device__ __forceinline__ int d_imax(int a, int b) { return a > b ? a : b; }
 
@@ -191,12 +201,10 @@ static __device__ __noinline__ int dv_count_bisect_lat(int n, const double2 *__r
   if (n > U) {
     const unsigned hp = dv_habs(pivmin);
     double y0 = dv_rcp_seed(t);
-    double2 v[U], nx[U];
+    double2 v[U];   // row j + u; a row read is replaced by the one U rows on
 #pragma unroll
     for (int u = 0; u < U; u++) v[u] = tp[1 + u];
     for (; j + U <= n; j += U) {
-#pragma unroll
-      for (int u = 0; u < U; u++) nx[u] = tp[d_imin(j + U + u, n - 1)];
       const double t0 = t;
       const int cnt0 = cnt;
       unsigned tmin = 0xffffffffu;
@@ -210,6 +218,7 @@ static __device__ __noinline__ int dv_count_bisect_lat(int n, const double2 *__r
         t = v[u].x - q - c;
         cnt += dv_signbit(t);
         tmin = min(tmin, dv_habs(t));
+        v[u] = tp[d_imin(j + U + u, n - 1)];
       }
       if (qdiv_failed(k) || tmin <= hp) {
         t = t0;
@@ -222,8 +231,6 @@ static __device__ __noinline__ int dv_count_bisect_lat(int n, const double2 *__r
         }
         y0 = dv_rcp_seed(t);
       }
-#pragma unroll
-      for (int u = 0; u < U; u++) v[u] = nx[u];
     }
   }
   for (; j < n; j++) {
@@ -267,12 +274,10 @@ static __device__ __noinline__ int dv_count_guess(int n, const double2 *__restri
   if (t <= pivmin) { cnt = 1; t = fmin(t, -pivmin); }
   int j = 1;
   if (n > U) {
-    double2 v[U], nx[U];
+    double2 v[U];
 #pragma unroll
     for (int u = 0; u < U; u++) v[u] = tp[1 + u];
     for (; j + U <= n; j += U) {
-#pragma unroll
-      for (int u = 0; u < U; u++) nx[u] = tp[d_imin(j + U + u, n - 1)];
       const double t0 = t;
       const int cnt0 = cnt;
 #pragma unroll
@@ -280,6 +285,7 @@ static __device__ __noinline__ int dv_count_guess(int n, const double2 *__restri
         const double y0 = dv_rcp_seed(t), e = __fma_rn(-t, y0, 1.0), qh = v[u].y * y0;
         t = __fma_rn(-qh, __fma_rn(e, e, e), (v[u].x - c) - qh);
         cnt += dv_signbit(t);
+        v[u] = tp[d_imin(j + U + u, n - 1)];
       }
       if (dv_habs(t) >= (0x7fe00000u << 1)) {   // infinite, NaN or about to be
         t = t0;
@@ -291,8 +297,6 @@ static __device__ __noinline__ int dv_count_guess(int n, const double2 *__restri
           if (t <= pivmin) { cnt++; t = fmin(t, -pivmin); }
         }
       }
-#pragma unroll
-      for (int u = 0; u < U; u++) v[u] = nx[u];
     }
   }
   for (; j < n; j++) {
@@ -383,13 +387,13 @@ static __device__ __noinline__ int dv_bisect_one(int n, const double2 *__restric
   return 0;
 }
 
-// dv_bisect_one by a group of L lanes (L = 4..32; groups independent): the
-// midpoints of the next log2(L) steps form a binary tree that follows from
-// the current interval; lane t of the group counts at node max(t,1) (its
-// interval computed along the node's path with the loop's operations), then
-// the group walks the tree, clamping each count to the walk's (na, nb) and
-// applying the loop's convergence test after each step, as the sequential
-// loop does.  The same sequence of intervals; log2(L) steps per count.  The
+// dv_bisect_one by a group of L lanes (L = 3..32; groups independent): the
+// midpoints of the next steps form a binary tree that follows from the
+// current interval; lane t of the group counts at node t + 1 (its interval
+// computed along the node's path with the loop's operations), then the group
+// walks the tree, clamping each count to the walk's (na, nb) and applying
+// the loop's convergence test after each step, as the sequential loop does.
+// The same sequence of intervals; about log2(L) steps per count.  The
 // counts are guessed; lanes 0 and 1 then confirm the two ends, and the walk
 // is repeated with exact counts if one fails.
 static __device__ __noinline__ void dv_bisect_tree(int L, int n, const double2 *__restrict__ tp,
@@ -397,9 +401,8 @@ static __device__ __noinline__ void dv_bisect_tree(int L, int n, const double2 *
                                             int j, double *a_, double *b_, const int na0,
                                             const int nb0, int *iters) {
   const int lane = threadIdx.x & 31;
-  const int t = lane & (L - 1), g0 = lane - t, depth = 31 - __clz(L);
+  const int t = lane % L, g0 = lane - t;
   const unsigned gm = ((L == 32) ? 0xffffffffu : ((1u << L) - 1u)) << g0;
-  const int node_t = t == 0 ? 1 : t;
   const double a0 = *a_, b0 = *b_;
   double a = a0, b = b0;
   int it = 0;
@@ -412,24 +415,21 @@ static __device__ __noinline__ void dv_bisect_tree(int L, int n, const double2 *
     it = 0;
     while (!done) {
       double l = a, r = b;
-      for (int k = 30 - __clz(node_t); k >= 0; k--) {
+      for (int k = 30 - __clz(t + 1); k >= 0; k--) {
         const double m = 0.5 * (l + r);
-        if ((node_t >> k) & 1) l = m; else r = m;
+        if (((t + 1) >> k) & 1) l = m; else r = m;
       }
       const double x = 0.5 * (l + r);
       const int raw = pass == 0 ? dv_count_guess(n, tp, pivmin, x)
                                 : dv_count_bisect_lat(n, tp, pivmin, x);
-      int node = 1;
-      for (int d = 0; d < depth; d++) {
-        const int cv = __shfl_sync(gm, raw, g0 + node);
-        if (!done) {
-          const double c = 0.5 * (a + b);
-          const int cnt = d_imin(nb, d_imax(na, cv));
-          if (j <= cnt) { b = c; nb = cnt; node = 2 * node; } else { a = c; na = cnt; node = 2 * node + 1; }
-          it++;
-          const double w = fabs(b - a), tt = fmax(fabs(b), fabs(a));
-          if (w < fmax(fmax(abstol, pivmin), reltol * tt) || na >= nb || it >= itmax) done = true;
-        }
+      for (int node = 1; node <= L && !done;) {
+        const int cv = __shfl_sync(gm, raw, g0 + node - 1);
+        const double c = 0.5 * (a + b);
+        const int cnt = d_imin(nb, d_imax(na, cv));
+        if (j <= cnt) { b = c; nb = cnt; node = 2 * node; } else { a = c; na = cnt; node = 2 * node + 1; }
+        it++;
+        const double w = fabs(b - a), tt = fmax(fabs(b), fabs(a));
+        if (w < fmax(fmax(abstol, pivmin), reltol * tt) || na >= nb || it >= itmax) done = true;
       }
     }
     if (pass == 1) { it += 2; break; }
@@ -453,7 +453,7 @@ static __device__ __noinline__ void dv_bisect_tree(int L, int n, const double2 *
 // row loop, best when a warp's threads all read the same rows (a block's
 // root representation) and fill the SM.
 template <int U>
-static __device__ __noinline__ int dv_dlaneg(int n, const double2 *__restrict__ P, int ps, double sigma,
+static __device__ __forceinline__ int dv_dlaneg_inl(int n, const double2 *__restrict__ P, int ps, double sigma,
                                       int r) {
   static_assert(128 % U == 0, "chunks must not straddle the 128-row blocks");
   const int blklen = 128;
@@ -517,7 +517,7 @@ static __device__ __noinline__ int dv_dlaneg(int n, const double2 *__restrict__ 
   }
   if (r - 1 >= 1) {
     const int last = r - 1;
-    double2 c[U], nx[U];
+    double2 c[U];   // row j + u; a row read is replaced by the one U rows on
 #pragma unroll
     for (int u = 0; u < U; u++) c[u] = P[(size_t)(d_imin(1 + u, last) - 1) * ps];
     double y0 = dv_rcp_seed(c[0].x + t);
@@ -526,8 +526,6 @@ static __device__ __noinline__ int dv_dlaneg(int n, const double2 *__restrict__ 
       int neg1 = 0, j = bj;
       const double bsav = t;
       for (; j + U - 1 <= jend; j += U) {
-#pragma unroll
-        for (int u = 0; u < U; u++) nx[u] = P[(size_t)(d_imin(j + U + u, last) - 1) * ps];
         const double t0 = t;
         const int n0 = neg1;
         qdiv_chk k;
@@ -537,9 +535,10 @@ static __device__ __noinline__ int dv_dlaneg(int n, const double2 *__restrict__ 
           const double dplus = c[u].x + t;
           double qt;
           const double tmp = dv_qdiv(t, dplus, y0, &k, &qt);
-          y0 = dv_rcp_seed((u + 1 < U ? c[u + 1].x : nx[0].x) + (qt * c[u].y - sigma));
+          y0 = dv_rcp_seed(c[(u + 1) % U].x + (qt * c[u].y - sigma));
           neg1 += dv_signbit(dplus);
           t = tmp * c[u].y - sigma;
+          c[u] = P[(size_t)(d_imin(j + U + u, last) - 1) * ps];
         }
         if (qdiv_failed(k)) {
           t = t0;
@@ -552,10 +551,8 @@ static __device__ __noinline__ int dv_dlaneg(int n, const double2 *__restrict__ 
             const double tmp = t / dplus;
             t = tmp * v.y - sigma;
           }
-          y0 = dv_rcp_seed(nx[0].x + t);
+          y0 = dv_rcp_seed(c[0].x + t);
         }
-#pragma unroll
-        for (int u = 0; u < U; u++) c[u] = nx[u];
       }
       for (; j <= jend; j++) {   // the last rows, fewer than a chunk
         const double2 v = P[(size_t)(j - 1) * ps];
@@ -582,7 +579,7 @@ static __device__ __noinline__ int dv_dlaneg(int n, const double2 *__restrict__ 
   }
   double p = P[(size_t)(n - 1) * ps].x - sigma;
   if (n - 1 >= r) {
-    double2 c[U], nx[U];
+    double2 c[U];
 #pragma unroll
     for (int u = 0; u < U; u++) c[u] = P[(size_t)(d_imax(n - 1 - u, r) - 1) * ps];
     double y0 = dv_rcp_seed(c[0].y + p);
@@ -591,8 +588,6 @@ static __device__ __noinline__ int dv_dlaneg(int n, const double2 *__restrict__ 
       int neg2 = 0, j = bj;
       const double bsav = p;
       for (; j - U + 1 >= jend; j -= U) {
-#pragma unroll
-        for (int u = 0; u < U; u++) nx[u] = P[(size_t)(d_imax(j - U - u, r) - 1) * ps];
         const double p0 = p;
         const int n0 = neg2;
         qdiv_chk k;
@@ -602,9 +597,10 @@ static __device__ __noinline__ int dv_dlaneg(int n, const double2 *__restrict__ 
           const double dminus = c[u].y + p;
           double qt;
           const double tmp = dv_qdiv(p, dminus, y0, &k, &qt);
-          y0 = dv_rcp_seed((u + 1 < U ? c[u + 1].y : nx[0].y) + (qt * c[u].x - sigma));
+          y0 = dv_rcp_seed(c[(u + 1) % U].y + (qt * c[u].x - sigma));
           neg2 += dv_signbit(dminus);
           p = tmp * c[u].x - sigma;
+          c[u] = P[(size_t)(d_imax(j - U - u, r) - 1) * ps];
         }
         if (qdiv_failed(k)) {
           p = p0;
@@ -617,10 +613,8 @@ static __device__ __noinline__ int dv_dlaneg(int n, const double2 *__restrict__ 
             const double tmp = p / dminus;
             p = tmp * v.x - sigma;
           }
-          y0 = dv_rcp_seed(nx[0].y + p);
+          y0 = dv_rcp_seed(c[0].y + p);
         }
-#pragma unroll
-        for (int u = 0; u < U; u++) c[u] = nx[u];
       }
       for (; j >= jend; j--) {
         const double2 v = P[(size_t)(j - 1) * ps];
@@ -648,6 +642,12 @@ static __device__ __noinline__ int dv_dlaneg(int n, const double2 *__restrict__ 
   double gamma = (t + sigma) + p;
   if (gamma < 0.0) negcnt++;
   return negcnt;
+}
+
+template <int U>
+static __device__ __noinline__ int dv_dlaneg(int n, const double2 *__restrict__ P, int ps, double sigma,
+                                      int r) {
+  return dv_dlaneg_inl<U>(n, P, ps, sigma, r);
 }
 
 // One interval of dlarrb (SRC/LAPACK/odrrb.f:136-293).  Intervals of one
@@ -706,118 +706,146 @@ static __device__ __noinline__ int dv_dlarrb_one(int n, const double2 *__restric
   return status;
 }
 
-// dv_dlarrb_one for one interval per group of L lanes (L = 4, 8, 16 or 32,
-// the same for the whole warp; every lane of a group calls it with the same
-// arguments and gets the same results; groups are independent, a group may
-// skip the call).  The bisection
-// midpoints of the next log2(L) steps form a binary tree whose nodes follow
-// from the current interval alone: lane t of the group evaluates the count
-// at node max(t,1) (heap numbering, computed along the node's path with the
-// same operations the sequential loop uses), then the group walks the tree
+// dv_dlarrb_one for one interval per group of L lanes (L = 3..32, the same
+// for the whole warp: 32 / L groups, the lanes left over in none).  Every
+// lane of the warp calls it; the lanes of a group pass the same arguments and
+// get the same results, and groups with act = false (the lanes left over
+// among them) have no interval.  The bisection
+// midpoints of the next steps form a binary tree whose nodes follow from the
+// current interval alone: lane t of the group evaluates the count at node
+// t + 1 (heap numbering, computed along the node's path with the same
+// operations the sequential loop uses), then the group walks the tree
 // with the counts, applying the sequential loop's convergence test before
 // each step (and before the next pass, which it may spare).  The first pass
 // counts at the two ends (lanes 0 and 1) and, for the usual case that
 // neither has to be widened, at nodes 1..L-2 of the tree between them.  The
 // widening loops are evaluated the same way, L/2 candidate ends per side in
 // one sweep.  The sequence of intervals is exactly the sequential one.
-static __device__ __noinline__ int dv_dlarrb_tree(int L, int n, const double2 *__restrict__ R, int ps,
-                                           int i, int first, int has_left, double rgap_own,
-                                           double lgap_in, double rtol1, double rtol2,
-                                           double pivmin, int maxitr, int r, double *w,
-                                           double *werr, int *ncount) {
+//
+// The passes are the warp's: a group that widens counts beside groups that
+// bisect.  (With a loop per group, groups once apart never met again and
+// counted one after the other: twice the time for the slowest warps of
+// k_refine_cl on the n = 20010 problem.)
+static __device__ __forceinline__ void dv_dlarrb_tree(bool act, int L, int n,
+                                            const double2 *__restrict__ R, int ps, int i, int first,
+                                            int has_left, double rgap_own, double lgap_in,
+                                            double rtol1, double rtol2, double pivmin, int maxitr,
+                                            int r, double *w, double *werr, int *ncount) {
+  enum { ENDS, WIDEN, TREE, DONE };
   const int lane = threadIdx.x & 31;
-  const int t = lane & (L - 1), g0 = lane - t, half = L >> 1;
+  const int t = lane % L, g0 = lane - t, half = L >> 1;
   const unsigned gbits = (L == 32) ? 0xffffffffu : ((1u << L) - 1u);
-  const unsigned full = gbits << g0;   // the group's lanes: groups run independently
+  const unsigned gm = gbits << g0;   // (the lanes left over: theirs)
   const double mnwdth = 2.0 * pivmin;
   double left = *w - *werr, right = *w + *werr;
-  int status = 0;
-  // the count at this lane's point: an end, a candidate end or a tree node
-  auto node_mid = [&](int node) {
-    double l = left, rr = right;
-    for (int b = 30 - __clz(node); b >= 0; b--) {
-      const double m = 0.5 * (l + rr);
-      if ((node >> b) & 1) l = m; else rr = m;
+  // widening: the first L/2 lanes hold the left end after the next 0..L/2-1
+  // widening steps, the others the right end; the first candidate that
+  // passes is the end the sequential loop stops at
+  const int side = t >= half, wk = t - side * half;
+  bool need0 = false, need1 = false;
+  double xs0 = 0.0, xs1 = 0.0, bs0 = 0.0, bs1 = 0.0;
+  int steps0 = 0, steps1 = 0;
+  int phase = act ? ENDS : DONE, iter = 0, nc = 0;
+  while (__any_sync(0xffffffffu, phase != DONE)) {
+    // this lane's point: an end, a candidate end or a tree node
+    double x = 0.0, back = 0.0;
+    bool mine = phase != DONE;
+    if (phase == ENDS && t < 2) {
+      x = t == 0 ? left : right;
+    } else if (phase == WIDEN) {
+      x = side ? xs1 : xs0;
+      back = side ? bs1 : bs0;
+      for (int k = 0; k < wk; k++) { x = side ? x + back : x - back; back = 2.0 * back; }
+      mine = wk < half && (side ? need1 : need0);
+    } else if (mine) {
+      const int node = phase == ENDS ? t - 1 : t + 1;
+      double l = left, rr = right;
+      for (int b = 30 - __clz(node); b >= 0; b--) {
+        const double m = 0.5 * (l + rr);
+        if ((node >> b) & 1) l = m; else rr = m;
+      }
+      x = 0.5 * (l + rr);
     }
-    return 0.5 * (l + rr);
-  };
-  int cnt = dv_dlaneg<QDIV_U>(n, R, ps, t == 0 ? left : t == 1 ? right : node_mid(t - 1), r);
-  bool need0 = __shfl_sync(full, cnt, g0) > i - 1, need1 = __shfl_sync(full, cnt, g0 + 1) < i;
-  *ncount += 2;
-  int shift = 1, known = L - 2;   // lane of node v: v + shift; nodes counted
-  if (need0 || need1) {
-    // widening: the first L/2 lanes hold the left end after the next 0..L/2-1
-    // widening steps, the others the right end; the first candidate that
-    // passes is the end the sequential loop stops at
-    known = 0;
-    const int side = t >= half, k = t & (half - 1);
-    double xs0 = need0 ? left - *werr : left, xs1 = need1 ? right + *werr : right;
-    double bs0 = 2.0 * *werr, bs1 = 2.0 * *werr;
-    int steps0 = 1, steps1 = 1;
-    while (need0 || need1) {
-      double x = side ? xs1 : xs0, back = side ? bs1 : bs0;
-      for (int j = 0; j < k; j++) { x = side ? x + back : x - back; back = 2.0 * back; }
-      const bool mine = side ? need1 : need0;
-      int c = 0;
-      if (mine) c = dv_dlaneg<QDIV_U>(n, R, ps, x, r);
-      const bool ok = mine && (side ? (c >= i) : (c <= i - 1));
-      const unsigned gb = (__ballot_sync(full, ok) >> g0) & gbits;
-      for (int sd = 0; sd < 2; sd++) {
-        const unsigned pass = (gb >> (half * sd)) & ((1u << half) - 1u);
-        const int k0 = pass ? __ffs(pass) - 1 : half - 1;
-        const double xsrc = __shfl_sync(full, x, g0 + half * sd + k0);
-        const double bsrc = __shfl_sync(full, back, g0 + half * sd + k0);
-        bool &need = sd ? need1 : need0;
-        double &xs = sd ? xs1 : xs0, &bs = sd ? bs1 : bs0;
-        int &steps = sd ? steps1 : steps0;
-        if (!need) continue;
-        if (pass) {
-          *ncount += k0 + 1;
-          xs = xsrc;
-          need = false;
+    int cnt = 0;
+    if (mine) cnt = dv_dlaneg_inl<QDIV_U>(n, R, ps, x, r);
+    __syncwarp();
+    if (phase != DONE) {
+      int shift = -1, known = L;      // lane of node v: v + shift; nodes counted
+      bool start = false;             // the ends are now those of the main loop
+      if (phase == ENDS) {
+        need0 = __shfl_sync(gm, cnt, g0) > i - 1;
+        need1 = __shfl_sync(gm, cnt, g0 + 1) < i;
+        nc += 2;
+        shift = 1;
+        known = L - 2;
+        if (need0 || need1) {
+          xs0 = need0 ? left - *werr : left;
+          xs1 = need1 ? right + *werr : right;
+          bs0 = bs1 = 2.0 * *werr;
+          steps0 = steps1 = 1;
+          phase = WIDEN;
         } else {
-          *ncount += half;
-          xs = sd ? xsrc + bsrc : xsrc - bsrc;
-          bs = 2.0 * bsrc;
-          steps += half;
-          if (steps >= MR3_EXPAND_CAP) { status = -1; need = false; }
+          start = true;
+        }
+      } else if (phase == WIDEN) {
+        const bool ok = mine && (side ? (cnt >= i) : (cnt <= i - 1));
+        const unsigned gb = (__ballot_sync(gm, ok) >> g0) & gbits;
+        for (int sd = 0; sd < 2; sd++) {
+          const unsigned pass = (gb >> (half * sd)) & ((1u << half) - 1u);
+          const int k0 = pass ? __ffs(pass) - 1 : half - 1;
+          const double xsrc = __shfl_sync(gm, x, g0 + half * sd + k0);
+          const double bsrc = __shfl_sync(gm, back, g0 + half * sd + k0);
+          bool &need = sd ? need1 : need0;
+          double &xs = sd ? xs1 : xs0, &bs = sd ? bs1 : bs0;
+          int &steps = sd ? steps1 : steps0;
+          if (!need) continue;
+          if (pass) {
+            nc += k0 + 1;
+            xs = xsrc;
+            need = false;
+          } else {
+            nc += half;
+            xs = sd ? xsrc + bsrc : xsrc - bsrc;
+            bs = 2.0 * bsrc;
+            steps += half;
+            if (steps >= MR3_EXPAND_CAP) need = false;
+          }
+        }
+        if (!need0 && !need1) {
+          left = xs0;
+          right = xs1;
+          start = true;
+          known = 0;
+        }
+      }
+      if (start) {
+        const double gap = fmin(first ? rgap_own : lgap_in, rgap_own);
+        const double width = 0.5 * fabs(left - right), tmp = fmax(fabs(left), fabs(right));
+        // converged early: W, WERR kept
+        phase = width <= fmax(rtol1 * gap, rtol2 * tmp) || width <= mnwdth ? DONE : TREE;
+      }
+      if (phase == TREE) {   // walk the counted nodes
+        const double gap = fmin(has_left ? lgap_in : rgap_own, rgap_own);
+        for (int node = 1;;) {
+          const double mid = 0.5 * (left + right);
+          const double width = right - mid, tmp = fmax(fabs(left), fabs(right));
+          if (width <= fmax(rtol1 * gap, rtol2 * tmp) || width <= mnwdth || iter == maxitr) {
+            *w = mid;
+            *werr = right - mid;
+            phase = DONE;
+            break;
+          }
+          if (node > known) break;
+          const int c = __shfl_sync(gm, cnt, g0 + node + shift);
+          nc++;
+          iter++;
+          if (c <= i - 1) { left = mid; node = 2 * node + 1; } else { right = mid; node = 2 * node; }
         }
       }
     }
-    left = xs0;
-    right = xs1;
+    __syncwarp();
   }
-  double width = 0.5 * fabs(left - right);
-  double tmp = fmax(fabs(left), fabs(right));
-  double gap = fmin(first ? rgap_own : lgap_in, rgap_own);
-  double cvrgd = fmax(rtol1 * gap, rtol2 * tmp);
-  if (width <= cvrgd || width <= mnwdth) return status;   // W, WERR kept
-  gap = fmin(has_left ? lgap_in : rgap_own, rgap_own);
-  for (int iter = 0;;) {
-    // walk the counted nodes
-    int node = 1;
-    bool done = false;
-    double mid;
-    for (;;) {
-      mid = 0.5 * (left + right);
-      width = right - mid;
-      tmp = fmax(fabs(left), fabs(right));
-      cvrgd = fmax(rtol1 * gap, rtol2 * tmp);
-      done = width <= cvrgd || width <= mnwdth || iter == maxitr;
-      if (done || node > known) break;
-      const int c = __shfl_sync(full, cnt, g0 + node + shift);
-      *ncount += 1;
-      if (c <= i - 1) { left = mid; node = 2 * node + 1; } else { right = mid; node = 2 * node; }
-      iter++;
-    }
-    if (done) break;
-    cnt = dv_dlaneg<QDIV_U>(n, R, ps, node_mid(t == 0 ? 1 : t), r);
-    shift = 0;
-    known = L - 1;
-  }
-  *w = 0.5 * (left + right);
-  *werr = right - *w;
-  return status;
+  *ncount += nc;
 }
 
 /* ------------------------------------------------------------------------

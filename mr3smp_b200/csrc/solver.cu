@@ -35,19 +35,23 @@
 #ifndef MR3_BIS_MINB
 #define MR3_BIS_MINB 0
 #endif
-#ifndef MR3_REF_MINB
-#define MR3_REF_MINB 0
-#endif
 #if MR3_BIS_MINB > 0
 #define LB_BIS __launch_bounds__(128, MR3_BIS_MINB)
 #else
 #define LB_BIS __launch_bounds__(128)
 #endif
-#if MR3_REF_MINB > 0
-#define LB_REF __launch_bounds__(128, MR3_REF_MINB)
-#else
-#define LB_REF __launch_bounds__(128)
+// The lane-group forms (tree_lanes) run in blocks of TREE_T threads, two
+// warps, so that a launch spreads evenly over the quarter SMs; TREE_MINB
+// blocks an SM leave their sweeps 168 registers.  (k_refine_cl on the n =
+// 20010 problem: 54 ms, with 128-thread blocks of 128 registers 71; four
+// blocks of 255 registers the same, but k_bisect then needs a second wave.)
+#ifndef TREE_T
+#define TREE_T 64
 #endif
+#ifndef TREE_MINB
+#define TREE_MINB 6
+#endif
+#define LB_TREE __launch_bounds__(TREE_T, TREE_MINB)
 #ifndef MR3_RRF_MINB
 #define MR3_RRF_MINB 0
 #endif
@@ -580,13 +584,14 @@ k_blocks(ProbDev *probs, BlockDev *blocks, const double *D, double *E, const dou
 // counts at its ends (see dv_count_guess).
 // ------------------------------------------------------------------------
 // L lanes per eigenvalue (few eigenvalues: single large problems).
-__global__ void __launch_bounds__(128)
+__global__ void LB_TREE
 k_bisect(int N, int L, const ProbDev *probs, const BlockDev *blocks, const int *blk_of_row,
          const double2 *TP, double *Wt, double *Et, int *It, Tol tol, unsigned long long *stats) {
-  const long long gt = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  long long base;
+  const long long item = group_item(L, &base);
   unsigned long long work = 0;
-  if (gt / L < N) {
-    const int g = (int)(gt / L);
+  if (item >= 0 && item < N) {
+    const int g = (int)item;
     const BlockDev *B = &blocks[blk_of_row[g]];
     const ProbDev *p = &probs[B->prob];
     const int k = g - B->ibgn;
@@ -597,7 +602,7 @@ k_bisect(int N, int L, const ProbDev *probs, const BlockDev *blocks, const int *
       int itc = 0;
       dv_bisect_tree(L, B->nbl, TP + B->ibgn, p->pivmin, B->atoli, tol.bsrtol, B->itmax2, j, &a, &b,
                      B->nab1, B->nab2, &itc);
-      if ((gt % L) == 0) {
+      if ((threadIdx.x & 31) % L == 0) {
         Wt[g] = 0.5 * (a + b);
         Et[g] = 0.5 * fabs(a - b);
         It[g] = j;
@@ -1121,39 +1126,44 @@ __device__ __forceinline__ unsigned long long refine_root_body(int s, const Prob
 }
 
 template <bool TREE>
-__global__ void LB_REF
+__global__ void __launch_bounds__(TREE ? TREE_T : 128, TREE ? TREE_MINB : 7)
 k_refine_root(int N, int L, const ProbDev *probs, const BlockDev *blocks, const int *iblk,
               const double2 *RP, double *W, double *Werr, const double *Wgap, Tol tol,
               unsigned long long *stats) {
-  const long long gt = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  long long base;
+  const long long item = group_item(TREE ? L : 1, &base);
   unsigned long long work = 0;
   if (!TREE) {
-    if (gt < N) work = refine_root_body((int)gt, probs, blocks, iblk, RP, W, Werr, Wgap, tol);
-  } else if (gt / L < N) {
+    if (item < N) work = refine_root_body((int)item, probs, blocks, iblk, RP, W, Werr, Wgap, tol);
+  } else if (base < N) {
     // L lanes per eigenvalue (few eigenvalues: single large problems)
-    const int s = (int)(gt / L);
-    const bool ok = iblk[s] >= 0;
-    const BlockDev *B = ok ? &blocks[iblk[s]] : nullptr;
-    const ProbDev *p = ok ? &probs[B->prob] : nullptr;
-    if (ok && !p->status && B->nbl >= 2 && !B->dqds) {
+    const int s = (int)item;
+    const BlockDev *B = item >= 0 && item < N && iblk[s] >= 0 ? &blocks[iblk[s]] : nullptr;
+    const ProbDev *p = B ? &probs[B->prob] : nullptr;
+    const bool act = B && !p->status && B->nbl >= 2 && !B->dqds;
+    int i = 0, II = 0, maxitr = 0, nc = 0;
+    double w = 0.0, werr = 0.0, rgap = 0.0, lgap = 0.0, rtol1 = 0.0, rtol2 = 0.0, pivmin = 0.0;
+    if (act) {
       const bool onlyW = (p->jobz == MR3_JOB_N);
-      const int II = s - B->wbgn + 1;
-      const int i = B->ilow + II - 1;
-      double w = W[s] - B->sigma;
-      double werr = Werr[s] + fabs(w) * MR3_EPS;
-      const double rgap = Wgap[s];
-      const double lgap = (II > 1) ? Wgap[s - 1] : rgap;
-      const int maxitr = dv_itmax(B->spdiam + p->pivmin, p->pivmin);
-      const double rtol1 = onlyW ? 4.0 * MR3_EPS : tol.rtol1;
-      const double rtol2 = onlyW ? 4.0 * MR3_EPS : tol.rtol2;
-      int nc = 0;
-      dv_dlarrb_tree(L, B->nbl, RP + B->ibgn, 1, i, II == 1, II > 1, rgap, lgap, rtol1, rtol2,
-                     p->pivmin, maxitr, B->nbl, &w, &werr, &nc);
-      if ((gt % L) == 0) {
-        W[s] = w;
-        Werr[s] = werr;
-        work = (unsigned long long)nc * (unsigned long long)B->nbl;
-      }
+      II = s - B->wbgn + 1;
+      i = B->ilow + II - 1;
+      w = W[s] - B->sigma;
+      werr = Werr[s] + fabs(w) * MR3_EPS;
+      rgap = Wgap[s];
+      lgap = (II > 1) ? Wgap[s - 1] : rgap;
+      pivmin = p->pivmin;
+      maxitr = dv_itmax(B->spdiam + pivmin, pivmin);
+      rtol1 = onlyW ? 4.0 * MR3_EPS : tol.rtol1;
+      rtol2 = onlyW ? 4.0 * MR3_EPS : tol.rtol2;
+    }
+    const int nb = act ? B->nbl : 0;
+    __syncwarp();
+    dv_dlarrb_tree(act, L, nb, act ? RP + B->ibgn : RP, 1, i, II == 1, II > 1, rgap, lgap, rtol1,
+                   rtol2, pivmin, maxitr, nb, &w, &werr, &nc);
+    if (act && (threadIdx.x & 31) % L == 0) {
+      W[s] = w;
+      Werr[s] = werr;
+      work = (unsigned long long)nc * (unsigned long long)nb;
     }
   }
   stat_add(stats, KID_REFROOT * 4 + 1, work);
@@ -1517,16 +1527,17 @@ __device__ __forceinline__ void own_rrr(const ClusterDev &C, const BlockDev &B, 
 // Both calls see a zero right gap, so their convergence test does not depend
 // on any other gap and the two ends are independent.
 template <bool TREE>
-__global__ void LB_REF
+__global__ void __launch_bounds__(TREE ? TREE_T : 128, 4)
 k_cl_ext(int ncl, int L, const ClusterDev *cl, const ProbDev *probs, const BlockDev *blocks,
          const double2 *RP, const double2 *RQ, const double *arena_prev, const double *Wsh,
          const double *Werr, const int *Windex, double *xw, double *xe, Tol tol,
          unsigned long long *stats) {
-  // L lanes per cluster end (L = 1: a thread; L >= 4: dv_dlarrb_tree, for
+  // L lanes per cluster end (L = 1: a thread; else dv_dlarrb_tree, for
   // launches with few clusters, where the sequential steps are the cost)
-  const long long gt = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  const bool valid = gt / L < 2LL * ncl;
-  const int t = valid ? (int)(gt / L) : 2 * ncl - 1;   // spare lanes mirror the last end
+  long long base;
+  const long long item = group_item(TREE ? L : 1, &base);
+  const bool valid = item >= 0 && item < 2LL * ncl;
+  const int t = valid ? (int)item : 2 * ncl - 1;   // spare lanes: the last end's pointers
   const int w = t >> 1;
   unsigned long long work = 0;
   {
@@ -1547,10 +1558,11 @@ k_cl_ext(int ncl, int L, const ClusterDev *cl, const ProbDev *probs, const Block
         dv_dlarrb_one<QDIV_U>(nb, Pp, ps, i, 1, II > 1, 0.0, 0.0, tol.rqtol, tol.rqtol, p->pivmin,
                              maxitr, nb, &wv, &ev, &nc);
     } else {
-      dv_dlarrb_tree(L, nb, Pp, ps, i, 1, II > 1, 0.0, 0.0, tol.rqtol, tol.rqtol, p->pivmin, maxitr,
-                     nb, &wv, &ev, &nc);
+      __syncwarp();
+      dv_dlarrb_tree(valid, L, nb, Pp, ps, i, 1, II > 1, 0.0, 0.0, tol.rqtol, tol.rqtol, p->pivmin,
+                     maxitr, nb, &wv, &ev, &nc);
     }
-    if (valid && (gt % L) == 0) {
+    if (valid && (threadIdx.x & 31) % L == 0) {
       xw[t] = wv;
       xe[t] = ev;
       work = (unsigned long long)nc * nb;
@@ -1685,30 +1697,42 @@ __device__ __forceinline__ unsigned long long refine_cl_body(
 
 // Lanes per interval for a launch of `items` independent intervals: the
 // form with the shortest time per bisection step.  A group of L lanes takes
-// log2(L) steps per count, a thread (L = 1) one.  A count's row costs the
-// larger of the chain's latency and the FP64 pipe's time for the warps of a
+// log2(L + 1) steps per count (a part of a step where its nodes end within a
+// level), a thread (L = 1) one.  A count's row costs the larger of the
+// chain's latency and the FP64 pipe's time for the warps of the fullest
 // quarter SM.  So lanes are added while the chain's latency hides them and
-// not beyond: 9000 intervals take 4 lanes each (65 cycles a step; 32 lanes,
-// which fill the SM with 15 warps a quarter, 152), 1000 take 32.  Measured in
-// cycles a row: dlaneg 250 (thread, plain divisions) and 115-135 (checked;
-// more when the rows are strided), 50 a warp with the SM full for either;
-// the guessed counts of stage A 48 and 18.
+// not beyond: 10005 intervals take 3 lanes each (two warps a quarter, 65
+// cycles a step; 4 lanes three warps, 80), 1000 take 32.  Measured in cycles
+// a row: dlaneg 250 (thread, plain divisions) and 115-135 (checked; more when
+// the rows are strided), 60 a warp; the guessed counts of stage A 48 and 18.
 struct RowCost { int lat1, lat, pipe; };   // thread form, group form, per warp
 __host__ __device__ __forceinline__ int tree_lanes(long long items, int nsm, int maxL = 32,
-                                                   RowCost rc = {130, 130, 50}) {
+                                                   RowCost rc = {130, 130, 60}) {
   int best = 1;
-  double best_cost = 0.0;
-  for (int L = 1; L <= 32 && L <= maxL; L = L == 1 ? 4 : 2 * L) {
-    const double pipe = rc.pipe * (double)(items * L) / (32.0 * 4.0 * nsm);
-    const double lat = L == 1 ? rc.lat1 : rc.lat, row = lat > pipe ? lat : pipe;
-    const int steps = L == 32 ? 5 : L == 16 ? 4 : L == 8 ? 3 : L == 4 ? 2 : 1;
+  float best_cost = 0.f;
+  for (int L = 1; L <= 32 && L <= maxL; L = L == 1 ? 3 : L + 1) {
+    const int G = 32 / L;
+    if (L > 1 && 32 / (L + 1) == G && L < 32 && L < maxL) continue;   // more lanes for nothing
+    const long long warps = (items + G - 1) / G, quarter = (warps + 4 * nsm - 1) / (4 * nsm);
+    const float pipe = (float)rc.pipe * quarter;
+    const float lat = L == 1 ? rc.lat1 : rc.lat, row = lat > pipe ? lat : pipe;
+    // whole levels of the tree, and the share of the next one
+    int d = 0;
+    while ((2 << d) - 1 <= L) d++;
+    const float steps = L == 1 ? 1.f : d + (L - ((1 << d) - 1)) / (float)(1 << d);
     if (L == 1 || row / steps < best_cost) { best = L; best_cost = row / steps; }
   }
   return best;
 }
 
+// Blocks of TREE_T threads for `items` groups of L lanes.
+static int group_blocks(long long items, int L) {
+  const long long warps = (items + 32 / L - 1) / (32 / L);
+  return (int)((warps + TREE_T / 32 - 1) / (TREE_T / 32));
+}
+
 template <bool TREE>
-__global__ void LB_REF
+__global__ void __launch_bounds__(TREE ? TREE_T : 128, 4)
 k_refine_cl(const int *rl, const int *rl_n, const ClusterDev *cl, const ProbDev *probs,
             const BlockDev *blocks, const double *arena_cur, double *Wsh, double *Werr,
             const double *Wgap, const int *Windex, const int *cl_of_slot, const int *lvl_of_slot,
@@ -1718,14 +1742,12 @@ k_refine_cl(const int *rl, const int *rl_n, const ClusterDev *cl, const ProbDev 
   const int L0 = cnt > 0 ? tree_lanes(cnt, nsm, tree_max) : 1;
   if (cnt > 0 && (L0 > 1) == TREE) {   // the other instantiation has the other form
     const int L = L0;
-    const long long gt = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    const long long per = ((long long)gridDim.x * blockDim.x) / L;
-    for (long long b0 = 0; b0 < cnt; b0 += per) {
-      const long long it = b0 + gt / L;
-      const bool valid = it < cnt;
-      // a warp past the list's end has nothing to do (the spare groups of
-      // the last warp mirror its last interval)
-      if (b0 + (gt & ~31LL) / L >= cnt) break;
+    long long base;
+    const long long item = group_item(TREE ? L : 1, &base);
+    const long long per = (((long long)gridDim.x * blockDim.x) >> 5) * (32 / L);
+    for (long long b0 = 0; b0 + base < cnt; b0 += per) {
+      const long long it = b0 + item;
+      const bool valid = item >= 0 && it < cnt;
       const int s = rl[valid ? it : cnt - 1];
       if (!TREE) {
         if (valid)
@@ -1745,9 +1767,10 @@ k_refine_cl(const int *rl, const int *rl_n, const ClusterDev *cl, const ProbDev 
       const int maxitr = dv_itmax(C.bl_spdiam + p->pivmin, p->pivmin);
       double w = Wsh[s], e = Werr[s];
       int nc = 0;
-      dv_dlarrb_tree(L, B.nbl, P, ps, i, i == pidx, II > 1, rgap, lgap, tol.rtol1, tol.rtol2,
+      __syncwarp();
+      dv_dlarrb_tree(valid, L, B.nbl, P, ps, i, i == pidx, II > 1, rgap, lgap, tol.rtol1, tol.rtol2,
                      p->pivmin, maxitr, B.nbl, &w, &e, &nc);
-      if (valid && (gt % L) == 0) {
+      if (valid && (threadIdx.x & 31) % L == 0) {
         Wsh[s] = w;
         Werr[s] = e;
         work += (unsigned long long)nc * (unsigned long long)B.nbl;
@@ -2481,7 +2504,7 @@ k_sng_bisect(int out, const SngDev *sng, const ClusterDev *cl, const ProbDev *pr
     t0 = __shfl_sync(full, t0, 0);
     if (t0 >= nbs) break;
     const bool valid = t0 + gi < nbs;
-    const int idx = bsl[valid ? t0 + gi : t0];   // spare groups mirror a valid one
+    const int idx = bsl[valid ? t0 + gi : t0];   // spare groups: a valid one's pointers
     const SngDev S = sng[idx];
     const ClusterDev C = cl[S.cl];
     const BlockDev &B = blocks[C.blk];
@@ -2495,8 +2518,9 @@ k_sng_bisect(int out, const SngDev *sng, const ClusterDev *cl, const ProbDev *pr
     const int maxitr = dv_itmax(C.bl_spdiam + pivmin, pivmin);
     const int tw = (st.r < 1 || st.r > nb) ? nb : st.r;
     int nc = 0;
-    dv_dlarrb_tree(L, nb, P, ps, Windex[S.slot], 1, 0, 0.0, 0.0, 0.0, 2.0 * MR3_EPS, pivmin, maxitr,
-                   tw, &st.wsh, &st.werr, &nc);
+    __syncwarp();
+    dv_dlarrb_tree(valid, L, nb, P, ps, Windex[S.slot], 1, 0, 0.0, 0.0, 0.0, 2.0 * MR3_EPS, pivmin,
+                   maxitr, tw, &st.wsh, &st.werr, &nc);
     st.flags = (st.flags | SF_USEDBS) & ~SF_NEEDBS;
     st.lambda = st.wsh;
     st.r = 0;
@@ -2637,16 +2661,19 @@ k_sng_finish(int in, const SngDev *sng, const ClusterDev *cl, ProbDev *probs,
         }
         have = false;
       }
-    } else if (needbs) {
-      const int maxitr = dv_itmax(spd + pivmin, pivmin);
+    } else if (__any_sync(full, needbs)) {
+      const int maxitr = needbs ? dv_itmax(spd + pivmin, pivmin) : 0;
       const int tw = (st.r < 1 || st.r > nb) ? nb : st.r;
       int nc = 0;
-      dv_dlarrb_tree(L, nb, P, ps, wi, 1, 0, 0.0, 0.0, 0.0, 2.0 * MR3_EPS, pivmin, maxitr, tw,
-                     &st.wsh, &st.werr, &nc);
-      st.flags = (st.flags | SF_USEDBS) & ~SF_NEEDBS;
-      st.lambda = st.wsh;
-      st.r = 0;
-      if (t == 0) w_neg += (unsigned long long)nc * nb;
+      __syncwarp();
+      dv_dlarrb_tree(needbs, L, nb, P, ps, wi, 1, 0, 0.0, 0.0, 0.0, 2.0 * MR3_EPS, pivmin, maxitr,
+                     tw, &st.wsh, &st.werr, &nc);
+      if (needbs) {
+        st.flags = (st.flags | SF_USEDBS) & ~SF_NEEDBS;
+        st.lambda = st.wsh;
+        st.r = 0;
+        if (t == 0) w_neg += (unsigned long long)nc * nb;
+      }
     }
     __syncwarp();
     if (!BISECT && !__any_sync(full, have)) continue;   // all sent to the second list
@@ -3575,7 +3602,7 @@ extern "C" int mr3_cuda_solve_cb(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void
       LAUNCH(k_bisect_cont, gN128, 128, NN, c->probs, c->blocks, c->blk_of_row, c->TP, c->Wt,
              c->Et, c->It, c->bis_st, tol, stats);
     } else
-      LAUNCH(k_bisect, (int)(((long long)NN * Lb + 127) / 128), 128, NN, Lb, c->probs,
+      LAUNCH(k_bisect, group_blocks(NN, Lb), TREE_T, NN, Lb, c->probs,
              c->blocks, c->blk_of_row, c->TP, c->Wt, c->Et, c->It, tol, stats);
   }
   LAUNCH(k_compact, L, MR3_THREADS, c->probs, c->blocks, c->D, c->Wt, c->Et, c->It, c->W, c->Werr,
@@ -3589,7 +3616,7 @@ extern "C" int mr3_cuda_solve_cb(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void
       LAUNCH(k_refine_root<false>, gN128, 128, NN, 1, c->probs, c->blocks, c->iblk, c->RP, c->W,
              c->Werr, c->Wgap, tol, stats);
     else
-      LAUNCH(k_refine_root<true>, (int)(((long long)NN * Lr + 127) / 128), 128, NN, Lr, c->probs,
+      LAUNCH(k_refine_root<true>, group_blocks(NN, Lr), TREE_T, NN, Lr, c->probs,
              c->blocks, c->iblk, c->RP, c->W, c->Werr, c->Wgap, tol, stats);
   }
   if (tol.nthreads < (1 << 30))
@@ -3638,7 +3665,7 @@ extern "C" int mr3_cuda_solve_cb(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void
                  c->blocks, c->RP, c->RQ, c->arena[nxt], c->Wsh, c->Werr, c->Windex, c->Wt, c->Et,
                  tol, stats);
         else
-          LAUNCH(k_cl_ext<true>, (int)((2LL * ncl * Lx + 127) / 128), 128, ncl, Lx, c->cl[cur],
+          LAUNCH(k_cl_ext<true>, group_blocks(2LL * ncl, Lx), TREE_T, ncl, Lx, c->cl[cur],
                  c->probs, c->blocks, c->RP, c->RQ, c->arena[nxt], c->Wsh, c->Werr, c->Windex, c->Wt,
                  c->Et, tol, stats);
         // two lanes per cluster when the clusters leave lanes idle
@@ -3664,7 +3691,7 @@ extern "C" int mr3_cuda_solve_cb(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void
         LAUNCH(k_refine_cl<false>, gN128, 128, c->rl, c->rl_n, c->cl[cur], c->probs, c->blocks,
                c->arena[cur], c->Wsh, c->Werr, c->Wgap, c->Windex, c->cl_of_slot, c->lvl_of_slot,
                level, tol, c->nsm, tree_max, stats);
-        LAUNCH(k_refine_cl<true>, (int)(lanes / 128), 128, c->rl, c->rl_n, c->cl[cur], c->probs,
+        LAUNCH(k_refine_cl<true>, (int)(lanes / TREE_T), TREE_T, c->rl, c->rl_n, c->cl[cur], c->probs,
                c->blocks, c->arena[cur], c->Wsh, c->Werr, c->Wgap, c->Windex, c->cl_of_slot,
                c->lvl_of_slot, level, tol, c->nsm, tree_max, stats);
         LAUNCH(k_gaps_cl, gN, 256, NN, c->cl[cur], c->Wsh, c->Werr, c->Wgap, c->W, c->cl_of_slot,

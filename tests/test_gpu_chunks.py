@@ -27,7 +27,7 @@ def _matrix(kind, n):
     return D - 2.0, E
 
 
-@pytest.mark.parametrize("lanes", ["1", "4", "32"])
+@pytest.mark.parametrize("lanes", ["1", "3", "5", "10", "32"])
 @pytest.mark.parametrize("kind", ["uniform", "wilkinson", "121"])
 def test_sizes_around_the_chunks(kind, lanes, monkeypatch):
     monkeypatch.setenv("MR3_TREE_LANES", lanes)
