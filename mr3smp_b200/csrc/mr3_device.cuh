@@ -10,6 +10,8 @@
 #include <math.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #define MR3_EPS    2.220446049250313080847e-16   // dlamch('P') = DBL_EPSILON
 #define MR3_SAFMIN 2.225073858507201383090e-308  // dlamch('S') = DBL_MIN
 #define MR3_MAX_GROWTH   64.0                    // INCLUDE/mrrr.h MAX_GROWTH
@@ -116,6 +118,15 @@ static __device__ __forceinline__ double dv_rcp_seed(double b) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
   return y;
+}
+
+// Element i of an array whose elements lie `stride` bytes apart: one widening
+// multiply-add.  (A lane that sweeps alone is bound by the instructions it
+// issues; 64-bit index arithmetic was a third of them.)
+template <typename T>
+static __device__ __forceinline__ T &dv_at(T *p, int i, unsigned stride) {
+  using B = typename std::conditional<std::is_const<T>::value, const char, char>::type;
+  return *reinterpret_cast<T *>(reinterpret_cast<B *>(p) + (unsigned long long)(unsigned)i * stride);
 }
 
 // The high word of |x| shifted left by one: ordered as |x| is.
@@ -515,11 +526,12 @@ static __device__ __forceinline__ int dv_dlaneg_inl(int n, const double2 *__rest
     if (gamma < 0.0) negcnt++;
     return negcnt;
   }
+  const unsigned sb = 16u * ps;   // bytes from row to row
   if (r - 1 >= 1) {
     const int last = r - 1;
     double2 c[U];   // row j + u; a row read is replaced by the one U rows on
 #pragma unroll
-    for (int u = 0; u < U; u++) c[u] = P[(size_t)(d_imin(1 + u, last) - 1) * ps];
+    for (int u = 0; u < U; u++) c[u] = dv_at(P, d_imin(1 + u, last) - 1, sb);
     double y0 = dv_rcp_seed(c[0].x + t);
     for (int bj = 1; bj <= last; bj += blklen) {
       const int jend = d_imin(bj + blklen - 1, last);
@@ -538,7 +550,7 @@ static __device__ __forceinline__ int dv_dlaneg_inl(int n, const double2 *__rest
           y0 = dv_rcp_seed(c[(u + 1) % U].x + (qt * c[u].y - sigma));
           neg1 += dv_signbit(dplus);
           t = tmp * c[u].y - sigma;
-          c[u] = P[(size_t)(d_imin(j + U + u, last) - 1) * ps];
+          c[u] = dv_at(P, d_imin(j + U + u, last) - 1, sb);
         }
         if (qdiv_failed(k)) {
           t = t0;
@@ -581,7 +593,7 @@ static __device__ __forceinline__ int dv_dlaneg_inl(int n, const double2 *__rest
   if (n - 1 >= r) {
     double2 c[U];
 #pragma unroll
-    for (int u = 0; u < U; u++) c[u] = P[(size_t)(d_imax(n - 1 - u, r) - 1) * ps];
+    for (int u = 0; u < U; u++) c[u] = dv_at(P, d_imax(n - 1 - u, r) - 1, sb);
     double y0 = dv_rcp_seed(c[0].y + p);
     for (int bj = n - 1; bj >= r; bj -= blklen) {
       const int jend = d_imax(bj - blklen + 1, r);
@@ -600,7 +612,7 @@ static __device__ __forceinline__ int dv_dlaneg_inl(int n, const double2 *__rest
           y0 = dv_rcp_seed(c[(u + 1) % U].y + (qt * c[u].x - sigma));
           neg2 += dv_signbit(dminus);
           p = tmp * c[u].x - sigma;
-          c[u] = P[(size_t)(d_imax(j - U - u, r) - 1) * ps];
+          c[u] = dv_at(P, d_imax(j - U - u, r) - 1, sb);
         }
         if (qdiv_failed(k)) {
           p = p0;
@@ -2688,14 +2700,13 @@ static __device__ __noinline__ void dv_r1s_call(bool active, int L, int n, doubl
   double sr1 = 0.0;     // SI of row r1-1 (0 for r1 = 1)
   if (t < 2) {
     const int m = up ? r2 - 1 : n - r1;   // rows of this lane's sweep
-    const long long first = up ? 0 : 2LL * (n - 2) * ps, step = up ? 2LL * ps : -2LL * ps;
+    // step k stands at the 0-based row k (upward) or n - 2 - k (downward)
+    const int row0 = up ? 0 : n - 2, dir = up ? 1 : -1;
+    const unsigned sb = 16u * ps, ob = 8u * b.st;   // bytes from row to row
     const double *Pd = reinterpret_cast<const double *>(P), *Qd = reinterpret_cast<const double *>(Q);
-    const double *pd = Pd + first + (up ? 0 : 1);
-    const double *pa = up ? Qd + 1 : Pd + first;
-    const double *pc = Qd + first;
-    const long long ostep = up ? st : -st;
-    double *__restrict__ o1 = up ? b.LP + st : b.UM + (n - 1) * st;
-    double *__restrict__ o2 = up ? b.SI + st : b.PA + (n - 1) * st;
+    const double *pd = Pd + (up ? 0 : 1), *pa = up ? Qd + 1 : Pd, *pc = Qd;
+    double *__restrict__ o1 = (up ? b.LP : b.UM) + st;
+    double *__restrict__ o2 = (up ? b.SI : b.PA) + st;
     const double x_in = up ? 0.0 - lambda : Pd[2LL * (n - 1) * ps] - lambda;
     if (!up) b.PA[n * st] = x_in;
     double x = x_in, v = 0.0;
@@ -2704,27 +2715,31 @@ static __device__ __noinline__ void dv_r1s_call(bool active, int L, int n, doubl
     auto plain = [&](int upto) {
 #pragma unroll 1
       for (; k < upto; k++) {
-        const double c = pc[k * step];
-        const double den = pd[k * step] + x;
-        const double q = pa[k * step] / den;
+        const int row = row0 + dir * k;
+        const double c = dv_at(pc, row, sb);
+        const double den = dv_at(pd, row, sb) + x;
+        const double q = dv_at(pa, row, sb) / den;
         neg += (den < 0.0);
         v = x * q * (up ? c : 1.0);
         x = v - lambda;
-        o1[k * ostep] = q * (up ? 1.0 : c);
-        o2[k * ostep] = up ? v : x;
+        dv_at(o1, row, ob) = q * (up ? 1.0 : c);
+        dv_at(o2, row, ob) = up ? v : x;
       }
     };
     if (m >= U) {
       double cd[U], ca[U], cc[U], nd[U], na[U], nc[U];
 #pragma unroll
-      for (int u = 0; u < U; u++) { cd[u] = pd[u * step]; ca[u] = pa[u * step]; cc[u] = pc[u * step]; }
+      for (int u = 0; u < U; u++) {
+        const int row = row0 + dir * u;
+        cd[u] = dv_at(pd, row, sb); ca[u] = dv_at(pa, row, sb); cc[u] = dv_at(pc, row, sb);
+      }
       double y0 = dv_rcp_seed(cd[0] + x);
 #pragma unroll 1
       while (k + U <= m) {
 #pragma unroll
         for (int u = 0; u < U; u++) {
-          const long long e = d_imin(k + U + u, m - 1) * step;
-          nd[u] = pd[e]; na[u] = pa[e]; nc[u] = pc[e];
+          const int row = row0 + dir * d_imin(k + U + u, m - 1);
+          nd[u] = dv_at(pd, row, sb); na[u] = dv_at(pa, row, sb); nc[u] = dv_at(pc, row, sb);
         }
         const double x0 = x, v0 = v;
         const int neg0 = neg;
@@ -2739,8 +2754,9 @@ static __device__ __noinline__ void dv_r1s_call(bool active, int L, int n, doubl
           neg += dv_signbit(den);
           v = x * q * f;
           x = v - lambda;
-          o1[(k + u) * ostep] = q * (up ? 1.0 : cc[u]);
-          o2[(k + u) * ostep] = up ? v : x;
+          const int row = row0 + dir * (k + u);
+          dv_at(o1, row, ob) = q * (up ? 1.0 : cc[u]);
+          dv_at(o2, row, ob) = up ? v : x;
         }
         if (qdiv_failed(ck)) {
           x = x0;
@@ -2762,21 +2778,22 @@ static __device__ __noinline__ void dv_r1s_call(bool active, int L, int n, doubl
       x = x_in;
       v = 0.0;
       for (k = 0; k < m; k++) {
-        const double c = pc[k * step], a = pa[k * step];
-        double den = pd[k * step] + x;
+        const int row = row0 + dir * k;
+        const double c = dv_at(pc, row, sb), a = dv_at(pa, row, sb);
+        double den = dv_at(pd, row, sb) + x;
         if (fabs(den) < pivmin) den = -pivmin;
         const double q = a / den;
         neg += (den < 0.0);
         if (up) {
           v = x * q * c;
-          if (q == 0.0) v = Pd[2LL * k * ps + 1];
+          if (q == 0.0) v = P[(size_t)k * ps].y;
           x = v - lambda;
-          o1[k * ostep] = q;
-          o2[k * ostep] = v;
+          dv_at(o1, row, ob) = q;
+          dv_at(o2, row, ob) = v;
         } else {
-          o1[k * ostep] = c * q;
+          dv_at(o1, row, ob) = c * q;
           x = q == 0.0 ? a - lambda : x * q - lambda;
-          o2[k * ostep] = x;
+          dv_at(o2, row, ob) = x;
         }
       }
     }
@@ -2819,26 +2836,27 @@ static __device__ __noinline__ void dv_r1s_call(bool active, int L, int n, doubl
   double ztz = 1.0;
   if (t < 2) {
     const int m = up ? r - 1 : n - r;
-    const double *Qd = reinterpret_cast<const double *>(Q);
-    const long long zs = up ? -st : st, qs = up ? -2LL * ps : 2LL * ps;
     // step k: row i = r-1-k (upward, z(i) from z(i+1)), r+k (downward, z(i+1) from z(i))
-    const double *pm = up ? b.LP + (r - 1) * st : b.UM + r * st;
-    const double *pq = Qd + 2LL * ((up ? r - 2 : r - 1)) * ps + 1;
-    double *pz = b.ZV + (up ? r - 1 : r + 1) * st;
+    const int i0 = up ? r - 1 : r, dir = up ? -1 : 1;
+    const unsigned sb = 16u * ps, zb = 8u * b.st;
+    const double *pm = up ? b.LP : b.UM;                                  // at row i
+    const double *pq = reinterpret_cast<const double *>(Q) + 1;           // at row i - 1
+    double *pz = b.ZV + (up ? 0 : st);                                    // at row i
     if (up) b.ZV[r * st] = 1.0;
     double z = 1.0;
     int k = 0;
     if (slow) {
       double zp = 0.0;   // the value before z
       for (; k < m; k++) {
-        const double ldi = pq[k * qs];
+        const int i = i0 + dir * k;
+        const double ldi = dv_at(pq, i - 1, sb);
         double zn;
         // a zero z: the quotient of the off-diagonals beside it
-        if (z == 0.0) zn = -(pq[(k - 1) * qs] / ldi) * zp;
-        else zn = -(pm[k * zs] * z);
+        if (z == 0.0) zn = -(dv_at(pq, i - 1 - dir, sb) / ldi) * zp;
+        else zn = -(dv_at(pm, i, zb) * z);
         if ((fabs(zn) + fabs(z)) * fabs(ldi) < gaptol) { stop = up ? r - k : r + k; break; }
         ztz = ztz + zn * zn;
-        pz[k * zs] = zn;
+        dv_at(pz, i, zb) = zn;
         zp = z;
         z = zn;
       }
@@ -2846,16 +2864,20 @@ static __device__ __noinline__ void dv_r1s_call(bool active, int L, int n, doubl
       double cm[U], cq[U], nm[U], nq[U];
       if (m >= U) {
 #pragma unroll
-        for (int u = 0; u < U; u++) { cm[u] = pm[u * zs]; cq[u] = pq[u * qs]; }
+        for (int u = 0; u < U; u++) {
+          const int i = i0 + dir * u;
+          cm[u] = dv_at(pm, i, zb);
+          cq[u] = dv_at(pq, i - 1, sb);
+        }
       }
       bool go = true;
 #pragma unroll 1
       for (; go && k + U <= m; k += U) {
 #pragma unroll
         for (int u = 0; u < U; u++) {
-          const long long e = d_imin(k + U + u, m - 1);
-          nm[u] = pm[e * zs];
-          nq[u] = pq[e * qs];
+          const int i = i0 + dir * d_imin(k + U + u, m - 1);
+          nm[u] = dv_at(pm, i, zb);
+          nq[u] = dv_at(pq, i - 1, sb);
         }
         double zz[U], zl = z;
         unsigned cut = 0u;
@@ -2869,7 +2891,7 @@ static __device__ __noinline__ void dv_r1s_call(bool active, int L, int n, doubl
 #pragma unroll
           for (int u = 0; u < U; u++) {
             ztz = ztz + zz[u] * zz[u];
-            pz[(k + u) * zs] = zz[u];
+            dv_at(pz, i0 + dir * (k + u), zb) = zz[u];
           }
           z = zl;
         } else {
@@ -2878,7 +2900,7 @@ static __device__ __noinline__ void dv_r1s_call(bool active, int L, int n, doubl
           for (int u = 0; u < U; u++)
             if (u < w) {
               ztz = ztz + zz[u] * zz[u];
-              pz[(k + u) * zs] = zz[u];
+              dv_at(pz, i0 + dir * (k + u), zb) = zz[u];
             }
           stop = up ? r - (k + w) : r + (k + w);
           go = false;
@@ -2887,10 +2909,11 @@ static __device__ __noinline__ void dv_r1s_call(bool active, int L, int n, doubl
         for (int u = 0; u < U; u++) { cm[u] = nm[u]; cq[u] = nq[u]; }
       }
       for (; go && k < m; k++) {
-        const double zn = -(pm[k * zs] * z), ldi = pq[k * qs];
+        const int i = i0 + dir * k;
+        const double zn = -(dv_at(pm, i, zb) * z), ldi = dv_at(pq, i - 1, sb);
         if ((fabs(zn) + fabs(z)) * fabs(ldi) < gaptol) { stop = up ? r - k : r + k; break; }
         ztz = ztz + zn * zn;
-        pz[k * zs] = zn;
+        dv_at(pz, i, zb) = zn;
         z = zn;
       }
     }
@@ -2936,6 +2959,7 @@ static __device__ __forceinline__ double rrf_sweep(int n, const double2 *__restr
                                                    double *__restrict__ dp,
                                                    double *__restrict__ lp, int os, bool *sawnan) {
   constexpr int U = QDIV_U;
+  const unsigned sb = 16u * ps, ob = 8u * os;   // bytes from row to row
   double s = -sig;
   double d = P[0].x + s;
   if (fabs(d) < pivmin) { d = -pivmin; *sawnan = true; }
@@ -2950,15 +2974,15 @@ static __device__ __forceinline__ double rrf_sweep(int n, const double2 *__restr
     double cp[U], np_[U];
 #pragma unroll
     for (int u = 0; u < U; u++) {
-      cq[u] = Q[(size_t)u * ps];
-      cp[u] = P[(size_t)(u + 1) * ps].x;
+      cq[u] = dv_at(Q, u, sb);
+      cp[u] = dv_at(P, u + 1, sb).x;
     }
     for (; i0 + U - 1 <= last; i0 += U) {
 #pragma unroll
       for (int u = 0; u < U; u++) {
         const int i = d_imin(i0 + U + u, last);
-        nq[u] = Q[(size_t)i * ps];
-        np_[u] = P[(size_t)(i + 1) * ps].x;
+        nq[u] = dv_at(Q, i, sb);
+        np_[u] = dv_at(P, i + 1, sb).x;
       }
       const double s0 = s, d0 = d, mx0 = mx;
       unsigned dmin = 0xffffffffu;
@@ -2969,11 +2993,11 @@ static __device__ __forceinline__ double rrf_sweep(int n, const double2 *__restr
         double qt;
         const double l = dv_qdiv(cq[u].y, d, y0, &k, &qt);
         y0 = dv_rcp_seed(cp[u] + (s * qt * cq[u].x - sig));
-        lp[(size_t)(i0 + u) * os] = l;
+        dv_at(lp, i0 + u, ob) = l;
         s = s * l * cq[u].x - sig;
         d = cp[u] + s;
         dmin = min(dmin, dv_habs(d));
-        dp[(size_t)(i0 + u + 1) * os] = d;
+        dv_at(dp, i0 + u + 1, ob) = d;
         mx = fmax(mx, fabs(d));
       }
       if (qdiv_failed(k) || dmin <= hp) {
