@@ -163,26 +163,10 @@ static __device__ __forceinline__ double dv_qdiv(double a, double b, double y0, 
   return q;
 }
 
-// Sturm count of T - x, IJOB=1 rule of dlaebz (SRC/LAPACK/odebz.f:255-270).
-// tp[j] = (d[j], e2[j-1]); tp[0].y unused.  The threads of a warp count the
-// same matrix, so every load is a broadcast that L1 serves; the plain loop
-// is faster here than the chunked sweeps used for per-lane data.
-static __device__ __noinline__ int dv_count_ijob1(int n, const double2 *__restrict__ tp,
-                                           double pivmin, double x) {
-  double2 v = tp[0];
-  double tmp = v.x - x;
-  if (fabs(tmp) < pivmin) tmp = -pivmin;
-  int cnt = (tmp <= 0.0);
-  for (int j = 1; j < n; j++) {
-    v = tp[j];
-    tmp = v.x - v.y / tmp - x;
-    if (fabs(tmp) < pivmin) tmp = -pivmin;
-    cnt += (tmp <= 0.0);
-  }
-  return cnt;
-}
-
-// Sturm count, IJOB=2/3 rule of dlaebz's serial loop (odebz.f loop 90).
+// Sturm count of T - c, IJOB=2/3 rule of dlaebz's serial loop (odebz.f loop
+// 90).  tp[j] = (d[j], e2[j-1]); tp[0].y unused.  The threads of a warp count
+// the same matrix, so every load is a broadcast that L1 serves; where they
+// fill the SM the plain loop is as fast as the checked chunks below.
 static __device__ __forceinline__ int dv_count_bisect(int n, const double2 *__restrict__ tp,
                                                double pivmin, double c) {
   double2 v = tp[0];
@@ -197,20 +181,44 @@ static __device__ __forceinline__ int dv_count_bisect(int n, const double2 *__re
   return cnt;
 }
 
-// dv_count_bisect for the launches that wait for the chain (a lane group
-// per interval): quotients by dv_qdiv, rows in checked chunks loaded one
-// chunk ahead.  The clamp at pivmin, 34 cycles of compare and select in the
-// chain, becomes part of the chunk's check: a pivot above pivmin in
-// magnitude is not changed by it, and its sign bit is its count.
-static __device__ __noinline__ int dv_count_bisect_lat(int n, const double2 *__restrict__ tp,
-                                                double pivmin, double c) {
+// Sturm counts of T - c for the launches that wait for the chain (a lane or a
+// lane group per interval): quotients by dv_qdiv, rows in checked chunks.
+// The clamp at pivmin, 34 cycles of compare and select in the chain, becomes
+// part of the chunk's check: a pivot above pivmin in magnitude is not changed
+// by it, and its sign bit is its count.  RULE: how a row forms, clamps and
+// counts its pivot.
+//   CNT_BISECT  dlaebz IJOB 2/3 (odebz.f loop 90): dv_count_bisect
+//   CNT_IJOB1   dlaebz IJOB 1 (odebz.f:255-270)
+//   CNT_LARRC   dlarrc 'T' (odrrc.f): (d - c) - q, pivots <= 0, no clamp
+//   CNT_LARRJ   dlarrj (odrrj.f): (d - c) - q, pivots < 0, no clamp
+enum { CNT_BISECT, CNT_IJOB1, CNT_LARRC, CNT_LARRJ };
+
+template <int RULE>
+static __device__ __forceinline__ double dv_pivot(double d, double q, double c) {
+  return RULE == CNT_BISECT || RULE == CNT_IJOB1 ? d - q - c : d - c - q;
+}
+
+template <int RULE>
+static __device__ __forceinline__ void dv_count_row(double *t, int *cnt, double pivmin) {
+  if (RULE == CNT_BISECT) {
+    if (*t <= pivmin) { (*cnt)++; *t = fmin(*t, -pivmin); }
+  } else {
+    if (RULE == CNT_IJOB1 && fabs(*t) < pivmin) *t = -pivmin;
+    *cnt += RULE == CNT_LARRJ ? *t < 0.0 : *t <= 0.0;
+  }
+}
+
+template <int RULE>
+static __device__ __noinline__ int dv_count_lat(int n, const double2 *__restrict__ tp, double pivmin,
+                                         double c) {
   constexpr int U = QDIV_U;
+  constexpr bool CLAMP = RULE == CNT_BISECT || RULE == CNT_IJOB1;
   double t = tp[0].x - c;
   int cnt = 0;
-  if (t <= pivmin) { cnt = 1; t = fmin(t, -pivmin); }
+  dv_count_row<RULE>(&t, &cnt, pivmin);
   int j = 1;
   if (n > U) {
-    const unsigned hp = dv_habs(pivmin);
+    const unsigned hp = CLAMP ? dv_habs(pivmin) : 0u;
     double y0 = dv_rcp_seed(t);
     double2 v[U];   // row j + u; a row read is replaced by the one U rows on
 #pragma unroll
@@ -225,8 +233,8 @@ static __device__ __noinline__ int dv_count_bisect_lat(int n, const double2 *__r
       for (int u = 0; u < U; u++) {
         double qt;
         const double q = dv_qdiv(v[u].y, t, y0, &k, &qt);
-        y0 = dv_rcp_seed(v[u].x - qt - c);
-        t = v[u].x - q - c;
+        y0 = dv_rcp_seed(dv_pivot<RULE>(v[u].x, qt, c));
+        t = dv_pivot<RULE>(v[u].x, q, c);
         cnt += dv_signbit(t);
         tmin = min(tmin, dv_habs(t));
         v[u] = tp[d_imin(j + U + u, n - 1)];
@@ -237,8 +245,8 @@ static __device__ __noinline__ int dv_count_bisect_lat(int n, const double2 *__r
 #pragma unroll 1
         for (int u = 0; u < U; u++) {
           const double2 w = tp[j + u];
-          t = w.x - w.y / t - c;
-          if (t <= pivmin) { cnt++; t = fmin(t, -pivmin); }
+          t = dv_pivot<RULE>(w.x, w.y / t, c);
+          dv_count_row<RULE>(&t, &cnt, pivmin);
         }
         y0 = dv_rcp_seed(t);
       }
@@ -246,8 +254,8 @@ static __device__ __noinline__ int dv_count_bisect_lat(int n, const double2 *__r
   }
   for (; j < n; j++) {
     const double2 w = tp[j];
-    t = w.x - w.y / t - c;
-    if (t <= pivmin) { cnt++; t = fmin(t, -pivmin); }
+    t = dv_pivot<RULE>(w.x, w.y / t, c);
+    dv_count_row<RULE>(&t, &cnt, pivmin);
   }
   return cnt;
 }
@@ -341,7 +349,7 @@ static __device__ __noinline__ void dv_ijob3_tree(int L, int n, const double2 *_
   int na = *na_, nb = *nb_, it = 0;
   bool done = nitmax < 1;
   if (!done) {   // the first step, at the given point
-    const int cnt = dv_count_bisect_lat(n, tp, pivmin, c);
+    const int cnt = dv_count_lat<CNT_BISECT>(n, tp, pivmin, c);
     if (cnt <= nval) { a = c; na = cnt; }
     if (cnt >= nval) { b = c; nb = cnt; }
     it = 1;
@@ -354,7 +362,7 @@ static __device__ __noinline__ void dv_ijob3_tree(int L, int n, const double2 *_
       const double m = 0.5 * (l + r);
       if ((node_t >> k) & 1) l = m; else r = m;
     }
-    const int raw = dv_count_bisect_lat(n, tp, pivmin, 0.5 * (l + r));
+    const int raw = dv_count_lat<CNT_BISECT>(n, tp, pivmin, 0.5 * (l + r));
     int node = 1;
     for (int d = 0; d < depth; d++) {
       const int cv = __shfl_sync(gm, raw, g0 + node);
@@ -432,7 +440,7 @@ static __device__ __noinline__ void dv_bisect_tree(int L, int n, const double2 *
       }
       const double x = 0.5 * (l + r);
       const int raw = pass == 0 ? dv_count_guess(n, tp, pivmin, x)
-                                : dv_count_bisect_lat(n, tp, pivmin, x);
+                                : dv_count_lat<CNT_BISECT>(n, tp, pivmin, x);
       for (int node = 1; node <= L && !done;) {
         const int cv = __shfl_sync(gm, raw, g0 + node - 1);
         const double c = 0.5 * (a + b);
@@ -444,7 +452,7 @@ static __device__ __noinline__ void dv_bisect_tree(int L, int n, const double2 *
       }
     }
     if (pass == 1) { it += 2; break; }
-    const int cv = t < 2 ? dv_count_bisect_lat(n, tp, pivmin, t == 0 ? a : b) : 0;
+    const int cv = t < 2 ? dv_count_lat<CNT_BISECT>(n, tp, pivmin, t == 0 ? a : b) : 0;
     const int ca = __shfl_sync(gm, cv, g0), cb = __shfl_sync(gm, cv, g0 + 1);
     it = 2;
     if (ca < j && cb >= j) break;
@@ -738,6 +746,10 @@ static __device__ __noinline__ int dv_dlarrb_one(int n, const double2 *__restric
 // bisect.  (With a loop per group, groups once apart never met again and
 // counted one after the other: twice the time for the slowest warps of
 // k_refine_cl on the n = 20010 problem.)
+// LARRJ: dlarrj (SRC/LAPACK/odrrj.f:100-281) on T's rows (d, e2) instead: its
+// count, one relative tolerance (rtol1) and no test between widening and
+// bisection; gaps, rtol2 and r are not used.
+template <bool LARRJ>
 static __device__ __forceinline__ void dv_dlarrb_tree(bool act, int L, int n,
                                             const double2 *__restrict__ R, int ps, int i, int first,
                                             int has_left, double rgap_own, double lgap_in,
@@ -758,6 +770,7 @@ static __device__ __forceinline__ void dv_dlarrb_tree(bool act, int L, int n,
   double xs0 = 0.0, xs1 = 0.0, bs0 = 0.0, bs1 = 0.0;
   int steps0 = 0, steps1 = 0;
   int phase = act ? ENDS : DONE, iter = 0, nc = 0;
+  if (LARRJ && act && right - *w < rtol1 * fmax(fabs(left), fabs(right))) phase = DONE;
   while (__any_sync(0xffffffffu, phase != DONE)) {
     // this lane's point: an end, a candidate end or a tree node
     double x = 0.0, back = 0.0;
@@ -779,7 +792,7 @@ static __device__ __forceinline__ void dv_dlarrb_tree(bool act, int L, int n,
       x = 0.5 * (l + rr);
     }
     int cnt = 0;
-    if (mine) cnt = dv_dlaneg_inl<QDIV_U>(n, R, ps, x, r);
+    if (mine) cnt = LARRJ ? dv_count_lat<CNT_LARRJ>(n, R, 0.0, x) : dv_dlaneg_inl<QDIV_U>(n, R, ps, x, r);
     __syncwarp();
     if (phase != DONE) {
       int shift = -1, known = L;      // lane of node v: v + shift; nodes counted
@@ -830,7 +843,9 @@ static __device__ __forceinline__ void dv_dlarrb_tree(bool act, int L, int n,
           known = 0;
         }
       }
-      if (start) {
+      if (start && LARRJ) {
+        phase = TREE;
+      } else if (start) {
         const double gap = fmin(first ? rgap_own : lgap_in, rgap_own);
         const double width = 0.5 * fabs(left - right), tmp = fmax(fabs(left), fabs(right));
         // converged early: W, WERR kept
@@ -841,7 +856,9 @@ static __device__ __forceinline__ void dv_dlarrb_tree(bool act, int L, int n,
         for (int node = 1;;) {
           const double mid = 0.5 * (left + right);
           const double width = right - mid, tmp = fmax(fabs(left), fabs(right));
-          if (width <= fmax(rtol1 * gap, rtol2 * tmp) || width <= mnwdth || iter == maxitr) {
+          const bool small = LARRJ ? width < rtol1 * tmp
+                                   : width <= fmax(rtol1 * gap, rtol2 * tmp) || width <= mnwdth;
+          if (small || iter == maxitr) {
             *w = mid;
             *werr = right - mid;
             phase = DONE;
@@ -3189,44 +3206,70 @@ static __device__ __noinline__ double dv_dlarrf(int n, const double2 *__restrict
   return sigma;
 }
 
-// One interval of dlarrj (SRC/LAPACK/odrrj.f:100-281): bisection on T to
-// relative tolerance rtol.  Intervals are independent (no gaps involved).
-// tp[j] = (d[j], e2[j-1]) of the unshifted matrix.
-static __device__ __forceinline__ int dv_count_rrj(int n, const double2 *__restrict__ tp, double s) {
-  double dplus = tp[0].x - s;
-  int cnt = (dplus < 0.0);
-  for (int j = 1; j < n; j++) {
-    const double2 v = tp[j];
-    dplus = v.x - s - v.y / dplus;
-    cnt += (dplus < 0.0);
+// The factorisation T - sigma I = L D L^T of compute_root_rrr's tries
+// (SRC/mrrr_val.c:838-870): dpiv_{j+1} = (D(j+1) - sigma) - E(j) (E(j) / dpiv_j),
+// the quotient as E(j) times 1 / dpiv_j, in checked chunks.  Every lane of a
+// warp may run a shift of its own on the same rows.  Lanes with `write` store
+// D and L; returns max |dpiv|, *bad: some sgn * dpiv < 0.
+static __device__ __noinline__ double dv_root_try(int n, const double *__restrict__ D,
+                                           const double *__restrict__ E, double sigma, int sgn,
+                                           bool write, double *__restrict__ Dt,
+                                           double *__restrict__ Lt, bool *bad) {
+  constexpr int U = QDIV_U;
+  double d = D[0] - sigma, dmax = fabs(d);
+  bool neg = sgn * d < 0.0;
+  if (write) Dt[0] = d;
+  int j = 0;   // rows j = 0..n-2 produce L(j), D(j+1)
+  const int last = n - 2;
+  auto plain = [&](int upto) {
+#pragma unroll 1
+    for (; j < upto; j++) {
+      const double ej = E[j];
+      const double inv = 1.0 / d;
+      const double t0 = ej * inv;
+      d = (D[j + 1] - sigma) - t0 * ej;
+      if (write) { Lt[j] = t0; Dt[j + 1] = d; }
+      dmax = fmax(dmax, fabs(d));
+      neg = neg || sgn * d < 0.0;
+    }
+  };
+  if (last + 1 >= U) {
+    double cd[U], ce[U];   // D(j + u + 1), E(j + u)
+#pragma unroll
+    for (int u = 0; u < U; u++) { cd[u] = D[u + 1]; ce[u] = E[u]; }
+    double y0 = dv_rcp_seed(d);
+#pragma unroll 1
+    while (j + U - 1 <= last) {
+      const double d0 = d, m0 = dmax;
+      const bool n0 = neg;
+      qdiv_chk k;
+      qdiv_begin(&k);
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        double qt;
+        const double inv = dv_qdiv(1.0, d, y0, &k, &qt);
+        y0 = dv_rcp_seed((cd[u] - sigma) - ce[u] * qt * ce[u]);
+        const double t0 = ce[u] * inv;
+        d = (cd[u] - sigma) - t0 * ce[u];
+        if (write) { Lt[j + u] = t0; Dt[j + u + 1] = d; }
+        dmax = fmax(dmax, fabs(d));
+        neg = neg || sgn * d < 0.0;
+        const int i = d_imin(j + U + u, last);
+        cd[u] = D[i + 1];
+        ce[u] = E[i];
+      }
+      if (qdiv_failed(k)) {
+        d = d0;
+        dmax = m0;
+        neg = n0;
+        plain(j + U);
+        y0 = dv_rcp_seed(d);
+      } else {
+        j += U;
+      }
+    }
   }
-  return cnt;
-}
-
-static __device__ __noinline__ void dv_dlarrj_one(int n, const double2 *__restrict__ tp, int i,
-                                           double rtol, int maxitr, double *w, double *werr) {
-  double left = *w - *werr, mid = *w, right = *w + *werr;
-  double width = right - mid;
-  double tmp = fmax(fabs(left), fabs(right));
-  if (width < rtol * tmp) return;
-  double fac = 1.0;
-  for (int cap = 0; cap < MR3_EXPAND_CAP; cap++) {
-    if (dv_count_rrj(n, tp, left) > i - 1) { left = left - *werr * fac; fac = 2.0 * fac; }
-    else break;
-  }
-  fac = 1.0;
-  for (int cap = 0; cap < MR3_EXPAND_CAP; cap++) {
-    if (dv_count_rrj(n, tp, right) < i) { right = right + *werr * fac; fac = 2.0 * fac; }
-    else break;
-  }
-  for (int iter = 0; iter <= maxitr; iter++) {
-    mid = 0.5 * (left + right);
-    width = right - mid;
-    tmp = fmax(fabs(left), fabs(right));
-    if (width < rtol * tmp || iter == maxitr) break;
-    int cnt = dv_count_rrj(n, tp, mid);
-    if (cnt <= i - 1) left = mid; else right = mid;
-  }
-  *w = 0.5 * (left + right);
-  *werr = right - *w;
+  plain(last + 1);
+  *bad = neg;
+  return dmax;
 }

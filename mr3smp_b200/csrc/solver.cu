@@ -431,8 +431,10 @@ k_prologue(ProbDev *probs, BlockDev *blocks, int *blk_of_row, double *D, double 
   if (irange == MR3_RANGE_A) {
     if (tid == 0) { p->il_out = 1; p->iu_out = n; }
   } else if (irange == MR3_RANGE_V) {
-    if (tid == 0) p->il_out = dv_count_ijob1(n, TP + off, pivmin, p->vl) + 1;
-    if (tid == 32) p->iu_out = dv_count_ijob1(n, TP + off, pivmin, p->vu);
+    if (tid < 2) {   // lanes 0 and 1 count at vl and vu
+      const int c = dv_count_lat<CNT_IJOB1>(n, TP + off, pivmin, tid == 0 ? p->vl : p->vu);
+      if (tid == 0) p->il_out = c + 1; else p->iu_out = c;
+    }
   } else {
     if (tid == 0) { p->il_out = p->il; p->iu_out = p->iu; }
   }
@@ -506,9 +508,9 @@ k_blocks(ProbDev *probs, BlockDev *blocks, const double *D, double *E, const dou
     int ilow = 1, iupp = nbl;
     if (irange != MR3_RANGE_A) {
       int c = 0;
-      if (lane == 0) c = dv_count_ijob1(nbl, TP + ibgn, pivmin, fmax(wl, bglf)) + 1;
-      if (lane == 1) c = dv_count_ijob1(nbl, TP + ibgn, pivmin, fmin(wu, bguf));
-      ilow = __shfl_sync(0xffffffffu, c, 0);
+      if (lane < 2)
+        c = dv_count_lat<CNT_IJOB1>(nbl, TP + ibgn, pivmin, lane == 0 ? fmax(wl, bglf) : fmin(wu, bguf));
+      ilow = __shfl_sync(0xffffffffu, c, 0) + 1;
       iupp = __shfl_sync(0xffffffffu, c, 1);
     }
     const int mbl = iupp - ilow + 1;
@@ -532,13 +534,9 @@ k_blocks(ProbDev *probs, BlockDev *blocks, const double *D, double *E, const dou
       int itmax = dv_itmax(tnb + pivmin, pivmin);
       double a = gl2, bq = gu2;
       int na = -1, nb = nbl + 1;
-      // the two searches by half-warps, each with the tree form
-      if (lane < 16)
-        dv_ijob3_tree(16, nbl, TP + ibgn, pivmin, atoli, tol.bsrtol, itmax, ilow - 1, gl2, &a, &bq,
-                      &na, &nb);
-      else
-        dv_ijob3_tree(16, nbl, TP + ibgn, pivmin, atoli, tol.bsrtol, itmax, iupp, gu2, &a, &bq,
-                      &na, &nb);
+      // the two searches by half-warps at once, each with the tree form
+      dv_ijob3_tree(16, nbl, TP + ibgn, pivmin, atoli, tol.bsrtol, itmax,
+                    lane < 16 ? ilow - 1 : iupp, lane < 16 ? gl2 : gu2, &a, &bq, &na, &nb);
       double a0 = __shfl_sync(0xffffffffu, a, 0), b0 = __shfl_sync(0xffffffffu, bq, 0);
       double a1 = __shfl_sync(0xffffffffu, a, 16), b1 = __shfl_sync(0xffffffffu, bq, 16);
       int nwl = __shfl_sync(0xffffffffu, na, 0), nwu = __shfl_sync(0xffffffffu, nb, 16);
@@ -559,8 +557,7 @@ k_blocks(ProbDev *probs, BlockDev *blocks, const double *D, double *E, const dou
     int nab1 = 0, nab2 = 0;
     if (!none) {
       int c = 0;
-      if (lane == 0) c = dv_count_ijob1(nbl, TP + ibgn, pivmin, gl3);
-      if (lane == 1) c = dv_count_ijob1(nbl, TP + ibgn, pivmin, gu3);
+      if (lane < 2) c = dv_count_lat<CNT_IJOB1>(nbl, TP + ibgn, pivmin, lane == 0 ? gl3 : gu3);
       nab1 = __shfl_sync(0xffffffffu, c, 0);
       nab2 = __shfl_sync(0xffffffffu, c, 1);
       nwlb = nab1; nwub = nab2;
@@ -948,7 +945,7 @@ __global__ void k_gaps_init(int N, const ProbDev *probs, const BlockDev *blocks,
 // ------------------------------------------------------------------------
 // Stage A4: root representation L D L^T = T - sigma I of each block
 // (compute_root_rrr, bisection branch, SRC/mrrr_val.c:717-948).
-// One warp per block; the factorisation tries are serial on lane 0.
+// One warp per block.
 // ------------------------------------------------------------------------
 __global__ void __launch_bounds__(MR3_THREADS)
 k_root(ProbDev *probs, BlockDev *blocks, double *D, double *E, const double2 *TP, double *Dt,
@@ -989,83 +986,68 @@ k_root(ProbDev *probs, BlockDev *blocks, double *D, double *E, const double2 *TP
       s2 = fmin(isright, vup) - 0.25 * tmp0;
     }
     int cnt = 0;
-    if (mbl > 1 && lane < 2) {   // dlarrc('T'): lane 0 counts at s1, lane 1 at s2
-      const double x = (lane == 0) ? s1 : s2;
-      const double2 *tp = TP + ibgn;
-      double piv = tp[0].x - x;
-      cnt = (piv <= 0.0);
-      for (int i = 0; i < nbl - 1; i++) {
-        double ee = E[ibgn + i];
-        double t = ee * ee;
-        piv = (tp[i + 1].x - x) - t / piv;
-        cnt += (piv <= 0.0);
+    if (mbl > 1 && lane < 2)   // dlarrc('T'): lane 0 counts at s1, lane 1 at s2
+      cnt = dv_count_lat<CNT_LARRC>(nbl, TP + ibgn, 0.0, lane == 0 ? s1 : s2);
+    int lcnt = __shfl_sync(0xffffffffu, cnt, 0), rcnt = __shfl_sync(0xffffffffu, cnt, 1);
+    double sigma;
+    int sgndef;
+    if (mbl == 1) { sigma = gl; sgndef = 1; }
+    else if ((lcnt - B->ilow) >= (B->iupp - rcnt)) {
+      sigma = allno ? fmax(isleft, gl) : (dqds ? isleft : fmax(isleft, vlp));
+      sgndef = 1;
+    } else {
+      sigma = allno ? fmin(isright, gu) : (dqds ? isright : fmin(isright, vup));
+      sgndef = -1;
+    }
+    double tau;
+    if (dqds) {
+      tau = spdiam * MR3_EPS * nbl + 2.0 * pivmin;
+      tau = fmax(tau, 2 * MR3_EPS * fabs(sigma));
+    } else if (mbl > 1) {
+      double clwdth = W[wend] + Werr[wend] - W[wbgn] - Werr[wbgn];
+      double avgap = fabs(clwdth / (double)(wend - wbgn));
+      if (sgndef > 0) { tau = fmax(Wgap[wbgn], avgap); tau *= 0.5; tau = fmax(tau, Werr[wbgn]); }
+      else { tau = fmax(Wgap[wend - 1], avgap); tau *= 0.5; tau = fmax(tau, Werr[wend]); }
+    } else {
+      tau = Werr[wbgn];
+    }
+    // The shifts of the MAX_TRY_ROOT tries follow from the first one, so lane
+    // k factors at the k-th shift and all tries cost one sweep; the first
+    // lane whose factors are a representation has the sequential loop's
+    // shift.  Lane 0 stores its factors as it goes; a later lane's are
+    // computed once more for the store.
+    for (int jtry = 0; jtry < lane && jtry < MR3_MAX_TRY_ROOT - 1; jtry++) {
+      if (jtry == MR3_MAX_TRY_ROOT - 2) {
+        if (sgndef == 1) sigma = gl - 2.0 * spdiam * MR3_EPS * nbl - 2.0 * 2.0 * pivmin;
+        else sigma = gu + 2.0 * spdiam * MR3_EPS * nbl + 2.0 * 2.0 * pivmin;
+      } else {
+        sigma -= sgndef * tau;
+        tau *= 2.0;
       }
     }
-    int lcnt = __shfl_sync(0xffffffffu, cnt, 0), rcnt = __shfl_sync(0xffffffffu, cnt, 1);
-    int ok = 1;
-    double sigma = 0.0;
+    bool rep = false;
+    if (lane < MR3_MAX_TRY_ROOT) {
+      bool bad;
+      const double dmax = dv_root_try(nbl, D + ibgn, E + ibgn, sigma, sgndef, lane == 0, Dt + ibgn,
+                                      Lt + ibgn, &bad);
+      // dqds needs a definite representation
+      rep = !(dmax > MR3_MAX_GROWTH * spdiam) && !(dqds && bad);
+    }
+    const unsigned reps = __ballot_sync(0xffffffffu, rep);
+    const int first = reps ? __ffs(reps) - 1 : MR3_MAX_TRY_ROOT - 1;
+    sigma = __shfl_sync(0xffffffffu, sigma, first);
     if (lane == 0) {
-      int sgndef;
-      if (mbl == 1) { sigma = gl; sgndef = 1; }
-      else if ((lcnt - B->ilow) >= (B->iupp - rcnt)) {
-        sigma = allno ? fmax(isleft, gl) : (dqds ? isleft : fmax(isleft, vlp));
-        sgndef = 1;
-      } else {
-        sigma = allno ? fmin(isright, gu) : (dqds ? isright : fmin(isright, vup));
-        sgndef = -1;
-      }
-      double tau;
-      if (dqds) {
-        tau = spdiam * MR3_EPS * nbl + 2.0 * pivmin;
-        tau = fmax(tau, 2 * MR3_EPS * fabs(sigma));
-      } else if (mbl > 1) {
-        double clwdth = W[wend] + Werr[wend] - W[wbgn] - Werr[wbgn];
-        double avgap = fabs(clwdth / (double)(wend - wbgn));
-        if (sgndef > 0) { tau = fmax(Wgap[wbgn], avgap); tau *= 0.5; tau = fmax(tau, Werr[wbgn]); }
-        else { tau = fmax(Wgap[wend - 1], avgap); tau *= 0.5; tau = fmax(tau, Werr[wend]); }
-      } else {
-        tau = Werr[wbgn];
-      }
-      ok = 0;
-      for (int jtry = 0; jtry < MR3_MAX_TRY_ROOT; jtry++) {
-        double dpiv = D[ibgn] - sigma;
-        Dt[ibgn] = dpiv;
-        double dmax = fabs(dpiv);
-        for (int i = 0; i < nbl - 1; i++) {
-          int j = ibgn + i;
-          double ej = E[j];
-          double inv = 1.0 / dpiv;
-          double t0 = ej * inv;
-          Lt[j] = t0;
-          dpiv = (D[j + 1] - sigma) - t0 * ej;
-          Dt[j + 1] = dpiv;
-          dmax = fmax(dmax, fabs(dpiv));
-        }
-        bool norep = dmax > MR3_MAX_GROWTH * spdiam;
-        if (dqds && !norep)   // dqds needs a definite representation
-          for (int i = 0; i < nbl; i++)
-            if (sgndef * Dt[ibgn + i] < 0.0) norep = true;
-        if (!norep) { ok = 1; break; }
-        if (jtry == MR3_MAX_TRY_ROOT - 2) {
-          if (sgndef == 1) sigma = gl - 2.0 * spdiam * MR3_EPS * nbl - 2.0 * 2.0 * pivmin;
-          else sigma = gu + 2.0 * spdiam * MR3_EPS * nbl + 2.0 * 2.0 * pivmin;
-        } else if (jtry == MR3_MAX_TRY_ROOT - 1) {
-          break;
-        } else {
-          sigma -= sgndef * tau;
-          tau *= 2.0;
-        }
-      }
-      if (!ok) set_status(p, MR3_EMISC);
+      bool bad;
+      if (first != 0)
+        dv_root_try(nbl, D + ibgn, E + ibgn, sigma, sgndef, true, Dt + ibgn, Lt + ibgn, &bad);
+      if (!reps) set_status(p, MR3_EMISC);
       B->sigma = sigma;
       B->spdiam = spdiam;
       B->dqds = dqds;
       B->sgndef = sgndef;
     }
-    ok = __shfl_sync(0xffffffffu, ok, 0);
-    sigma = __shfl_sync(0xffffffffu, sigma, 0);
     __syncwarp();
-    if (!ok) continue;
+    if (!reps) continue;
     // store the root, perturb it by 8*eps relative noise from dlarnv(2) with
     // seed (1,1,1,1) (SRC/mrrr_val.c:927-941), and pack its rows
     const unsigned long long seed = (1ULL << 36) | (1ULL << 24) | (1ULL << 12) | 1ULL;
@@ -1158,7 +1140,7 @@ k_refine_root(int N, int L, const ProbDev *probs, const BlockDev *blocks, const 
     }
     const int nb = act ? B->nbl : 0;
     __syncwarp();
-    dv_dlarrb_tree(act, L, nb, act ? RP + B->ibgn : RP, 1, i, II == 1, II > 1, rgap, lgap, rtol1,
+    dv_dlarrb_tree<false>(act, L, nb, act ? RP + B->ibgn : RP, 1, i, II == 1, II > 1, rgap, lgap, rtol1,
                    rtol2, pivmin, maxitr, nb, &w, &werr, &nc);
     if (act && (threadIdx.x & 31) % L == 0) {
       W[s] = w;
@@ -1307,23 +1289,37 @@ __global__ void k_shift_w(int N, const ProbDev *probs, const BlockDev *blocks, c
   W[s] += E[B->iend];
 }
 
-// refine_to_highrac (SRC/mrrr.c:452-520): dlarrj on the scaled input T,
-// one thread per eigenvalue.
-__global__ void k_highrac(int N, const ProbDev *probs, const BlockDev *blocks, const int *iblk,
-                          const int *Windex, const double2 *TPc, double *W, double *Werr) {
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= N || iblk[s] < 0) return;
-  const BlockDev *B = &blocks[iblk[s]];
-  const ProbDev *p = &probs[B->prob];
-  if (p->status || !p->tryrac_out || p->jobz == MR3_JOB_C) return;
-  // ilow = smallest local index of the block's values; values are stored in
-  // increasing local index, so it is the index of the first one.
-  const int i = Windex[B->wbgn] + (s - B->wbgn);
-  const int maxitr = dv_itmax(p->spdiam + p->pivmin, p->pivmin);
-  double w = W[s], we = Werr[s];
-  dv_dlarrj_one(B->nbl, TPc + B->ibgn, i, 4.0 * MR3_EPS, maxitr, &w, &we);
-  W[s] = w;
-  Werr[s] = we;
+// refine_to_highrac (SRC/mrrr.c:452-520): dlarrj on the scaled input T, L
+// lanes per eigenvalue (tree_lanes; one by one the n = 1500 graded matrix took
+// 6.2 ms, 20 counts of 300 cycles a row each).
+__global__ void LB_TREE
+k_highrac(int N, int L, const ProbDev *probs, const BlockDev *blocks, const int *iblk,
+          const int *Windex, const double2 *TPc, double *W, double *Werr) {
+  long long base;
+  const long long item = group_item(L, &base);
+  if (base >= N) return;
+  const int s = (int)item;
+  const BlockDev *B = item >= 0 && item < N && iblk[s] >= 0 ? &blocks[iblk[s]] : nullptr;
+  const ProbDev *p = B ? &probs[B->prob] : nullptr;
+  const bool act = B && !p->status && p->tryrac_out && p->jobz != MR3_JOB_C;
+  int i = 0, maxitr = 0, n = 0, nc = 0;
+  double w = 0.0, we = 0.0;
+  if (act) {
+    // ilow = smallest local index of the block's values; values are stored in
+    // increasing local index, so it is the index of the first one.
+    i = Windex[B->wbgn] + (s - B->wbgn);
+    maxitr = dv_itmax(p->spdiam + p->pivmin, p->pivmin);
+    n = B->nbl;
+    w = W[s];
+    we = Werr[s];
+  }
+  __syncwarp();
+  dv_dlarrb_tree<true>(act, L, n, act ? TPc + B->ibgn : TPc, 1, i, 0, 0, 0.0, 0.0, 4.0 * MR3_EPS, 0.0,
+                       0.0, maxitr, 0, &w, &we, &nc);
+  if (act && (threadIdx.x & 31) % L == 0) {
+    W[s] = w;
+    Werr[s] = we;
+  }
 }
 
 __global__ void k_invscale(int N, const ProbDev *probs, const BlockDev *blocks, const int *iblk,
@@ -1559,7 +1555,7 @@ k_cl_ext(int ncl, int L, const ClusterDev *cl, const ProbDev *probs, const Block
                              maxitr, nb, &wv, &ev, &nc);
     } else {
       __syncwarp();
-      dv_dlarrb_tree(valid, L, nb, Pp, ps, i, 1, II > 1, 0.0, 0.0, tol.rqtol, tol.rqtol, p->pivmin,
+      dv_dlarrb_tree<false>(valid, L, nb, Pp, ps, i, 1, II > 1, 0.0, 0.0, tol.rqtol, tol.rqtol, p->pivmin,
                      maxitr, nb, &wv, &ev, &nc);
     }
     if (valid && (threadIdx.x & 31) % L == 0) {
@@ -1768,7 +1764,7 @@ k_refine_cl(const int *rl, const int *rl_n, const ClusterDev *cl, const ProbDev 
       double w = Wsh[s], e = Werr[s];
       int nc = 0;
       __syncwarp();
-      dv_dlarrb_tree(valid, L, B.nbl, P, ps, i, i == pidx, II > 1, rgap, lgap, tol.rtol1, tol.rtol2,
+      dv_dlarrb_tree<false>(valid, L, B.nbl, P, ps, i, i == pidx, II > 1, rgap, lgap, tol.rtol1, tol.rtol2,
                      p->pivmin, maxitr, B.nbl, &w, &e, &nc);
       if (valid && (threadIdx.x & 31) % L == 0) {
         Wsh[s] = w;
@@ -2519,7 +2515,7 @@ k_sng_bisect(int out, const SngDev *sng, const ClusterDev *cl, const ProbDev *pr
     const int tw = (st.r < 1 || st.r > nb) ? nb : st.r;
     int nc = 0;
     __syncwarp();
-    dv_dlarrb_tree(valid, L, nb, P, ps, Windex[S.slot], 1, 0, 0.0, 0.0, 0.0, 2.0 * MR3_EPS, pivmin,
+    dv_dlarrb_tree<false>(valid, L, nb, P, ps, Windex[S.slot], 1, 0, 0.0, 0.0, 0.0, 2.0 * MR3_EPS, pivmin,
                    maxitr, tw, &st.wsh, &st.werr, &nc);
     st.flags = (st.flags | SF_USEDBS) & ~SF_NEEDBS;
     st.lambda = st.wsh;
@@ -2666,7 +2662,7 @@ k_sng_finish(int in, const SngDev *sng, const ClusterDev *cl, ProbDev *probs,
       const int tw = (st.r < 1 || st.r > nb) ? nb : st.r;
       int nc = 0;
       __syncwarp();
-      dv_dlarrb_tree(needbs, L, nb, P, ps, wi, 1, 0, 0.0, 0.0, 0.0, 2.0 * MR3_EPS, pivmin, maxitr,
+      dv_dlarrb_tree<false>(needbs, L, nb, P, ps, wi, 1, 0, 0.0, 0.0, 0.0, 2.0 * MR3_EPS, pivmin, maxitr,
                      tw, &st.wsh, &st.werr, &nc);
       if (needbs) {
         st.flags = (st.flags | SF_USEDBS) & ~SF_NEEDBS;
@@ -3844,9 +3840,11 @@ extern "C" int mr3_cuda_solve_cb(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void
 
   // ---- post-processing (SRC/mrrr.c:262-285)
   if (anyN) LAUNCH(k_shift_w, gN, 256, NN, c->probs, c->blocks, c->iblk, c->E, c->W);
-  if (anyTry)
-    LAUNCH(k_highrac, gN128, 128, NN, c->probs, c->blocks, c->iblk, c->Windex, c->TPc, c->W,
-           c->Werr);
+  if (anyTry) {
+    const int Lj = std::max(3, tree_lanes(nwant, c->nsm, std::max(tree_max, 3), RowCost{193, 95, 55}));
+    LAUNCH(k_highrac, group_blocks(NN, Lj), TREE_T, NN, Lj, c->probs, c->blocks, c->iblk, c->Windex,
+           c->TPc, c->W, c->Werr);
+  }
   LAUNCH(k_invscale, gN, 256, NN, c->probs, c->blocks, c->iblk, c->W);
   if (anyV) {
     LAUNCH(k_place_w, gN, 256, NN, c->probs, c->prob_of_slot, c->W, c->Zindex, c->Wout);
