@@ -2826,12 +2826,22 @@ static __device__ __noinline__ void dv_r1s_call(bool active, int L, int n, doubl
   // ---- the twist index: gamma(i) = SI(i-1) + P(i-1) for i in (r1, r2]
   double best = 0.0;
   int rbest = 0;
-#pragma unroll 4
-  for (int i = r1 + 1 + t; i <= r2; i += L) {
-    const double sprev = b.SI[(i - 1) * st];
-    double c = sprev + b.PA[i * st];
-    if (c == 0.0) c = eps * sprev;
-    if (!isnan(c) && (rbest == 0 || fabs(c) <= fabs(best))) { best = c; rbest = i; }   // i increases
+  for (int i0 = r1 + 1 + t; i0 <= r2; i0 += U * L) {
+    double si[U], pi[U];   // the chunk's loads are issued together
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int i = d_imin(i0 + u * L, r2);
+      si[u] = dv_at(b.SI, i - 1, 8u * b.st);
+      pi[u] = dv_at(b.PA, i, 8u * b.st);
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int i = i0 + u * L;
+      double c = si[u] + pi[u];
+      if (c == 0.0) c = eps * si[u];
+      // i increases; a NaN is never smaller
+      if (i <= r2 && (rbest == 0 ? c == c : fabs(c) <= fabs(best))) { best = c; rbest = i; }
+    }
   }
   for (int s = L >> 1; s > 0; s >>= 1) {
     const double ob = __shfl_xor_sync(gm, best, s);

@@ -2557,10 +2557,10 @@ k_sng_bisect(int out, const SngDev *sng, const ClusterDev *cl, const ProbDev *pr
 #define FIN_CTAS 1
 #endif
 #ifndef FIN_MAXG
-#define FIN_MAXG 8
+#define FIN_MAXG 16
 #endif
 #ifndef FIN_LIST
-#define FIN_LIST 16      // singletons per warp up to which a list is taken
+#define FIN_LIST 64      // singletons per warp up to which a list is taken
 #endif
 enum { FIN_LATER = 0, FIN_FIRST = 1, FIN_BISECT = 2 };
 
