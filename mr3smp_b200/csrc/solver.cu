@@ -2553,8 +2553,14 @@ k_sng_bisect(int out, const SngDev *sng, const ClusterDev *cl, const ProbDev *pr
 // the others would wait for each group's, so singletons that need one leave
 // their group for a second list (bsl) and FIN_BISECT serves that: all groups
 // of a warp bisect at the same time, then make the one or two calls left.
+#ifndef FIN_WARPS
+#define FIN_WARPS 4      // warps per CTA
+#endif
 #ifndef FIN_CTAS
-#define FIN_CTAS 1
+#define FIN_CTAS 2       // CTAs per SM
+#endif
+#ifndef FIN_HALF
+#define FIN_HALF 8       // singletons per warp up to which one CTA an SM is enough
 #endif
 #ifndef FIN_MAXG
 #define FIN_MAXG 16
@@ -2583,7 +2589,7 @@ __device__ __forceinline__ int fin_groups(int n, int nwarps, int maxG, bool bise
 }
 
 template <int KIND>
-__global__ void __launch_bounds__(SNG_WARPS * 32, FIN_CTAS)
+__global__ void __launch_bounds__(FIN_WARPS * 32, FIN_CTAS)
 k_sng_finish(int in, const SngDev *sng, const ClusterDev *cl, ProbDev *probs,
              const BlockDev *blocks, const double2 *RP, const double2 *RQ, const double *arena,
              double *W, double *Wsh, double *Werr, double *Wgap, const int *Windex,
@@ -3732,23 +3738,32 @@ extern "C" int mr3_cuda_solve_cb(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void
         const int bis_ctas = c->nsm * 4;
         const int nblk = (nsng + LIST_T - 1) / LIST_T;
         // k_sng_finish: fw warps of up to maxG groups each, their row scratch
-        // (5 (nmax + 2) doubles a group) within 2 GB (one group a warp at least)
+        // (5 (nmax + 2) doubles a group) within half the bound of the rounds'
+        // scratch, at least 2 GB (one group a warp at least).  A list of at
+        // most FIN_HALF singletons per warp of one CTA an SM gets no second
+        // one, and no more CTAs than it fills with a singleton a warp: the
+        // registers left go to the next level's kernels and to other solves
+        // (mixed_9000 66.7 -> 63 ms, glued_20010 214 -> 206).
         const size_t per = 5ull * ((size_t)nmaxV + 2) * sizeof(double);
-        const size_t fw = (size_t)c->nsm * FIN_CTAS * SNG_WARPS;
+        const size_t fin_bound = std::max((size_t)2 << 30, c->round_scratch / 2);
+        const size_t fw_all = (size_t)c->nsm * FIN_CTAS * FIN_WARPS;
+        size_t fw = fw_all;
+        if ((size_t)nsng <= fw / FIN_CTAS * FIN_HALF) fw /= FIN_CTAS;
+        fw = std::min(fw, ((size_t)nsng + FIN_WARPS - 1) / FIN_WARPS * FIN_WARPS);
         int maxG = FIN_MAXG;
-        while (maxG > 1 && (fw * maxG * per > ((size_t)2 << 30) || fw * (maxG / 2) >= (size_t)nsng))
-          maxG >>= 1;
-        const int fin_ctas = (int)(fw / SNG_WARPS);
+        while (maxG > 1 && (fw * maxG * per > fin_bound || fw * (maxG / 2) >= (size_t)nsng)) maxG >>= 1;
+        const int fin_ctas = (int)(fw / FIN_WARPS);
         if (fw * maxG * per > c->capFscratch) {
+          const size_t sz = std::max(fw * maxG * per, std::min(fin_bound, c->capFscratch * 3 / 2));
           CK(cudaStreamSynchronize(c->own), "fscratch sync");
           CK(cudaStreamSynchronize(c->rnd), "fscratch sync");
-          CK(regrow(&c->fscratch, fw * maxG * per / sizeof(double)), "fscratch");
-          c->capFscratch = fw * maxG * per;
+          CK(regrow(&c->fscratch, sz / sizeof(double)), "fscratch");
+          c->capFscratch = sz;
         }
         // a list of at most this many singletons is finished in one launch
         // (k_sng_finish), from the level's start or after some rounds;
         // MR3_FINISH_MAX overrides it (0: never)
-        int finish_max = (int)std::min<size_t>(FIN_LIST * fw, 1u << 30);
+        int finish_max = (int)std::min<size_t>(FIN_LIST * fw_all, 1u << 30);
         if (const char *ev = getenv("MR3_FINISH_MAX")) finish_max = atoi(ev);
         const bool direct = nsng <= finish_max;
         if (!direct && nwarps * per_warp > c->capScratch) {
@@ -3764,17 +3779,17 @@ extern "C" int mr3_cuda_solve_cb(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void
           const int in = rd & 1, last = rd == SNG_ROUNDS - 1;
           LAUNCH(k_round_reset, 1, 1, c->sc, in, rd == 0);
           if (direct)
-            LAUNCH(k_sng_finish<FIN_FIRST>, fin_ctas, SNG_WARPS * 32, in, c->sng, c->cl[cur], c->probs,
+            LAUNCH(k_sng_finish<FIN_FIRST>, fin_ctas, FIN_WARPS * 32, in, c->sng, c->cl[cur], c->probs,
                    c->blocks, c->RP, c->RQ, c->arena[cur], c->W, c->Wsh, c->Werr, c->Wgap,
                    c->Windex, c->Zindex, c->sst, c->act[0], c->act[1], c->bsl, c->sc, c->fscratch,
                    (long long)nmaxV, maxG, c->done_list, c->tile_left, stats);
           else if (rd > 0)
-            LAUNCH(k_sng_finish<FIN_LATER>, fin_ctas, SNG_WARPS * 32, in, c->sng, c->cl[cur], c->probs,
+            LAUNCH(k_sng_finish<FIN_LATER>, fin_ctas, FIN_WARPS * 32, in, c->sng, c->cl[cur], c->probs,
                    c->blocks, c->RP, c->RQ, c->arena[cur], c->W, c->Wsh, c->Werr, c->Wgap,
                    c->Windex, c->Zindex, c->sst, c->act[0], c->act[1], c->bsl, c->sc, c->fscratch,
                    (long long)nmaxV, maxG, c->done_list, c->tile_left, stats);
           if (maxG > 1 && (direct || rd > 0))
-            LAUNCH(k_sng_finish<FIN_BISECT>, fin_ctas, SNG_WARPS * 32, in, c->sng, c->cl[cur], c->probs,
+            LAUNCH(k_sng_finish<FIN_BISECT>, fin_ctas, FIN_WARPS * 32, in, c->sng, c->cl[cur], c->probs,
                    c->blocks, c->RP, c->RQ, c->arena[cur], c->W, c->Wsh, c->Werr, c->Wgap,
                    c->Windex, c->Zindex, c->sst, c->act[0], c->act[1], c->bsl, c->sc, c->fscratch,
                    (long long)nmaxV, maxG, c->done_list, c->tile_left, stats);
