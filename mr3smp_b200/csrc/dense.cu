@@ -172,7 +172,43 @@ int range_code(char c) {
   return -1;
 }
 
-// Device buffers of one call, released on every exit path.
+// Device buffers and library handles of a call.  Creating and destroying
+// the cuSOLVER handle and allocating and freeing a dozen buffers took 5.5 of
+// the 15.7 ms of an n = 700 dsyeig, so a call borrows them: finished calls
+// leave theirs in a list of at most KEEP_SETS per process, with at most
+// KEEP_BYTES each; what is above that, and a set whose call failed, is freed.
+// A set belongs to one call at a time and to the device it was made on; its
+// buffers' contents do not outlive a call.
+const int KEEP_SETS = 4;
+const size_t KEEP_BYTES = (size_t)256 << 20;
+enum { BUF_A, BUF_B, BUF_AP, BUF_D, BUF_E, BUF_TAU, BUF_W, BUF_Z, BUF_WORK, BUF_ZSUPP, BUF_FLAGS,
+       BUF_COUNT };
+
+struct DenseSet {
+  int device = 0;
+  void *buf[BUF_COUNT] = {};
+  size_t cap[BUF_COUNT] = {};
+  cusolverDnHandle_t h = nullptr;
+  cublasHandle_t hb = nullptr;
+  void drop_buffers() {
+    for (int k = 0; k < BUF_COUNT; k++) {
+      if (buf[k]) cudaFree(buf[k]);
+      buf[k] = nullptr;
+      cap[k] = 0;
+    }
+  }
+  void drop() {
+    drop_buffers();
+    if (h) g_cs.destroy(h);
+    if (hb) g_cs.bdestroy(hb);
+    h = nullptr;
+    hb = nullptr;
+  }
+};
+DenseSet *g_kept[KEEP_SETS];
+pthread_mutex_t g_kept_mu = PTHREAD_MUTEX_INITIALIZER;
+
+// The buffers of one call; the set goes back on every exit path.
 struct DenseBufs {
   double *A = nullptr, *B = nullptr, *AP = nullptr, *D = nullptr, *E = nullptr, *tau = nullptr,
          *W = nullptr, *Z = nullptr, *work = nullptr;
@@ -180,12 +216,57 @@ struct DenseBufs {
   unsigned long long *maxbits = nullptr;
   cusolverDnHandle_t h = nullptr;
   cublasHandle_t hb = nullptr;
+  DenseSet *set = nullptr;
+  bool good = false;   // the call ended well: its set may be kept
+
+  void borrow(int device) {
+    pthread_mutex_lock(&g_kept_mu);
+    for (int k = 0; k < KEEP_SETS && !set; k++)
+      if (g_kept[k] && g_kept[k]->device == device) {
+        set = g_kept[k];
+        g_kept[k] = nullptr;
+      }
+    pthread_mutex_unlock(&g_kept_mu);
+    if (!set) {
+      set = new DenseSet();
+      set->device = device;
+    }
+  }
+  // Buffer `which` with room for `bytes`.
+  template <typename T>
+  cudaError_t get(int which, size_t bytes, T **p) {
+    if (bytes > set->cap[which] || !set->buf[which]) {
+      if (set->buf[which]) cudaFree(set->buf[which]);
+      set->buf[which] = nullptr;
+      set->cap[which] = 0;
+      const cudaError_t e = cudaMalloc(&set->buf[which], bytes > 0 ? bytes : 1);
+      if (e != cudaSuccess) return e;
+      set->cap[which] = bytes;
+    }
+    *p = (T *)set->buf[which];
+    return cudaSuccess;
+  }
   ~DenseBufs() {
-    void *p[] = {A, B, AP, D, E, tau, W, Z, work, Zsupp, info, nan, maxbits};
-    for (void *q : p)
-      if (q) cudaFree(q);
-    if (h) g_cs.destroy(h);
-    if (hb) g_cs.bdestroy(hb);
+    if (!set) return;
+    set->h = h;
+    set->hb = hb;
+    bool kept = false;
+    if (good) {
+      size_t total = 0;
+      for (size_t c : set->cap) total += c;
+      if (total > KEEP_BYTES) set->drop_buffers();
+      pthread_mutex_lock(&g_kept_mu);
+      for (int k = 0; k < KEEP_SETS && !kept; k++)
+        if (!g_kept[k]) {
+          g_kept[k] = set;
+          kept = true;
+        }
+      pthread_mutex_unlock(&g_kept_mu);
+    }
+    if (!kept) {
+      set->drop();
+      delete set;
+    }
   }
 };
 
@@ -219,22 +300,27 @@ int check_common(int jz, int rg, int n, const double *vl, const double *vu, cons
 int start(DenseBufs &b, int n, int jz, int ncols) {
   pthread_once(&g_cs_once, load_cusolver);
   if (!g_cs.ok) return 2;
-  DCK(cudaSetDevice(device_id()));
-  const size_t nn = (size_t)n * n;
-  DCK(cudaMalloc((void **)&b.A, nn * sizeof(double)));
-  DCK(cudaMalloc((void **)&b.D, n * sizeof(double)));
-  DCK(cudaMalloc((void **)&b.E, n * sizeof(double)));
-  DCK(cudaMalloc((void **)&b.tau, n * sizeof(double)));
-  DCK(cudaMalloc((void **)&b.W, n * sizeof(double)));
-  DCK(cudaMalloc((void **)&b.Zsupp, 2 * (size_t)n * sizeof(int)));
-  DCK(cudaMalloc((void **)&b.info, sizeof(int)));
-  DCK(cudaMalloc((void **)&b.nan, sizeof(int)));
-  DCK(cudaMalloc((void **)&b.maxbits, sizeof(unsigned long long)));
-  if (jz == MR3_JOB_V) DCK(cudaMalloc((void **)&b.Z, (size_t)n * ncols * sizeof(double)));
-  DCK(cudaMemset(b.E, 0, n * sizeof(double)));
-  DCK(cudaMemset(b.nan, 0, sizeof(int)));
-  DCK(cudaMemset(b.maxbits, 0, sizeof(unsigned long long)));
-  SCK(g_cs.create(&b.h));
+  const int device = device_id();
+  DCK(cudaSetDevice(device));
+  b.borrow(device);
+  b.h = b.set->h;
+  b.hb = b.set->hb;
+  const size_t nn = (size_t)n * n, nd = n * sizeof(double);
+  char *flags;
+  DCK(b.get(BUF_A, nn * sizeof(double), &b.A));
+  DCK(b.get(BUF_D, nd, &b.D));
+  DCK(b.get(BUF_E, nd, &b.E));
+  DCK(b.get(BUF_TAU, nd, &b.tau));
+  DCK(b.get(BUF_W, nd, &b.W));
+  DCK(b.get(BUF_ZSUPP, 2 * (size_t)n * sizeof(int), &b.Zsupp));
+  DCK(b.get(BUF_FLAGS, 16, &flags));   // max-norm bits, NaN flag, info
+  b.maxbits = (unsigned long long *)flags;
+  b.nan = (int *)(flags + 8);
+  b.info = (int *)(flags + 12);
+  if (jz == MR3_JOB_V) DCK(b.get(BUF_Z, (size_t)n * ncols * sizeof(double), &b.Z));
+  DCK(cudaMemset(b.E, 0, nd));
+  DCK(cudaMemset(flags, 0, 16));
+  if (!b.h) SCK(g_cs.create(&b.h));
   return 0;
 }
 
@@ -249,12 +335,10 @@ int dense_core(DenseBufs &b, int jz, int rg, bool lower, int n, int ncols, doubl
   const double rmin = sqrt(smlnum), rmax = fmin(sqrt(bignum), 1.0 / sqrt(sqrt(DBL_MIN)));
   k_tri_absmax<<<kGrid, 256>>>(n, b.A, lower, b.maxbits, b.nan);
   DCK(cudaGetLastError());
-  unsigned long long bits = 0;
-  int sawnan = 0;
-  DCK(cudaMemcpy(&bits, b.maxbits, sizeof(bits), cudaMemcpyDeviceToHost));
-  DCK(cudaMemcpy(&sawnan, b.nan, sizeof(int), cudaMemcpyDeviceToHost));
-  double norm;
-  memcpy(&norm, &bits, sizeof(norm));
+  struct { double norm; int nan, info; } flags;
+  DCK(cudaMemcpy(&flags, b.maxbits, sizeof(flags), cudaMemcpyDeviceToHost));
+  double norm = flags.norm;
+  const int sawnan = flags.nan;
   if (sawnan) norm = NAN;
   double sigma = 1.0;
   bool scaled = false;
@@ -281,9 +365,7 @@ int dense_core(DenseBufs &b, int jz, int rg, bool lower, int n, int ncols, doubl
   if (n > 1 && jz == MR3_JOB_V)
     SCK(g_cs.ormtr_ws(b.h, CUBLAS_SIDE_LEFT, fill, CUBLAS_OP_N, n, ncols, b.A, n, b.tau, b.Z, n,
                       &lw2));
-  if (b.work) cudaFree(b.work);
-  b.work = nullptr;
-  DCK(cudaMalloc((void **)&b.work, (size_t)(lw1 > lw2 ? lw1 : lw2) * sizeof(double) + 8));
+  DCK(b.get(BUF_WORK, (size_t)(lw1 > lw2 ? lw1 : lw2) * sizeof(double) + 8, &b.work));
   int hinfo = 0;
   if (n > 1) {
     SCK(g_cs.sytrd(b.h, fill, n, b.A, n, b.D, b.E, b.tau, b.work, lw1, b.info));
@@ -340,13 +422,13 @@ int reduce_generalized(DenseBufs &b, int itype, bool lower, int n) {
   const cublasFillMode_t fill = lower ? CUBLAS_FILL_MODE_LOWER : CUBLAS_FILL_MODE_UPPER;
   int lw = 0, hinfo = 0;
   SCK(g_cs.potrf_ws(b.h, fill, n, b.B, n, &lw));
-  DCK(cudaMalloc((void **)&b.work, (size_t)lw * sizeof(double) + 8));
+  DCK(b.get(BUF_WORK, (size_t)lw * sizeof(double) + 8, &b.work));
   SCK(g_cs.potrf(b.h, fill, n, b.B, n, b.work, lw, b.info));
   DCK(cudaMemcpy(&hinfo, b.info, sizeof(int), cudaMemcpyDeviceToHost));
   if (hinfo != 0) return 2;   // B is not positive definite
   k_symmetrize<<<kGrid, 256>>>(n, b.A, lower);
   DCK(cudaGetLastError());
-  BCK(g_cs.bcreate(&b.hb));
+  if (!b.hb) BCK(g_cs.bcreate(&b.hb));
   const double one = 1.0;
   const cublasDiagType_t nu = CUBLAS_DIAG_NON_UNIT;
   if (itype == 1) {
@@ -411,6 +493,7 @@ extern "C" int dsyeig(char *jobz, char *range, char *uplo, int *np, double *A, i
   if (jz == MR3_JOB_V && *mp > 0)
     DCK(cudaMemcpy2D(Z, (size_t)*ldzp * sizeof(double), b.Z, n * sizeof(double),
                      n * sizeof(double), *mp, cudaMemcpyDeviceToHost));
+  b.good = true;
   return 0;
 }
 
@@ -431,7 +514,7 @@ extern "C" int dspeig(char *jobz, char *range, char *uplo, int *np, double *AP, 
   int rc = start(b, n, jz, ncols);
   if (rc) return rc;
   const size_t np_ = (size_t)n * (n + 1) / 2;
-  DCK(cudaMalloc((void **)&b.AP, np_ * sizeof(double)));
+  DCK(b.get(BUF_AP, np_ * sizeof(double), &b.AP));
   DCK(cudaMemcpy(b.AP, AP, np_ * sizeof(double), cudaMemcpyHostToDevice));
   k_packed<<<kGrid, 256>>>(n, b.AP, b.A, lower, 0);
   DCK(cudaGetLastError());
@@ -439,6 +522,7 @@ extern "C" int dspeig(char *jobz, char *range, char *uplo, int *np, double *AP, 
   if (jz == MR3_JOB_V && *mp > 0)
     DCK(cudaMemcpy2D(Z, (size_t)*ldzp * sizeof(double), b.Z, n * sizeof(double),
                      n * sizeof(double), *mp, cudaMemcpyDeviceToHost));
+  b.good = true;
   return 0;
 }
 
@@ -457,7 +541,7 @@ extern "C" int dsygeig(int *itype, char *jobz, char *range, char *uplo, int *np,
   const int ncols = rg == MR3_RANGE_I ? *iup - *ilp + 1 : n;
   int rc = start(b, n, jz, ncols);
   if (rc) return rc;
-  DCK(cudaMalloc((void **)&b.B, (size_t)n * n * sizeof(double)));
+  DCK(b.get(BUF_B, (size_t)n * n * sizeof(double), &b.B));
   DCK(cudaMemcpy2D(b.A, n * sizeof(double), A, (size_t)*ldap * sizeof(double), n * sizeof(double),
                    n, cudaMemcpyHostToDevice));
   DCK(cudaMemcpy2D(b.B, n * sizeof(double), B, (size_t)*ldbp * sizeof(double), n * sizeof(double),
@@ -475,6 +559,7 @@ extern "C" int dsygeig(int *itype, char *jobz, char *range, char *uplo, int *np,
   if (jz == MR3_JOB_V && *mp > 0)
     DCK(cudaMemcpy2D(A, (size_t)*ldap * sizeof(double), b.Z, n * sizeof(double),
                      n * sizeof(double), *mp, cudaMemcpyDeviceToHost));
+  b.good = true;
   return 0;
 }
 
@@ -493,8 +578,8 @@ extern "C" int dspgeig(int *itype, char *jobz, char *range, char *uplo, int *np,
   int rc = start(b, n, jz, ncols);
   if (rc) return rc;
   const size_t np_ = (size_t)n * (n + 1) / 2;
-  DCK(cudaMalloc((void **)&b.B, (size_t)n * n * sizeof(double)));
-  DCK(cudaMalloc((void **)&b.AP, np_ * sizeof(double)));
+  DCK(b.get(BUF_B, (size_t)n * n * sizeof(double), &b.B));
+  DCK(b.get(BUF_AP, np_ * sizeof(double), &b.AP));
   DCK(cudaMemset(b.B, 0, (size_t)n * n * sizeof(double)));
   DCK(cudaMemcpy(b.AP, AP, np_ * sizeof(double), cudaMemcpyHostToDevice));
   k_packed<<<kGrid, 256>>>(n, b.AP, b.A, lower, 0);
@@ -516,6 +601,7 @@ extern "C" int dspgeig(int *itype, char *jobz, char *range, char *uplo, int *np,
   if (jz == MR3_JOB_V && *mp > 0)
     DCK(cudaMemcpy2D(Z, (size_t)*ldzp * sizeof(double), b.Z, n * sizeof(double),
                      n * sizeof(double), *mp, cudaMemcpyDeviceToHost));
+  b.good = true;
   return 0;
 }
 
