@@ -415,6 +415,34 @@ static __device__ __noinline__ int dv_bisect_one(int n, const double2 *__restric
 // The same sequence of intervals; about log2(L) steps per count.  The
 // counts are guessed; lanes 0 and 1 then confirm the two ends, and the walk
 // is repeated with exact counts if one fails.
+//
+// An eigenvalue far below the interval's ends in magnitude takes the walk
+// many steps, one per halving (a matrix graded over 280 decades up to 1000).
+// After BIS_LONG steps the group first brackets the eigenvalue with points of
+// its own choice, dv_bracket_mid, until the bracket is narrower than the walk's
+// last interval; the walk then goes on without counts, since its midpoints
+// lie beside the bracket (one inside is counted).  The turns and with them
+// the interval are the same.
+#ifndef BIS_LONG
+#ifndef BIS_LONG
+#ifndef BIS_LONG
+#define BIS_LONG 56
+#endif
+#endif
+#endif
+
+// A point between l and r that halves the bracket's exponent range while its
+// ends differ by more than a factor of four, else the bracket.
+static __device__ __forceinline__ double dv_bracket_mid(double l, double r) {
+  if (l < 0.0 && r > 0.0) return 0.0;
+  if (l >= 0.0) {
+    const double s = fmax(l, MR3_SAFMIN);
+    return r > 4.0 * s ? sqrt(s) * sqrt(r) : 0.5 * (l + r);
+  }
+  const double s = fmax(-r, MR3_SAFMIN);
+  return -l > 4.0 * s ? -(sqrt(s) * sqrt(-l)) : 0.5 * (l + r);
+}
+
 static __device__ __noinline__ void dv_bisect_tree(int L, int n, const double2 *__restrict__ tp,
                                             double pivmin, double abstol, double reltol, int itmax,
                                             int j, double *a_, double *b_, const int na0,
@@ -449,6 +477,36 @@ static __device__ __noinline__ void dv_bisect_tree(int L, int n, const double2 *
         it++;
         const double w = fabs(b - a), tt = fmax(fabs(b), fabs(a));
         if (w < fmax(fmax(abstol, pivmin), reltol * tt) || na >= nb || it >= itmax) done = true;
+      }
+      if (!done && pass == 0 && it >= BIS_LONG) {
+        // the bracket: guessed counts below j at lo, at least j at hi
+        double lo = a, hi = b;
+        bool more = true;
+        for (int q = 0; more && q < 64; q++) {
+          double bl = lo, br = hi;
+          for (int k = 30 - __clz(t + 1); k >= 0; k--) {
+            const double m = dv_bracket_mid(bl, br);
+            if (((t + 1) >> k) & 1) bl = m; else br = m;
+          }
+          const int rb = dv_count_guess(n, tp, pivmin, dv_bracket_mid(bl, br));
+          for (int node = 1; node <= L && more;) {
+            const int cv = __shfl_sync(gm, rb, g0 + node - 1);
+            const double m = dv_bracket_mid(lo, hi);
+            if (!(m > lo && m < hi)) { more = false; break; }
+            if (j <= cv) { hi = m; node = 2 * node; } else { lo = m; node = 2 * node + 1; }
+            const double tt = fmax(fabs(lo), fabs(hi));
+            more = hi - lo > 0.125 * fmax(fmax(abstol, pivmin), reltol * tt);
+          }
+        }
+        while (!done) {   // the rest of the walk
+          const double c = 0.5 * (a + b);
+          int cv = c >= hi ? nb : c <= lo ? na : dv_count_guess(n, tp, pivmin, c);
+          const int cnt = d_imin(nb, d_imax(na, cv));
+          if (j <= cnt) { b = c; nb = cnt; hi = fmin(hi, c); } else { a = c; na = cnt; lo = fmax(lo, c); }
+          it++;
+          const double w = fabs(b - a), tt = fmax(fabs(b), fabs(a));
+          if (w < fmax(fmax(abstol, pivmin), reltol * tt) || na >= nb || it >= itmax) done = true;
+        }
       }
     }
     if (pass == 1) { it += 2; break; }

@@ -78,3 +78,39 @@ def test_confirmed_guess_is_the_exact_bisection(name, T, err):
             assert (a, b) == bisect(lambda c: sturm(d, e2, c), j, lo, hi), (name, j)
     if err <= 1e-12 and name == "uniform":
         assert confirmed >= len(d) - 1
+
+
+def bracket_mid(l, r):
+    if l < 0.0 < r:
+        return 0.0
+    if l >= 0.0:
+        s = max(l, PIV)
+        return float(np.sqrt(s) * np.sqrt(r)) if r > 4.0 * s else 0.5 * (l + r)
+    return -bracket_mid(-r, -l)
+
+
+@pytest.mark.parametrize("sign", [1.0, -1.0])
+def test_bracketed_walk_is_the_bisection(sign):
+    """The walk of a long bisection from a bracket found at other points: the
+    intervals of the bisection that counts at every midpoint."""
+    g = 10.0 ** (-np.arange(24) * 11.0)
+    d, e2 = sign * 3.0 * g, g[:-1] * g[1:]
+    for j in range(1, 25):
+        a0, b0 = -4.5, 4.5
+        ref = bisect(lambda c: sturm(d, e2, c), j, a0, b0, itmax=1100)
+        lo, hi = a0, b0
+        counts = 0
+        while hi - lo > 0.125 * max(4 * PIV, 1.5e-8 * max(abs(lo), abs(hi))):
+            m = bracket_mid(lo, hi)
+            if not lo < m < hi:
+                break
+            counts += 1
+            if j <= sturm(d, e2, m):
+                hi = m
+            else:
+                lo = m
+        assert counts < 60
+
+        def count(c):
+            return j if c >= hi else j - 1 if c <= lo else sturm(d, e2, c)
+        assert bisect(count, j, a0, b0, itmax=1100) == ref, j
