@@ -14,6 +14,11 @@
 
 #include "mr3_b200.h"
 
+/* mr3_cuda_solve_cb without the device's screening for non-finite entries
+ * (solver.cu): the problems here have been screened on the host. */
+int mr3__cuda_solve_finite(mr3_cuda_ctx *ctx, int nprob, mr3_cuda_prob *probs, void *stream,
+                           mr3_cuda_done_fn done, void *user);
+
 #define POOL_MAX 64
 
 typedef struct {
@@ -274,7 +279,7 @@ __attribute__((visibility("hidden"))) int mr3__batched_on(mr3_cuda_ctx *ctx, int
     ec.dp = dp + cbeg[c];
     ec.copied = copied + cbeg[c];
     ec.rc = MR3_OK;
-    if (mr3_cuda_solve_cb(ctx, cbeg[c + 1] - cbeg[c], dp + cbeg[c], NULL, on_done, &ec) != MR3_OK ||
+    if (mr3__cuda_solve_finite(ctx, cbeg[c + 1] - cbeg[c], dp + cbeg[c], NULL, on_done, &ec) != MR3_OK ||
         ec.rc != MR3_OK || mr3_cuda_event(ctx, 2, MR3_STREAM_MAIN, MR3_STREAM_COPY) != MR3_OK) {
       rc = MR3_EMISC;
       goto done;

@@ -148,13 +148,21 @@ __device__ __forceinline__ void column_done(ProbDev *p, int prob, int zind, SngC
 // by the SMs straight into pinned host memory; null targets are skipped.
 // A copy-engine transfer would queue behind the eigenvector copies of
 // finished tiles that the caller may have started meanwhile.
-__global__ void k_export(const LevelCounters *lc, LevelCounters *hlc, SngCounters *sc,
-                         SngCounters *hsc, const int2 *done_list, int2 *hdone, int *hsnap) {
+// A level's export (lc) also clears the other LevelCounters and n_sng, which
+// the next level's classification counts in.
+__global__ void k_export(const LevelCounters *lc, LevelCounters *lc_next, LevelCounters *hlc,
+                         SngCounters *sc, SngCounters *hsc, const int2 *done_list, int2 *hdone, int *hsnap) {
   const int t = threadIdx.x, from = sc->done_exp, to = sc->done_n;
   if (t == 0) {
     if (hlc) *hlc = *lc;
     if (hsc) *hsc = *sc;
     if (hsnap) *hsnap = to;
+    if (lc_next) {
+      LevelCounters z;
+      z.n_cl = 0; z.err = 0; z.arena_need = 0;
+      *lc_next = z;
+      sc->n_sng = 0;
+    }
   }
   if (hdone)
     for (int i = from + t; i < to; i += blockDim.x) hdone[i] = done_list[i];
@@ -222,14 +230,17 @@ __device__ __forceinline__ void stat_add(unsigned long long *stats, int slot, un
 // Stage A0: per-problem prologue (SRC/mrrr.c:206-243, SRC/mrrr_val.c:167-329)
 // ------------------------------------------------------------------------
 __global__ void k_gather(ProbDev *probs, const double *const *Din, const double *const *Ein,
-                         double *D, double *E, int *prob_of_slot, int *iblk) {
+                         double *D, double *E, int *prob_of_slot, int *iblk, int *lvl_of_slot,
+                         int *flag) {
   ProbDev *p = &probs[blockIdx.x];
+  if (threadIdx.x == 0) flag[blockIdx.x] = 0;
   const double *di = Din[blockIdx.x], *ei = Ein[blockIdx.x];
   for (int i = threadIdx.x; i < p->n; i += blockDim.x) {
     D[p->off + i] = di[i];
     E[p->off + i] = ei[i];
     prob_of_slot[p->off + i] = blockIdx.x;
     iblk[p->off + i] = -1;
+    lvl_of_slot[p->off + i] = -1;
   }
 }
 
@@ -1379,6 +1390,41 @@ __global__ void k_merge_pass(int N, const ProbDev *probs, const int *prob_of_slo
   out[o + pos] = r;
 }
 
+// All passes of k_merge_pass for problems of at most cap eigenvalues in one
+// launch: a CTA per problem, the records in shared memory.  Bound by launches
+// and latency at these sizes: 11 launches' 0.09 ms become 0.03 at 1500
+// eigenvalues.
+#define SORT_CTA 2048
+__global__ void __launch_bounds__(512)
+k_sort_cta(const ProbDev *probs, SortRec *rec, int cap, int want_job, const int *flag) {
+  extern __shared__ SortRec sort_buf[];
+  const ProbDev *p = &probs[blockIdx.x];
+  if (p->trivial || p->status || p->jobz != want_job) return;
+  if (flag && !flag[blockIdx.x]) return;
+  const int m = p->m;
+  SortRec *in = sort_buf, *out = sort_buf + cap, *r = rec + p->off;
+  for (int k = threadIdx.x; k < m; k += blockDim.x) in[k] = r[k];
+  __syncthreads();
+  for (int width = 1; width < m; width *= 2) {
+    for (int k = threadIdx.x; k < m; k += blockDim.x) {
+      const int run0 = (k / (2 * width)) * (2 * width);
+      const int a1 = min(run0 + width, m), b1 = min(run0 + 2 * width, m);
+      const SortRec e = in[k];
+      const bool isA = k < a1;   // its place: its own rank plus the other run's smaller elements
+      int lo = isA ? a1 : run0, hi = isA ? b1 : a1;
+      const int first = lo;
+      while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (rec_less(in[mid], e)) lo = mid + 1; else hi = mid;
+      }
+      out[run0 + (isA ? k - run0 : k - a1) + (lo - first)] = e;
+    }
+    __syncthreads();
+    SortRec *t = in; in = out; out = t;
+  }
+  for (int k = threadIdx.x; k < m; k += blockDim.x) r[k] = in[k];
+}
+
 // Keys of init_zindex (SRC/mrrr_vec.c:380-416): the running maximum of
 // W + sigma inside each block; one warp per block.
 __global__ void k_zkeys(ProbDev *probs, const BlockDev *blocks, const double *W, const double *E,
@@ -1578,8 +1624,10 @@ template <bool PAIR>
 __global__ void LB_RRF
 k_cl_rrf(int ncl, ClusterDev *cl, const ProbDev *probs, const BlockDev *blocks, const double2 *RP,
          const double2 *RQ, const double *arena_prev, double *arena_cur, const double *xw,
-         const double *xe, double *Wsh, double *Werr, double *Wgap, unsigned long long *stats) {
+         const double *xe, double *Wsh, double *Werr, double *Wgap, int *rl_n,
+         unsigned long long *stats) {
   const int gt = blockIdx.x * blockDim.x + threadIdx.x;
+  if (gt == 0) *rl_n = 0;   // counted by k_cl_pack
   const int w = PAIR ? gt >> 1 : gt;
   const bool lead = !PAIR || (gt & 1) == 0;
   unsigned long long work = 0;
@@ -1857,6 +1905,27 @@ __global__ void __launch_bounds__(256) k_rl_scatter(int N, const int *lvl, int l
   }
 }
 
+// The same for few slots, in one launch of one CTA.
+#define RL_CTA 16384
+__global__ void __launch_bounds__(1024) k_rl_small(int N, const int *lvl, int level, int *rl) {
+  __shared__ int wcnt[32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  int pos = 0;
+  for (int b0 = 0; b0 < N; b0 += 1024) {
+    const int k = b0 + threadIdx.x;
+    const bool f = k < N && lvl[k] == level;
+    const unsigned b = __ballot_sync(0xffffffffu, f);
+    if (lane == 0) wcnt[wid] = __popc(b);
+    __syncthreads();
+    int before = lane < wid ? wcnt[lane] : 0, total = wcnt[lane];
+    before = __reduce_add_sync(0xffffffffu, before);
+    total = __reduce_add_sync(0xffffffffu, total);
+    if (f) rl[pos + before + __popc(b & ((1u << lane) - 1u))] = k;
+    pos += total;
+    __syncthreads();
+  }
+}
+
 __global__ void k_gaps_cl(int N, const ClusterDev *cl, const double *Wsh, const double *Werr,
                           double *Wgap, double *W, const int *cl_of_slot, const int *lvl_of_slot,
                           int level) {
@@ -2051,13 +2120,71 @@ __global__ void k_group_tasks(int ncl, const ClusterDev *cl, const BlockDev *blo
   for (int m = 0; m < C.G; m++) { xs.soff[w + m] = o; o += xs.ns[w + m]; }
 }
 
+// The round lists before a level's first round (or its finish).
+__device__ __forceinline__ void level_reset(SngCounters *sc, int n_sng) {
+  sc->nin = n_sng;
+  sc->act_next[0] = 0;
+  sc->bs_next = 0;
+  sc->fb_n = 0;
+  sc->fb_next = 0;
+  sc->mode = 0;
+  sc->fin_ctas = 0;
+}
+
 // bk[0..15]: counts per bucket; bk[16..31]: first record of each bucket,
 // largest blocks first; bk[32..47]: fill counters (zeroed with the counts).
-__global__ void k_bucket_scan(int *bk) {
+__global__ void k_bucket_scan(int *bk, SngCounters *sc) {
+  level_reset(sc, sc->n_sng);
   int run = 0;
   for (int b = SNG_BUCKETS - 1; b >= 0; b--) {
     bk[SNG_BUCKETS + b] = run;
     run += bk[b];
+  }
+}
+
+// The same for few clusters, in one launch of one CTA: five launches (with
+// the counts' clearing and the lists' reset) become one.  With the sort, the
+// refinement list below, one upload per solve and one wait at its end, a
+// solve of 33 rows went from 0.51 to 0.41 ms, one of 1000 from 3.30 to 3.15.
+// The line: a thread walks its clusters one after another, 4 passes at 4096.
+#define GROUP_CTA 4096
+__global__ void __launch_bounds__(1024)
+k_group_small(int ncl, const ClusterDev *cl, const BlockDev *blocks, ClsScratch xs, SngCounters *sc,
+              LevelCounters *lcn, int cap) {
+  __shared__ int cnt[SNG_BUCKETS], first[SNG_BUCKETS], total;
+  if (threadIdx.x < SNG_BUCKETS) cnt[threadIdx.x] = 0;
+  __syncthreads();
+  for (int pass = 0; pass < 2; pass++) {
+    for (int w = threadIdx.x; w < ncl; w += blockDim.x) {
+      if (cl[w].g != 0) continue;
+      const int G = cl[w].G;
+      int tot = 0;
+      for (int m = 0; m < G; m++) tot += xs.ns[w + m];
+      if (tot == 0) continue;
+      const int b = size_bucket(blocks[cl[w].blk].nbl);
+      const int at = atomicAdd(&cnt[b], tot);
+      if (pass == 0) continue;
+      int o = first[b] + at;
+      if (o + tot > cap) { atomicOr(&lcn->err, 1); continue; }
+      for (int m = 0; m < G; m++) { xs.soff[w + m] = o; o += xs.ns[w + m]; }
+    }
+    __syncthreads();
+    if (pass == 0) {
+      if (threadIdx.x == 0) {
+        int run = 0;
+        for (int b = SNG_BUCKETS - 1; b >= 0; b--) {
+          first[b] = run;
+          run += cnt[b];
+          cnt[b] = 0;
+        }
+        total = run;
+      }
+      __syncthreads();
+    }
+  }
+  if (threadIdx.x == 0) {
+    sc->n_sng = total;
+    level_reset(sc, total);
   }
 }
 
@@ -2111,13 +2238,13 @@ struct SngState {
   int r, k, flags, pad;
 };
 
-__global__ void k_round_reset(SngCounters *sc, int in, int first) {
-  sc->nin = first ? sc->n_sng : sc->act_n[in];
+// The lists of a round after the first.
+__global__ void k_round_reset(SngCounters *sc, int in) {
+  sc->nin = sc->act_n[in];
   sc->act_next[in] = 0;
   sc->bs_next = 0;
   sc->fb_n = 0;
   sc->fb_next = 0;
-  if (first) { sc->mode = 0; sc->fin_ctas = 0; }
 }
 
 // Stable compaction of a round's list: entry j of the list leaves the round
@@ -2924,10 +3051,12 @@ struct mr3_cuda_ctx {
   double *fscratch = nullptr;               // row scratch of the split finish
   size_t capFscratch = 0;
   size_t round_scratch = (size_t)8 << 30;   // bound of the round warps' checkpoint scratch
+  // a solve's problem records and array pointers, uploaded in one copy: probs,
+  // then Din, Ein, Wp, Dp, Ep, each as long as the solve's problem count
+  char *pk = nullptr, *h_pk = nullptr;      // device, page-locked host
   const double **Din = nullptr, **Ein = nullptr;
   double **Wp = nullptr, **Dp = nullptr, **Ep = nullptr;
-  // pinned host mirrors
-  ProbDev *h_probs = nullptr;
+  ProbDev *h_probs = nullptr;               // host views of pk
   void **h_ptrs = nullptr;
   LevelCounters *h_lc = nullptr, *d_hlc = nullptr;   // host pointer, device view
   SngCounters *h_sc = nullptr, *d_hsc = nullptr;
@@ -3058,23 +3187,32 @@ static int ensure_rows(mr3_cuda_ctx *c, size_t N, size_t P) {
   }
   if (P > c->capP) {
     size_t p = std::max(P, c->capP + c->capP / 2);
-    CK(regrow(&c->probs, p), "probs");
+    c->capP = 0;   // until all of it is there
+    const size_t rec = sizeof(ProbDev) + 5 * sizeof(void *);
+    CK(regrow(&c->pk, p * rec), "problem records");
     CK(regrow(&c->flag, p), "flag");
-
-    CK(regrow(&c->Din, p), "Din");
-    CK(regrow(&c->Ein, p), "Ein");
-    CK(regrow(&c->Wp, p), "Wp");
-    CK(regrow(&c->Dp, p), "Dp");
-    CK(regrow(&c->Ep, p), "Ep");
-    if (c->h_probs) cudaFreeHost(c->h_probs);
-    if (c->h_ptrs) cudaFreeHost(c->h_ptrs);
+    if (c->h_pk) cudaFreeHost(c->h_pk);
     if (c->h_flag) cudaFreeHost(c->h_flag);
-    CK(cudaMallocHost((void **)&c->h_probs, p * sizeof(ProbDev)), "h_probs");
-    CK(cudaMallocHost((void **)&c->h_ptrs, 5 * p * sizeof(void *)), "h_ptrs");
+    c->h_pk = nullptr;
+    c->h_flag = nullptr;
+    CK(cudaMallocHost((void **)&c->h_pk, p * rec), "h_pk");
     CK(cudaMallocHost((void **)&c->h_flag, p * sizeof(int)), "h_flag");
     c->capP = p;
   }
   return MR3_OK;
+}
+
+// Lays the upload out for n problems.
+static void layout_pk(mr3_cuda_ctx *c, int n) {
+  c->h_probs = (ProbDev *)c->h_pk;
+  c->h_ptrs = (void **)(c->h_pk + n * sizeof(ProbDev));
+  c->probs = (ProbDev *)c->pk;
+  double **ptr = (double **)(c->pk + n * sizeof(ProbDev));
+  c->Din = (const double **)ptr;
+  c->Ein = (const double **)(ptr + n);
+  c->Wp = ptr + 2 * n;
+  c->Dp = ptr + 3 * n;
+  c->Ep = ptr + 4 * n;
 }
 
 extern "C" int mr3_cuda_ctx_create(int device, mr3_cuda_ctx **out) {
@@ -3101,8 +3239,7 @@ extern "C" int mr3_cuda_ctx_create_prio(int device, int high, mr3_cuda_ctx **out
       cudaStreamCreateWithPriority(&c->aux, cudaStreamNonBlocking, prio) != cudaSuccess ||
       cudaStreamCreateWithPriority(&c->rnd, cudaStreamNonBlocking, prio) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->rnd_done, cudaEventDisableTiming) != cudaSuccess ||
-      cudaMalloc((void **)&c->lc, 2 * sizeof(LevelCounters)) != cudaSuccess ||
-      cudaMalloc((void **)&c->sc, sizeof(SngCounters)) != cudaSuccess ||
+      cudaMalloc((void **)&c->lc, 2 * sizeof(LevelCounters) + sizeof(SngCounters)) != cudaSuccess ||
       cudaMalloc((void **)&c->rl_n, sizeof(int)) != cudaSuccess ||
       cudaMalloc((void **)&c->bis_n, 2 * sizeof(int)) != cudaSuccess ||
       cudaMalloc((void **)&c->sbk, 3 * SNG_BUCKETS * sizeof(int)) != cudaSuccess ||
@@ -3119,8 +3256,11 @@ extern "C" int mr3_cuda_ctx_create_prio(int device, int high, mr3_cuda_ctx **out
     mr3_cuda_ctx_destroy(c);
     return MR3_EMISC;
   }
+  c->sc = reinterpret_cast<SngCounters *>(c->lc + 2);
   int nb = 0;
-  if (cudaFuncSetAttribute(k_sng_round<SNG_LATER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  if (cudaFuncSetAttribute(k_sort_cta, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           2 * SORT_CTA * (int)sizeof(SortRec)) != cudaSuccess ||
+      cudaFuncSetAttribute(k_sng_round<SNG_LATER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            SNG_TILE_BYTES) != cudaSuccess ||
       cudaFuncSetAttribute(k_sng_round<SNG_FIRST>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            SNG_TILE_BYTES) != cudaSuccess) {
@@ -3141,19 +3281,19 @@ extern "C" int mr3_cuda_ctx_create_prio(int device, int high, mr3_cuda_ctx **out
 extern "C" void mr3_cuda_ctx_destroy(mr3_cuda_ctx *c) {
   if (!c) return;
   cudaSetDevice(c->device);
-  void *dev[] = {c->probs, c->blocks, c->blk_of_row, c->Windex, c->iblk, c->It, c->Zindex,
+  void *dev[] = {c->pk, c->blocks, c->blk_of_row, c->Windex, c->iblk, c->It, c->Zindex,
                  c->prob_of_slot, c->cl_of_slot, c->lvl_of_slot, c->unit_list, c->flag, c->tmp2,
                  c->D, c->E, c->E2, c->Wt, c->Et, c->W, c->Werr, c->Wgap, c->Wcopy, c->Wsh,
                  c->Dt, c->Lt, c->Wout, c->gers, c->TP, c->TPc, c->RP, c->RQ, c->rec0, c->rec1,
                  c->cl[0], c->cl[1], c->sng, c->sst, c->act[0], c->act[1], c->bsl, c->sflag, c->sbcnt, c->rlcnt, c->rl, c->rl_n, c->sbk, c->done_list, c->tile_left,
-                 c->bis_nodes[0], c->bis_nodes[1], c->bis_cnt, c->bis_bcnt, c->bis_n, c->bis_st, c->lc, c->sc, c->scratch, c->arena[0],
+                 c->bis_nodes[0], c->bis_nodes[1], c->bis_cnt, c->bis_bcnt, c->bis_n, c->bis_st, c->lc, c->scratch, c->arena[0],
                  c->cls_ns, c->cls_soff, c->cls_cbase, c->cls_abase, c->qd, c->fscratch,
-                 c->arena[1], (void *)c->Din, (void *)c->Ein, c->Wp, c->Dp, c->Ep};
+                 c->arena[1]};
   for (void *q : dev)
     if (q) cudaFree(q);
   for (int i = 0; i < MR3_CUDA_WS_SLOTS; i++)
     if (c->ws[i]) cudaFree(c->ws[i]);
-  void *host[] = {c->h_probs, c->h_ptrs, c->h_lc, c->h_sc, c->h_flag, c->h_const, c->h_iconst, c->h_bisn,
+  void *host[] = {c->h_pk, c->h_lc, c->h_sc, c->h_flag, c->h_const, c->h_iconst, c->h_bisn,
                   c->h_done, c->h_snap};
   for (void *q : host)
     if (q) cudaFreeHost(q);
@@ -3331,9 +3471,15 @@ static int valid_prob(const mr3_cuda_prob &q) {
 
 // Sort the records of the problems selected by (want_job, flag) in place in
 // rec0/rec1; returns the buffer holding the result.
-static int merge_sort_impl(mr3_cuda_ctx *c, cudaStream_t st, int N, int mmax, int want_job,
+static int merge_sort_impl(mr3_cuda_ctx *c, cudaStream_t st, int L, int N, int mmax, int want_job,
                            const int *flag, SortRec **result) {
   SortRec *in = c->rec0, *out = c->rec1;
+  if (mmax <= SORT_CTA) {
+    LAUNCH_SMEM(k_sort_cta, L, 512, 2 * (size_t)mmax * sizeof(SortRec), c->probs, in, mmax, want_job,
+                flag);
+    *result = in;
+    return MR3_OK;
+  }
   // every pass writes every element of every selected problem
   for (int width = 1; width < mmax; width *= 2) {
     LAUNCH(k_merge_pass, (N + 255) / 256, 256, N, c->probs, c->prob_of_slot, in, out, width,
@@ -3344,10 +3490,10 @@ static int merge_sort_impl(mr3_cuda_ctx *c, cudaStream_t st, int N, int mmax, in
   return MR3_OK;
 }
 
-static SortRec *merge_sort(mr3_cuda_ctx *c, cudaStream_t st, int N, int mmax, int want_job,
+static SortRec *merge_sort(mr3_cuda_ctx *c, cudaStream_t st, int L, int N, int mmax, int want_job,
                            const int *flag, int *rc) {
   SortRec *r = c->rec0;
-  *rc = merge_sort_impl(c, st, N, mmax, want_job, flag, &r);
+  *rc = merge_sort_impl(c, st, L, N, mmax, want_job, flag, &r);
   return r;
 }
 
@@ -3355,8 +3501,24 @@ extern "C" int mr3_cuda_solve(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void *s
   return mr3_cuda_solve_cb(c, P, pr, stream, nullptr, nullptr);
 }
 
+static int solve_impl(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void *stream,
+                      mr3_cuda_done_fn done_fn, void *user, bool screen);
+
 extern "C" int mr3_cuda_solve_cb(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void *stream,
                                  mr3_cuda_done_fn done_fn, void *user) {
+  return solve_impl(c, P, pr, stream, done_fn, user, true);
+}
+
+// mr3_cuda_solve_cb for problems whose entries the host library has found
+// finite already (mr3__finite_input): no screening on the device, and no wait
+// for it.
+extern "C" __attribute__((visibility("hidden"))) int mr3__cuda_solve_finite(
+    mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void *stream, mr3_cuda_done_fn done_fn, void *user) {
+  return solve_impl(c, P, pr, stream, done_fn, user, false);
+}
+
+static int solve_impl(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void *stream,
+                      mr3_cuda_done_fn done_fn, void *user, bool screen) {
   if (!c) return MR3_EMISC;
   cudaStream_t st = stream ? (cudaStream_t)stream : c->own;
   // MR3_TREE_LANES caps the lanes per bisection interval (1: a thread each);
@@ -3419,21 +3581,18 @@ extern "C" int mr3_cuda_solve_cb(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void
     if (live[i]) idx.push_back(i);
   int rc = ensure_rows(c, 0, (size_t)nlive);
   if (rc != MR3_OK) return rc;
-  {
+  if (screen) {
     // a problem with a non-finite entry is refused (info 2) before the
     // solve, so that it cannot disturb the others of the batch
     const int Lc = nlive;
+    layout_pk(c, Lc);
     for (int k = 0; k < Lc; k++) {
       c->h_probs[k].n = pr[idx[k]].n;
       c->h_ptrs[k] = (void *)pr[idx[k]].D;
       c->h_ptrs[Lc + k] = (void *)pr[idx[k]].E;
     }
-    CK(cudaMemcpyAsync(c->probs, c->h_probs, Lc * sizeof(ProbDev), cudaMemcpyHostToDevice, st),
-       "screen probs");
-    CK(cudaMemcpyAsync(c->Din, c->h_ptrs, Lc * sizeof(void *), cudaMemcpyHostToDevice, st),
-       "screen D");
-    CK(cudaMemcpyAsync(c->Ein, c->h_ptrs + Lc, Lc * sizeof(void *), cudaMemcpyHostToDevice, st),
-       "screen E");
+    CK(cudaMemcpyAsync(c->pk, c->h_pk, Lc * (sizeof(ProbDev) + 2 * sizeof(void *)),
+                       cudaMemcpyHostToDevice, st), "screen records");
     LAUNCH(k_finite, Lc, 256, c->probs, c->Din, c->Ein, c->flag);
     CK(cudaMemcpyAsync(c->h_flag, c->flag, Lc * sizeof(int), cudaMemcpyDeviceToHost, st),
        "screen flags");
@@ -3463,6 +3622,7 @@ extern "C" int mr3_cuda_solve_cb(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void
   const int L = nlive;
   rc = ensure_rows(c, N, (size_t)L);
   if (rc != MR3_OK) return rc;
+  layout_pk(c, L);
   // column tiles of the problems whose column count is known up front
   // (jobz V, range A or I); finished tiles are reported to done_fn at the
   // host's syncs (the kernels that wrote them have finished)
@@ -3520,8 +3680,8 @@ extern "C" int mr3_cuda_solve_cb(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void
   // the counters (and the tiles finished since the last export) go to the
   // host through k_export; the host waits for it, reporting the tiles of
   // the rounds before it as they complete
-  auto sync_counters = [&](LevelCounters *lc, const char *what) -> int {
-    LAUNCH(k_export, 1, 256, lc, lc ? c->d_hlc : nullptr, c->sc, c->d_hsc, c->done_list,
+  auto sync_counters = [&](LevelCounters *lc, LevelCounters *lc_next, const char *what) -> int {
+    LAUNCH(k_export, 1, 256, lc, lc_next, lc ? c->d_hlc : nullptr, c->sc, c->d_hsc, c->done_list,
            tiles ? c->d_hdone : nullptr, nullptr);
     for (int i = 0; i < npend; i++) {
       CK(cudaEventSynchronize(c->rev[i]), "round event");
@@ -3552,12 +3712,8 @@ extern "C" int mr3_cuda_solve_cb(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void
       c->h_ptrs[4 * L + k] = (void *)q.E;
     }
   }
-  CK(cudaMemcpyAsync(c->probs, c->h_probs, L * sizeof(ProbDev), cudaMemcpyHostToDevice, st), "probs");
-  CK(cudaMemcpyAsync(c->Din, c->h_ptrs, L * sizeof(void *), cudaMemcpyHostToDevice, st), "Din");
-  CK(cudaMemcpyAsync(c->Ein, c->h_ptrs + L, L * sizeof(void *), cudaMemcpyHostToDevice, st), "Ein");
-  CK(cudaMemcpyAsync(c->Wp, c->h_ptrs + 2 * L, L * sizeof(void *), cudaMemcpyHostToDevice, st), "Wp");
-  CK(cudaMemcpyAsync(c->Dp, c->h_ptrs + 3 * L, L * sizeof(void *), cudaMemcpyHostToDevice, st), "Dp");
-  CK(cudaMemcpyAsync(c->Ep, c->h_ptrs + 4 * L, L * sizeof(void *), cudaMemcpyHostToDevice, st), "Ep");
+  CK(cudaMemcpyAsync(c->pk, c->h_pk, L * (sizeof(ProbDev) + 5 * sizeof(void *)),
+                     cudaMemcpyHostToDevice, st), "problem records");
 
   Tol tol;
   tol.rtol1 = fmin(sqrt(2.220446049250313e-16), 1e-2 * 1e-3);
@@ -3573,7 +3729,8 @@ extern "C" int mr3_cuda_solve_cb(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void
   const int gN = (NN + 255) / 256, gN128 = (NN + 127) / 128;
 
   // ---- stage A: eigenvalues
-  LAUNCH(k_gather, L, 256, c->probs, c->Din, c->Ein, c->D, c->E, c->prob_of_slot, c->iblk);
+  LAUNCH(k_gather, L, 256, c->probs, c->Din, c->Ein, c->D, c->E, c->prob_of_slot, c->iblk,
+         c->lvl_of_slot, c->flag);
   LAUNCH(k_prologue, L, MR3_THREADS, c->probs, c->blocks, c->blk_of_row, c->D, c->E, c->E2,
          c->gers, c->TP, c->TPc, tol);
   LAUNCH(k_blocks, L, MR3_THREADS, c->probs, c->blocks, c->D, c->E, c->gers, c->TP, tol);
@@ -3631,15 +3788,14 @@ extern "C" int mr3_cuda_solve_cb(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void
   // ---- stage B: eigenvectors
   if (anyV) {
     LAUNCH(k_zkeys, L, MR3_THREADS, c->probs, c->blocks, c->W, c->E, c->Windex, c->rec0);
-    SortRec *sorted = merge_sort(c, st, NN, mmax, MR3_JOB_V, nullptr, &rc);
+    SortRec *sorted = merge_sort(c, st, L, NN, mmax, MR3_JOB_V, nullptr, &rc);
     if (rc != MR3_OK) { snprintf(c->err, sizeof(c->err), "merge sort"); return rc; }
     LAUNCH(k_zindex_from_sorted, gN, 256, NN, c->probs, c->prob_of_slot, sorted, c->Zindex);
-    CK(cudaMemsetAsync(c->lc, 0, 2 * sizeof(LevelCounters), st), "lc");
-    CK(cudaMemsetAsync(c->sc, 0, sizeof(SngCounters), st), "sc");
-    CK(cudaMemsetAsync(c->lvl_of_slot, 0xff, N * sizeof(int), st), "lvl");
+    // (the two LevelCounters and the SngCounters lie side by side)
+    CK(cudaMemsetAsync(c->lc, 0, 2 * sizeof(LevelCounters) + sizeof(SngCounters), st), "counters");
     LAUNCH(k_level0, L, MR3_THREADS, c->probs, c->blocks, c->E, c->gers, c->W, c->Werr, c->Wsh,
            c->cl[0], &c->lc[0], c->sc, c->unit_list);
-    if ((rc = sync_counters(c->lc, "level0 sync")) != MR3_OK) return rc;
+    if ((rc = sync_counters(c->lc, nullptr, "level0 sync")) != MR3_OK) return rc;
     if (c->h_sc->n_unit > 0)
       LAUNCH(k_unitvec, c->h_sc->n_unit, 256, c->unit_list, c->sc, c->probs, c->blocks, c->iblk,
              c->Zindex, c->done_list, c->tile_left);
@@ -3674,23 +3830,28 @@ extern "C" int mr3_cuda_solve_cb(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void
         if (2LL * ncl <= lanes)
           LAUNCH(k_cl_rrf<true>, (int)((2LL * ncl + 127) / 128), 128, ncl, c->cl[cur], c->probs,
                  c->blocks, c->RP, c->RQ, c->arena[nxt], c->arena[cur], c->Wt, c->Et, c->Wsh,
-                 c->Werr, c->Wgap, stats);
+                 c->Werr, c->Wgap, c->rl_n, stats);
         else
           LAUNCH(k_cl_rrf<false>, (ncl + 127) / 128, 128, ncl, c->cl[cur], c->probs, c->blocks,
                  c->RP, c->RQ, c->arena[nxt], c->arena[cur], c->Wt, c->Et, c->Wsh, c->Werr,
-                 c->Wgap, stats);
-        CK(cudaMemsetAsync(c->rl_n, 0, sizeof(int), st), "rl_n");
+                 c->Wgap, c->rl_n, stats);
         LAUNCH(k_cl_pack, std::min(ncl, 65535 * 16), 256, ncl, c->cl[cur], c->blocks, c->arena[cur],
                c->Wsh, c->Werr, c->cl_of_slot, c->lvl_of_slot, level, c->rl_n);
-        {
+        if (NN <= RL_CTA) {
+          LAUNCH(k_rl_small, 1, 1024, NN, c->lvl_of_slot, level, c->rl);
+        } else {
           const int nrb = (int)((NN + RL_T - 1) / RL_T);
           LAUNCH(k_rl_count, nrb, 256, NN, c->lvl_of_slot, level, c->rlcnt);
           LAUNCH(k_rl_scan, 1, 1024, nrb, c->rlcnt);
           LAUNCH(k_rl_scatter, nrb, 256, NN, c->lvl_of_slot, level, c->rlcnt, c->rl);
         }
         // both forms are launched; the one that does not match the list's
-        // length returns at once (the length is known on the device only)
-        LAUNCH(k_refine_cl<false>, gN128, 128, c->rl, c->rl_n, c->cl[cur], c->probs, c->blocks,
+        // length returns at once (the length is known on the device only).
+        // Up to two threads' warps a quarter SM (the thread form's row costs
+        // its latency), a list shorter than one for lane groups is one too.
+        const bool all_tree = NN <= 2LL * 32 * 4 * c->nsm && tree_lanes(NN, c->nsm, tree_max) > 1;
+        if (!all_tree)
+          LAUNCH(k_refine_cl<false>, gN128, 128, c->rl, c->rl_n, c->cl[cur], c->probs, c->blocks,
                c->arena[cur], c->Wsh, c->Werr, c->Wgap, c->Windex, c->cl_of_slot, c->lvl_of_slot,
                level, tol, c->nsm, tree_max, stats);
         LAUNCH(k_refine_cl<true>, (int)(lanes / TREE_T), TREE_T, c->rl, c->rl_n, c->cl[cur], c->probs,
@@ -3705,19 +3866,21 @@ extern "C" int mr3_cuda_solve_cb(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void
         CK(cudaStreamWaitEvent(st, c->rnd_done, 0), "rounds wait");
         rounds_pending = false;
       }
-      CK(cudaMemsetAsync(&c->lc[nxt], 0, sizeof(LevelCounters), st), "lcn");
-      CK(cudaMemsetAsync(&c->sc->n_sng, 0, sizeof(int), st), "scn");
       LAUNCH(k_classify<0>, gW, MR3_THREADS, ncl, c->cl[cur], c->blocks, c->Wsh, c->Wgap,
              c->cl[nxt], c->sng, &c->lc[nxt], xs, NN);
-      CK(cudaMemsetAsync(c->sbk, 0, 3 * SNG_BUCKETS * sizeof(int), st), "sbk");
-      LAUNCH(k_group_tasks<0>, (ncl + 127) / 128, 128, ncl, c->cl[cur], c->blocks, xs, c->sc, c->sbk,
-             &c->lc[nxt], NN);
-      LAUNCH(k_bucket_scan, 1, 1, c->sbk);
-      LAUNCH(k_group_tasks<1>, (ncl + 127) / 128, 128, ncl, c->cl[cur], c->blocks, xs, c->sc, c->sbk,
-             &c->lc[nxt], NN);
+      if (ncl <= GROUP_CTA) {
+        LAUNCH(k_group_small, 1, 1024, ncl, c->cl[cur], c->blocks, xs, c->sc, &c->lc[nxt], NN);
+      } else {
+        CK(cudaMemsetAsync(c->sbk, 0, 3 * SNG_BUCKETS * sizeof(int), st), "sbk");
+        LAUNCH(k_group_tasks<0>, (ncl + 127) / 128, 128, ncl, c->cl[cur], c->blocks, xs, c->sc, c->sbk,
+               &c->lc[nxt], NN);
+        LAUNCH(k_bucket_scan, 1, 1, c->sbk, c->sc);
+        LAUNCH(k_group_tasks<1>, (ncl + 127) / 128, 128, ncl, c->cl[cur], c->blocks, xs, c->sc, c->sbk,
+               &c->lc[nxt], NN);
+      }
       LAUNCH(k_classify<1>, gW, MR3_THREADS, ncl, c->cl[cur], c->blocks, c->Wsh, c->Wgap,
              c->cl[nxt], c->sng, &c->lc[nxt], xs, NN);
-      if ((rc = sync_counters(&c->lc[nxt], "level sync")) != MR3_OK) return rc;
+      if ((rc = sync_counters(&c->lc[nxt], &c->lc[cur], "level sync")) != MR3_OK) return rc;
       if (c->h_lc->err) { snprintf(c->err, sizeof(c->err), "queue overflow"); return MR3_EMISC; }
       if ((rc = report_done()) != MR3_OK) return rc;
       if (c->h_sc->err) { snprintf(c->err, sizeof(c->err), "singleton rounds exhausted"); return MR3_EMISC; }
@@ -3777,7 +3940,7 @@ extern "C" int mr3_cuda_solve_cb(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void
         trace_t0 = std::chrono::steady_clock::now();
         for (int rd = 0; rd < SNG_ROUNDS; rd++) {
           const int in = rd & 1, last = rd == SNG_ROUNDS - 1;
-          LAUNCH(k_round_reset, 1, 1, c->sc, in, rd == 0);
+          if (rd > 0) LAUNCH(k_round_reset, 1, 1, c->sc, in);
           if (direct)
             LAUNCH(k_sng_finish<FIN_FIRST>, fin_ctas, FIN_WARPS * 32, in, c->sng, c->cl[cur], c->probs,
                    c->blocks, c->RP, c->RQ, c->arena[cur], c->W, c->Wsh, c->Werr, c->Wgap,
@@ -3806,7 +3969,7 @@ extern "C" int mr3_cuda_solve_cb(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void
                         c->sflag, c->sc, c->scratch, (long long)nmaxV, c->done_list, c->tile_left,
                         stats);
           if (tiles) {
-            LAUNCH(k_export, 1, 256, nullptr, nullptr, c->sc, nullptr, c->done_list, c->d_hdone,
+            LAUNCH(k_export, 1, 256, nullptr, nullptr, nullptr, c->sc, nullptr, c->done_list, c->d_hdone,
                    c->d_hsnap + npend);
             CK(cudaEventRecord(c->rev[npend], st), "round record");
             npend++;
@@ -3848,9 +4011,6 @@ extern "C" int mr3_cuda_solve_cb(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void
       }
     }
     if (rounds_pending) CK(cudaStreamWaitEvent(st, c->rnd_done, 0), "rounds wait");
-    if ((rc = sync_counters(nullptr, "rounds sync")) != MR3_OK) return rc;
-    if (c->h_sc->err) { snprintf(c->err, sizeof(c->err), "singleton rounds exhausted"); return MR3_EMISC; }
-    if ((rc = report_done()) != MR3_OK) return rc;
   }
 
   // ---- post-processing (SRC/mrrr.c:262-285)
@@ -3863,17 +4023,30 @@ extern "C" int mr3_cuda_solve_cb(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void
   LAUNCH(k_invscale, gN, 256, NN, c->probs, c->blocks, c->iblk, c->W);
   if (anyV) {
     LAUNCH(k_place_w, gN, 256, NN, c->probs, c->prob_of_slot, c->W, c->Zindex, c->Wout);
-    CK(cudaMemsetAsync(c->flag, 0, L * sizeof(int), st), "flag");
     LAUNCH(k_check_sorted, gN, 256, NN, c->probs, c->prob_of_slot, c->Wout, c->flag);
     CK(cudaMemcpyAsync(c->h_flag, c->flag, L * sizeof(int), cudaMemcpyDeviceToHost, st), "flag d2h");
-    CK(cudaStreamSynchronize(st), "flag sync");
+  }
+  if (anyN) {
+    LAUNCH(k_wkeys, gN, 256, NN, c->probs, c->prob_of_slot, c->W, c->rec0, MR3_JOB_N, nullptr);
+    SortRec *sorted = merge_sort(c, st, L, NN, mmax, MR3_JOB_N, nullptr, &rc);
+    if (rc != MR3_OK) return rc;
+    LAUNCH(k_sorted_to_w, gN, 256, NN, c->probs, c->prob_of_slot, sorted, c->Wout, MR3_JOB_N, nullptr);
+  }
+  LAUNCH(k_scatter, L, 256, c->probs, c->Wp, c->Dp, c->Ep, c->Wout, c->D, c->E);
+  CK(cudaMemcpyAsync(c->h_probs, c->probs, L * sizeof(ProbDev), cudaMemcpyDeviceToHost, st), "probs d2h");
+  if (!anyV) {
+    CK(cudaStreamSynchronize(st), "final sync");
+  } else {
+    if ((rc = sync_counters(nullptr, nullptr, "final sync")) != MR3_OK) return rc;
+    if (c->h_sc->err) { snprintf(c->err, sizeof(c->err), "singleton rounds exhausted"); return MR3_EMISC; }
+    if ((rc = report_done()) != MR3_OK) return rc;
     bool anyUnsorted = false;
     for (int k = 0; k < L; k++) anyUnsorted |= (c->h_flag[k] != 0);
     if (anyUnsorted) {
       // bubble fix-up of sort_eigenpairs == stable sort by value of the
       // columns in output order; permute W, Zsupp and the Z columns
       LAUNCH(k_wkeys, gN, 256, NN, c->probs, c->prob_of_slot, c->Wout, c->rec0, MR3_JOB_V, c->flag);
-      SortRec *sorted = merge_sort(c, st, NN, mmax, MR3_JOB_V, c->flag, &rc);
+      SortRec *sorted = merge_sort(c, st, L, NN, mmax, MR3_JOB_V, c->flag, &rc);
       if (rc != MR3_OK) return rc;
       LAUNCH(k_sorted_to_w, gN, 256, NN, c->probs, c->prob_of_slot, sorted, c->Wout, MR3_JOB_V, c->flag);
       LAUNCH(k_perm_zsupp, gN, 256, NN, c->probs, c->prob_of_slot, sorted, c->flag, c->tmp2);
@@ -3916,17 +4089,10 @@ extern "C" int mr3_cuda_solve_cb(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void
           done_fn(user, c->h_dprob.data(), c->h_dcol.data(), c->h_dcnt.data(),
                   (int)c->h_dprob.size());
       }
+      LAUNCH(k_scatter, L, 256, c->probs, c->Wp, c->Dp, c->Ep, c->Wout, c->D, c->E);
+      CK(cudaStreamSynchronize(st), "order sync");
     }
   }
-  if (anyN) {
-    LAUNCH(k_wkeys, gN, 256, NN, c->probs, c->prob_of_slot, c->W, c->rec0, MR3_JOB_N, nullptr);
-    SortRec *sorted = merge_sort(c, st, NN, mmax, MR3_JOB_N, nullptr, &rc);
-    if (rc != MR3_OK) return rc;
-    LAUNCH(k_sorted_to_w, gN, 256, NN, c->probs, c->prob_of_slot, sorted, c->Wout, MR3_JOB_N, nullptr);
-  }
-  LAUNCH(k_scatter, L, 256, c->probs, c->Wp, c->Dp, c->Ep, c->Wout, c->D, c->E);
-  CK(cudaMemcpyAsync(c->h_probs, c->probs, L * sizeof(ProbDev), cudaMemcpyDeviceToHost, st), "probs d2h");
-  CK(cudaStreamSynchronize(st), "final sync");
   if (c->prof) prof_flush(c);
 
   for (int k = 0; k < L; k++) {
