@@ -326,56 +326,102 @@ static __device__ __noinline__ int dv_count_guess(int n, const double2 *__restri
   return cnt;
 }
 
-// One interval of dlaebz IJOB=3 from the user-supplied point c, by a group of
-// L lanes (L = 2..32, a power of two; every lane of the group passes the same
-// arguments and gets the same results).  The first count is at the given
-// point c, as in the sequential loop; after it the points are midpoints, and the midpoints of the next log2(L) steps form a binary
-// tree that follows from the current interval: lane t of the group counts
-// at node max(t,1) (heap numbering; its interval computed along the node's
-// path with the loop's operations), then the group walks the tree applying
-// the loop's updates and tests after each step.  A count equal to nval
-// closes the interval (a = b = c), which the width test then stops.  The
+// One step of dlaebz IJOB=3: the count cv at the point c closes the interval
+// from one side, from both when it equals nval.  True when the loop ends.
+static __device__ __forceinline__ bool ijob3_step(double c, int cv, int nval, double tol0,
+                                                  double reltol, int nitmax, double *a, double *b,
+                                                  int *na, int *nb, int *it) {
+  if (cv <= nval) { *a = c; *na = cv; }
+  if (cv >= nval) { *b = c; *nb = cv; }
+  ++*it;
+  const double w = fabs(*b - *a), tt = fmax(fabs(*b), fabs(*a));
+  return w < fmax(tol0, reltol * tt) || *na >= *nb || *it >= nitmax;
+}
+
+// One interval of dlaebz IJOB=3 from the user-supplied point c, by L lanes
+// that follow one another (every lane of the group passes the same arguments
+// and gets the same results).  The first step is at the given point c, whose
+// count the caller passes (cnt0), as in the sequential loop; after it the
+// points are midpoints, and the midpoints of the next log2(L) steps form a
+// binary tree that follows from the current interval: lane t of the group
+// counts at node max(t,1) (heap numbering; its interval computed along the
+// node's path with the loop's operations), then the group walks the tree
+// applying the loop's updates and tests after each step.  A count equal to
+// nval closes the interval (a = b = c), which the width test then stops.  The
 // same points, counts and results as the loop; log2(L) steps per count.
-static __device__ __noinline__ void dv_ijob3_tree(int L, int n, const double2 *__restrict__ tp,
+//   Down to a relative width of 2^-36 the counts are guessed (dv_count_guess:
+// half the latency, a third of the FP64 operations, so that half a CTA walks
+// 7 steps in less than a warp's 5 took).  Then one pass of exact counts at the
+// last points below and above nval and at a closing one confirms the walk: the
+// Sturm count does not decrease with the point, so the exact counts at all
+// earlier points lie on the same sides.  An unconfirmed walk is repeated with
+// exact counts, as the steps below that width are.
+//   cnt == nullptr: L = 2..32, a power of two; the whole warp calls.
+//   cnt != nullptr: shared memory of an int per thread; L a multiple of 32 and
+//   a power of two; the whole CTA calls, its groups one behind the other.
+// The groups go on together until the last is done.
+#define IJOB3_WIDTH 1.4551915228366852e-11   // 2^-36
+static __device__ __noinline__ void dv_ijob3_tree(int L, int *cnt, int n, const double2 *__restrict__ tp,
                                            double pivmin, double abstol, double reltol,
-                                           int nitmax, int nval, double c, double *a_,
+                                           int nitmax, int nval, double c, int cnt0, double *a_,
                                            double *b_, int *na_, int *nb_) {
-  const int lane = threadIdx.x & 31;
-  const int t = lane & (L - 1), g0 = lane - t, depth = 31 - __clz(L);
-  const unsigned gm = ((L == 32) ? 0xffffffffu : ((1u << L) - 1u)) << g0;
+  const int tid = cnt ? (int)threadIdx.x : (int)(threadIdx.x & 31);
+  const int t = tid & (L - 1), g0 = tid - t, depth = 31 - __clz(L);
   const int node_t = t == 0 ? 1 : t;
   const double tol0 = fmax(abstol, pivmin);
   double a = *a_, b = *b_;
   int na = *na_, nb = *nb_, it = 0;
   bool done = nitmax < 1;
-  if (!done) {   // the first step, at the given point
-    const int cnt = dv_count_lat<CNT_BISECT>(n, tp, pivmin, c);
-    if (cnt <= nval) { a = c; na = cnt; }
-    if (cnt >= nval) { b = c; nb = cnt; }
-    it = 1;
-    const double w = fabs(b - a), tt = fmax(fabs(b), fabs(a));
-    if (w < fmax(tol0, reltol * tt) || na >= nb || it >= nitmax) done = true;
-  }
-  while (!done) {
-    double l = a, r = b;
-    for (int k = 30 - __clz(node_t); k >= 0; k--) {
-      const double m = 0.5 * (l + r);
-      if ((node_t >> k) & 1) l = m; else r = m;
-    }
-    const int raw = dv_count_lat<CNT_BISECT>(n, tp, pivmin, 0.5 * (l + r));
-    int node = 1;
-    for (int d = 0; d < depth; d++) {
-      const int cv = __shfl_sync(gm, raw, g0 + node);
-      if (!done) {
-        const double cm = 0.5 * (a + b);
-        if (cv <= nval) { a = cm; na = cv; }
-        if (cv >= nval) { b = cm; nb = cv; }
-        node = (cv < nval) ? 2 * node + 1 : 2 * node;
-        it++;
-        const double w = fabs(b - a), tt = fmax(fabs(b), fabs(a));
-        if (w < fmax(tol0, reltol * tt) || na >= nb || it >= nitmax) done = true;
+  if (!done) done = ijob3_step(c, cnt0, nval, tol0, reltol, nitmax, &a, &b, &na, &nb, &it);
+  const double sa = a, sb = b;
+  const int sna = na, snb = nb, sit = it;
+  const bool sdone = done;
+  for (int pass = 0; pass < 2; pass++) {   // guessed, then exact
+    bool stop = done;
+    while (cnt ? __syncthreads_or(!stop) : __any_sync(0xffffffffu, !stop)) {
+      double l = a, r = b;
+      for (int k = 30 - __clz(node_t); k >= 0; k--) {
+        const double m = 0.5 * (l + r);
+        if ((node_t >> k) & 1) l = m; else r = m;
+      }
+      const double x = 0.5 * (l + r);
+      const int raw = pass == 0 ? dv_count_guess(n, tp, pivmin, x)
+                                : dv_count_lat<CNT_BISECT>(n, tp, pivmin, x);
+      if (cnt) {
+        cnt[tid] = raw;
+        __syncthreads();
+      }
+      int node = 1;
+      for (int d = 0; d < depth; d++) {
+        const int cv = cnt ? cnt[g0 + node] : __shfl_sync(0xffffffffu, raw, g0 + node);
+        if (!stop) {
+          done = ijob3_step(0.5 * (a + b), cv, nval, tol0, reltol, nitmax, &a, &b, &na, &nb, &it);
+          node = (cv < nval) ? 2 * node + 1 : 2 * node;
+          stop = done || (pass == 0 &&
+                          !(fabs(b - a) > IJOB3_WIDTH * fmax(fabs(b), fabs(a))));
+        }
       }
     }
+    if (pass == 1) break;
+    // lane 0 counts at a, lane 1 at b (the same point when one closed it)
+    const bool walked = it > sit;
+    if (!(cnt ? __syncthreads_or(walked) : __any_sync(0xffffffffu, walked))) continue;
+    const int raw = dv_count_lat<CNT_BISECT>(n, tp, pivmin, (t & 1) ? b : a);
+    if (cnt) {
+      cnt[tid] = raw;
+      __syncthreads();
+    }
+    const int ea = cnt ? cnt[g0] : __shfl_sync(0xffffffffu, raw, g0);
+    const int eb = cnt ? cnt[g0 + 1] : __shfl_sync(0xffffffffu, raw, g0 + 1);
+    const bool closed = walked && na == nval && nb == nval;
+    bool ok = true;
+    if (closed) ok = ea == nval;
+    else {
+      if (a != sa || na != sna) { ok &= ea < nval; na = ea; }
+      if (b != sb || nb != snb) { ok &= eb > nval; nb = eb; }
+    }
+    if (!ok) { a = sa; b = sb; na = sna; nb = snb; it = sit; done = sdone; }
+    if (cnt) __syncthreads();
   }
   *a_ = a;
   *b_ = b;

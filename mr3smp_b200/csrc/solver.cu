@@ -265,9 +265,9 @@ __global__ void k_finite(const ProbDev *probs, const double *const *Din, const d
 
 __global__ void __launch_bounds__(MR3_THREADS)
 k_prologue(ProbDev *probs, BlockDev *blocks, int *blk_of_row, double *D, double *E, double *E2,
-           double2 *gers, double2 *TP, double2 *TPc, Tol tol) {
+           double2 *gers, double2 *TP, double2 *TPc, Tol tol, int wide) {
   __shared__ double sred[32];
-  __shared__ int sint[64];
+  __shared__ int sint[64], cnt_sh[MR3_THREADS];
   __shared__ int sflag;
   ProbDev *p = &probs[blockIdx.x];
   const int n = p->n, off = p->off, tid = threadIdx.x, nt = blockDim.x;
@@ -460,41 +460,54 @@ k_prologue(ProbDev *probs, BlockDev *blocks, int *blk_of_row, double *D, double 
   }
   if (p->jobz == MR3_JOB_C) return;
   // ---- range I: the interval holding eigenvalues il..iu (SRC/mrrr_val.c:295-319),
-  // the two searches by warps 0 and 1, each with the tree form
-  if (irange == MR3_RANGE_I && tid < 64) {
+  // the two searches by half a CTA each, by warps 0 and 1 in larger batches
+  // (`wide` and its line: see k_blocks).  Half a CTA: 13.1 -> 12.5 ms for the
+  // 20010 rows of a glued matrix, whose searches run to the last bits, which
+  // take exact counts.
+  if (irange == MR3_RANGE_I && (wide || tid < 64)) {
+    const int L = wide ? MR3_THREADS / 2 : 32;
+    const bool up = tid >= L;
     int itmax = (int)((dv_log(p->tnorm + pivmin) - dv_log(pivmin)) / dv_log(2.0) + 2);
     double atoli = 2 * (2 * MR3_SAFMIN + 2 * pivmin);
     double a = p->gl, bq = p->gu;
     int na = -1, nb = n + 1;
-    if (tid < 32) {
-      dv_ijob3_tree(32, n, TP + off, pivmin, atoli, tol.rqtol, itmax, p->il - 1, p->gl, &a, &bq,
-                    &na, &nb);
-      if (tid == 0) { p->wl = a; p->wlu = bq; p->nwl = na; p->vl_out = a; }
-    } else {
-      dv_ijob3_tree(32, n, TP + off, pivmin, atoli, tol.rqtol, itmax, p->iu, p->gu, &a, &bq, &na,
-                    &nb);
-      if (tid == 32) { p->wul = a; p->wu = bq; p->nwu = nb; p->vu_out = bq; }
-    }
+    const double c0 = up ? bq : a;
+    const int cnt0 = dv_count_lat<CNT_BISECT>(n, TP + off, pivmin, c0);
+    dv_ijob3_tree(L, wide ? cnt_sh : nullptr, n, TP + off, pivmin, atoli, tol.rqtol, itmax,
+                  up ? p->iu : p->il - 1, c0, cnt0, &a, &bq, &na, &nb);
+    if (tid == 0) { p->wl = a; p->wlu = bq; p->nwl = na; p->vl_out = a; }
+    if (tid == L) { p->wul = a; p->wu = bq; p->nwu = nb; p->vu_out = bq; }
   }
 }
 
 // ------------------------------------------------------------------------
 // Stage A1: per-block setup (SRC/mrrr_val.c:340-412 and the set-up part of
-// dlarrd, SRC/LAPACK/odrrd.f:283-450).  One warp per block.
+// dlarrd, SRC/LAPACK/odrrd.f:283-450).  One warp per block; with `wide` (no
+// more problems than SMs) a problem's only block gets the whole CTA: every
+// warp runs the same operations on the same values, warps 0 and 1 count the
+// four first points side by side, the two searches have half the CTA each.
+// Bound by the latency of the counts (95 cycles a row, one after another).
+// Two warps a scheduler fit into a guessed row's 48 cycles, so that a CTA's
+// wide search costs one CTA an SM nothing and would cost a second one.  The
+// interval of a 2000-row matrix: 1.03 -> 0.49 ms (half-warps, exact counts
+// before); half CTAs with exact counts were no faster than half-warps.
 // ------------------------------------------------------------------------
 __global__ void __launch_bounds__(MR3_THREADS)
 k_blocks(ProbDev *probs, BlockDev *blocks, const double *D, double *E, const double2 *gers,
-         const double2 *TP, Tol tol) {
+         const double2 *TP, Tol tol, int wide) {
   ProbDev *p = &probs[blockIdx.x];
   if (p->trivial || p->jobz == MR3_JOB_C) return;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const double pivmin = p->pivmin, tnorm = p->tnorm, wl = p->wl, wu = p->wu;
   const int irange = p->irange;
-  for (int b = wid; b < p->nsplit; b += nw) {
+  __shared__ int cnt_sh[MR3_THREADS], first_sh[4];
+  if (p->nsplit != 1) wide = 0;
+  const bool lead = lane == 0 && (!wide || wid == 0);   // writes the block's record
+  for (int b = wide ? 0 : wid; b < p->nsplit; b += nw) {
     BlockDev *B = &blocks[p->off + b];
     const int ibgn = B->ibgn, iend = B->iend, nbl = B->nbl;
     if (nbl == 1) {
-      if (lane == 0) {
+      if (lead) {
         double dv = D[ibgn];
         bool take = (irange == MR3_RANGE_A) || (irange == MR3_RANGE_V && dv > wl && dv <= wu) ||
                     (irange == MR3_RANGE_I && (dv + pivmin) > wl && (dv - pivmin) <= wu);
@@ -516,16 +529,35 @@ k_blocks(ProbDev *probs, BlockDev *blocks, const double *D, double *E, const dou
     bgu = warp_max(bgu);
     const double bglf = bgl - 2 * tnorm * MR3_EPS * nbl - 4 * pivmin;
     const double bguf = bgu + 2 * tnorm * MR3_EPS * nbl + 4 * pivmin;
-    int ilow = 1, iupp = nbl;
+    const double tnb = fmax(fabs(bgl), fabs(bgu));
+    const double gl2 = bgl - 2.0 * tnb * MR3_EPS * nbl - 2.0 * 2.0 * pivmin;
+    const double gu2 = bgu + 2.0 * tnb * MR3_EPS * nbl + 2.0 * 2.0 * pivmin;
+    int ilow = 1, iupp = nbl, cl0 = 0, cu0 = 0;   // cl0, cu0: counts at gl2, gu2
     if (irange != MR3_RANGE_A) {
-      int c = 0;
-      if (lane < 2)
-        c = dv_count_lat<CNT_IJOB1>(nbl, TP + ibgn, pivmin, lane == 0 ? fmax(wl, bglf) : fmin(wu, bguf));
-      ilow = __shfl_sync(0xffffffffu, c, 0) + 1;
-      iupp = __shfl_sync(0xffffffffu, c, 1);
+      if (!wide || wid == 0) {
+        int c = 0;
+        if (lane < 2)
+          c = dv_count_lat<CNT_IJOB1>(nbl, TP + ibgn, pivmin,
+                                      lane == 0 ? fmax(wl, bglf) : fmin(wu, bguf));
+        ilow = __shfl_sync(0xffffffffu, c, 0) + 1;
+        iupp = __shfl_sync(0xffffffffu, c, 1);
+      }
+      if (wide && wid == 1) {
+        int c = 0;
+        if (lane < 2) c = dv_count_lat<CNT_BISECT>(nbl, TP + ibgn, pivmin, lane == 0 ? gl2 : gu2);
+        cl0 = __shfl_sync(0xffffffffu, c, 0);
+        cu0 = __shfl_sync(0xffffffffu, c, 1);
+      }
+      if (wide) {
+        if (threadIdx.x == 0) { first_sh[0] = ilow; first_sh[1] = iupp; }
+        if (threadIdx.x == 32) { first_sh[2] = cl0; first_sh[3] = cu0; }
+        __syncthreads();
+        ilow = first_sh[0]; iupp = first_sh[1];
+        cl0 = first_sh[2]; cu0 = first_sh[3];
+      }
     }
     const int mbl = iupp - ilow + 1;
-    if (lane == 0) {
+    if (lead) {
       B->bgl = bglf; B->bgu = bguf; B->spdiam = bguf - bglf;
       B->ilow = ilow; B->iupp = iupp; B->mbl = mbl;
       B->none = 1; B->nab1 = 0; B->nab2 = 0;
@@ -535,9 +567,6 @@ k_blocks(ProbDev *probs, BlockDev *blocks, const double *D, double *E, const dou
     if (mbl <= 0) continue;
     // dlarrd("I","B") set-up on this block
     const int brange = (ilow == 1 && iupp == nbl) ? MR3_RANGE_A : MR3_RANGE_I;
-    const double tnb = fmax(fabs(bgl), fabs(bgu));
-    const double gl2 = bgl - 2.0 * tnb * MR3_EPS * nbl - 2.0 * 2.0 * pivmin;
-    const double gu2 = bgu + 2.0 * tnb * MR3_EPS * nbl + 2.0 * 2.0 * pivmin;
     const double atoli = 2.0 * 2.0 * MR3_SAFMIN + 2.0 * 2.0 * pivmin;
     double wlb = gl2, wub = gu2, wlub = 0.0, wulb = 0.0;
     int bad = 0;
@@ -545,12 +574,26 @@ k_blocks(ProbDev *probs, BlockDev *blocks, const double *D, double *E, const dou
       int itmax = dv_itmax(tnb + pivmin, pivmin);
       double a = gl2, bq = gu2;
       int na = -1, nb = nbl + 1;
-      // the two searches by half-warps at once, each with the tree form
-      dv_ijob3_tree(16, nbl, TP + ibgn, pivmin, atoli, tol.bsrtol, itmax,
-                    lane < 16 ? ilow - 1 : iupp, lane < 16 ? gl2 : gu2, &a, &bq, &na, &nb);
-      double a0 = __shfl_sync(0xffffffffu, a, 0), b0 = __shfl_sync(0xffffffffu, bq, 0);
-      double a1 = __shfl_sync(0xffffffffu, a, 16), b1 = __shfl_sync(0xffffffffu, bq, 16);
-      int nwl = __shfl_sync(0xffffffffu, na, 0), nwu = __shfl_sync(0xffffffffu, nb, 16);
+      // the two searches at once, by half-warps or half CTAs
+      const int L = wide ? MR3_THREADS / 2 : 16;
+      const bool up = wide ? (int)threadIdx.x >= L : lane >= L;
+      if (!wide) cl0 = cu0 = dv_count_lat<CNT_BISECT>(nbl, TP + ibgn, pivmin, up ? gu2 : gl2);
+      dv_ijob3_tree(L, wide ? cnt_sh : nullptr, nbl, TP + ibgn, pivmin, atoli, tol.bsrtol, itmax,
+                    up ? iupp : ilow - 1, up ? gu2 : gl2, up ? cu0 : cl0, &a, &bq, &na, &nb);
+      double a0, b0, a1, b1;
+      int nwl, nwu;
+      if (wide) {
+        __shared__ double ab_sh[4];
+        if (threadIdx.x == 0) { ab_sh[0] = a; ab_sh[1] = bq; first_sh[0] = na; }
+        if ((int)threadIdx.x == L) { ab_sh[2] = a; ab_sh[3] = bq; first_sh[1] = nb; }
+        __syncthreads();
+        a0 = ab_sh[0]; b0 = ab_sh[1]; a1 = ab_sh[2]; b1 = ab_sh[3];
+        nwl = first_sh[0]; nwu = first_sh[1];
+      } else {
+        a0 = __shfl_sync(0xffffffffu, a, 0); b0 = __shfl_sync(0xffffffffu, bq, 0);
+        a1 = __shfl_sync(0xffffffffu, a, 16); b1 = __shfl_sync(0xffffffffu, bq, 16);
+        nwl = __shfl_sync(0xffffffffu, na, 0); nwu = __shfl_sync(0xffffffffu, nb, 16);
+      }
       wlb = a0; wlub = b0; wulb = a1; wub = b1;
       if (nwl < 0 || nwl >= nbl || nwu < 1 || nwu > nbl) bad = 1;
     }
@@ -566,14 +609,14 @@ k_blocks(ProbDev *probs, BlockDev *blocks, const double *D, double *E, const dou
       }
     }
     int nab1 = 0, nab2 = 0;
-    if (!none) {
+    if (!none && (!wide || wid == 0)) {   // the record's writer
       int c = 0;
       if (lane < 2) c = dv_count_lat<CNT_IJOB1>(nbl, TP + ibgn, pivmin, lane == 0 ? gl3 : gu3);
       nab1 = __shfl_sync(0xffffffffu, c, 0);
       nab2 = __shfl_sync(0xffffffffu, c, 1);
       nwlb = nab1; nwub = nab2;
     }
-    if (lane == 0) {
+    if (lead) {
       B->irange = brange;
       B->gl3 = gl3; B->gu3 = gu3; B->atoli = atoli;
       B->wlu = wlub; B->wul = wulb;
@@ -1215,75 +1258,130 @@ __global__ void k_gaps_root(int N, const ProbDev *probs, const BlockDev *blocks,
 // (SRC/mrrr_val.c:515-626).  One thread per problem; runs only when the
 // blocks together produced more than nvals values.
 // ------------------------------------------------------------------------
-__global__ void k_discard(ProbDev *probs, int nprob, BlockDev *blocks, double *W, double *Werr,
-                          double *Wgap, int *Windex, int *iblk, double *Wcopy) {
-  int pi = blockIdx.x * blockDim.x + threadIdx.x;
-  if (pi >= nprob) return;
-  ProbDev *p = &probs[pi];
+// A CTA per problem.  A problem with a surplus (clusters at the interval's
+// ends) is compacted by the CTA in chunks of MR3_THREADS entries, each read
+// whole before it is written at or below its place.  A serial chain of
+// loads before: 6.5 -> 0.05 ms for 10005 entries of a glued matrix.
+__global__ void __launch_bounds__(MR3_THREADS)
+k_discard(ProbDev *probs, BlockDev *blocks, double *W, double *Werr, double *Wgap, int *Windex,
+          int *iblk, double *Wcopy) {
+  __shared__ int wcnt[MR3_THREADS / 32];
+  __shared__ double wval[MR3_THREADS / 32];
+  ProbDev *p = &probs[blockIdx.x];
   if (p->trivial || p->jobz == MR3_JOB_C || p->status) return;
-  int mp = p->m;
-  if (!(mp > p->nvals && p->irange == MR3_RANGE_I)) {
-    if (mp < p->nvals) set_status(p, MR3_EMISC);
+  const int m0 = p->m, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int nvals = p->nvals;
+  __syncthreads();   // m and status are read before thread 0 writes them
+  if (!(m0 > nvals && p->irange == MR3_RANGE_I)) {
+    if (tid == 0 && m0 < nvals) set_status(p, MR3_EMISC);
     return;
   }
   const int o = p->off;
   double *w = W + o, *we = Werr + o, *wg = Wgap + o, *wc = Wcopy + o;
   int *wi = Windex + o, *ib = iblk + o;
-  int idiscl = p->il_out - 1 - p->nwl, idiscu = p->nwu - p->iu_out, im;
-#define MOVE(dst, src) { w[dst] = w[src]; wc[dst] = wc[src]; we[dst] = we[src]; wg[dst] = wg[src]; \
-                         wi[dst] = wi[src]; ib[dst] = ib[src]; }
-  if (idiscl > 0) {
-    im = 0;
-    for (int je = 0; je < mp; je++) {
-      if (wc[je] < p->wlu && idiscl > 0) idiscl--;
-      else { MOVE(im, je); im++; }
+  int mp = m0;
+  // the rank of this thread among the CTA's flagged threads, and their number
+  auto rank_of = [&](bool f, int *total) -> int {
+    const unsigned b = __ballot_sync(0xffffffffu, f);
+    if (lane == 0) wcnt[wid] = __popc(b);
+    __syncthreads();
+    int before = 0, all = 0;
+    for (int v = 0; v < MR3_THREADS / 32; v++) {
+      if (v < wid) before += wcnt[v];
+      all += wcnt[v];
+    }
+    __syncthreads();
+    *total = all;
+    return before + __popc(b & ((1u << lane) - 1u));
+  };
+  // keeps the entries 0..mp-1 for which drop(entry, its rank among the
+  // entries with cand(entry)) does not hold; mp becomes their number
+  auto compact = [&](auto cand, auto drop) {
+    int im = 0, seen = 0;
+    for (int j0 = 0; j0 < mp; j0 += MR3_THREADS) {
+      const int je = j0 + tid;
+      const bool in = je < mp;
+      int nc, nk;
+      const bool isc = in && cand(je);
+      const int r = seen + rank_of(isc, &nc);
+      const bool keep = in && !(isc && drop(r));
+      double v0 = 0, v1 = 0, v2 = 0, v3 = 0;
+      int v4 = 0, v5 = 0;
+      if (keep) { v0 = w[je]; v1 = wc[je]; v2 = we[je]; v3 = wg[je]; v4 = wi[je]; v5 = ib[je]; }
+      const int at = im + rank_of(keep, &nk);   // ends with a barrier: all have read
+      if (keep) { w[at] = v0; wc[at] = v1; we[at] = v2; wg[at] = v3; wi[at] = v4; ib[at] = v5; }
+      seen += nc;
+      im += nk;
     }
     mp = im;
-  }
-  if (idiscu > 0) {
-    im = mp;
-    for (int je = mp - 1; je >= 0; je--) {
-      if (wc[je] > p->wul && idiscu > 0) idiscu--;
-      else { im--; MOVE(im, je); }
+    __syncthreads();
+  };
+  auto count_of = [&](auto cand) -> int {
+    int total = 0;
+    for (int j0 = 0; j0 < mp; j0 += MR3_THREADS) {
+      int nc;
+      rank_of(j0 + tid < mp && cand(j0 + tid), &nc);
+      total += nc;
     }
-    int jee = 0;
-    for (int je = im; je < mp; je++) { MOVE(jee, je); jee++; }
-    mp -= im;
+    return total;
+  };
+  int idiscl = p->il_out - 1 - p->nwl, idiscu = p->nwu - p->iu_out;
+  const double wlu = p->wlu, wul = p->wul;
+  if (idiscl > 0) {   // the first idiscl entries below wlu
+    auto low = [&](int je) { return wc[je] < wlu; };
+    const int total = count_of(low);
+    compact(low, [&](int r) { return r < idiscl; });
+    idiscl -= min(idiscl, total);
+  }
+  if (idiscu > 0) {   // the last idiscu entries above wul
+    auto high = [&](int je) { return wc[je] > wul; };
+    const int total = count_of(high);
+    compact(high, [&](int r) { return r >= total - idiscu; });
+    idiscu -= min(idiscu, total);
   }
   if (idiscl > 0 || idiscu > 0) {
-    if (idiscl > 0) {
-      double wkill = p->wu;
-      for (int jd = 0; jd < idiscl; jd++) {
-        int iw = -1;
-        for (int je = 0; je < mp; je++)
-          if (ib[je] >= 0 && (wc[je] < wkill || iw == -1)) { iw = je; wkill = wc[je]; }
-        if (iw >= 0) ib[iw] = -2;
+    // still too many: the smallest, then the largest ones, each time the
+    // first of equals
+    for (int side = 0; side < 2; side++)
+      for (int jd = side ? idiscu : idiscl; jd > 0; jd--) {
+        double best = 0.0;
+        int bi = -1;
+        for (int je = tid; je < mp; je += MR3_THREADS) {
+          const double v = side ? -wc[je] : wc[je];
+          if (ib[je] >= 0 && (bi < 0 || v < best)) { best = v; bi = je; }
+        }
+        for (int d = 16; d > 0; d >>= 1) {
+          const double ov = __shfl_xor_sync(0xffffffffu, best, d);
+          const int oi = __shfl_xor_sync(0xffffffffu, bi, d);
+          if (oi >= 0 && (bi < 0 || ov < best || (ov == best && oi < bi))) { best = ov; bi = oi; }
+        }
+        if (lane == 0) { wval[wid] = best; wcnt[wid] = bi; }
+        __syncthreads();
+        if (tid == 0) {
+          for (int v = 1; v < MR3_THREADS / 32; v++)
+            if (wcnt[v] >= 0 && (bi < 0 || wval[v] < best || (wval[v] == best && wcnt[v] < bi))) {
+              best = wval[v];
+              bi = wcnt[v];
+            }
+          if (bi >= 0) ib[bi] = -2;
+        }
+        __syncthreads();
       }
-    }
-    if (idiscu > 0) {
-      double wkill = p->wl;
-      for (int jd = 0; jd < idiscu; jd++) {
-        int iw = -1;
-        for (int je = 0; je < mp; je++)
-          if (ib[je] >= 0 && (wc[je] > wkill || iw == -1)) { iw = je; wkill = wc[je]; }
-        if (iw >= 0) ib[iw] = -2;
-      }
-    }
-    im = 0;
-    for (int je = 0; je < mp; je++)
-      if (ib[je] >= 0) { MOVE(im, je); im++; }
-    mp = im;
+    compact([&](int je) { return ib[je] < 0; }, [&](int) { return true; });
   }
-#undef MOVE
-  for (int je = mp; je < p->m; je++) ib[je] = -1;
-  p->m = mp;
-  if (mp < p->nvals) set_status(p, MR3_EMISC);
-  // block W ranges after the removal: recomputed from iblk (SRC/mrrr_vec.c:335-338)
-  for (int b = 0; b < p->nsplit; b++) blocks[o + b].mbl = 0;
-  for (int je = 0; je < mp; je++) {
+  for (int je = mp + tid; je < m0; je += MR3_THREADS) ib[je] = -1;
+  if (tid == 0) {
+    p->m = mp;
+    if (mp < nvals) set_status(p, MR3_EMISC);
+  }
+  // block W ranges after the removal: recomputed from iblk (SRC/mrrr_vec.c:335-338);
+  // a block's entries follow one another
+  for (int b = tid; b < p->nsplit; b += MR3_THREADS) blocks[o + b].mbl = 0;
+  __syncthreads();
+  for (int je = tid; je < mp; je += MR3_THREADS) {
     BlockDev *B = &blocks[ib[je]];
-    if (B->mbl == 0) B->wbgn = o + je;
-    B->mbl++;
+    if (je == 0 || ib[je - 1] != ib[je]) { B->wbgn = o + je; atomicSub(&B->mbl, je); }
+    if (je == mp - 1 || ib[je + 1] != ib[je]) atomicAdd(&B->mbl, je + 1);
   }
 }
 
@@ -3729,11 +3827,12 @@ static int solve_impl(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void *stream,
   const int gN = (NN + 255) / 256, gN128 = (NN + 127) / 128;
 
   // ---- stage A: eigenvalues
+  const int wide = L <= c->nsm;   // see k_blocks
   LAUNCH(k_gather, L, 256, c->probs, c->Din, c->Ein, c->D, c->E, c->prob_of_slot, c->iblk,
          c->lvl_of_slot, c->flag);
   LAUNCH(k_prologue, L, MR3_THREADS, c->probs, c->blocks, c->blk_of_row, c->D, c->E, c->E2,
-         c->gers, c->TP, c->TPc, tol);
-  LAUNCH(k_blocks, L, MR3_THREADS, c->probs, c->blocks, c->D, c->E, c->gers, c->TP, tol);
+         c->gers, c->TP, c->TPc, tol, wide);
+  LAUNCH(k_blocks, L, MR3_THREADS, c->probs, c->blocks, c->D, c->E, c->gers, c->TP, tol, wide);
   unsigned long long *stats = c->prof ? c->stats : nullptr;
   {
     const int Lb = tree_lanes(nwant, c->nsm, tree_max, RowCost{48, 48, 18});
@@ -3782,8 +3881,8 @@ static int solve_impl(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void *stream,
     LAUNCH(k_dqds, gN, 256, NN, c->probs, c->blocks, c->blk_of_row, c->D, c->E, c->W, c->Werr,
            c->qd);
   LAUNCH(k_gaps_root, gN, 256, NN, c->probs, c->blocks, c->iblk, c->W, c->Werr, c->Wgap);
-  LAUNCH(k_discard, (L + 127) / 128, 128, c->probs, L, c->blocks, c->W, c->Werr, c->Wgap,
-         c->Windex, c->iblk, c->Wcopy);
+  LAUNCH(k_discard, L, MR3_THREADS, c->probs, c->blocks, c->W, c->Werr, c->Wgap, c->Windex, c->iblk,
+         c->Wcopy);
 
   // ---- stage B: eigenvectors
   if (anyV) {
