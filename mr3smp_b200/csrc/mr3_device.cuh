@@ -774,67 +774,22 @@ static __device__ __noinline__ int dv_dlaneg(int n, const double2 *__restrict__ 
   return dv_dlaneg_inl<U>(n, P, ps, sigma, r);
 }
 
-// One interval of dlarrb (SRC/LAPACK/odrrb.f:136-293).  Intervals of one
-// dlarrb call never read each other's state: the convergence test reads the
-// gaps of the input WGAP, which dlarrb rewrites only after every interval has
-// converged.  So one thread per interval yields the sequential result.
+// Intervals of dlarrb (SRC/LAPACK/odrrb.f:136-293), one per group of L lanes
+// (the same L for the whole warp: 32 / L groups, the lanes left over in none).
+// Intervals of one dlarrb call never read each other's state: the convergence
+// test reads the gaps of the input WGAP, which dlarrb rewrites only after every
+// interval has converged.  So an interval by itself yields the sequential
+// result.
 //   i      : 1-based eigenvalue index of this interval (IFIRST..ILAST)
 //   first  : i == IFIRST (initial-phase left gap is then the own right gap)
 //   has_left: II > 1 (main-loop left gap is WGAP(II-1))
 //   w, werr: in/out; updated only if the interval went through the main loop
-// Returns the number of counts spent, or -1 if a widening loop hit its cap.
-template <int U>
-static __device__ __noinline__ int dv_dlarrb_one(int n, const double2 *__restrict__ R, int ps, int i,
-                                          int first,
-                                          int has_left, double rgap_own, double lgap_in,
-                                          double rtol1, double rtol2, double pivmin,
-                                          int maxitr, int r, double *w, double *werr,
-                                          int *ncount) {
-  double mnwdth = 2.0 * pivmin;
-  double left = *w - *werr, right = *w + *werr;
-  double gap = fmin(first ? rgap_own : lgap_in, rgap_own);
-  double back = *werr;
-  int negcnt, cap, status = 0;
-  int nc = 0;
-  for (cap = 0; cap < MR3_EXPAND_CAP; cap++) {
-    negcnt = dv_dlaneg<U>(n, R, ps, left, r);
-    nc++;
-    if (negcnt > i - 1) { left = left - back; back = 2.0 * back; } else break;
-  }
-  if (cap == MR3_EXPAND_CAP) status = -1;
-  back = *werr;
-  for (cap = 0; cap < MR3_EXPAND_CAP; cap++) {
-    negcnt = dv_dlaneg<U>(n, R, ps, right, r);
-    nc++;
-    if (negcnt < i) { right = right + back; back = 2.0 * back; } else break;
-  }
-  if (cap == MR3_EXPAND_CAP) status = -1;
-  *ncount += nc;
-  double width = 0.5 * fabs(left - right);
-  double tmp = fmax(fabs(left), fabs(right));
-  double cvrgd = fmax(rtol1 * gap, rtol2 * tmp);
-  if (width <= cvrgd || width <= mnwdth) return status;   // converged early: W, WERR kept
-  gap = fmin(has_left ? lgap_in : rgap_own, rgap_own);
-  for (int iter = 0; iter <= maxitr; iter++) {
-    double mid = 0.5 * (left + right);
-    width = right - mid;
-    tmp = fmax(fabs(left), fabs(right));
-    cvrgd = fmax(rtol1 * gap, rtol2 * tmp);
-    if (width <= cvrgd || width <= mnwdth || iter == maxitr) break;
-    negcnt = dv_dlaneg<U>(n, R, ps, mid, r);
-    *ncount += 1;
-    if (negcnt <= i - 1) left = mid; else right = mid;
-  }
-  *w = 0.5 * (left + right);
-  *werr = right - *w;
-  return status;
-}
-
-// dv_dlarrb_one for one interval per group of L lanes (L = 3..32, the same
-// for the whole warp: 32 / L groups, the lanes left over in none).  Every
-// lane of the warp calls it; the lanes of a group pass the same arguments and
-// get the same results, and groups with act = false (the lanes left over
-// among them) have no interval.  The bisection
+// Every lane of the warp calls it; the lanes of a group pass the same
+// arguments and get the same results, groups with act = false (the lanes left
+// over among them) have no interval.
+//
+// ONE (L = 1): a thread per interval; its ends are widened by itself, the main
+// loop's steps are the warp's.  Else (L = 3..32) the bisection
 // midpoints of the next steps form a binary tree whose nodes follow from the
 // current interval alone: lane t of the group evaluates the count at node
 // t + 1 (heap numbering, computed along the node's path with the same
@@ -849,11 +804,19 @@ static __device__ __noinline__ int dv_dlarrb_one(int n, const double2 *__restric
 // The passes are the warp's: a group that widens counts beside groups that
 // bisect.  (With a loop per group, groups once apart never met again and
 // counted one after the other: twice the time for the slowest warps of
-// k_refine_cl on the n = 20010 problem.)
+// k_refine_cl on the n = 20010 problem.)  A pass costs the warp the same
+// however many of its groups still count, and most intervals end long before
+// the few next to the representation's shift, whose relative tolerance is
+// small.  So once the groups left could have lanes for a whole tree level
+// more, they move: the q-th of them to the lanes of the q-th group of the
+// larger size, its result back to its own lanes when it ends.  1024 mixed
+// problems: k_refine_cl 25.8 -> 20.8 ms, k_sng_finish's bisections 24.0 ->
+// 22.5, the ends of the clusters 14.6 -> 13.9; k_refine_root 23.5 -> 24.3 there
+// and 4.25 -> 3.75 for 200 problems.
 // LARRJ: dlarrj (SRC/LAPACK/odrrj.f:100-281) on T's rows (d, e2) instead: its
 // count, one relative tolerance (rtol1) and no test between widening and
 // bisection; gaps, rtol2 and r are not used.
-template <bool LARRJ>
+template <bool LARRJ, bool ONE = false, int U = QDIV_U>
 static __device__ __forceinline__ void dv_dlarrb_tree(bool act, int L, int n,
                                             const double2 *__restrict__ R, int ps, int i, int first,
                                             int has_left, double rgap_own, double lgap_in,
@@ -861,11 +824,14 @@ static __device__ __forceinline__ void dv_dlarrb_tree(bool act, int L, int n,
                                             int r, double *w, double *werr, int *ncount) {
   enum { ENDS, WIDEN, TREE, DONE };
   const int lane = threadIdx.x & 31;
-  const int t = lane % L, g0 = lane - t, half = L >> 1;
+  int t = lane % L, g0 = lane - t;
+  const int half = L >> 1;
   const unsigned gbits = (L == 32) ? 0xffffffffu : ((1u << L) - 1u);
-  const unsigned gm = gbits << g0;   // (the lanes left over: theirs)
-  const double mnwdth = 2.0 * pivmin;
+  unsigned gm = gbits << g0;   // (the lanes left over: theirs)
+  double mnwdth = 2.0 * pivmin;
   double left = *w - *werr, right = *w + *werr;
+  const double gap0 = fmin(first ? rgap_own : lgap_in, rgap_own);
+  double gap = fmin(has_left ? lgap_in : rgap_own, rgap_own);
   // widening: the first L/2 lanes hold the left end after the next 0..L/2-1
   // widening steps, the others the right end; the first candidate that
   // passes is the end the sequential loop stops at
@@ -874,14 +840,75 @@ static __device__ __forceinline__ void dv_dlarrb_tree(bool act, int L, int n,
   double xs0 = 0.0, xs1 = 0.0, bs0 = 0.0, bs1 = 0.0;
   int steps0 = 0, steps1 = 0;
   int phase = act ? ENDS : DONE, iter = 0, nc = 0;
+  if (ONE && act) {
+    double back = *werr;
+    for (int cap = 0; cap < MR3_EXPAND_CAP; cap++) {
+      nc++;
+      if (dv_dlaneg<U>(n, R, ps, left, r) <= i - 1) break;
+      left = left - back;
+      back = 2.0 * back;
+    }
+    back = *werr;
+    for (int cap = 0; cap < MR3_EXPAND_CAP; cap++) {
+      nc++;
+      if (dv_dlaneg<U>(n, R, ps, right, r) >= i) break;
+      right = right + back;
+      back = 2.0 * back;
+    }
+    const double width = 0.5 * fabs(left - right), tmp = fmax(fabs(left), fabs(right));
+    phase = width <= fmax(rtol1 * gap0, rtol2 * tmp) || width <= mnwdth ? DONE : TREE;
+    if (phase == TREE) {   // the loop's first test
+      const double mid = 0.5 * (left + right);
+      if (right - mid <= fmax(rtol1 * gap, rtol2 * tmp) || right - mid <= mnwdth || maxitr == 0) {
+        *w = mid;
+        *werr = right - mid;
+        phase = DONE;
+      }
+    }
+  }
+  if (ONE) __syncwarp();
   if (LARRJ && act && right - *w < rtol1 * fmax(fabs(left), fabs(right))) phase = DONE;
-  while (__any_sync(0xffffffffu, phase != DONE)) {
+  // after the groups moved: Lc lanes each, own the lane that gets the result
+  // of this lane's group, nco the counts of the interval this lane began with
+  int Lc = L, own = g0, nco = 0;
+  bool moved = false;
+  for (;;) {
+    const unsigned am = __ballot_sync(0xffffffffu, phase != DONE && t == 0);
+    if (am == 0) break;
+    const int na = __popc(am);
+    if (na * (2 * Lc + 1) <= 32 && !__any_sync(0xffffffffu, phase < TREE)) {
+      if (!moved) { nco = nc; nc = 0; }
+      moved = true;
+      Lc = 32 / na;
+      const int q = lane / Lc, src = q < na ? (int)__fns(am, 0, q + 1) : 0;
+      phase = __shfl_sync(0xffffffffu, phase, src);
+      left = __shfl_sync(0xffffffffu, left, src);
+      right = __shfl_sync(0xffffffffu, right, src);
+      gap = __shfl_sync(0xffffffffu, gap, src);
+      rtol1 = __shfl_sync(0xffffffffu, rtol1, src);
+      rtol2 = __shfl_sync(0xffffffffu, rtol2, src);
+      mnwdth = __shfl_sync(0xffffffffu, mnwdth, src);
+      R = reinterpret_cast<const double2 *>(
+          __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(R), src));
+      n = __shfl_sync(0xffffffffu, n, src);
+      ps = __shfl_sync(0xffffffffu, ps, src);
+      i = __shfl_sync(0xffffffffu, i, src);
+      r = __shfl_sync(0xffffffffu, r, src);
+      maxitr = __shfl_sync(0xffffffffu, maxitr, src);
+      iter = __shfl_sync(0xffffffffu, iter, src);
+      nc = __shfl_sync(0xffffffffu, nc, src);
+      own = __shfl_sync(0xffffffffu, own, src);
+      if (q >= na) phase = DONE;
+      t = lane % Lc;
+      g0 = lane - t;
+      gm = ((Lc == 32) ? 0xffffffffu : ((1u << Lc) - 1u)) << g0;
+    }
     // this lane's point: an end, a candidate end or a tree node
     double x = 0.0, back = 0.0;
     bool mine = phase != DONE;
-    if (phase == ENDS && t < 2) {
+    if (!ONE && phase == ENDS && t < 2) {
       x = t == 0 ? left : right;
-    } else if (phase == WIDEN) {
+    } else if (!ONE && phase == WIDEN) {
       x = side ? xs1 : xs0;
       back = side ? bs1 : bs0;
       for (int k = 0; k < wk; k++) { x = side ? x + back : x - back; back = 2.0 * back; }
@@ -896,12 +923,14 @@ static __device__ __forceinline__ void dv_dlarrb_tree(bool act, int L, int n,
       x = 0.5 * (l + rr);
     }
     int cnt = 0;
-    if (mine) cnt = LARRJ ? dv_count_lat<CNT_LARRJ>(n, R, 0.0, x) : dv_dlaneg_inl<QDIV_U>(n, R, ps, x, r);
+    if (mine) cnt = LARRJ ? dv_count_lat<CNT_LARRJ>(n, R, 0.0, x) : dv_dlaneg_inl<U>(n, R, ps, x, r);
     __syncwarp();
+    bool ended = false;
+    double wnew = 0.0, enew = 0.0;
     if (phase != DONE) {
-      int shift = -1, known = L;      // lane of node v: v + shift; nodes counted
+      int shift = -1, known = Lc;     // lane of node v: v + shift; nodes counted
       bool start = false;             // the ends are now those of the main loop
-      if (phase == ENDS) {
+      if (!ONE && phase == ENDS) {
         need0 = __shfl_sync(gm, cnt, g0) > i - 1;
         need1 = __shfl_sync(gm, cnt, g0 + 1) < i;
         nc += 2;
@@ -916,7 +945,7 @@ static __device__ __forceinline__ void dv_dlarrb_tree(bool act, int L, int n,
         } else {
           start = true;
         }
-      } else if (phase == WIDEN) {
+      } else if (!ONE && phase == WIDEN) {
         const bool ok = mine && (side ? (cnt >= i) : (cnt <= i - 1));
         const unsigned gb = (__ballot_sync(gm, ok) >> g0) & gbits;
         for (int sd = 0; sd < 2; sd++) {
@@ -950,21 +979,20 @@ static __device__ __forceinline__ void dv_dlarrb_tree(bool act, int L, int n,
       if (start && LARRJ) {
         phase = TREE;
       } else if (start) {
-        const double gap = fmin(first ? rgap_own : lgap_in, rgap_own);
         const double width = 0.5 * fabs(left - right), tmp = fmax(fabs(left), fabs(right));
         // converged early: W, WERR kept
-        phase = width <= fmax(rtol1 * gap, rtol2 * tmp) || width <= mnwdth ? DONE : TREE;
+        phase = width <= fmax(rtol1 * gap0, rtol2 * tmp) || width <= mnwdth ? DONE : TREE;
       }
       if (phase == TREE) {   // walk the counted nodes
-        const double gap = fmin(has_left ? lgap_in : rgap_own, rgap_own);
         for (int node = 1;;) {
           const double mid = 0.5 * (left + right);
           const double width = right - mid, tmp = fmax(fabs(left), fabs(right));
           const bool small = LARRJ ? width < rtol1 * tmp
                                    : width <= fmax(rtol1 * gap, rtol2 * tmp) || width <= mnwdth;
           if (small || iter == maxitr) {
-            *w = mid;
-            *werr = right - mid;
+            wnew = mid;
+            enew = right - mid;
+            ended = true;
             phase = DONE;
             break;
           }
@@ -977,6 +1005,22 @@ static __device__ __forceinline__ void dv_dlarrb_tree(bool act, int L, int n,
       }
     }
     __syncwarp();
+    if (!moved) {
+      if (ended) { *w = wnew; *werr = enew; }
+    } else {
+      for (unsigned em = __ballot_sync(0xffffffffu, ended && t == 0); em; em &= em - 1) {
+        const int f = __ffs(em) - 1;
+        const double wv = __shfl_sync(0xffffffffu, wnew, f), ev = __shfl_sync(0xffffffffu, enew, f);
+        const int to = __shfl_sync(0xffffffffu, own, f), k = __shfl_sync(0xffffffffu, nc, f);
+        if (lane == to) { *w = wv; *werr = ev; nco += k; }
+      }
+    }
+  }
+  if (moved) {   // to the other lanes of the interval's first group
+    const int lead = lane - lane % L;
+    *w = __shfl_sync(0xffffffffu, *w, lead);
+    *werr = __shfl_sync(0xffffffffu, *werr, lead);
+    nc = __shfl_sync(0xffffffffu, nco, lead);
   }
   *ncount += nc;
 }

@@ -1134,31 +1134,17 @@ k_root(ProbDev *probs, BlockDev *blocks, double *D, double *E, const double2 *TP
 // Stage A5: refine the approximations w.r.t. the root representation
 // (refine_eigval_approx, unchunked dlarrb, SRC/mrrr_val.c:992-1082).
 // ------------------------------------------------------------------------
-__device__ __forceinline__ unsigned long long refine_root_body(int s, const ProbDev *probs,
-                                                               const BlockDev *blocks,
-                                                               const int *iblk, const double2 *RP,
-                                                               double *W, double *Werr,
-                                                               const double *Wgap, Tol tol) {
-  if (iblk[s] < 0) return 0;
-  const BlockDev *B = &blocks[iblk[s]];
-  const ProbDev *p = &probs[B->prob];
-  if (p->status || B->nbl < 2 || B->dqds) return 0;
-  const bool onlyW = (p->jobz == MR3_JOB_N);   // rtol1 = rtol2 = 4 eps (SRC/mrrr.c:230-232)
-  const int II = s - B->wbgn + 1;
-  const int i = B->ilow + II - 1;
-  double w = W[s] - B->sigma;
-  double werr = Werr[s] + fabs(w) * MR3_EPS;
-  const double rgap = Wgap[s];
-  const double lgap = (II > 1) ? Wgap[s - 1] : rgap;
-  const int maxitr = dv_itmax(B->spdiam + p->pivmin, p->pivmin);
-  const double rtol1 = onlyW ? 4.0 * MR3_EPS : tol.rtol1;
-  const double rtol2 = onlyW ? 4.0 * MR3_EPS : tol.rtol2;
-  int nc = 0;
-  dv_dlarrb_one<1>(B->nbl, RP + B->ibgn, 1, i, II == 1, II > 1, rgap, lgap, rtol1, rtol2, p->pivmin,
-                maxitr, B->nbl, &w, &werr, &nc);
-  W[s] = w;
-  Werr[s] = werr;
-  return (unsigned long long)nc * (unsigned long long)B->nbl;
+// The item of a group (group_item) when the groups of a warp take items
+// ROOT_STEP apart: windows of ROOT_STEP warps, whose items they share.  Further
+// apart, a batch's warps hold problems of different sizes (60 requests of 64 to
+// 16384 rows: 2.2 ms with 32, 2.9 with 128) and gain on one large problem (glued
+// 20010 rows: neighbours 36.8 ms, 27.5 with 32, 21.1 with 128).
+#define ROOT_STEP 32
+__device__ __forceinline__ long long spread_item(long long item, long long base, int L) {
+  if (item < 0) return -1;
+  const int G = 32 / L;
+  const long long w = base / G, w0 = w - w % ROOT_STEP;
+  return w0 * G + (item - base) * ROOT_STEP + (w - w0);
 }
 
 template <bool TREE>
@@ -1167,20 +1153,22 @@ k_refine_root(int N, int L, const ProbDev *probs, const BlockDev *blocks, const 
               const double2 *RP, double *W, double *Werr, const double *Wgap, Tol tol,
               unsigned long long *stats) {
   long long base;
-  const long long item = group_item(TREE ? L : 1, &base);
+  if (!TREE) L = 1;
+  const long long item = group_item(L, &base);
   unsigned long long work = 0;
-  if (!TREE) {
-    if (item < N) work = refine_root_body((int)item, probs, blocks, iblk, RP, W, Werr, Wgap, tol);
-  } else if (base < N) {
-    // L lanes per eigenvalue (few eigenvalues: single large problems)
-    const int s = (int)item;
-    const BlockDev *B = item >= 0 && item < N && iblk[s] >= 0 ? &blocks[iblk[s]] : nullptr;
+  if (TREE || base < N) {
+    // L lanes per eigenvalue (few eigenvalues: single large problems), or one.
+    // The groups of a warp take eigenvalues ROOT_STEP apart: the eigenvalues
+    // next to the root's shift need many steps, and each gets the more lanes
+    // the fewer of them are in a warp.
+    const int s = (int)(TREE ? spread_item(item, base, L) : item);
+    const BlockDev *B = s >= 0 && s < N && iblk[s] >= 0 ? &blocks[iblk[s]] : nullptr;
     const ProbDev *p = B ? &probs[B->prob] : nullptr;
     const bool act = B && !p->status && B->nbl >= 2 && !B->dqds;
     int i = 0, II = 0, maxitr = 0, nc = 0;
     double w = 0.0, werr = 0.0, rgap = 0.0, lgap = 0.0, rtol1 = 0.0, rtol2 = 0.0, pivmin = 0.0;
     if (act) {
-      const bool onlyW = (p->jobz == MR3_JOB_N);
+      const bool onlyW = (p->jobz == MR3_JOB_N);   // rtol1 = rtol2 = 4 eps (SRC/mrrr.c:230-232)
       II = s - B->wbgn + 1;
       i = B->ilow + II - 1;
       w = W[s] - B->sigma;
@@ -1194,8 +1182,9 @@ k_refine_root(int N, int L, const ProbDev *probs, const BlockDev *blocks, const 
     }
     const int nb = act ? B->nbl : 0;
     __syncwarp();
-    dv_dlarrb_tree<false>(act, L, nb, act ? RP + B->ibgn : RP, 1, i, II == 1, II > 1, rgap, lgap, rtol1,
-                   rtol2, pivmin, maxitr, nb, &w, &werr, &nc);
+    dv_dlarrb_tree<false, !TREE, TREE ? QDIV_U : 1>(act, L, nb, act ? RP + B->ibgn : RP, 1, i, II == 1,
+                                                    II > 1, rgap, lgap, rtol1, rtol2, pivmin, maxitr,
+                                                    nb, &w, &werr, &nc);
     if (act && (threadIdx.x & 31) % L == 0) {
       W[s] = w;
       Werr[s] = werr;
@@ -1693,15 +1682,9 @@ k_cl_ext(int ncl, int L, const ClusterDev *cl, const ProbDev *probs, const Block
     const int maxitr = dv_itmax(C.bl_spdiam + p->pivmin, p->pivmin);
     double wv = Wsh[sx], ev = Werr[sx];
     int nc = 0;
-    if (!TREE) {
-      if (valid)
-        dv_dlarrb_one<QDIV_U>(nb, Pp, ps, i, 1, II > 1, 0.0, 0.0, tol.rqtol, tol.rqtol, p->pivmin,
-                             maxitr, nb, &wv, &ev, &nc);
-    } else {
-      __syncwarp();
-      dv_dlarrb_tree<false>(valid, L, nb, Pp, ps, i, 1, II > 1, 0.0, 0.0, tol.rqtol, tol.rqtol, p->pivmin,
-                     maxitr, nb, &wv, &ev, &nc);
-    }
+    __syncwarp();
+    dv_dlarrb_tree<false, !TREE>(valid, TREE ? L : 1, nb, Pp, ps, i, 1, II > 1, 0.0, 0.0, tol.rqtol,
+                                 tol.rqtol, p->pivmin, maxitr, nb, &wv, &ev, &nc);
     if (valid && (threadIdx.x & 31) % L == 0) {
       xw[t] = wv;
       xe[t] = ev;
@@ -1811,32 +1794,6 @@ __global__ void k_cl_pack(int ncl, const ClusterDev *cl, const BlockDev *blocks,
   }
 }
 
-// Refinement of a level's clusters w.r.t. their new representation
-// (refine_eigvals without R-tasks, SRC/process_cluster.c:394-428).
-__device__ __forceinline__ unsigned long long refine_cl_body(
-    int s, const ClusterDev *cl, const ProbDev *probs, const BlockDev *blocks,
-    const double *arena_cur, double *Wsh, double *Werr, const double *Wgap, const int *Windex,
-    const int *cl_of_slot, const int *lvl_of_slot, int level, Tol tol) {
-  if (lvl_of_slot[s] != level) return 0;
-  const ClusterDev C = cl[cl_of_slot[s]];
-  const BlockDev &B = blocks[C.blk];
-  const ProbDev *p = &probs[B.prob];
-  const int pidx = Windex[C.begin], i = Windex[s], II = i - (pidx - 1);
-  const double2 *P, *Q;
-  int ps;
-  own_rrr(C, B, nullptr, nullptr, arena_cur, &P, &Q, &ps);
-  const double rgap = Wgap[s];
-  const double lgap = (II > 1) ? Wgap[s - 1] : rgap;
-  const int maxitr = dv_itmax(C.bl_spdiam + p->pivmin, p->pivmin);
-  double w = Wsh[s], e = Werr[s];
-  int nc = 0;
-  dv_dlarrb_one<QDIV_U>(B.nbl, P, ps, i, i == pidx, II > 1, rgap, lgap, tol.rtol1, tol.rtol2, p->pivmin,
-                maxitr, B.nbl, &w, &e, &nc);
-  Wsh[s] = w;
-  Werr[s] = e;
-  return (unsigned long long)nc * (unsigned long long)B.nbl;
-}
-
 // Lanes per interval for a launch of `items` independent intervals: the
 // form with the shortest time per bisection step.  A group of L lanes takes
 // log2(L + 1) steps per count (a part of a step where its nodes end within a
@@ -1873,6 +1830,10 @@ static int group_blocks(long long items, int L) {
   return (int)((warps + TREE_T / 32 - 1) / (TREE_T / 32));
 }
 
+// Refinement of a level's clusters w.r.t. their new representation
+// (refine_eigvals without R-tasks, SRC/process_cluster.c:394-428).  (Groups of
+// a warp apart from one another, as in k_refine_root, read rows of different
+// representations: glued 20010 rows 49 -> 51 ms, mixed 9000 19 -> 20.)
 template <bool TREE>
 __global__ void __launch_bounds__(TREE ? TREE_T : 128, 4)
 k_refine_cl(const int *rl, const int *rl_n, const ClusterDev *cl, const ProbDev *probs,
@@ -1891,12 +1852,6 @@ k_refine_cl(const int *rl, const int *rl_n, const ClusterDev *cl, const ProbDev 
       const long long it = b0 + item;
       const bool valid = item >= 0 && it < cnt;
       const int s = rl[valid ? it : cnt - 1];
-      if (!TREE) {
-        if (valid)
-          work += refine_cl_body(s, cl, probs, blocks, arena_cur, Wsh, Werr, Wgap, Windex,
-                                 cl_of_slot, lvl_of_slot, level, tol);
-        continue;
-      }
       const ClusterDev C = cl[cl_of_slot[s]];
       const BlockDev &B = blocks[C.blk];
       const ProbDev *p = &probs[B.prob];
@@ -1910,8 +1865,8 @@ k_refine_cl(const int *rl, const int *rl_n, const ClusterDev *cl, const ProbDev 
       double w = Wsh[s], e = Werr[s];
       int nc = 0;
       __syncwarp();
-      dv_dlarrb_tree<false>(valid, L, B.nbl, P, ps, i, i == pidx, II > 1, rgap, lgap, tol.rtol1, tol.rtol2,
-                     p->pivmin, maxitr, B.nbl, &w, &e, &nc);
+      dv_dlarrb_tree<false, !TREE>(valid, TREE ? L : 1, B.nbl, P, ps, i, i == pidx, II > 1, rgap, lgap,
+                                   tol.rtol1, tol.rtol2, p->pivmin, maxitr, B.nbl, &w, &e, &nc);
       if (valid && (threadIdx.x & 31) % L == 0) {
         Wsh[s] = w;
         Werr[s] = e;
@@ -3874,7 +3829,7 @@ static int solve_impl(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void *stream,
       LAUNCH(k_refine_root<false>, gN128, 128, NN, 1, c->probs, c->blocks, c->iblk, c->RP, c->W,
              c->Werr, c->Wgap, tol, stats);
     else
-      LAUNCH(k_refine_root<true>, group_blocks(NN, Lr), TREE_T, NN, Lr, c->probs,
+      LAUNCH(k_refine_root<true>, group_blocks(NN + ROOT_STEP * (32 / Lr) - 1, Lr), TREE_T, NN, Lr, c->probs,
              c->blocks, c->iblk, c->RP, c->W, c->Werr, c->Wgap, tol, stats);
   }
   if (tol.nthreads < (1 << 30))
