@@ -6,10 +6,12 @@
 // SRC/process_{cluster,singleton,refinement}.c) executed in one fixed,
 // order-independent way, so the output does not depend on how the GPU
 // schedules the work:
-//   - bisection (dlarrd) and root refinement (dlarrb) are not chunked: one
-//     thread per eigenvalue gives exactly the unchunked sequential result;
-//   - the eigenvalue stage always bisects (the reference's choice once
-//     nthreads > 12*m/n, SRC/mrrr_val.c:281-285); there is no dqds;
+//   - bisection (dlarrd) and root refinement (dlarrb) are not chunked: each
+//     eigenvalue by itself, by one thread or a group of lanes, gives exactly
+//     the unchunked sequential result;
+//   - the eigenvalue stage bisects (the reference's choice once
+//     nthreads > 12*m/n, SRC/mrrr_val.c:281-285) unless MR3_NTHREADS asks for
+//     the other;
 //   - every singleton is its own task and cluster refinement is never split;
 //     a cluster is classified completely before its singletons run.
 // The pthread task queue becomes a device work queue drained level by level:
@@ -2725,9 +2727,10 @@ k_sng_bisect(int out, const SngDev *sng, const ClusterDev *cl, const ProbDev *pr
 // A warp holds G = 32 / L groups in lock-step; a group that finishes its
 // singleton takes the next one of the list.  A sweep's row takes one warp
 // about 110 cycles of latency and 45 of issue, whatever its number of groups,
-// so two warps a quarter SM fill it (one CTA of 8 warps per SM: 8 against 16
-// warps, 4.5 and 5.7 ms for the n = 1000 problem, 343 and 378 for the glued
-// n = 20010 one) and a longer list gets more groups per warp, not more warps.
+// so two warps a quarter SM fill it (8 against 16 warps an SM: 4.5 and 5.7 ms
+// for the n = 1000 problem, 343 and 378 for the glued n = 20010 one) and a
+// longer list gets more groups per warp, not more warps.  The eight are two
+// CTAs of four, one for a short list (FIN_HALF).
 //
 // A bisection takes as long as about ten calls.  With several groups a warp
 // the others would wait for each group's, so singletons that need one leave
