@@ -2991,6 +2991,9 @@ __global__ void k_place_w(int N, const ProbDev *probs, const int *prob_of_slot, 
   else Wout[s] = W[s];
 }
 
+// Flags the problems with eigenvectors whose values are out of order, for the
+// fix-up below (eigenvalues alone are sorted by themselves; their Wout still
+// lies block after block here, and they have neither Z nor Zsupp).
 __global__ void k_check_sorted(int N, ProbDev *probs, const int *prob_of_slot, const double *Wout,
                                int *unsorted) {
   int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2999,7 +3002,7 @@ __global__ void k_check_sorted(int N, ProbDev *probs, const int *prob_of_slot, c
   if (pi < 0) return;
   const ProbDev *p = &probs[pi];
   int k = s - p->off;
-  if (k + 1 >= p->m || p->status || p->jobz == MR3_JOB_C) return;
+  if (k + 1 >= p->m || p->status || p->jobz != MR3_JOB_V) return;
   if (Wout[s] > Wout[s + 1]) atomicOr(&unsorted[pi], 1);
 }
 
@@ -3036,7 +3039,7 @@ __global__ void k_perm_zsupp(int N, const ProbDev *probs, const int *prob_of_slo
   if (pi < 0 || !flag[pi]) return;
   const ProbDev *p = &probs[pi];
   int k = s - p->off;
-  if (k >= p->m) return;
+  if (k >= p->m || p->jobz != MR3_JOB_V) return;
   int src = rec[s].idx;
   tmp2[2 * (size_t)s] = p->Zsupp[2 * (size_t)src];
   tmp2[2 * (size_t)s + 1] = p->Zsupp[2 * (size_t)src + 1];
@@ -3049,7 +3052,7 @@ __global__ void k_perm_zsupp2(int N, const ProbDev *probs, const int *prob_of_sl
   if (pi < 0 || !flag[pi]) return;
   const ProbDev *p = &probs[pi];
   int k = s - p->off;
-  if (k >= p->m) return;
+  if (k >= p->m || p->jobz != MR3_JOB_V) return;
   p->Zsupp[2 * (size_t)k] = tmp2[2 * (size_t)s];
   p->Zsupp[2 * (size_t)k + 1] = tmp2[2 * (size_t)s + 1];
 }
@@ -4120,7 +4123,7 @@ static int solve_impl(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void *stream,
       CK(cudaMemcpyAsync(c->h_probs, c->probs, L * sizeof(ProbDev), cudaMemcpyDeviceToHost, st), "probs m");
       CK(cudaStreamSynchronize(st), "perm sync");
       for (int k = 0; k < L; k++) {
-        if (!c->h_flag[k]) continue;
+        if (!c->h_flag[k] || c->h_probs[k].jobz != MR3_JOB_V) continue;
         const ProbDev &h = c->h_probs[k];
         std::vector<int> moved;
         for (int j = 0; j < h.m; j++)
@@ -4144,7 +4147,7 @@ static int solve_impl(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void *stream,
         c->h_dcol.clear();
         c->h_dcnt.clear();
         for (int k = 0; k < L; k++)
-          if (c->h_flag[k] && c->h_probs[k].m > 0) {
+          if (c->h_flag[k] && c->h_probs[k].jobz == MR3_JOB_V && c->h_probs[k].m > 0) {
             c->h_dprob.push_back(idx[k]);
             c->h_dcol.push_back(0);
             c->h_dcnt.push_back(c->h_probs[k].m);
