@@ -354,9 +354,11 @@ static __device__ __forceinline__ bool ijob3_step(double c, int cv, int nval, do
 // 7 steps in less than a warp's 5 took).  Then one pass of exact counts at the
 // last points below and above nval and at a closing one confirms the walk: the
 // Sturm count does not decrease with the point, so the exact counts at all
-// earlier points lie on the same sides.  An unconfirmed walk is repeated with
-// exact counts, as the steps below that width are.
-//   cnt == nullptr: L = 2..32, a power of two; the whole warp calls.
+// earlier points lie on the same sides.  (The closing count alone would not do:
+// it may be nval although an earlier point, guessed below or above nval, has
+// that count too and would have closed the interval there.)  An unconfirmed
+// walk is repeated with exact counts, as the steps below that width are.
+//   cnt == nullptr: L = 4..32, a power of two; the whole warp calls.
 //   cnt != nullptr: shared memory of an int per thread; L a multiple of 32 and
 //   a power of two; the whole CTA calls, its groups one behind the other.
 // The groups go on together until the last is done.
@@ -376,6 +378,8 @@ static __device__ __noinline__ void dv_ijob3_tree(int L, int *cnt, int n, const 
   const double sa = a, sb = b;
   const int sna = na, snb = nb, sit = it;
   const bool sdone = done;
+  double pa = a, pb = b;   // the ends before the last step
+  int pna = na, pnb = nb;
   for (int pass = 0; pass < 2; pass++) {   // guessed, then exact
     bool stop = done;
     while (cnt ? __syncthreads_or(!stop) : __any_sync(0xffffffffu, !stop)) {
@@ -395,6 +399,7 @@ static __device__ __noinline__ void dv_ijob3_tree(int L, int *cnt, int n, const 
       for (int d = 0; d < depth; d++) {
         const int cv = cnt ? cnt[g0 + node] : __shfl_sync(0xffffffffu, raw, g0 + node);
         if (!stop) {
+          pa = a; pb = b; pna = na; pnb = nb;
           done = ijob3_step(0.5 * (a + b), cv, nval, tol0, reltol, nitmax, &a, &b, &na, &nb, &it);
           node = (cv < nval) ? 2 * node + 1 : 2 * node;
           stop = done || (pass == 0 &&
@@ -403,23 +408,25 @@ static __device__ __noinline__ void dv_ijob3_tree(int L, int *cnt, int n, const 
       }
     }
     if (pass == 1) break;
-    // lane 0 counts at a, lane 1 at b (the same point when one closed it)
+    // lane 0 counts at the last point below nval, lane 1 at the last above,
+    // lane 2 at the closing one
     const bool walked = it > sit;
     if (!(cnt ? __syncthreads_or(walked) : __any_sync(0xffffffffu, walked))) continue;
-    const int raw = dv_count_lat<CNT_BISECT>(n, tp, pivmin, (t & 1) ? b : a);
+    const bool closed = walked && na == nval && nb == nval;
+    if (!closed) { pa = a; pb = b; pna = na; pnb = nb; }
+    const int raw = dv_count_lat<CNT_BISECT>(n, tp, pivmin, t == 0 ? pa : t == 1 ? pb : a);
     if (cnt) {
       cnt[tid] = raw;
       __syncthreads();
     }
     const int ea = cnt ? cnt[g0] : __shfl_sync(0xffffffffu, raw, g0);
     const int eb = cnt ? cnt[g0 + 1] : __shfl_sync(0xffffffffu, raw, g0 + 1);
-    const bool closed = walked && na == nval && nb == nval;
-    bool ok = true;
-    if (closed) ok = ea == nval;
-    else {
-      if (a != sa || na != sna) { ok &= ea < nval; na = ea; }
-      if (b != sb || nb != snb) { ok &= eb > nval; nb = eb; }
-    }
+    const int ec = cnt ? cnt[g0 + 2] : __shfl_sync(0xffffffffu, raw, g0 + 2);
+    // (an end that has not moved was counted exactly or given)
+    bool ok = !closed || ec == nval;
+    if (pa != sa || pna != sna) { ok &= ea < nval; pna = ea; }
+    if (pb != sb || pnb != snb) { ok &= eb > nval; pnb = eb; }
+    if (!closed) { na = pna; nb = pnb; }
     if (!ok) { a = sa; b = sb; na = sna; nb = snb; it = sit; done = sdone; }
     if (cnt) __syncthreads();
   }
