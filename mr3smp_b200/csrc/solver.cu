@@ -3164,10 +3164,13 @@ static void prof_flush(mr3_cuda_ctx *c) {
   c->evnext = 0;
 }
 
+// (the runtime keeps a failed call's error for the next cudaGetLastError,
+// which would be the check of a later solve's first launch: it is cleared)
 #define CK(call, what)                                                    \
   do {                                                                    \
     cudaError_t e_ = (call);                                              \
     if (e_ != cudaSuccess) {                                              \
+      (void)cudaGetLastError();                                           \
       snprintf(c->err, sizeof(c->err), "%s: %s", what, cudaGetErrorString(e_)); \
       return MR3_EMISC;                                                   \
     }                                                                     \
@@ -3193,6 +3196,8 @@ static void prof_flush(mr3_cuda_ctx *c) {
     }                                                                     \
   } while (0)
 
+// The old buffer is gone whatever becomes of the new one, so a caller that
+// keeps a capacity sets it to zero first and to the new size afterwards.
 template <typename T>
 static cudaError_t regrow(T **p, size_t count) {
   if (*p) cudaFree(*p);
@@ -3203,6 +3208,7 @@ static cudaError_t regrow(T **p, size_t count) {
 static int ensure_rows(mr3_cuda_ctx *c, size_t N, size_t P) {
   if (N > c->capN) {
     size_t n = std::max(N, c->capN + c->capN / 2);
+    c->capN = 0;   // until all of it is there
     CK(regrow(&c->blocks, n), "blocks");
     CK(regrow(&c->blk_of_row, n), "blk_of_row");
     CK(regrow(&c->Windex, n), "Windex");
@@ -3246,7 +3252,7 @@ static int ensure_rows(mr3_cuda_ctx *c, size_t N, size_t P) {
   }
   if (P > c->capP) {
     size_t p = std::max(P, c->capP + c->capP / 2);
-    c->capP = 0;   // until all of it is there
+    c->capP = 0;
     const size_t rec = sizeof(ProbDev) + 5 * sizeof(void *);
     CK(regrow(&c->pk, p * rec), "problem records");
     CK(regrow(&c->flag, p), "flag");
@@ -3313,6 +3319,7 @@ extern "C" int mr3_cuda_ctx_create_prio(int device, int high, mr3_cuda_ctx **out
       cudaHostGetDevicePointer((void **)&c->d_hsc, c->h_sc, 0) != cudaSuccess ||
       cudaHostGetDevicePointer((void **)&c->d_hsnap, c->h_snap, 0) != cudaSuccess) {
     mr3_cuda_ctx_destroy(c);
+    (void)cudaGetLastError();
     return MR3_EMISC;
   }
   c->sc = reinterpret_cast<SngCounters *>(c->lc + 2);
@@ -3324,6 +3331,7 @@ extern "C" int mr3_cuda_ctx_create_prio(int device, int high, mr3_cuda_ctx **out
       cudaFuncSetAttribute(k_sng_round<SNG_FIRST>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            SNG_TILE_BYTES) != cudaSuccess) {
     mr3_cuda_ctx_destroy(c);
+    (void)cudaGetLastError();
     return MR3_EMISC;
   }
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_sng_round<SNG_LATER>, SNG_WARPS * 32,
@@ -3387,6 +3395,8 @@ extern "C" void *mr3_cuda_ws(mr3_cuda_ctx *c, int slot, size_t bytes) {
     c->ws_cap[slot] = 0;
     size_t sz = std::max<size_t>(bytes, 256);
     if (cudaMalloc(&c->ws[slot], sz) != cudaSuccess) {
+      (void)cudaGetLastError();
+      c->ws[slot] = nullptr;
       snprintf(c->err, sizeof(c->err), "workspace of %zu bytes", sz);
       return nullptr;
     }
@@ -3476,6 +3486,7 @@ extern "C" void *mr3_cuda_host_ws(mr3_cuda_ctx *c, size_t bytes) {
     c->hws_cap = 0;
     size_t sz = std::max<size_t>(bytes, 4096);
     if (cudaMallocHost(&c->hws, sz) != cudaSuccess) {
+      (void)cudaGetLastError();
       c->hws = nullptr;
       snprintf(c->err, sizeof(c->err), "page-locked buffer of %zu bytes", sz);
       return nullptr;
@@ -3697,6 +3708,7 @@ static int solve_impl(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void *stream,
   }
   if (done_fn && ntiles > c->capTiles) {
     CK(cudaStreamSynchronize(st), "tiles sync");
+    c->capTiles = 0;
     CK(regrow(&c->tile_left, ntiles), "tile_left");
     CK(regrow(&c->done_list, ntiles), "done_list");
     if (c->h_done) cudaFreeHost(c->h_done);
@@ -3987,6 +3999,7 @@ static int solve_impl(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void *stream,
           const size_t sz = std::max(fw * maxG * per, std::min(fin_bound, c->capFscratch * 3 / 2));
           CK(cudaStreamSynchronize(c->own), "fscratch sync");
           CK(cudaStreamSynchronize(c->rnd), "fscratch sync");
+          c->capFscratch = 0;
           CK(regrow(&c->fscratch, sz / sizeof(double)), "fscratch");
           c->capFscratch = sz;
         }
@@ -3998,6 +4011,7 @@ static int solve_impl(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void *stream,
         const bool direct = nsng <= finish_max;
         if (!direct && nwarps * per_warp > c->capScratch) {
           CK(cudaStreamSynchronize(st), "scratch sync");
+          c->capScratch = 0;
           CK(regrow(&c->scratch, nwarps * per_warp), "scratch");
           c->capScratch = nwarps * per_warp;
         }
@@ -4073,6 +4087,7 @@ static int solve_impl(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void *stream,
       if (ncl > 0 && need > c->capArena[nxt]) {
         CK(cudaStreamSynchronize(st), "arena sync");
         size_t nsz = std::max(need, c->capArena[nxt] + c->capArena[nxt] / 2);
+        c->capArena[nxt] = 0;
         CK(regrow(&c->arena[nxt], nsz), "arena");
         c->capArena[nxt] = nsz;
       }

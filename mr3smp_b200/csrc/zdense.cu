@@ -204,9 +204,10 @@ struct ZBufs {
   }
 };
 
-#define DCK(x)                          \
-  do {                                  \
-    if ((x) != cudaSuccess) return 2;   \
+// (a failed call's error is not left for the check of a later launch)
+#define DCK(x)                                                        \
+  do {                                                                \
+    if ((x) != cudaSuccess) { (void)cudaGetLastError(); return 2; }   \
   } while (0)
 #define SCK(x)                                            \
   do {                                                    \
