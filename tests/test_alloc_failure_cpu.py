@@ -34,7 +34,9 @@ def lib(tmp_path_factory):
     if not build.up_to_date() or not os.path.exists(obj):
         build.build(force=True)
     so = str(tmp_path_factory.mktemp("fake") / "solver_fake.so")
-    subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-I/usr/local/cuda/include", "-o", so,
+    # (-Bsymbolic: its own runtime, whatever libraries the process has loaded)
+    subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-Wl,-Bsymbolic",
+                    "-I/usr/local/cuda/include", "-o", so,
                     os.path.join(ROOT, "tests", "fake_cudart.cpp"), obj], check=True)
     L = C.CDLL(so)
     L.fake_launches.restype = C.c_char_p
