@@ -94,7 +94,10 @@ static __device__ __forceinline__ int dv_itmax(double a, double b) {
 // and NaN divisors; |a| and |q| >= 2^-960, so that r does not underflow)
 // are only recorded (qdiv_chk); a sweep tests them once per chunk of rows
 // and repeats a chunk that fails, 1.5e-5 per division, with plain
-// divisions.  So every result is that of a / b, whatever the seed.
+// divisions.  A quotient that overflows comes out as a NaN whose test value is
+// the same NaN; it makes the next row's divisor a NaN, which is recorded, and
+// in a chunk's last row the value carried to the next chunk (`last`), which
+// must be finite.  So every result is that of a / b, whatever the seed.
 //
 // The seed of the next row may come from a divisor predicted with *qt =
 // qh (1 + e), 40 bits of the quotient two operations earlier, which takes
@@ -108,6 +111,7 @@ static __device__ __forceinline__ int dv_itmax(double a, double b) {
 #define QDIV_KK   1.0000152587890625      // 1 + 2^-16
 #define QDIV_EMAX (0x3ee00000u << 1)      // high word of 2^-17, sign shifted out
 #define QDIV_AMIN (0x03f00000u << 1)      // high word of 2^-960
+#define QDIV_INF  (0x7ff00000u << 1)      // high word of infinity
 #define QDIV_U    8                       // rows per checked chunk
 
 struct qdiv_chk {
@@ -144,8 +148,9 @@ static __device__ __forceinline__ void qdiv_begin(qdiv_chk *k) {
   k->amin = 0xffffffffu;
 }
 
-static __device__ __forceinline__ bool qdiv_failed(const qdiv_chk &k) {
-  return k.acc != 0u || k.emax >= QDIV_EMAX || k.amin < QDIV_AMIN;
+// last: what the chunk's last quotient went into (NaN if that was).
+static __device__ __forceinline__ bool qdiv_failed(const qdiv_chk &k, double last) {
+  return k.acc != 0u || k.emax >= QDIV_EMAX || k.amin < QDIV_AMIN || dv_habs(last) >= QDIV_INF;
 }
 
 static __device__ __forceinline__ double dv_qdiv(double a, double b, double y0, qdiv_chk *k,
@@ -239,7 +244,7 @@ static __device__ __noinline__ int dv_count_lat(int n, const double2 *__restrict
         tmin = min(tmin, dv_habs(t));
         v[u] = tp[d_imin(j + U + u, n - 1)];
       }
-      if (qdiv_failed(k) || tmin <= hp) {
+      if (qdiv_failed(k, t) || tmin <= hp) {
         t = t0;
         cnt = cnt0;
 #pragma unroll 1
@@ -671,7 +676,7 @@ static __device__ __forceinline__ int dv_dlaneg_inl(int n, const double2 *__rest
           t = tmp * c[u].y - sigma;
           c[u] = dv_at(P, d_imin(j + U + u, last) - 1, sb);
         }
-        if (qdiv_failed(k)) {
+        if (qdiv_failed(k, t)) {
           t = t0;
           neg1 = n0;
 #pragma unroll 1
@@ -733,7 +738,7 @@ static __device__ __forceinline__ int dv_dlaneg_inl(int n, const double2 *__rest
           p = tmp * c[u].x - sigma;
           c[u] = dv_at(P, d_imax(j - U - u, r) - 1, sb);
         }
-        if (qdiv_failed(k)) {
+        if (qdiv_failed(k, p)) {
           p = p0;
           neg2 = n0;
 #pragma unroll 1
@@ -2930,7 +2935,7 @@ static __device__ __noinline__ void dv_r1s_call(bool active, int L, int n, doubl
           dv_at(o1, row, ob) = q * (up ? 1.0 : cc[u]);
           dv_at(o2, row, ob) = up ? v : x;
         }
-        if (qdiv_failed(ck)) {
+        if (qdiv_failed(ck, x)) {
           x = x0;
           v = v0;
           neg = neg0;
@@ -3182,7 +3187,7 @@ static __device__ __forceinline__ double rrf_sweep(int n, const double2 *__restr
         dv_at(dp, i0 + u + 1, ob) = d;
         mx = fmax(mx, fabs(d));
       }
-      if (qdiv_failed(k) || dmin <= hp) {
+      if (qdiv_failed(k, d) || dmin <= hp) {
         s = s0;
         d = d0;
         mx = mx0;
@@ -3423,7 +3428,7 @@ static __device__ __noinline__ double dv_root_try(int n, const double *__restric
         cd[u] = D[i + 1];
         ce[u] = E[i];
       }
-      if (qdiv_failed(k)) {
+      if (qdiv_failed(k, d)) {
         d = d0;
         dmax = m0;
         neg = n0;
