@@ -115,6 +115,13 @@ int dsyeig(char *jobz, char *range, char *uplo, int *n, double *A, int *lda,
            double *vl, double *vu, int *il, int *iu, int *m, double *W,
            double *Z, int *ldz);
 
+/* Gives back the device buffers and library handles that finished calls of
+ * dsyeig, dspeig, dsygeig and dspgeig keep for the next one (at most four sets
+ * of at most 256 MB per process); later calls allocate theirs anew.  Returns
+ * the number of sets freed.  Safe beside calls of other threads.  No
+ * counterpart in the reference. */
+int mr3_dense_release(void);
+
 /* Replaces the Fortran binding dsyeig_ of SRC/dense.c:1037-1043. */
 void dsyeig_(char *jobz, char *range, char *uplo, int *n, double *A, int *lda,
              double *vl, double *vu, int *il, int *iu, int *m, double *W,

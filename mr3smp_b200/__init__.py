@@ -179,6 +179,12 @@ def dsyeig(jobz: str, rng: str, uplo: str, A, vl: float = 0.0, vu: float = 0.0, 
     return out
 
 
+def dense_release() -> int:
+    """Gives back the device buffers that the real dense drivers keep for their
+    next call; returns the number of sets freed."""
+    return int(lib().mr3_dense_release())
+
+
 def pack(A, uplo: str):
     """The uplo triangle of a square array in LAPACK packed storage."""
     A = np.asarray(A, dtype=np.float64)

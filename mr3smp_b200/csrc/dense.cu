@@ -29,6 +29,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include "alloc.h"
 #include "mr3_b200.h"
 
 namespace {
@@ -177,8 +178,9 @@ int range_code(char c) {
 // the 15.7 ms of an n = 700 dsyeig, so a call borrows them: finished calls
 // leave theirs in a list of at most KEEP_SETS per process, with at most
 // KEEP_BYTES each; what is above that, and a set whose call failed, is freed.
-// A set belongs to one call at a time and to the device it was made on; its
-// buffers' contents do not outlive a call.
+// mr3_dense_release() gives the idle ones back, and so does an allocation of
+// the library that finds no memory.  A set belongs to one call at a time and
+// to the device it was made on; its buffers' contents do not outlive a call.
 const int KEEP_SETS = 4;
 const size_t KEEP_BYTES = (size_t)256 << 20;
 enum { BUF_A, BUF_B, BUF_AP, BUF_D, BUF_E, BUF_TAU, BUF_W, BUF_Z, BUF_WORK, BUF_ZSUPP, BUF_FLAGS,
@@ -197,15 +199,18 @@ struct DenseSet {
       cap[k] = 0;
     }
   }
-  void drop() {
+  // Frees everything, on the set's own device.
+  ~DenseSet() {
+    int cur = device;
+    cudaGetDevice(&cur);
+    if (cur != device) cudaSetDevice(device);
     drop_buffers();
     if (h) g_cs.destroy(h);
     if (hb) g_cs.bdestroy(hb);
-    h = nullptr;
-    hb = nullptr;
+    if (cur != device) cudaSetDevice(cur);
   }
 };
-DenseSet *g_kept[KEEP_SETS];
+KeptList<DenseSet, KEEP_SETS> g_kept;
 pthread_mutex_t g_kept_mu = PTHREAD_MUTEX_INITIALIZER;
 
 // The buffers of one call; the set goes back on every exit path.
@@ -221,11 +226,7 @@ struct DenseBufs {
 
   void borrow(int device) {
     pthread_mutex_lock(&g_kept_mu);
-    for (int k = 0; k < KEEP_SETS && !set; k++)
-      if (g_kept[k] && g_kept[k]->device == device) {
-        set = g_kept[k];
-        g_kept[k] = nullptr;
-      }
+    set = g_kept.take(device);
     pthread_mutex_unlock(&g_kept_mu);
     if (!set) {
       set = new DenseSet();
@@ -239,8 +240,11 @@ struct DenseBufs {
       if (set->buf[which]) cudaFree(set->buf[which]);
       set->buf[which] = nullptr;
       set->cap[which] = 0;
-      const cudaError_t e = cudaMalloc(&set->buf[which], bytes > 0 ? bytes : 1);
-      if (e != cudaSuccess) return e;
+      const cudaError_t e = mr3__alloc(&set->buf[which], bytes > 0 ? bytes : 1);
+      if (e != cudaSuccess) {
+        set->buf[which] = nullptr;
+        return e;
+      }
       set->cap[which] = bytes;
     }
     *p = (T *)set->buf[which];
@@ -250,23 +254,16 @@ struct DenseBufs {
     if (!set) return;
     set->h = h;
     set->hb = hb;
-    bool kept = false;
+    DenseSet *out = set;
     if (good) {
       size_t total = 0;
       for (size_t c : set->cap) total += c;
       if (total > KEEP_BYTES) set->drop_buffers();
       pthread_mutex_lock(&g_kept_mu);
-      for (int k = 0; k < KEEP_SETS && !kept; k++)
-        if (!g_kept[k]) {
-          g_kept[k] = set;
-          kept = true;
-        }
+      out = g_kept.give(set);
       pthread_mutex_unlock(&g_kept_mu);
     }
-    if (!kept) {
-      set->drop();
-      delete set;
-    }
+    delete out;
   }
 };
 
@@ -468,6 +465,18 @@ int backtransform_generalized(DenseBufs &b, int itype, bool lower, int n, int m)
 }
 
 }  // namespace
+
+// The idle sets are taken out one by one, so that calls of other threads keep
+// theirs.
+extern "C" int mr3_dense_release(void) {
+  for (int count = 0;; count++) {
+    pthread_mutex_lock(&g_kept_mu);
+    DenseSet *set = g_kept.take_any();
+    pthread_mutex_unlock(&g_kept_mu);
+    if (!set) return count;
+    delete set;
+  }
+}
 
 extern "C" int dsyeig(char *jobz, char *range, char *uplo, int *np, double *A, int *ldap,
                       double *vlp, double *vup, int *ilp, int *iup, int *mp, double *W,

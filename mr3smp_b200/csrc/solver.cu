@@ -28,6 +28,7 @@
 #include <string>
 #include <vector>
 
+#include "alloc.h"
 #include "mr3_cuda.h"
 #include "mr3_device.cuh"
 
@@ -3202,7 +3203,7 @@ template <typename T>
 static cudaError_t regrow(T **p, size_t count) {
   if (*p) cudaFree(*p);
   *p = nullptr;
-  return cudaMalloc((void **)p, std::max<size_t>(count, 1) * sizeof(T));
+  return mr3__alloc((void **)p, std::max<size_t>(count, 1) * sizeof(T));
 }
 
 static int ensure_rows(mr3_cuda_ctx *c, size_t N, size_t P) {
@@ -3394,7 +3395,7 @@ extern "C" void *mr3_cuda_ws(mr3_cuda_ctx *c, int slot, size_t bytes) {
     c->ws[slot] = nullptr;
     c->ws_cap[slot] = 0;
     size_t sz = std::max<size_t>(bytes, 256);
-    if (cudaMalloc(&c->ws[slot], sz) != cudaSuccess) {
+    if (mr3__alloc(&c->ws[slot], sz) != cudaSuccess) {
       (void)cudaGetLastError();
       c->ws[slot] = nullptr;
       snprintf(c->err, sizeof(c->err), "workspace of %zu bytes", sz);
@@ -4146,7 +4147,7 @@ static int solve_impl(mr3_cuda_ctx *c, int P, mr3_cuda_prob *pr, void *stream,
         if (moved.empty()) continue;
         double *tmp = nullptr;
         size_t colsz = (size_t)h.n;
-        CK(cudaMalloc((void **)&tmp, moved.size() * colsz * sizeof(double)), "perm tmp");
+        CK(mr3__alloc((void **)&tmp, moved.size() * colsz * sizeof(double)), "perm tmp");
         for (size_t t = 0; t < moved.size(); t++)
           CK(cudaMemcpyAsync(tmp + t * colsz, h.Z + (size_t)hrec[h.off + moved[t]].idx * h.ldz,
                              colsz * sizeof(double), cudaMemcpyDeviceToDevice, st), "perm gather");

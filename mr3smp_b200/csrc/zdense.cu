@@ -26,6 +26,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include "alloc.h"
 #include "mr3_b200.h"
 
 namespace {
@@ -236,18 +237,18 @@ int zstart(ZBufs &b, int n, int jz, int ncols) {
   pthread_once(&g_z_once, load_libs);
   if (!g_z.ok) return 2;
   DCK(cudaSetDevice(device_id()));
-  DCK(cudaMalloc((void **)&b.A, (size_t)n * n * kC));
-  DCK(cudaMalloc((void **)&b.tau, (size_t)n * kC));
-  DCK(cudaMalloc((void **)&b.D, n * sizeof(double)));
-  DCK(cudaMalloc((void **)&b.E, n * sizeof(double)));
-  DCK(cudaMalloc((void **)&b.W, n * sizeof(double)));
-  DCK(cudaMalloc((void **)&b.Zsupp, 2 * (size_t)n * sizeof(int)));
-  DCK(cudaMalloc((void **)&b.info, sizeof(int)));
-  DCK(cudaMalloc((void **)&b.nan, sizeof(int)));
-  DCK(cudaMalloc((void **)&b.maxbits, sizeof(unsigned long long)));
+  DCK(mr3__alloc((void **)&b.A, (size_t)n * n * kC));
+  DCK(mr3__alloc((void **)&b.tau, (size_t)n * kC));
+  DCK(mr3__alloc((void **)&b.D, n * sizeof(double)));
+  DCK(mr3__alloc((void **)&b.E, n * sizeof(double)));
+  DCK(mr3__alloc((void **)&b.W, n * sizeof(double)));
+  DCK(mr3__alloc((void **)&b.Zsupp, 2 * (size_t)n * sizeof(int)));
+  DCK(mr3__alloc((void **)&b.info, sizeof(int)));
+  DCK(mr3__alloc((void **)&b.nan, sizeof(int)));
+  DCK(mr3__alloc((void **)&b.maxbits, sizeof(unsigned long long)));
   if (jz == MR3_JOB_V) {
-    DCK(cudaMalloc((void **)&b.Zr, (size_t)n * ncols * sizeof(double)));
-    DCK(cudaMalloc((void **)&b.Z, (size_t)n * ncols * kC));
+    DCK(mr3__alloc((void **)&b.Zr, (size_t)n * ncols * sizeof(double)));
+    DCK(mr3__alloc((void **)&b.Z, (size_t)n * ncols * kC));
   }
   DCK(cudaMemset(b.E, 0, n * sizeof(double)));
   DCK(cudaMemset(b.nan, 0, sizeof(int)));
@@ -301,7 +302,7 @@ int zcore(ZBufs &b, int jz, int rg, bool lower, int n, int ncols, double *vlp, d
                      &lw2));
   if (b.work) cudaFree(b.work);
   b.work = nullptr;
-  DCK(cudaMalloc((void **)&b.work, (size_t)(lw1 > lw2 ? lw1 : lw2) * kC + 16));
+  DCK(mr3__alloc((void **)&b.work, (size_t)(lw1 > lw2 ? lw1 : lw2) * kC + 16));
   if (n > 1) {
     SCK(g_z.hetrd(b.h, fill, n, b.A, n, b.D, b.E, b.tau, b.work, lw1, b.info));
     DCK(cudaMemcpy(&hinfo, b.info, sizeof(int), cudaMemcpyDeviceToHost));
@@ -356,7 +357,7 @@ int zreduce(ZBufs &b, int itype, bool lower, int n) {
   const cublasFillMode_t fill = lower ? CUBLAS_FILL_MODE_LOWER : CUBLAS_FILL_MODE_UPPER;
   int lw = 0, hinfo = 0;
   SCK(g_z.potrf_ws(b.h, fill, n, b.B, n, &lw));
-  DCK(cudaMalloc((void **)&b.work, (size_t)lw * kC + 16));
+  DCK(mr3__alloc((void **)&b.work, (size_t)lw * kC + 16));
   SCK(g_z.potrf(b.h, fill, n, b.B, n, b.work, lw, b.info));
   DCK(cudaMemcpy(&hinfo, b.info, sizeof(int), cudaMemcpyDeviceToHost));
   if (hinfo != 0) return 2;   // B is not positive definite
@@ -444,7 +445,7 @@ extern "C" int zhpeig(char *jobz, char *range, char *uplo, int *np, void *AP, do
   int rc = zstart(b, n, jz, ncols);
   if (rc) return rc;
   const size_t np_ = (size_t)n * (n + 1) / 2;
-  DCK(cudaMalloc((void **)&b.AP, np_ * kC));
+  DCK(mr3__alloc((void **)&b.AP, np_ * kC));
   DCK(cudaMemcpy(b.AP, AP, np_ * kC, cudaMemcpyHostToDevice));
   k_herm_packed<<<kGrid, 256>>>(n, b.AP, b.A, lower, 0);
   DCK(cudaGetLastError());
@@ -465,7 +466,7 @@ extern "C" int zhegeig(int *itype, char *jobz, char *range, char *uplo, int *np,
   const int ncols = rg == MR3_RANGE_I ? *iup - *ilp + 1 : n;
   int rc = zstart(b, n, jz, ncols);
   if (rc) return rc;
-  DCK(cudaMalloc((void **)&b.B, (size_t)n * n * kC));
+  DCK(mr3__alloc((void **)&b.B, (size_t)n * n * kC));
   DCK(cudaMemcpy2D(b.A, n * kC, A, (size_t)*ldap * kC, n * kC, n, cudaMemcpyHostToDevice));
   DCK(cudaMemcpy2D(b.B, n * kC, B, (size_t)*ldbp * kC, n * kC, n, cudaMemcpyHostToDevice));
   if ((rc = zreduce(b, *itype, lower, n))) return rc;
@@ -494,8 +495,8 @@ extern "C" int zhpgeig(int *itype, char *jobz, char *range, char *uplo, int *np,
   int rc = zstart(b, n, jz, ncols);
   if (rc) return rc;
   const size_t np_ = (size_t)n * (n + 1) / 2;
-  DCK(cudaMalloc((void **)&b.B, (size_t)n * n * kC));
-  DCK(cudaMalloc((void **)&b.AP, np_ * kC));
+  DCK(mr3__alloc((void **)&b.B, (size_t)n * n * kC));
+  DCK(mr3__alloc((void **)&b.AP, np_ * kC));
   DCK(cudaMemset(b.B, 0, (size_t)n * n * kC));
   DCK(cudaMemcpy(b.AP, AP, np_ * kC, cudaMemcpyHostToDevice));
   k_herm_packed<<<kGrid, 256>>>(n, b.AP, b.A, lower, 0);

@@ -11,6 +11,7 @@
 static std::map<const void *, std::string> g_names;
 static cudaError_t g_last = cudaSuccess;
 static long g_allocs, g_fail_at = -1;
+static int g_idle;           // idle buffer sets of the dense drivers
 struct Launch { std::string name; std::vector<void *> args; };
 static std::vector<Launch> g_launches;
 static std::map<std::string, std::vector<int>> g_ptr_args;   // positions of pointer parameters
@@ -26,6 +27,8 @@ static cudaError_t alloc(void **p, size_t n) {
 }
 extern "C" {
 // test controls
+void fake_idle(int n) { g_idle = n; }
+int mr3_dense_release() { const int n = g_idle; g_idle = 0; return n; }
 void fake_fail(long k) { g_allocs = 0; g_fail_at = k; }
 long fake_allocs() { return g_allocs; }
 void fake_levels(const int *v, int n) { g_levels.assign(v, v + n); g_at = 0; }
