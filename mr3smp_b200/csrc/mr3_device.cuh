@@ -3315,6 +3315,8 @@ static __device__ __noinline__ double dv_dlarrf(int n, const double2 *__restrict
       const unsigned pm = 3u << ((threadIdx.x & 31) & ~1);   // this lane pair
       const bool right = (threadIdx.x & 1) != 0;
       bool sn = false;
+      // (the partner may still read the last try's factors for its growth quantity)
+      __syncwarp(pm);
       const double mx = rrf_sweep(n, P, Q, ps, right ? rsigma : lsigma, pivmin, right ? wk_ : dp_,
                                   right ? wk_ + (size_t)n * os : lp_, os, &sn);
       const int src = (threadIdx.x & 31) & ~1;
