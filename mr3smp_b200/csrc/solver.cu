@@ -13,7 +13,9 @@
 //     nthreads > 12*m/n, SRC/mrrr_val.c:281-285) unless MR3_NTHREADS asks for
 //     the other;
 //   - every singleton is its own task and cluster refinement is never split;
-//     a cluster is classified completely before its singletons run.
+//     a cluster is classified completely before its singletons run;
+//   - every eigenvalue is refined as its own local index, also where the removal
+//     of surplus ones (k_discard) left a hole in a cluster's indices.
 // The pthread task queue becomes a device work queue drained level by level:
 // a level's clusters compute their child representations and refine their
 // eigenvalues; a classification kernel appends child clusters and singleton
