@@ -802,12 +802,12 @@ def main():
             # DRAM bytes per dlar1v row of the singleton kernels, measured with
             # ncu (dram__bytes_read.sum + dram__bytes_write.sum) on a
             # 256-problem mixed batch (n <= 4096), scaled by this run's rows
-            traffic = {"bytes_per_launch": 48.4 * ctr[4][2] / max(tcnt, 1),
+            traffic = {"bytes_per_launch": 50.4 * ctr[4][2] / max(tcnt, 1),
                        "algorithmic_bytes_per_launch": zbytes / max(tcnt, 1),   # the Z write
-                       "source": "ncu on a 256-problem mixed batch (n <= 4096): 48.4 B per "
-                                 "dlar1v row (checkpoints and child representations; the "
-                                 "Z write is about 3 B per row), scaled by the live "
-                                 "dlar1v-row counter"}
+                       "source": "ncu on a 256-problem mixed batch (n <= 4096): 50.4 B per "
+                                 "dlar1v row (checkpoints, the finish's row values and "
+                                 "child representations; the Z write is about 3 B per "
+                                 "row), scaled by the live dlar1v-row counter"}
         roof = {"bound": "fp64-div", "kernel": tname, "achieved": achieved,
                 "peak": div_gops, "unit": "Gdiv/s",
                 "frac": (achieved / div_gops) if div_gops else None,

@@ -482,11 +482,7 @@ static __device__ __noinline__ int dv_bisect_one(int n, const double2 *__restric
 // lie beside the bracket (one inside is counted).  The turns and with them
 // the interval are the same.
 #ifndef BIS_LONG
-#ifndef BIS_LONG
-#ifndef BIS_LONG
 #define BIS_LONG 56
-#endif
-#endif
 #endif
 
 // A point between l and r that halves the bracket's exponent range while its

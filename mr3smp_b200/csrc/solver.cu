@@ -1805,11 +1805,19 @@ __global__ void k_cl_pack(int ncl, const ClusterDev *cl, const BlockDev *blocks,
 // level), a thread (L = 1) one.  A count's row costs the larger of the
 // chain's latency and the FP64 pipe's time for the warps of the fullest
 // quarter SM.  So lanes are added while the chain's latency hides them and
-// not beyond: 10005 intervals take 3 lanes each (two warps a quarter, 65
-// cycles a step; 4 lanes three warps, 80), 1000 take 32.  Measured in cycles
-// a row: dlaneg 250 (thread, plain divisions) and 115-135 (checked; more when
-// the rows are strided), 60 a warp; the guessed counts of stage A 48 and 18.
-struct RowCost { int lat1, lat, pipe; };   // thread form, group form, per warp
+// not beyond: 10005 intervals of dlarrb take 3 lanes each (two warps a quarter,
+// 65 cycles a step; 4 lanes three warps, 80), 1000 take 32.  The callers' costs,
+// measured in cycles a row (one warp; one more warp a quarter SM):
+//   cluster ends, k_refine_cl  130 130 60  checked dlaneg, rows strided, both forms
+//   k_refine_root              250 115 50  rows from L1; plain divisions by thread
+//   k_bisect                    48  48 18  guessed counts, both forms
+//   k_highrac                  193  95 55  counts of T, plain by thread, checked
+// Against the best of all limits (MR3_TREE_LANES 1 to 32; one matrix of n rows,
+// eigenvalues only, ms): k_refine_root 0.68 of 0.68 at n = 1500 (a thread each
+// 4.5), 1.55 of 1.55 at 3001 (9.3), 4.6 of 4.6 at 6000 (19), 8.5 of 8.5 at 10005
+// (32), 17.7 of 17.7 at 16000 (73); k_bisect 0.59 of 0.52, 1.52 of 1.27, 3.4 of 3.4,
+// 7.9 of 7.0 and 15.5 of 15.5 (a thread each, after shared levels, 1.4 to 19.9).
+struct RowCost { int lat1, lat, pipe; };   // thread form, group form, a further warp
 __host__ __device__ __forceinline__ int tree_lanes(long long items, int nsm, int maxL = 32,
                                                    RowCost rc = {130, 130, 60}) {
   int best = 1;
@@ -2751,6 +2759,14 @@ k_sng_bisect(int out, const SngDev *sng, const ClusterDev *cl, const ProbDev *pr
 #ifndef FIN_MAXG
 #define FIN_MAXG 16
 #endif
+// FIN_LIST: a longer list (75776 singletons on 148 SMs) starts with rounds.
+// Measured on batches of one total number of rows, ms a solve, every list
+// through the finish against this line: problems of 32 to 1024 rows even at
+// 90 000 rows, 15.0 against 14.3 at 120 000, 26.3 against 24.6 at 300 000; of 200
+// rows 3.4 and 3.6 at 90 000, 6.3 and 6.0 at 220 000; of 20 to 200 rows 2.8 and
+// 3.4, 4.5 and 4.8.  Rounds alone took 2 to 3 times as long at 75 000 rows (35.9
+// against 11.3, 6.3 and 3.0, 8.2 and 2.6).  So the line lies where the larger
+// problems, whose solves are the longer ones, begin to lose.
 #ifndef FIN_LIST
 #define FIN_LIST 64      // singletons per warp up to which a list is taken
 #endif
@@ -3110,7 +3126,7 @@ struct mr3_cuda_ctx {
   SngCounters *sc = nullptr;
   double *scratch = nullptr, *arena[2] = {nullptr, nullptr};
   double *qd = nullptr;                     // dqds arrays (4 doubles per row)
-  double *fscratch = nullptr;               // row scratch of the split finish
+  double *fscratch = nullptr;               // row scratch of the finish
   size_t capFscratch = 0;
   size_t round_scratch = (size_t)8 << 30;   // bound of the round warps' checkpoint scratch
   // a solve's problem records and array pointers, uploaded in one copy: probs,
@@ -3307,17 +3323,17 @@ extern "C" int mr3_cuda_ctx_create_prio(int device, int high, mr3_cuda_ctx **out
       cudaStreamCreateWithPriority(&c->aux, cudaStreamNonBlocking, prio) != cudaSuccess ||
       cudaStreamCreateWithPriority(&c->rnd, cudaStreamNonBlocking, prio) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->rnd_done, cudaEventDisableTiming) != cudaSuccess ||
-      cudaMalloc((void **)&c->lc, 2 * sizeof(LevelCounters) + sizeof(SngCounters)) != cudaSuccess ||
-      cudaMalloc((void **)&c->rl_n, sizeof(int)) != cudaSuccess ||
-      cudaMalloc((void **)&c->bis_n, 2 * sizeof(int)) != cudaSuccess ||
-      cudaMalloc((void **)&c->sbk, 3 * SNG_BUCKETS * sizeof(int)) != cudaSuccess ||
+      mr3__alloc((void **)&c->lc, 2 * sizeof(LevelCounters) + sizeof(SngCounters)) != cudaSuccess ||
+      mr3__alloc((void **)&c->rl_n, sizeof(int)) != cudaSuccess ||
+      mr3__alloc((void **)&c->bis_n, 2 * sizeof(int)) != cudaSuccess ||
+      mr3__alloc((void **)&c->sbk, 3 * SNG_BUCKETS * sizeof(int)) != cudaSuccess ||
       cudaMallocHost((void **)&c->h_lc, 2 * sizeof(LevelCounters)) != cudaSuccess ||
       cudaMallocHost((void **)&c->h_sc, sizeof(SngCounters)) != cudaSuccess ||
       cudaMallocHost((void **)&c->h_snap, SNG_ROUNDS * sizeof(int)) != cudaSuccess ||
       cudaMallocHost((void **)&c->h_const, sizeof(double)) != cudaSuccess ||
       cudaMallocHost((void **)&c->h_iconst, 2 * sizeof(int)) != cudaSuccess ||
       cudaMallocHost((void **)&c->h_bisn, sizeof(int)) != cudaSuccess ||
-      cudaMalloc((void **)&c->stats, KID_COUNT * 4 * sizeof(unsigned long long)) != cudaSuccess ||
+      mr3__alloc((void **)&c->stats, KID_COUNT * 4 * sizeof(unsigned long long)) != cudaSuccess ||
       cudaHostGetDevicePointer((void **)&c->d_hlc, c->h_lc, 0) != cudaSuccess ||
       cudaHostGetDevicePointer((void **)&c->d_hsc, c->h_sc, 0) != cudaSuccess ||
       cudaHostGetDevicePointer((void **)&c->d_hsnap, c->h_snap, 0) != cudaSuccess) {
