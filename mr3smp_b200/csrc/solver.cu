@@ -514,8 +514,13 @@ k_blocks(ProbDev *probs, BlockDev *blocks, const double *D, double *E, const dou
     if (nbl == 1) {
       if (lead) {
         double dv = D[ibgn];
+        // Range I: the counts at wl and wu took a value within pivmin of the
+        // point as one below it (dv_count_row), so it is not taken at wl.  (The
+        // reference takes it, SRC/mrrr_val.c:340-412, and then returns more than
+        // iu-il+1 values: the integer matrix diag(1, 0, -1), eigenvalue 3, whose
+        // search ends at wl = 0, gets two.)
         bool take = (irange == MR3_RANGE_A) || (irange == MR3_RANGE_V && dv > wl && dv <= wu) ||
-                    (irange == MR3_RANGE_I && (dv + pivmin) > wl && (dv - pivmin) <= wu);
+                    (irange == MR3_RANGE_I && !(dv - wl <= pivmin) && dv - wu <= pivmin);
         B->mbl = take ? 1 : 0;
         B->ilow = 1; B->iupp = take ? 1 : 0;
         B->nab1 = 0; B->nab2 = 0; B->none = 1;
@@ -1249,8 +1254,10 @@ __global__ void k_gaps_root(int N, const ProbDev *probs, const BlockDev *blocks,
 
 // ------------------------------------------------------------------------
 // Range I: drop surplus eigenvalues found near wl/wu
-// (SRC/mrrr_val.c:515-626).  One thread per problem; runs only when the
-// blocks together produced more than nvals values.
+// (SRC/mrrr_val.c:515-626).  Runs only when the blocks together produced more
+// than nvals values.  A problem that has another number than nvals at the end
+// (counts that contradict one another, near the underflow threshold) is given
+// status 2: Z has nvals columns.
 // ------------------------------------------------------------------------
 // A CTA per problem.  A problem with a surplus (clusters at the interval's
 // ends) is compacted by the CTA in chunks of MR3_THREADS entries, each read
@@ -1366,7 +1373,7 @@ k_discard(ProbDev *probs, BlockDev *blocks, double *W, double *Werr, double *Wga
   for (int je = mp + tid; je < m0; je += MR3_THREADS) ib[je] = -1;
   if (tid == 0) {
     p->m = mp;
-    if (mp < nvals) set_status(p, MR3_EMISC);
+    if (mp != nvals) set_status(p, MR3_EMISC);
   }
   // block W ranges after the removal: recomputed from iblk (SRC/mrrr_vec.c:335-338);
   // a block's entries follow one another

@@ -126,10 +126,9 @@ def _call(fn, jobz, rng, D, E, vl=0.0, vu=0.0, il=1, iu=1, tryrac=0, ldz=None):
     ldz = n if ldz is None else ldz
     want_z = jobz[0] in "Vv"
     W = np.zeros(max(n, 1))
-    nz = max(n, 1)
-    if want_z and rng[0] in "Ii":
-        nz = iu - il + 1
-    Z = np.zeros((nz if want_z else 1) * (ldz if want_z else 1))
+    # n columns also for range I: the reference may return more than iu-il+1
+    # eigenpairs (an uncoupled row's value where the search for il ends)
+    Z = np.zeros((max(n, 1) if want_z else 1) * (ldz if want_z else 1))
     Zs = np.zeros(2 * max(n, 1), dtype=np.int32)
     n_ = C.c_int(n)
     vl_ = C.c_double(vl)
